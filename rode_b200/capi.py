@@ -27,7 +27,7 @@ C_ABI_SYMBOLS = (
     "rode_last_error", "rode_version", "rode_preprocess_workspace_bytes", "rode_preprocess_capacity",
     "rode_preprocess", "rode_preprocess_noalloc", "rode_preprocess_cpu", "rode_spmm_workspace_bytes", "rode_spmm_f32", "rode_spmm_f64",
     "rode_sddmm_f32", "rode_hot_columns_workspace_bytes", "rode_hot_columns_words", "rode_hot_columns",
-    "rode_spmm_f32_hot", "rode_spmm_f64_hot",
+    "rode_spmm_f32_hot", "rode_spmm_f64_hot", "rode_spmm_f32_all", "rode_spmm_f64_all",
 )
 # Itanium-ABI names of the C++ entry points declared in RoDeSpmm.h / RoDeSddmm.h /
 # RoDePreprocess.h; identical to the names the reference's own objects export.
@@ -81,10 +81,12 @@ def load() -> ctypes.CDLL:
     lib.rode_hot_columns.argtypes = [ctypes.c_longlong, ci, vp, sz, sz, vp, vp, sz, vp]
     lib.rode_spmm_f32_hot.argtypes = [ci, ci, ci, ci, vp, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp, vp, vp]
     lib.rode_spmm_f64_hot.argtypes = lib.rode_spmm_f32_hot.argtypes
+    lib.rode_spmm_f32_all.argtypes = [ci, ci, ci, ci, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp, vp, vp]
+    lib.rode_spmm_f64_all.argtypes = lib.rode_spmm_f32_all.argtypes
     for name in ("rode_preprocess_workspace_bytes", "rode_preprocess_capacity", "rode_preprocess",
                  "rode_preprocess_noalloc", "rode_preprocess_cpu", "rode_spmm_workspace_bytes", "rode_spmm_f32", "rode_spmm_f64",
                  "rode_sddmm_f32", "rode_hot_columns_workspace_bytes", "rode_hot_columns_words", "rode_hot_columns",
-                 "rode_spmm_f32_hot", "rode_spmm_f64_hot"):
+                 "rode_spmm_f32_hot", "rode_spmm_f64_hot", "rode_spmm_f32_all", "rode_spmm_f64_all"):
         getattr(lib, name).restype = ci
     _lib = lib
     return lib
@@ -237,6 +239,14 @@ def spmm_raw(dtype, m1, m2, k, n, values, col, row_ptr, blk, res, st, B, C, work
                  _stream(stream1), _stream(stream2)))
 
 
+def spmm_all_raw(dtype, M, m1, k, n, values, col, row_ptr, blk, st, B, C, workspace, workspace_bytes, stream1=None,
+                 stream2=None, hot=None) -> None:
+    """rode_spmm_f32_all / _f64_all on raw device addresses: C may hold anything, every row is written."""
+    fn = load().rode_spmm_f32_all if dtype == torch.float32 else load().rode_spmm_f64_all
+    check(fn(M, m1, k, n, values, col, row_ptr, blk, st, B, C, workspace, workspace_bytes, hot, _stream(stream1),
+             _stream(stream2)))
+
+
 def hot_columns_raw(nnz, n_cols, col, dense_row_bytes, budget_bytes, bitmap, workspace, workspace_bytes,
                     stream=None) -> None:
     check(load().rode_hot_columns(nnz, n_cols, col, dense_row_bytes, budget_bytes, bitmap, workspace,
@@ -269,7 +279,8 @@ def spmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torch
          C: Optional[torch.Tensor] = None, workspace: Optional[torch.Tensor] = None, stream1=None,
          stream2=None, hot: Optional[torch.Tensor] = None) -> torch.Tensor:
     """C = S @ B through rode_spmm_f32 / rode_spmm_f64.  Asynchronous on the two streams
-    (default: torch's current stream for both).  ``C`` defaults to a fresh zero tensor.
+    (default: torch's current stream for both).  A given ``C`` must be zero in the rows without a
+    nonzero, which are not written; by default C is a fresh tensor of which every row is written.
     ``hot``: popularity bitmap from ``hot_columns`` (same results, fewer DRAM bytes)."""
     M = row_ptr.numel() - 1
     k, n = B.shape
@@ -282,8 +293,9 @@ def spmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torch
         cur = torch.cuda.current_stream(dev)
         s1 = cur if stream1 is None else stream1
         s2 = cur if stream2 is None else stream2
+        whole = C is None and (meta.m1 > 0 or meta.m2 > 0)
         if C is None:
-            C = torch.zeros((M, n), dtype=B.dtype, device=dev)
+            C = (torch.empty if whole else torch.zeros)((M, n), dtype=B.dtype, device=dev)
         need = spmm_workspace_bytes(meta.m1, n, B.element_size())
         if workspace is None and need:
             workspace = torch.empty(need, dtype=torch.uint8, device=dev)
@@ -294,6 +306,11 @@ def spmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torch
                 if isinstance(s, torch.cuda.Stream) and s != cur:
                     workspace.record_stream(s)
         ws_bytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
+        if whole:
+            spmm_all_raw(B.dtype, M, meta.m1, k, n, values.data_ptr(), col.data_ptr(), row_ptr.data_ptr(),
+                         meta.block_r_ind.data_ptr(), meta.st_off.data_ptr(), B.data_ptr(), C.data_ptr(),
+                         _ptr(workspace), ws_bytes, s1, s2, hot=_ptr(hot))
+            return C
         spmm_raw(B.dtype, meta.m1, meta.m2, k, n, values.data_ptr(), col.data_ptr(), row_ptr.data_ptr(),
                  meta.block_r_ind.data_ptr(), meta.residue_r_ind.data_ptr(), meta.st_off.data_ptr(), B.data_ptr(),
                  C.data_ptr(), _ptr(workspace), ws_bytes, s1, s2, hot=_ptr(hot))
@@ -318,8 +335,8 @@ def sddmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torc
         cur = torch.cuda.current_stream(dev)
         s1 = cur if stream1 is None else stream1
         s2 = cur if stream2 is None else stream2
-        if out is None:
-            out = torch.zeros(values.numel(), dtype=torch.float32, device=dev)
+        if out is None:  # every stored entry lies in a block segment or a residue row, so all of it is written
+            out = torch.empty(values.numel(), dtype=torch.float32, device=dev)
         sddmm_raw(meta.m1, meta.m2, rhs.shape[0], k, meta.block_r_ind.data_ptr(), meta.residue_r_ind.data_ptr(),
                   meta.st_off.data_ptr(), row_ptr.data_ptr(), col.data_ptr(), values.data_ptr(), lhs.data_ptr(),
                   rhs.data_ptr(), out.data_ptr(), s1, s2)

@@ -288,7 +288,37 @@ __device__ __forceinline__ unsigned group_mask(int lane) {
     }
 }
 
+// ---------------------------------------------------------------------------------------
+// The kernels of one call as a chain of programmatic dependents on one stream: each grid lets the next
+// one start as soon as all its own CTAs have started (chain_begin), so the chain runs like grids on
+// several streams but costs one launch call per grid and no events.  A grid that completes lets the
+// stream move on, so one warp or CTA of every grid that has nothing (more) to do waits for the grid
+// before it (chain_wait): no grid of the chain completes before all earlier ones have completed and
+// flushed their stores.  In the kernels whose code generation suffers from a common exit (the per-row
+// kernel of the stencil 0.695 -> 0.750 ms) that is a CTA of its own behind the last row.  Launched without
+// the attribute, both are no-ops.
+__device__ __forceinline__ void chain_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 #endif  // __CUDACC__
+
+#ifdef __CUDACC__
+// kernel<<<grid, block, 0, stream>>>(args...), with `chained` as a programmatic dependent of the grid
+// before it on the stream.
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t stream, bool chained, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+#endif
 
 // Number of SMs of the current device (looked up once per device; 148 if the query fails).
 inline int sm_count() {

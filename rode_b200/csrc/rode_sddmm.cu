@@ -231,7 +231,8 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
     const int g = lane / L, l = lane % L;
     const unsigned gmask = group_mask<L>(lane);
     const long long item0 = static_cast<long long>(blockIdx.x) * items_per_warp;
-    if (item0 >= n_items) return;
+    chain_begin();
+    if (item0 >= n_items) return chain_wait();  // the CTA behind the items
 
     // ---- descriptors: lane j owns item item0 + j --------------------------------------------
     int row = 0, begin = 0, len = 0;
@@ -444,6 +445,7 @@ sddmm_block(int m1, const int *__restrict__ block_r_ind, const int *__restrict__
     const int l = lane % L;
     const int gbase = lane - l;  // first lane (= first nonzero of the chunk) of this group
     const unsigned gmask = group_mask<L>(lane);
+    chain_begin();
     int seg = blockIdx.x;
     while (seg < m1) {
     int claimed = INT_MAX;  // never used in arithmetic: the loop test compares it with m1 as it is
@@ -609,9 +611,9 @@ int launch_k(int m1, int m2, int seg_cap, const int *block_r_ind, const int *res
     }
     if (m2 > 0) {
         const int per = items_per_warp(m2, 32);
-        sddmm_items<L, VPL, false, false, RL, RVPL><<<(m2 + per - 1) / per, 32, 0, s2>>>(
-            m2, per, residue_r_ind, nullptr, row_offsets, col, values, lhs, rhs, out, L * VPL,
-            RODE_SDDMM_ROW_MODE_MIN);
+        RODE_CUDA_TRY(launch_chained(sddmm_items<L, VPL, false, false, RL, RVPL>, dim3((m2 + per - 1) / per + 1), dim3(32), s2,
+                                     m1 > 0 && s1 == s2, m2, per, residue_r_ind, nullptr, row_offsets, col, values, lhs,
+                                     rhs, out, L * VPL, RODE_SDDMM_ROW_MODE_MIN));
         RODE_CHECK_LAUNCH("rode::sddmm_items<rows>");
     }
     return RODE_OK;
@@ -632,9 +634,9 @@ int launch_ragged(int m1, int m2, int k, const int *block_r_ind, const int *resi
     }
     if (m2 > 0) {
         const int per = items_per_warp(m2, 32);
-        sddmm_items<32, 2, false, true><<<(m2 + per - 1) / per, 32, 0, s2>>>(m2, per, residue_r_ind, nullptr,
-                                                                              row_offsets, col, values, lhs, rhs, out,
-                                                                              row_vecs, 0);
+        RODE_CUDA_TRY(launch_chained(sddmm_items<32, 2, false, true>, dim3((m2 + per - 1) / per + 1), dim3(32), s2,
+                                     m1 > 0 && s1 == s2, m2, per, residue_r_ind, nullptr, row_offsets, col, values, lhs,
+                                     rhs, out, row_vecs, 0));
         RODE_CHECK_LAUNCH("rode::sddmm_items<rows, any k>");
     }
     return RODE_OK;

@@ -158,11 +158,7 @@ spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ 
     constexpr int kSteps = 32 / G;        // nonzeros per group per 32-nonzero chunk
     constexpr int NB = (kSteps + U - 1) / U;
     constexpr unsigned kFull = 0xffffffffu;
-    // Programmatic dependent launch: as soon as every CTA of this grid has started, the fix-up
-    // grid may be scheduled into free slots.  Its warps look for rows that were cut into
-    // several segments; those that find none exit at once, the others wait for this grid to
-    // complete before they read the workspace.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const int g = lane / L, l = lane % L;
     // Chunk staging (two buffers, so one __syncwarp per chunk orders both the reads after the
@@ -312,43 +308,85 @@ spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ 
 }
 
 // ---------------------------------------------------------------------------------------
-// Sums the workspace slots of every row that was cut into several segments.  A one-warp CTA
-// looks at 32 consecutive segments; a lane whose segment is the first of a split row flags
-// it, and the warp then adds that row's slots (fp64 accumulation, eight slots in flight per
-// lane; the order is fixed by the code, so the result is deterministic).
-constexpr int kFixupThreads = 32;
-constexpr int kFixupUnroll = 8;  // workspace slots in flight per lane
+// Sums the workspace slots of every row that was cut into several segments, with fp64
+// accumulation and in an order that the code fixes, so the result is deterministic.
+//
+// What bounds it: latency, at the very end of the call (its time is not hidden behind anything).  A CTA
+// looks at up to kFixupThreads consecutive segments, one per thread, and lists the rows that begin among
+// them and were cut; its warps then take the listed rows one each, eight slots of 16 bytes per lane in
+// flight, and rows of more than kFixupWideSlots slots are taken by all warps together.  (One warp for 32
+// segments, which added its rows one after the other with 4-byte loads, took 7 us after the block grid's
+// end on the Zipf matrix, 25 us on Pareto 2^20 and 74 to 140 us on R-MAT scale 23, whose longest row has 470
+// slots.)
+constexpr int kFixupThreads = 256;
+constexpr int kFixupWarps = kFixupThreads / 32;
+constexpr int kFixupUnroll = 8;      // workspace slots in flight per lane
+constexpr int kFixupWideSlots = 24;  // rows with more slots are summed by the whole CTA
+
+// Sum over the slots s = s0, s0 + step, ... < cnt of vector x of a split row, `row_slots` = its first slot.
+template <typename T>
+__device__ __forceinline__ void fixup_sum(const typename Vec16<T>::type *__restrict__ row_slots, size_t row_vecs, int x,
+                                          int s0, int step, int cnt, double (&acc)[Vec16<T>::kLen]) {
+    using V = typename Vec16<T>::type;
+#pragma unroll
+    for (int j = 0; j < Vec16<T>::kLen; ++j) acc[j] = 0.0;
+    for (int s = s0; s < cnt; s += step * kFixupUnroll) {
+        V v[kFixupUnroll];
+#pragma unroll
+        for (int u = 0; u < kFixupUnroll; ++u) {
+            v[u] = vzero(static_cast<V *>(nullptr));
+            if (s + u * step < cnt) v[u] = __ldcg(row_slots + static_cast<size_t>(s + u * step) * row_vecs + x);
+        }
+#pragma unroll
+        for (int u = 0; u < kFixupUnroll; ++u) {
+            __align__(16) T e[Vec16<T>::kLen];
+            *reinterpret_cast<V *>(e) = v[u];
+#pragma unroll
+            for (int j = 0; j < Vec16<T>::kLen; ++j) acc[j] += static_cast<double>(e[j]);
+        }
+    }
+}
 
 template <typename T>
 __global__ void __launch_bounds__(kFixupThreads)
-spmm_fixup(int m1, int n, const int *__restrict__ row_offsets, const int *__restrict__ block_r_ind,
+spmm_fixup(int m1, int segs_per_cta, int n, const int *__restrict__ row_offsets, const int *__restrict__ block_r_ind,
            const int *__restrict__ st_off, const T *__restrict__ partial, T *__restrict__ C) {
+    using V = typename Vec16<T>::type;
+    constexpr int kLen = Vec16<T>::kLen;
     constexpr unsigned kFull = 0xffffffffu;
-    const int lane = threadIdx.x;
-    const int seg = blockIdx.x * 32 + lane;
-    bool head = false;
-    int row = 0, count = 0;
-    if (seg < m1) {
-        row = __ldg(block_r_ind + seg);
+    // split rows that begin in this CTA's range: narrow ones from the front, wide ones from the back
+    __shared__ int s_row[kFixupThreads], s_first[kFixupThreads], s_cnt[kFixupThreads];
+    __shared__ int n_narrow, n_wide;
+    __shared__ double s_part[kFixupWarps][32][kLen];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) n_narrow = n_wide = 0;
+    __syncthreads();
+    const int seg = blockIdx.x * segs_per_cta + threadIdx.x;
+    if (static_cast<int>(threadIdx.x) < segs_per_cta && seg < m1) {
+        const int row = __ldg(block_r_ind + seg);
         const int off = __ldg(st_off + seg);
         const int next = (seg + 1 < m1) ? __ldg(st_off + seg + 1) : INT_MAX;
         const int row_begin = __ldg(row_offsets + row);
         const int row_end = __ldg(row_offsets + row + 1);
-        head = (off == row_begin) && (next < row_end);
-        if (head) {
+        if ((off == row_begin) && (next < row_end)) {
             // number of segments of the row = pieces of (next - aligned start) nonzeros
-            const int piece = next - (row_begin - row_begin % 4);
-            count = (row_end - (row_begin - row_begin % 4) + piece - 1) / piece;
+            const int aligned = row_begin - row_begin % 4;
+            const int piece = next - aligned;
+            int count = (row_end - aligned + piece - 1) / piece;
             // the last piece is a segment only if it is >= 32 long; otherwise it was a
             // residue tail that the previous segment consumed
-            const int last_len = row_end - (row_begin - row_begin % 4) - (count - 1) * piece;
-            if (last_len < 32) --count;
+            if (row_end - aligned - (count - 1) * piece < 32) --count;
+            const int slot = count > kFixupWideSlots ? kFixupThreads - 1 - atomicAdd(&n_wide, 1) : atomicAdd(&n_narrow, 1);
+            s_row[slot] = row;
+            s_first[slot] = seg;
+            s_cnt[slot] = count;
         }
     }
-    unsigned todo = __ballot_sync(kFull, head);
-    if (todo == 0) {
-        // No split row among these 32 segments: nothing to read from the workspace.  The first
-        // CTA still waits for the block grid, so that this grid as a whole cannot complete
+    __syncthreads();
+    const int narrow = n_narrow, wide = n_wide;
+    if (narrow + wide == 0) {
+        // No split row begins among these segments: nothing to read from the workspace.  The first
+        // CTA still waits for the grids before this one, so that this grid as a whole cannot complete
         // before spmm_block has completed and flushed its stores: whatever the caller enqueues
         // on the stream afterwards (an event, a copy of C, the next kernel) is then ordered
         // after the block grid through this grid, as with a plain launch.
@@ -358,52 +396,63 @@ spmm_fixup(int m1, int n, const int *__restrict__ row_offsets, const int *__rest
     // Everything above read only the caller's metadata; the workspace is written by the
     // preceding spmm_block grid: wait for it (no-op when launched without the attribute).
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    while (todo) {
-        const int src = __ffs(todo) - 1;
-        todo &= todo - 1;
-        const int first = blockIdx.x * 32 + src;
-        const int r = __shfl_sync(kFull, row, src);
-        const int cnt = __shfl_sync(kFull, count, src);
-        // 4 columns per lane.  Rows narrower than 128 columns leave lanes over: those form
-        // 32 / (n/4) groups that take alternate slots and are combined by shuffles.
-        const int quads = n / 4;
-        const int width = (quads == 8 || quads == 16) ? quads : 32;  // lanes per slot
-        const int groups = 32 / width;
-        const int g = lane / width, l = lane % width;
-        for (int x = l * 4; x < n; x += 128) {
-            double acc[4] = {0.0, 0.0, 0.0, 0.0};
-            for (int s0 = g; s0 < cnt; s0 += groups * kFixupUnroll) {
-                T v[kFixupUnroll][4];
+
+    // `width` lanes cover a row of up to 32 vectors; narrower rows leave 32 / width groups of lanes that
+    // take alternate slots and are combined by shuffles.
+    const int row_vecs = n / kLen;
+    int width = 1;
+    while (width < row_vecs && width < 32) width <<= 1;
+    const int groups = 32 / width;
+    const int g = lane / width, l = lane % width;
+    auto combine_groups = [&](double (&acc)[kLen]) {
+        for (int w = width; w < 32; w <<= 1)
 #pragma unroll
-                for (int u = 0; u < kFixupUnroll; ++u) {
-                    const int s = s0 + u * groups;
+            for (int j = 0; j < kLen; ++j) acc[j] += __shfl_xor_sync(kFull, acc[j], w);
+    };
+    auto store = [&](int row, int x, const double (&acc)[kLen]) {
+        __align__(16) T e[kLen];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) v[u][j] = T(0);
-                    if (s < cnt) {
-                        const T *src_row = partial + static_cast<size_t>(first + s) * n + x;
+        for (int j = 0; j < kLen; ++j) e[j] = static_cast<T>(acc[j]);
+        st_stream(reinterpret_cast<V *>(C) + static_cast<size_t>(row) * row_vecs + x, *reinterpret_cast<const V *>(e));
+    };
+    for (int i = warp; i < narrow; i += kFixupWarps) {
+        const V *slots = reinterpret_cast<const V *>(partial) + static_cast<size_t>(s_first[i]) * row_vecs;
+        const int row = s_row[i], cnt = s_cnt[i];
+        for (int x0 = 0; x0 < row_vecs; x0 += 32) {
+            const int x = x0 + l;
+            double acc[kLen];
+            fixup_sum<T>(slots, row_vecs, x, x < row_vecs ? g : cnt, groups, cnt, acc);
+            combine_groups(acc);
+            if (g == 0 && x < row_vecs) store(row, x, acc);
+        }
+    }
+    for (int i = 0; i < wide; ++i) {
+        const int at = kFixupThreads - 1 - i;
+        const V *slots = reinterpret_cast<const V *>(partial) + static_cast<size_t>(s_first[at]) * row_vecs;
+        const int row = s_row[at], cnt = s_cnt[at];
+        for (int x0 = 0; x0 < row_vecs; x0 += 32) {
+            const int x = x0 + l;
+            double acc[kLen];
+            fixup_sum<T>(slots, row_vecs, x, x < row_vecs ? warp * groups + g : cnt, kFixupWarps * groups, cnt, acc);
+            combine_groups(acc);
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) v[u][j] = src_row[j];
-                    }
-                }
+            for (int j = 0; j < kLen; ++j) s_part[warp][lane][j] = acc[j];
+            __syncthreads();
+            if (warp == 0 && g == 0 && x < row_vecs) {
+                for (int w = 1; w < kFixupWarps; ++w)
 #pragma unroll
-                for (int u = 0; u < kFixupUnroll; ++u)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) acc[j] += static_cast<double>(v[u][j]);
+                    for (int j = 0; j < kLen; ++j) acc[j] += s_part[w][lane][j];
+                store(row, x, acc);
             }
-            for (int w = width; w < 32; w <<= 1)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[j] += __shfl_xor_sync(kFull, acc[j], w);
-            if (g == 0) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) C[static_cast<size_t>(r) * n + x + j] = static_cast<T>(acc[j]);
-            }
+            __syncthreads();
         }
     }
 }
 
 // ---------------------------------------------------------------------------------------
-// Residue rows without a block part.  One lane group per L consecutive entries of
-// residue_r_ind; grid.y walks the column tiles.
+// Rows without a block part: the entries of residue_r_ind, or, where that is null, all rows of the matrix
+// (n_items = their number; rows with a block part are skipped, rows without a nonzero stored as zeros).
+// One lane group per L consecutive entries; grid.y walks the column tiles.
 template <typename T, int L, bool kRagged>
 __global__ void __launch_bounds__(kCtaThreads, (sizeof(T) == 4 ? 32 : 16) / kCtaWarps)  // fp32: 64 registers
 spmm_rows(int m2, int rows_per_group, int n, const T *__restrict__ values,
@@ -416,6 +465,7 @@ spmm_rows(int m2, int rows_per_group, int n, const T *__restrict__ values,
     constexpr int NB = (L + U - 1) / U;  // batches per L-nonzero chunk
     constexpr int kAlign = 4;            // vec_len of the preprocessing
     constexpr int kBlockK = 32;          // k_block of the preprocessing
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const int l = lane % L;
     const unsigned gmask = group_mask<L>(lane);
@@ -443,12 +493,14 @@ spmm_rows(int m2, int rows_per_group, int n, const T *__restrict__ values,
 
     // ---- descriptors: lane j of the group owns residue row item0 + j -----------------------
     int row = 0, begin = 0, len = 0;
+    bool empty = false;  // all-rows form: a row of zeros
     if (l < rows_per_group && item0 + l < m2) {
-        row = __ldg(residue_r_ind + item0 + l);
+        row = residue_r_ind != nullptr ? __ldg(residue_r_ind + item0 + l) : item0 + l;
         begin = __ldg(row_offsets + row);
         const int end = __ldg(row_offsets + row + 1);
         // aligned length >= k_block: a block part exists and its last segment took the tail
         if (end - begin + (begin % kAlign) < kBlockK) len = end - begin;
+        empty = end == begin && residue_r_ind == nullptr;
     }
     int start = len;  // exclusive prefix sum of len inside the group
 #pragma unroll
@@ -467,8 +519,12 @@ spmm_rows(int m2, int rows_per_group, int n, const T *__restrict__ values,
     const bool inside = !kRagged || col_vec < row_vecs;  // ragged widths: lanes beyond the row's end idle
 
     // Rows of the list without a nonzero are left alone: C arrives zero-filled (the contract of
-    // the reference's entry points), and on graphs with many empty rows the zero rows were half
-    // of this kernel's DRAM writes.
+    // the reference's entry points).  In the all-rows form C arrives with any contents, and the rows
+    // without a nonzero, which are in no list when they start at a multiple of four, are stored here.
+    for (unsigned zeros = (__ballot_sync(gmask, empty) & gmask) >> gshift; zeros != 0; zeros &= zeros - 1) {
+        const int r = item0 + __ffs(zeros) - 1;
+        if (inside) st_stream(c_lane + static_cast<size_t>(r) * row_vecs, vzero(static_cast<V *>(nullptr)));
+    }
     unsigned todo = (__ballot_sync(gmask, len > 0) & gmask) >> gshift;  // rows with nonzeros, in order
     if (todo == 0) return;
 
@@ -559,6 +615,7 @@ spmm_rows(int m2, int rows_per_group, int n, const T *__restrict__ values,
     }();
     group = kClaim ? __shfl_sync(gmask, claimed, 0, L) : n_groups;
     }  // bundles of this group
+    if (blockIdx.x == 0 && blockIdx.y == 0) chain_wait();
 }
 
 // ---------------------------------------------------------------------------------------
@@ -586,6 +643,8 @@ spmm_rows_simple(int m2, int n, const T *__restrict__ values, const int *__restr
     constexpr int U = (kInFlight < L) ? kInFlight : L;
     constexpr int kAlign = 4;    // vec_len of the preprocessing
     constexpr int kBlockK = 32;  // k_block of the preprocessing
+    chain_begin();
+    if (blockIdx.x == gridDim.x - 1) return chain_wait();  // the CTA behind the rows
     const long long item_ll = (static_cast<long long>(blockIdx.x) * kRowsCtaThreads + threadIdx.x) / L;
     if (item_ll >= m2) return;
     const int item = static_cast<int>(item_ll);
@@ -593,12 +652,12 @@ spmm_rows_simple(int m2, int n, const T *__restrict__ values, const int *__restr
     const int l = lane % L;
     const unsigned gmask = group_mask<L>(lane);
 
-    const int row = __ldg(residue_r_ind + item);
+    const int row = residue_r_ind != nullptr ? __ldg(residue_r_ind + item) : item;
     const int begin = __ldg(row_offsets + row);
     const int end = __ldg(row_offsets + row + 1);
     // aligned length >= k_block: a block part exists and its last segment took the tail;
-    // no nonzero: the row stays as the caller zero-filled it
-    if (end - begin + (begin % kAlign) >= kBlockK || end == begin) return;
+    // list form, no nonzero: the row stays as the caller zero-filled it (all rows: zeros are stored below)
+    if (end - begin + (begin % kAlign) >= kBlockK || (end == begin && residue_r_ind != nullptr)) return;
 
     // (this kernel keeps the 64-bit index form of the dense-row address: the 32 x 32 -> 64 bit form of
     // the other kernels measured 2.7 % slower here, stencil N = 64 0.692 -> 0.711 ms)
@@ -695,17 +754,19 @@ spmm_rows_wide(int m2, int n, const T *__restrict__ values, const int *__restric
     constexpr int kAlign = 4;    // vec_len of the preprocessing
     constexpr int kBlockK = 32;  // k_block of the preprocessing
     constexpr unsigned kFull = 0xffffffffu;
+    chain_begin();
+    if (blockIdx.x == gridDim.x - 1) return chain_wait();  // the CTA behind the rows
     const int item = blockIdx.x * kSmallGridWarps + (threadIdx.x >> 5);
     if (item >= m2) return;
     const int lane = threadIdx.x & 31;
     const int g = lane / L, l = lane % L;
 
-    const int row = __ldg(residue_r_ind + item);
+    const int row = residue_r_ind != nullptr ? __ldg(residue_r_ind + item) : item;
     const int begin = __ldg(row_offsets + row);
     const int end = __ldg(row_offsets + row + 1);
     if (end - begin + (begin % kAlign) >= kBlockK) return;  // the block part took this row's tail
     const int len = end - begin;                            // < 32
-    if (len == 0) return;                                   // stays as the caller zero-filled it
+    if (len == 0 && residue_r_ind != nullptr) return;
 
     int c = 0;
     T val = T(0);
@@ -718,6 +779,16 @@ spmm_rows_wide(int m2, int n, const T *__restrict__ values, const int *__restric
     const size_t col_vec = static_cast<size_t>(blockIdx.y) * L * VPL + l;
     const V *b_lane = reinterpret_cast<const V *>(B) + col_vec;
     auto inside = [&](int v) { return !kRagged || col_vec + v * L < row_vecs; };
+    if (len == 0) {  // (list form: stays as the caller zero-filled it, returned above)
+        if (g == 0) {
+#pragma unroll
+            for (int v = 0; v < VPL; ++v)
+                if (inside(v))
+                    st_stream(reinterpret_cast<V *>(C) + static_cast<size_t>(row) * row_vecs + col_vec + v * L,
+                              vzero(static_cast<V *>(nullptr)));
+        }
+        return;
+    }
 
     int cc[L];
     T vv[L];
@@ -752,7 +823,7 @@ spmm_rows_wide(int m2, int n, const T *__restrict__ values, const int *__restric
 
 template <typename T, int VB, int L, int VPL, bool kRagged>
 int launch_rows(int m2, int n, const T *values, const int *col, const int *row_offsets, const int *residue_r_ind,
-                const T *B, T *C, int *counters, cudaStream_t s2);
+                const T *B, T *C, int *counters, bool chained, bool counters_clear, cudaStream_t s2);
 
 // Block kernel of shape (VB bytes per load, L lanes, VPL loads per lane) and residue-row kernel
 // of shape (RVB, RL, RVPL); both cover the same column tile.
@@ -768,6 +839,8 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
     constexpr int USmall = (kChunkSteps * VPL <= kSmallCap) ? kChunkSteps : kSmallCap / VPL;
     // ragged widths: the last tile is partly empty
     const unsigned tiles = static_cast<unsigned>(kRagged ? (n + kTileWidth - 1) / kTileWidth : n / kTileWidth);
+    const bool chained = s1 == s2 && m1 > 0;
+    bool counters_clear = false;  // the residue kernel's claim counters have been zeroed already
     if (m1 > 0) {
         // Fewer warps than two full waves of 32 per SM: the latency of the longest segment
         // rules, so batches are larger.  CTAs stay one warp: with 4-warp CTAs the Zipf matrix
@@ -784,10 +857,11 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
                                 tiles <= kMaxCounterTiles / 2 &&
                                 ctas_needed > kPersistentMinWaves * (resident / static_cast<int>(tiles));
         int *claim = nullptr;
-        if (persistent) {
-            RODE_CUDA_TRY(cudaMemsetAsync(counters, 0, sizeof(int) * tiles, s1));
-            claim = counters;
-        }
+        // in a chain the residue kernel's counters are zeroed here too: nothing may stand between two of its grids
+        counters_clear = chained && counters != nullptr && m2 > 32LL * kPersistentMinWaves * (resident / static_cast<int>(tiles));
+        if (persistent || counters_clear)
+            RODE_CUDA_TRY(cudaMemsetAsync(counters, 0, counters_clear ? kCounterBytes : sizeof(int) * tiles, s1));
+        if (persistent) claim = counters;
         dim3 grid(persistent ? (resident + tiles - 1) / tiles : ctas_needed, tiles);
         bool launched = false;
         // Popularity hints: block kernel of the 512-byte tile only.  In the residue-row kernel
@@ -809,67 +883,64 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
                 m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0, claim);
         }
         RODE_CHECK_LAUNCH("rode::spmm_block");
-        // fix-up as a programmatic dependent of spmm_block: its launch latency and its
-        // metadata prologue overlap the tail of the block grid
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((m1 + kFixupThreads - 1) / kFixupThreads);
-        cfg.blockDim = dim3(kFixupThreads);
-        cfg.dynamicSmemBytes = 0;
-        cfg.stream = s1;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
+    }
+    // Rows: on the block kernel's own stream they are chained behind it (see chain_begin), on another one
+    // they are a plain launch.
+    if (m2 > 0) {
+        if (int rc = launch_rows<T, RVB, RL, RVPL, kRagged>(m2, n, values, col, row_offsets, residue_r_ind, B, C, counters,
+                                                            chained, counters_clear, s2))
+            return rc;
+    }
+    if (m1 > 0) {
+        // fix-up last, chained behind the block grid (and the rows): its launch latency and its
+        // metadata prologue overlap the tail of those grids
+        int per = (m1 / (4 * sm_count()) + 31) / 32 * 32;  // segments per CTA: about four CTAs per SM
+        per = per < 32 ? 32 : (per > kFixupThreads ? kFixupThreads : per);
         const T *partial_in = partial;
-        RODE_CUDA_TRY(cudaLaunchKernelEx(&cfg, spmm_fixup<T>, m1, n, row_offsets, block_r_ind, st_off, partial_in,
-                                         C));
+        RODE_CUDA_TRY(launch_chained(spmm_fixup<T>, dim3((m1 + per - 1) / per), dim3(kFixupThreads), s1, true, m1, per, n,
+                                     row_offsets, block_r_ind, st_off, partial_in, C));
         RODE_CHECK_LAUNCH("rode::spmm_fixup");
     }
-    if (m2 > 0)
-        return launch_rows<T, RVB, RL, RVPL, kRagged>(m2, n, values, col, row_offsets, residue_r_ind, B, C, counters, s2);
     return RODE_OK;
 }
 
 template <typename T, int VB, int L, int VPL, bool kRagged>
 int launch_rows(int m2, int n, const T *values, const int *col, const int *row_offsets, const int *residue_r_ind,
-                const T *B, T *C, int *counters, cudaStream_t s2) {
+                const T *B, T *C, int *counters, bool chained, bool counters_clear, cudaStream_t s2) {
     constexpr int kTileWidth = L * VPL * VecB<T, VB>::kLen;
     const unsigned tiles = static_cast<unsigned>(kRagged ? (n + kTileWidth - 1) / kTileWidth : n / kTileWidth);
-    {
-        if constexpr (VB == 16 && L == 32 && VPL == 1) {
-            // 32 rows per warp when the list is long; fewer (shorter dependent chains, more
-            // warps) when the warps would not fill the GPU twice over
-            const long long slots = 2LL * 28 * sm_count() * (kCtaThreads / 32);
-            int per_group = static_cast<int>((m2 + slots - 1) / slots);
-            per_group = per_group < 4 ? 4 : (per_group > 32 ? 32 : per_group);
-            const long long groups = (static_cast<long long>(m2) + per_group - 1) / per_group;
-            constexpr int kGroupsPerCta = kCtaThreads / 32;
-            const long long ctas_needed = (groups + kGroupsPerCta - 1) / kGroupsPerCta;
-            const long long resident = static_cast<long long>(RODE_SPMM_PERSISTENT_CTAS_PER_SM) * sm_count();
-            const bool persistent = RODE_SPMM_PERSISTENT_ROWS != 0 && sizeof(T) == 4 && counters != nullptr &&
-                                    tiles <= kMaxCounterTiles / 2 &&
-                                    ctas_needed > kPersistentMinWaves * (resident / tiles);
-            int *claim = nullptr;
-            if (persistent) {
-                claim = counters + kMaxCounterTiles / 2;  // second half: the residue kernel's counters
-                RODE_CUDA_TRY(cudaMemsetAsync(claim, 0, sizeof(int) * tiles, s2));
-            }
-            dim3 grid(static_cast<unsigned>(persistent ? (resident + tiles - 1) / tiles : ctas_needed), tiles);
-            spmm_rows<T, 32, kRagged><<<grid, kCtaThreads, 0, s2>>>(m2, per_group, n, values, col, row_offsets,
-                                                           residue_r_ind, B, C, claim);
-        } else if (static_cast<long long>(m2) * tiles <= RODE_SPMM_WIDE_ROWS_WAVES * 32LL * sm_count()) {
-            dim3 grid((m2 + kSmallGridWarps - 1) / kSmallGridWarps, tiles);
-            spmm_rows_wide<T, VB, L, VPL, kRagged><<<grid, 32 * kSmallGridWarps, 0, s2>>>(m2, n, values, col, row_offsets,
-                                                                                 residue_r_ind, B, C);
-        } else {
-            constexpr int kRowsPerCta = kRowsCtaThreads / L;
-            dim3 grid((m2 + kRowsPerCta - 1) / kRowsPerCta, tiles);
-            spmm_rows_simple<T, VB, L, VPL, kRagged><<<grid, kRowsCtaThreads, 0, s2>>>(m2, n, values, col, row_offsets,
-                                                                              residue_r_ind, B, C);
+    if constexpr (VB == 16 && L == 32 && VPL == 1) {
+        // 32 rows per warp when the list is long; fewer (shorter dependent chains, more
+        // warps) when the warps would not fill the GPU twice over
+        const long long slots = 2LL * 28 * sm_count() * (kCtaThreads / 32);
+        int per_group = static_cast<int>((m2 + slots - 1) / slots);
+        per_group = per_group < 4 ? 4 : (per_group > 32 ? 32 : per_group);
+        const long long groups = (static_cast<long long>(m2) + per_group - 1) / per_group;
+        constexpr int kGroupsPerCta = kCtaThreads / 32;
+        const long long ctas_needed = (groups + kGroupsPerCta - 1) / kGroupsPerCta;
+        const long long resident = static_cast<long long>(RODE_SPMM_PERSISTENT_CTAS_PER_SM) * sm_count();
+        const bool persistent = RODE_SPMM_PERSISTENT_ROWS != 0 && sizeof(T) == 4 && counters != nullptr &&
+                                tiles <= kMaxCounterTiles / 2 && (!chained || counters_clear) &&
+                                ctas_needed > kPersistentMinWaves * (resident / tiles);
+        int *claim = nullptr;
+        if (persistent) {
+            claim = counters + kMaxCounterTiles / 2;  // second half: the residue kernel's counters
+            if (!counters_clear) RODE_CUDA_TRY(cudaMemsetAsync(claim, 0, sizeof(int) * tiles, s2));
         }
-        RODE_CHECK_LAUNCH("rode::spmm_rows");
+        const dim3 grid(static_cast<unsigned>(persistent ? (resident + tiles - 1) / tiles : ctas_needed), tiles);
+        RODE_CUDA_TRY(launch_chained(spmm_rows<T, 32, kRagged>, grid, dim3(kCtaThreads), s2, chained, m2, per_group, n, values,
+                                     col, row_offsets, residue_r_ind, B, C, claim));
+    } else if (static_cast<long long>(m2) * tiles <= RODE_SPMM_WIDE_ROWS_WAVES * 32LL * sm_count()) {
+        const dim3 grid((m2 + kSmallGridWarps - 1) / kSmallGridWarps + 1, tiles);
+        RODE_CUDA_TRY(launch_chained(spmm_rows_wide<T, VB, L, VPL, kRagged>, grid, dim3(32 * kSmallGridWarps), s2, chained, m2,
+                                     n, values, col, row_offsets, residue_r_ind, B, C));
+    } else {
+        constexpr int kRowsPerCta = kRowsCtaThreads / L;
+        const dim3 grid((m2 + kRowsPerCta - 1) / kRowsPerCta + 1, tiles);
+        RODE_CUDA_TRY(launch_chained(spmm_rows_simple<T, VB, L, VPL, kRagged>, grid, dim3(kRowsCtaThreads), s2, chained, m2, n,
+                                     values, col, row_offsets, residue_r_ind, B, C));
     }
+    RODE_CHECK_LAUNCH("rode::spmm_rows");
     return RODE_OK;
 }
 
@@ -881,7 +952,8 @@ constexpr int wide_vpl(int shape) { return (shape % 100) % 2 == 0 ? (shape % 100
 template <typename T>
 int spmm(int m1, int m2, int k, int n, const T *values, const int *col, const int *row_offsets,
          const int *block_r_ind, const int *residue_r_ind, const int *st_off, const T *B, T *C, void *workspace,
-         size_t workspace_bytes, const unsigned *hot, rode_stream_t stream1, rode_stream_t stream2) {
+         size_t workspace_bytes, const unsigned *hot, rode_stream_t stream1, rode_stream_t stream2,
+         bool all_rows = false) {
     constexpr int kLen = Vec16<T>::kLen;
     if (m1 < 0 || m2 < 0 || n <= 0) return fail(RODE_ERR_INVALID_ARGUMENT, "spmm: m1, m2 >= 0 and n > 0 required");
     if (hot != nullptr && k <= 0)
@@ -889,9 +961,10 @@ int spmm(int m1, int m2, int k, int n, const T *values, const int *col, const in
                                                "when hot_columns is given");
     if (n % 4 != 0) return fail(RODE_ERR_INVALID_ARGUMENT, "spmm: n = %d is not a multiple of 4", n);
     if (m1 == 0 && m2 == 0) return RODE_OK;
-    if (!values || !col || !row_offsets || !B || !C) return fail(RODE_ERR_INVALID_ARGUMENT, "spmm: null array");
+    const bool may_be_empty = all_rows && m1 == 0;  // rows of zeros only: nothing of the three arrays is read
+    if (!row_offsets || !C || (!may_be_empty && (!values || !col || !B))) return fail(RODE_ERR_INVALID_ARGUMENT, "spmm: null array");
     if (m1 > 0 && (!block_r_ind || !st_off)) return fail(RODE_ERR_INVALID_ARGUMENT, "spmm: null block metadata");
-    if (m2 > 0 && !residue_r_ind) return fail(RODE_ERR_INVALID_ARGUMENT, "spmm: null residue metadata");
+    if (m2 > 0 && !residue_r_ind && !all_rows) return fail(RODE_ERR_INVALID_ARGUMENT, "spmm: null residue metadata");
     if (!aligned_to(B, 16) || !aligned_to(C, 16))
         return fail(RODE_ERR_INVALID_ARGUMENT, "spmm: B and C must be 16-byte aligned");
     if ((n + 8 * kLen - 1) / (8 * kLen) > 65535)
@@ -1008,6 +1081,22 @@ int rode_spmm_f64_hot(int m1, int m2, int k, int n, const double *values, const 
                       const unsigned *hot_columns, rode_stream_t stream1, rode_stream_t stream2) {
     return rode::spmm<double>(m1, m2, k, n, values, column_indices, row_offsets, block_r_ind, residue_r_ind,
                               st_off, B, C, workspace, workspace_bytes, hot_columns, stream1, stream2);
+}
+
+int rode_spmm_f32_all(int M, int m1, int k, int n, const float *values, const int *column_indices,
+                      const int *row_offsets, const int *block_r_ind, const int *st_off, const float *B, float *C,
+                      void *workspace, size_t workspace_bytes, const unsigned *hot_columns, rode_stream_t stream1,
+                      rode_stream_t stream2) {
+    return rode::spmm<float>(m1, M, k, n, values, column_indices, row_offsets, block_r_ind, nullptr, st_off, B, C,
+                             workspace, workspace_bytes, hot_columns, stream1, stream2, /*all_rows=*/true);
+}
+
+int rode_spmm_f64_all(int M, int m1, int k, int n, const double *values, const int *column_indices,
+                      const int *row_offsets, const int *block_r_ind, const int *st_off, const double *B, double *C,
+                      void *workspace, size_t workspace_bytes, const unsigned *hot_columns, rode_stream_t stream1,
+                      rode_stream_t stream2) {
+    return rode::spmm<double>(m1, M, k, n, values, column_indices, row_offsets, block_r_ind, nullptr, st_off, B, C,
+                              workspace, workspace_bytes, hot_columns, stream1, stream2, /*all_rows=*/true);
 }
 
 }  // extern "C"

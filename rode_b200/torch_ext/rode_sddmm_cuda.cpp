@@ -10,14 +10,12 @@
 //     reference's calling convention) is copied to the current CUDA device, decomposed
 //     there, and the results are returned as CPU tensors; a CUDA row_offsets tensor gives
 //     CUDA results without any host round trip except the two counts.
-//   * sddmm_forward launches on torch's current stream (block part) and one side stream
-//     from torch's pool (residue part) joined back with an event, instead of creating,
-//     synchronising and destroying two streams per call
-//     (RoDe_SDDMM/rode_sddmm_cuda.cu:203-246); it does not block the host.
+//   * sddmm_forward launches on torch's current stream, where block and residue part run side by
+//     side as programmatic dependents, instead of creating, synchronising and destroying two
+//     streams per call (RoDe_SDDMM/rode_sddmm_cuda.cu:203-246); it does not block the host.
 //   * k_version may also be 64.
 //   * spmm_forward and hot_columns are new: the reference has no Python entry for SpMM.
 #include <ATen/cuda/CUDAContext.h>
-#include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
@@ -37,20 +35,6 @@ namespace {
 #define RODE_CHECK_INT(x) TORCH_CHECK((x).dtype() == torch::kInt32, #x " must be int32")
 
 void check_status(int status) { TORCH_CHECK(status == RODE_OK, "rode_b200: ", rode_last_error()); }
-
-// Runs `launch(stream1, stream2)` with the block work on the current stream and the residue
-// work on a pool stream forked from it and joined back into it.
-template <typename F>
-void fork_join(const c10::Device &device, F launch) {
-    auto cur = at::cuda::getCurrentCUDAStream(device.index());
-    auto side = at::cuda::getStreamFromPool(false, device.index());
-    at::cuda::CUDAEvent fork, join;
-    fork.record(cur);
-    fork.block(side);
-    launch(cur.stream(), side.stream());
-    join.record(side);
-    join.block(cur);
-}
 
 std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, int, int> py_preprocess(torch::Tensor row_offsets, int nnz,
                                                                                  int seg_length, int k_block,
@@ -119,15 +103,14 @@ torch::Tensor py_sddmm_forward(torch::Tensor block_indices, torch::Tensor residu
     TORCH_CHECK(row_offsets.size(0) == m + 1, "row_offsets must have m + 1 entries");
 
     const c10::cuda::CUDAGuard guard(values.device());
-    torch::Tensor out = torch::zeros({values.size(0)}, values.options());
-    if (m1 == 0 && m2 == 0) return out;
-    fork_join(values.device(), [&](cudaStream_t s1, cudaStream_t s2) {
-        check_status(rode_sddmm_f32(m1, m2, n, k, block_indices.data_ptr<int>(), residue_indices.data_ptr<int>(),
-                                    st_offsets.data_ptr<int>(), row_offsets.data_ptr<int>(),
-                                    column_indices.data_ptr<int>(), values.data_ptr<float>(),
-                                    lhs_matrix.data_ptr<float>(), rhs_matrix.data_ptr<float>(), out.data_ptr<float>(),
-                                    s1, s2));
-    });
+    if (m1 == 0 && m2 == 0) return torch::zeros({values.size(0)}, values.options());
+    // every stored entry lies in a block segment or a residue row, so every element is written
+    torch::Tensor out = torch::empty({values.size(0)}, values.options());
+    const cudaStream_t s = at::cuda::getCurrentCUDAStream(values.device().index()).stream();
+    check_status(rode_sddmm_f32(m1, m2, n, k, block_indices.data_ptr<int>(), residue_indices.data_ptr<int>(),
+                                st_offsets.data_ptr<int>(), row_offsets.data_ptr<int>(), column_indices.data_ptr<int>(),
+                                values.data_ptr<float>(), lhs_matrix.data_ptr<float>(), rhs_matrix.data_ptr<float>(),
+                                out.data_ptr<float>(), s, s));
     return out;
 }
 
@@ -179,8 +162,8 @@ torch::Tensor py_spmm_forward(torch::Tensor block_indices, torch::Tensor residue
     const int n = static_cast<int>(dense.size(1));
 
     const c10::cuda::CUDAGuard guard(values.device());
-    torch::Tensor out = torch::zeros({m, n}, dense.options());
-    if (m1 == 0 && m2 == 0) return out;
+    if (m1 == 0 && m2 == 0) return torch::zeros({m, n}, dense.options());
+    torch::Tensor out = torch::empty({m, n}, dense.options());  // every row is written
     size_t ws_bytes = 0;
     check_status(rode_spmm_workspace_bytes(m1, n, static_cast<int>(dense.element_size()), &ws_bytes));
     torch::Tensor ws = torch::empty({static_cast<long long>(std::max<size_t>(ws_bytes, 16))},
@@ -193,23 +176,17 @@ torch::Tensor py_spmm_forward(torch::Tensor block_indices, torch::Tensor residue
                     "hot_columns must come from hot_columns() for this matrix");
         hot = reinterpret_cast<const unsigned *>(hot_columns->data_ptr<int>());
     }
-    fork_join(values.device(), [&](cudaStream_t s1, cudaStream_t s2) {
-        if (dense.dtype() == torch::kFloat32)
-            check_status(rode_spmm_f32_hot(m1, m2, k, n, values.data_ptr<float>(), column_indices.data_ptr<int>(),
-                                           row_offsets.data_ptr<int>(), block_indices.data_ptr<int>(),
-                                           residue_indices.data_ptr<int>(), st_offsets.data_ptr<int>(),
-                                           dense.data_ptr<float>(), out.data_ptr<float>(), ws.data_ptr(), ws_bytes,
-                                           hot, s1, s2));
-        else
-            check_status(rode_spmm_f64_hot(m1, m2, k, n, values.data_ptr<double>(), column_indices.data_ptr<int>(),
-                                           row_offsets.data_ptr<int>(), block_indices.data_ptr<int>(),
-                                           residue_indices.data_ptr<int>(), st_offsets.data_ptr<int>(),
-                                           dense.data_ptr<double>(), out.data_ptr<double>(), ws.data_ptr(), ws_bytes,
-                                           hot, s1, s2));
-    });
-    // The workspace is used by the block and fix-up kernels on the current stream and, for its
-    // claim counters, by the residue kernel on the side stream; the side stream was joined back
-    // into the current one, so the caching allocator may reuse the buffer after this call.
+    const cudaStream_t s = at::cuda::getCurrentCUDAStream(values.device().index()).stream();
+    if (dense.dtype() == torch::kFloat32)
+        check_status(rode_spmm_f32_all(m, m1, k, n, values.data_ptr<float>(), column_indices.data_ptr<int>(),
+                                       row_offsets.data_ptr<int>(), block_indices.data_ptr<int>(),
+                                       st_offsets.data_ptr<int>(), dense.data_ptr<float>(), out.data_ptr<float>(),
+                                       ws.data_ptr(), ws_bytes, hot, s, s));
+    else
+        check_status(rode_spmm_f64_all(m, m1, k, n, values.data_ptr<double>(), column_indices.data_ptr<int>(),
+                                       row_offsets.data_ptr<int>(), block_indices.data_ptr<int>(),
+                                       st_offsets.data_ptr<int>(), dense.data_ptr<double>(), out.data_ptr<double>(),
+                                       ws.data_ptr(), ws_bytes, hot, s, s));
     return out;
 }
 
