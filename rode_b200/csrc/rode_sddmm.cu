@@ -47,29 +47,7 @@
 namespace rode {
 namespace {
 
-// Shape of a lane group per K: L lanes x VPL 16-byte vectors per lane (K = 4 * L * VPL),
-// encoded as L * 100 + VPL.  A batch holds 8 / VPL nonzeros, so a lane always has 8 loads
-// in flight.
-#ifndef RODE_SDDMM_SHAPE_32
-#define RODE_SDDMM_SHAPE_32 801
-#endif
-#ifndef RODE_SDDMM_SHAPE_64
-#define RODE_SDDMM_SHAPE_64 1601
-#endif
-#ifndef RODE_SDDMM_SHAPE_128
-#define RODE_SDDMM_SHAPE_128 3201
-#endif
-// Shape of a lane group in the row-per-group mode of the residue-row kernel (0 = no such mode),
-// and the mean number of nonzeros per row from which a warp uses it.
-#ifndef RODE_SDDMM_ROW_SHAPE_32
-#define RODE_SDDMM_ROW_SHAPE_32 801
-#endif
-#ifndef RODE_SDDMM_ROW_SHAPE_64
-#define RODE_SDDMM_ROW_SHAPE_64 802
-#endif
-#ifndef RODE_SDDMM_ROW_SHAPE_128
-#define RODE_SDDMM_ROW_SHAPE_128 0
-#endif
+// Mean number of nonzeros per row from which a warp of the residue-row kernel takes its rows one by one.
 #ifndef RODE_SDDMM_ROW_MODE_MIN
 #define RODE_SDDMM_ROW_MODE_MIN 6
 #endif
@@ -81,9 +59,6 @@ namespace {
 // Lane-group sizes L of the stream kernel for which it stages (bit mask: 8 | 16 | 32).
 #ifndef RODE_SDDMM_ITEMS_SMEM_MASK
 #define RODE_SDDMM_ITEMS_SMEM_MASK (8 | 16 | 32)
-#endif
-#ifndef RODE_SDDMM_LONG_SEGMENTS_BY_WARP
-#define RODE_SDDMM_LONG_SEGMENTS_BY_WARP 1
 #endif
 constexpr int kLoadsInFlight = 8;  // 16-byte loads per lane per batch
 constexpr unsigned kFull = 0xffffffffu;
@@ -120,22 +95,25 @@ __device__ __forceinline__ float reduce_batch(float (&p)[NB], int l, unsigned gm
 // `stage` = 2 x 32 ints of shared memory owned by this warp (two chunk buffers), `stage_buf` the
 // buffer to use next; both are carried from row to row so that a group never stores into a
 // buffer that one of its lanes may still read.
-template <int L, int VPL, bool kStageAllowed>
-__device__ __forceinline__ void sddmm_one_row(int row, int begin, int end, int lane,
+// kRagged: the dense rows hold row_vecs_arg <= L * VPL vectors, the rest of the lanes idle.
+template <int L, int VPL, bool kStageAllowed, bool kRagged>
+__device__ __forceinline__ void sddmm_one_row(int row, int begin, int end, int lane, int row_vecs_arg,
                                               const int *__restrict__ column_indices,
                                               const float *__restrict__ values, const float *__restrict__ lhs,
                                               const float *__restrict__ rhs, float *__restrict__ out, int *stage,
                                               int &stage_buf) {
     constexpr int kBatch = (kLoadsInFlight / VPL < L) ? kLoadsInFlight / VPL : L;
     constexpr bool kStage = RODE_SDDMM_COLUMNS_IN_SMEM != 0 && kStageAllowed && (kBatch % 4 == 0);
-    constexpr size_t kRowVecs = L * VPL;
+    const unsigned row_vecs = kRagged ? row_vecs_arg : L * VPL;
     const int l = lane % L;
     const unsigned gmask = group_mask<L>(lane);
     const float4 *rhs_lane = reinterpret_cast<const float4 *>(rhs) + l;
+    auto inside = [&](int v) { return !kRagged || static_cast<unsigned>(l + v * L) < row_vecs; };
     float4 a[VPL];
 #pragma unroll
     for (int v = 0; v < VPL; ++v)
-        a[v] = __ldg(reinterpret_cast<const float4 *>(lhs) + static_cast<size_t>(row) * kRowVecs + v * L + l);
+        a[v] = inside(v) ? __ldg(reinterpret_cast<const float4 *>(lhs) + static_cast<size_t>(row) * row_vecs + v * L + l)
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
     int c_nxt = 0;
     float v_nxt = 0.f;
     if (begin + l < end) {
@@ -173,7 +151,8 @@ __device__ __forceinline__ void sddmm_one_row(int row, int begin, int end, int l
 #pragma unroll
                     for (int v = 0; v < VPL; ++v) {
                         bb[u][v] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (t < cnt) bb[u][v] = ld_dense(rhs_lane + static_cast<size_t>(cc[u]) * kRowVecs + v * L);
+                        if (t < cnt && inside(v))
+                            bb[u][v] = ld_dense(rhs_lane + static_cast<size_t>(cc[u]) * row_vecs + v * L);
                     }
                 }
                 float p[kBatch];
@@ -213,14 +192,14 @@ __device__ __forceinline__ void sddmm_one_row(int row, int begin, int end, int l
 #define RODE_SDDMM_ITEMS_MIN_CTAS 28
 #endif
 template <int L, int VPL, bool kSegments, bool kRagged = false, int LB = 0, int VPLB = 1>
-__global__ void __launch_bounds__(32, kRagged ? 24 : RODE_SDDMM_ITEMS_MIN_CTAS)
+__global__ void __launch_bounds__(32, VPL > 1 ? 24 : RODE_SDDMM_ITEMS_MIN_CTAS)
 sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, const int *__restrict__ st_off,
             const int *__restrict__ row_offsets, const int *__restrict__ column_indices,
             const float *__restrict__ values, const float *__restrict__ lhs, const float *__restrict__ rhs,
             float *__restrict__ out, int row_vecs_arg, int row_mode_min) {
     constexpr int G = 32 / L;
     constexpr int kBatch = kLoadsInFlight / VPL;  // nonzeros per batch
-    const size_t kRowVecs = kRagged ? static_cast<size_t>(row_vecs_arg) : L * VPL;  // float4 per dense row (K / 4)
+    const size_t row_vecs = kRagged ? static_cast<unsigned>(row_vecs_arg) : L * VPL;  // float4 per dense row (K / 4)
     constexpr int kAlign = 4;             // vec_len of the preprocessing
     constexpr int kBlockK = 32;           // k_block of the preprocessing
     __shared__ int s_end[32];             // stream position where item j ends
@@ -261,7 +240,7 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
     start -= len;
     const unsigned nonempty = __ballot_sync(kFull, len > 0);
     if (total == 0) return;
-    if constexpr (LB > 0 && !kSegments && !kRagged) {
+    if constexpr (LB > 0 && !kSegments) {
         static_assert(LB * VPLB == L * VPL, "both lane-group shapes must cover the same dense row");
         // (full warps of 32 rows only: short lists give a warp fewer rows than it has groups, and
         // there the stream's even split of the nonzeros is what shortens the dependent chain)
@@ -274,8 +253,8 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
                 const int b0 = __shfl_sync(kFull, begin, j & 31);
                 const int n0 = __shfl_sync(kFull, len, j & 31);
                 if (j < items_per_warp && n0 > 0)
-                    sddmm_one_row<LB, VPLB, ((RODE_SDDMM_ITEMS_SMEM_MASK) & L) != 0>(r, b0, b0 + n0, lane, column_indices, values, lhs, rhs, out, &s_col[0][0],
-                                            stage_buf);
+                    sddmm_one_row<LB, VPLB, ((RODE_SDDMM_ITEMS_SMEM_MASK) & L) != 0, kRagged>(
+                        r, b0, b0 + n0, lane, row_vecs_arg, column_indices, values, lhs, rhs, out, &s_col[0][0], stage_buf);
             }
             return;
         }
@@ -311,9 +290,9 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
     const float4 *lhs_lane = reinterpret_cast<const float4 *>(lhs) + l;
     const float4 *rhs_lane = reinterpret_cast<const float4 *>(rhs) + l;
     // vector v of this lane lies inside the dense row
-    auto inside = [&](int v) { return !kRagged || static_cast<size_t>(l + v * L) < kRowVecs; };
+    auto inside = [&](int v) { return !kRagged || static_cast<size_t>(l + v * L) < row_vecs; };
     auto load_lhs = [&](int item, int v) {
-        return inside(v) ? __ldg(lhs_lane + static_cast<size_t>(s_row[item]) * kRowVecs + v * L)
+        return inside(v) ? __ldg(lhs_lane + static_cast<size_t>(s_row[item]) * row_vecs + v * L)
                          : make_float4(0.f, 0.f, 0.f, 0.f);
     };
 
@@ -372,7 +351,7 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
                     for (int v = 0; v < VPL; ++v) {
                         bb[u][v] = make_float4(0.f, 0.f, 0.f, 0.f);
                         if (t < cnt && inside(v))
-                            bb[u][v] = ld_dense(rhs_lane + static_cast<size_t>(cc[u]) * kRowVecs + v * L);
+                            bb[u][v] = ld_dense(rhs_lane + static_cast<size_t>(cc[u]) * row_vecs + v * L);
                     }
                 }
                 float p[kBatch];
@@ -430,14 +409,14 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
 // claims further ones from *next_segment; the claim is issued before the segment's work and
 // read after it.  One-warp CTAs of one segment each live a few microseconds, and a fifth of the
 // warp slots stood empty waiting for the next CTA to be launched into them.
-template <int L, int VPL, bool kClaim>
-__global__ void __launch_bounds__(32, 32)  // 64 registers: 32 one-warp CTAs per SM
+template <int L, int VPL, bool kClaim, bool kRagged = false>
+__global__ void __launch_bounds__(32, VPL == 1 ? 32 : 24)  // 64 registers: 32 one-warp CTAs per SM
 sddmm_block(int m1, const int *__restrict__ block_r_ind, const int *__restrict__ st_off,
             const int *__restrict__ row_offsets, const int *__restrict__ column_indices,
             const float *__restrict__ values, const float *__restrict__ lhs, const float *__restrict__ rhs,
-            float *__restrict__ out, int *__restrict__ next_segment) {
+            float *__restrict__ out, int *__restrict__ next_segment, int row_vecs_arg) {
     constexpr int kBatch = kLoadsInFlight / VPL;
-    constexpr size_t kRowVecs = L * VPL;
+    const size_t row_vecs = kRagged ? static_cast<unsigned>(row_vecs_arg) : L * VPL;
     constexpr bool kStage = RODE_SDDMM_COLUMNS_IN_SMEM != 0 && (kBatch % 4 == 0);
     __shared__ __align__(16) int s_col[2][32];  // column indices of the current chunk, two buffers
     int stage_buf = 0;
@@ -459,10 +438,12 @@ sddmm_block(int m1, const int *__restrict__ block_r_ind, const int *__restrict__
     const int end = min(__ldg(row_offsets + row + 1), next);
 
     const float4 *rhs_lane = reinterpret_cast<const float4 *>(rhs) + l;
+    auto inside = [&](int v) { return !kRagged || static_cast<size_t>(l + v * L) < row_vecs; };
     float4 a[VPL];
 #pragma unroll
     for (int v = 0; v < VPL; ++v)
-        a[v] = __ldg(reinterpret_cast<const float4 *>(lhs) + static_cast<size_t>(row) * kRowVecs + v * L + l);
+        a[v] = inside(v) ? __ldg(reinterpret_cast<const float4 *>(lhs) + static_cast<size_t>(row) * row_vecs + v * L + l)
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
 
     int c_cur = 0, c_nxt = 0;
     float v_cur = 0.f, v_nxt = 0.f;
@@ -500,8 +481,8 @@ sddmm_block(int m1, const int *__restrict__ block_r_ind, const int *__restrict__
 #pragma unroll
                     for (int v = 0; v < VPL; ++v) {
                         bb[u][v] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (gbase + t < cnt)
-                            bb[u][v] = ld_dense(rhs_lane + static_cast<size_t>(cc[u]) * kRowVecs + v * L);
+                        if (gbase + t < cnt && inside(v))
+                            bb[u][v] = ld_dense(rhs_lane + static_cast<size_t>(cc[u]) * row_vecs + v * L);
                     }
                 }
                 float p[kBatch];
@@ -582,62 +563,42 @@ int items_per_warp(int n_items, int cap) {
     return static_cast<int>(per);
 }
 
-template <int L, int VPL, int RL, int RVPL>
-int launch_k(int m1, int m2, int seg_cap, const int *block_r_ind, const int *residue_r_ind, const int *st_off,
-             const int *row_offsets, const int *col, const float *values, const float *lhs, const float *rhs,
-             float *out, cudaStream_t s1, cudaStream_t s2) {
+// L lanes x VPL vectors for the segments and the streams, RL x RVPL (RL = 0: none) for the row mode of the
+// residue kernel.  kLongSegments: a warp per segment, else up to 32 segments per warp.
+template <int L, int VPL, int RL, int RVPL, bool kRagged, bool kLongSegments>
+int launch_k(int m1, int m2, int k, const int *block_r_ind, const int *residue_r_ind,
+             const int *st_off, const int *row_offsets, const int *col, const float *values, const float *lhs,
+             const float *rhs, float *out, cudaStream_t s1, cudaStream_t s2) {
+    const int row_vecs = k / 4;
     if (m1 > 0) {
-        if (seg_cap < 32 && RODE_SDDMM_LONG_SEGMENTS_BY_WARP) {
-            const int resident = 32 * sm_count();
+        if constexpr (kLongSegments) {
+            const int resident = (VPL == 1 ? 32 : 24) * sm_count();
             int *claim = nullptr;
             if (RODE_SDDMM_PERSISTENT && m1 > 16 * resident) {  // from about 16 segments per warp on it pays
                 if (int rc = claim_counters(s1, s2, &claim)) return rc;
             }
             if (claim != nullptr) {
                 RODE_CUDA_TRY(cudaMemsetAsync(claim, 0, sizeof(int), s1));
-                sddmm_block<L, VPL, true><<<resident, 32, 0, s1>>>(m1, block_r_ind, st_off, row_offsets, col, values, lhs,
-                                                                   rhs, out, claim);
+                sddmm_block<L, VPL, true, kRagged><<<resident, 32, 0, s1>>>(m1, block_r_ind, st_off, row_offsets, col, values,
+                                                                            lhs, rhs, out, claim, row_vecs);
             } else {
-                sddmm_block<L, VPL, false><<<m1, 32, 0, s1>>>(m1, block_r_ind, st_off, row_offsets, col, values, lhs, rhs,
-                                                              out, nullptr);
+                sddmm_block<L, VPL, false, kRagged><<<m1, 32, 0, s1>>>(m1, block_r_ind, st_off, row_offsets, col, values, lhs,
+                                                                       rhs, out, nullptr, row_vecs);
             }
             RODE_CHECK_LAUNCH("rode::sddmm_block");
         } else {
-            const int per = items_per_warp(m1, seg_cap);
-            sddmm_items<L, VPL, true><<<(m1 + per - 1) / per, 32, 0, s1>>>(m1, per, block_r_ind, st_off, row_offsets,
-                                                                            col, values, lhs, rhs, out, L * VPL, 0);
+            const int per = items_per_warp(m1, 32);
+            sddmm_items<L, VPL, true, kRagged><<<(m1 + per - 1) / per, 32, 0, s1>>>(
+                m1, per, block_r_ind, st_off, row_offsets, col, values, lhs, rhs, out, row_vecs, 0);
             RODE_CHECK_LAUNCH("rode::sddmm_items<segments>");
         }
     }
     if (m2 > 0) {
         const int per = items_per_warp(m2, 32);
-        RODE_CUDA_TRY(launch_chained(sddmm_items<L, VPL, false, false, RL, RVPL>, dim3((m2 + per - 1) / per + 1), dim3(32), s2,
+        RODE_CUDA_TRY(launch_chained(sddmm_items<L, VPL, false, kRagged, RL, RVPL>, dim3((m2 + per - 1) / per + 1), dim3(32), s2,
                                      m1 > 0 && s1 == s2, m2, per, residue_r_ind, nullptr, row_offsets, col, values, lhs,
-                                     rhs, out, L * VPL, RODE_SDDMM_ROW_MODE_MIN));
+                                     rhs, out, row_vecs, RODE_SDDMM_ROW_MODE_MIN));
         RODE_CHECK_LAUNCH("rode::sddmm_items<rows>");
-    }
-    return RODE_OK;
-}
-
-// Any other K that is a multiple of 4, up to 256: 32 lanes x 2 vectors per lane, vectors beyond
-// the row's end masked.  Both item lists run through sddmm_items (a few segments per warp when
-// segments are long).
-int launch_ragged(int m1, int m2, int k, const int *block_r_ind, const int *residue_r_ind, const int *st_off,
-                  const int *row_offsets, const int *col, const float *values, const float *lhs, const float *rhs,
-                  float *out, cudaStream_t s1, cudaStream_t s2) {
-    const int row_vecs = k / 4;
-    if (m1 > 0) {
-        const int per = items_per_warp(m1, 4);
-        sddmm_items<32, 2, true, true><<<(m1 + per - 1) / per, 32, 0, s1>>>(m1, per, block_r_ind, st_off, row_offsets,
-                                                                             col, values, lhs, rhs, out, row_vecs, 0);
-        RODE_CHECK_LAUNCH("rode::sddmm_items<segments, any k>");
-    }
-    if (m2 > 0) {
-        const int per = items_per_warp(m2, 32);
-        RODE_CUDA_TRY(launch_chained(sddmm_items<32, 2, false, true>, dim3((m2 + per - 1) / per + 1), dim3(32), s2,
-                                     m1 > 0 && s1 == s2, m2, per, residue_r_ind, nullptr, row_offsets, col, values, lhs,
-                                     rhs, out, row_vecs, 0));
-        RODE_CHECK_LAUNCH("rode::sddmm_items<rows, any k>");
     }
     return RODE_OK;
 }
@@ -661,25 +622,20 @@ extern "C" int rode_sddmm_f32(int m1, int m2, int n, int k, const int *block_r_i
     if (m2 > 0 && !residue_r_ind) return fail(RODE_ERR_INVALID_ARGUMENT, "sddmm: null residue metadata");
     if (!aligned_to(lhs, 16) || !aligned_to(rhs, 16))
         return fail(RODE_ERR_INVALID_ARGUMENT, "sddmm: lhs and rhs must be 16-byte aligned");
-    switch (k) {
-        // segments per warp in sddmm_items: few when segments are long (512), 32 when short
-        case 32:
-            return launch_k<RODE_SDDMM_SHAPE_32 / 100, RODE_SDDMM_SHAPE_32 % 100, RODE_SDDMM_ROW_SHAPE_32 / 100,
-                            RODE_SDDMM_ROW_SHAPE_32 % 100>(
-                m1, m2, 4, block_r_ind, residue_r_ind, st_off, row_offsets, column_indices, values, lhs, rhs, out,
-                stream1, stream2);
-        case 64:
-            return launch_k<RODE_SDDMM_SHAPE_64 / 100, RODE_SDDMM_SHAPE_64 % 100, RODE_SDDMM_ROW_SHAPE_64 / 100,
-                            RODE_SDDMM_ROW_SHAPE_64 % 100>(
-                m1, m2, 4, block_r_ind, residue_r_ind, st_off, row_offsets, column_indices, values, lhs, rhs, out,
-                stream1, stream2);
-        case 128:
-            return launch_k<RODE_SDDMM_SHAPE_128 / 100, RODE_SDDMM_SHAPE_128 % 100, RODE_SDDMM_ROW_SHAPE_128 / 100,
-                            RODE_SDDMM_ROW_SHAPE_128 == 0 ? 1 : RODE_SDDMM_ROW_SHAPE_128 % 100>(
-                m1, m2, 32, block_r_ind, residue_r_ind, st_off, row_offsets, column_indices, values, lhs, rhs, out,
-                stream1, stream2);
-        default:
-            return launch_ragged(m1, m2, k, block_r_ind, residue_r_ind, st_off, row_offsets, column_indices, values,
-                                 lhs, rhs, out, stream1, stream2);
-    }
+#define RODE_SDDMM_LAUNCH(L, VPL, RL, RVPL, ragged, long_segments)                                                    \
+    launch_k<L, VPL, RL, RVPL, ragged, long_segments>(m1, m2, k, block_r_ind, residue_r_ind, st_off, row_offsets,    \
+                                       column_indices, values, lhs, rhs, out, stream1, stream2)
+    // The narrowest lane group that covers the dense row; where it does not fit exactly the lanes beyond the
+    // row's end idle (ragged).  (One form of 32 lanes x 2 vectors for all of those widths took 0.209 ms on
+    // the 100003 x 50021 Zipf matrix at K = 96, the 32 x 1 form 0.117 ms.)  The decomposition that goes with
+    // K = 128 has 32-long segments, all others 512-long ones.
+    const int vecs = k / 4;
+    if (vecs == 8) return RODE_SDDMM_LAUNCH(8, 1, 8, 1, false, true);
+    if (vecs == 16) return RODE_SDDMM_LAUNCH(16, 1, 8, 2, false, true);
+    if (vecs == 32) return RODE_SDDMM_LAUNCH(32, 1, 0, 1, false, false);
+    if (vecs < 8) return RODE_SDDMM_LAUNCH(8, 1, 8, 1, true, true);
+    if (vecs < 16) return RODE_SDDMM_LAUNCH(16, 1, 8, 2, true, true);
+    if (vecs < 32) return RODE_SDDMM_LAUNCH(32, 1, 0, 1, true, true);
+    return RODE_SDDMM_LAUNCH(32, 2, 0, 1, true, true);
+#undef RODE_SDDMM_LAUNCH
 }

@@ -233,3 +233,19 @@ def test_sddmm_calls_on_different_stream_pairs_run_side_by_side():
         torch.cuda.synchronize()
         for out in outs:
             assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("k", [4, 28, 36, 60, 68, 96, 124, 132, 252, 256])
+@pytest.mark.parametrize("family", ["power law", "mesh"])    # long segments and streams; the row mode
+def test_sddmm_widths_that_leave_lanes_idle(oracle_cpu, family, k):
+    A = W.pareto_rows(m=40001, n=3001, mean=20, cap=1400, seed=k) if family == "power law" else W.stencil27(33, seed=k)
+    d = A.to("cuda")
+    meta = capi.preprocess(d.row_ptr, d.nnz, 512, 32, 4)
+    lhs, rhs = W.dense(A.m, k, seed=k), W.dense(A.n, k, seed=k + 1)
+    out = torch.full((A.nnz + 2,), float("nan"), device="cuda")
+    capi.sddmm(meta, d.row_ptr, d.col, d.val, lhs.cuda(), rhs.cuda(), out=out[1:-1])
+    rp, col, val = A.row_ptr.numpy(), A.col.numpy(), A.val.numpy()
+    truth = oracle_cpu.sddmm_f64acc(rp, col, val, lhs.numpy(), rhs.numpy(), threads=oracle_cpu.max_threads())
+    assert_close_to_truth(out[1:-1].cpu().numpy(), truth, sddmm_abs_scale(rp, col, val, lhs.numpy(), rhs.numpy()),
+                          f"{family} k={k}")
+    assert bool(torch.isnan(out[0])) and bool(torch.isnan(out[-1]))
