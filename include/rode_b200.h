@@ -104,8 +104,7 @@ int rode_preprocess(int seg_len, int k_block, int vec_len, int M, const int *row
  *             the life of the process: after a cudaDeviceReset in the same process it is
  *             stale, so do not call this entry point again after resetting a device.
  *   Sharing   all calls on a device use the same array and it keeps the previous call's
- *             contents.  The caller clears nothing (the call itself zeroes its 8-byte
- *             counter with a memset node on the stream, and every other entry that is read is
+ *             contents.  The caller clears nothing (every entry that is read is
  *             written first by the same call), but two calls that overlap in time on one GPU,
  *             e.g. on two streams, race on it: serialise them. */
 int rode_preprocess_noalloc(int seg_len, int k_block, int vec_len, int M, const int *row_ptr,

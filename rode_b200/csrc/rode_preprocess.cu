@@ -9,44 +9,23 @@
 // The reference's device version (count kernel _preprocess.cu:244-274, two CUB scans
 // :330-334, fill kernel :275-322) keeps its prefix sums in the output arrays and overwrites
 // them in place across thread blocks.  Here the prefix sums live in a separate scratch
-// array, so the two kernels below are race-free:
-//
-//   count_tiles   one CTA per tile of kTile rows: per-row (bn, rn), tile totals -> scratch.  The
-//                 CTA that finishes last (a counter in the scratch tells it) turns the totals
-//                 into exclusive tile offsets and writes n_blk, n_res and the end sentinel.
-//   fill_tiles    one CTA per tile: in-tile exclusive scan + tile offset; the tile's residue rows
-//                 and segments are put in order in shared memory and copied out with coalesced
-//                 stores; rows with many segments are written by a whole warp.  Launched as a
-//                 programmatic dependent of count_tiles: its CTAs read their rows and scan them
-//                 while the count grid drains, and wait for it only before they need the tile offset.
-//
-// HBM traffic: row_ptr is read twice (8 B/row), outputs written once (8 B/segment,
-// 4 B/residue row), scratch is 8 B per 2048 rows.
+// array, the totals of each tile of rows: count_tiles writes them, fill_tiles adds up those before its
+// tile and writes the outputs; a matrix of a few tiles needs fill_tiles only.
 #include <climits>
 #include <mutex>
+
+#include <cooperative_groups.h>
 
 #include "rode_common.cuh"
 
 namespace rode {
 namespace {
 
-// CTAs per SM the register budget must allow: the count kernel fits 32 registers (8 CTAs) without
-// spilling, the fill kernel 48 (5 CTAs).
-#ifndef RODE_PRE_COUNT_MIN_CTAS
-#define RODE_PRE_COUNT_MIN_CTAS 8
-#endif
-#ifndef RODE_PRE_FILL_MIN_CTAS
-#define RODE_PRE_FILL_MIN_CTAS 5
-#endif
 constexpr int kThreads = 256;
-#ifndef RODE_PRE_ROWS_PER_THREAD
-#define RODE_PRE_ROWS_PER_THREAD 8
-#endif
-constexpr int kRowsPerThread = RODE_PRE_ROWS_PER_THREAD;
-constexpr int kTile = kThreads * kRowsPerThread;  // rows per CTA
+constexpr int kTile = 2048;    // rows per CTA
 constexpr int kWarps = kThreads / 32;
-constexpr int kLongRow = 8;  // rows with more segments than this are written by a warp
-// Scratch layout: slot 0 = {count of finished count_tiles CTAs, unused}, slot 1 + t = tile t.
+constexpr int kShortRow = 8;   // rows of up to so many segments are written by one thread, others by a warp
+// Scratch: running sums of the tiles, one int2 each (callers provide for one more).
 constexpr int kScratchHeader = 1;
 
 // The three parameters of the decomposition.  kPow2 = all of them are powers of two (every
@@ -75,7 +54,8 @@ __device__ __forceinline__ void row_counts(int off, int next, const Params &p, i
         // one form for both cases of the spec loop: with a <= seg_len the quotient is 0 and the
         // remainder is a itself, except a == seg_len, where quotient 1 + remainder 0 gives the same
         // single segment; and (a % seg_len) % k_block == a % k_block because k_block divides seg_len
-        bn = (a >> p.seg_shift) + ((a & (p.seg_len - 1)) >= p.k_block ? 1 : 0);
+        // (a / seg_len, plus one where the remainder reaches k_block = one division of a sum)
+        bn = static_cast<int>((static_cast<unsigned>(a) + (p.seg_len - p.k_block)) >> p.seg_shift);
         rn = (a & (p.k_block - 1)) != 0 ? 1 : 0;
     } else if (a > p.seg_len) {
         const int rest = a % p.seg_len;
@@ -87,153 +67,6 @@ __device__ __forceinline__ void row_counts(int off, int next, const Params &p, i
     }
 }
 
-// Inclusive scan of (x, y) over a CTA of kW warps; returns the exclusive prefix of this
-// thread and the CTA totals.  smem: 2 * kW ints.
-template <int kW = kWarps>
-__device__ __forceinline__ void block_exclusive_scan2(int x, int y, int *smem, int &ex, int &ey, int &tx,
-                                                      int &ty) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int ix = x, iy = y;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int ux = __shfl_up_sync(0xffffffffu, ix, d);
-        const int uy = __shfl_up_sync(0xffffffffu, iy, d);
-        if (lane >= d) {
-            ix += ux;
-            iy += uy;
-        }
-    }
-    if (lane == 31) {
-        smem[warp] = ix;
-        smem[kW + warp] = iy;
-    }
-    __syncthreads();
-    int wx = 0, wy = 0;
-    tx = 0;
-    ty = 0;
-#pragma unroll
-    for (int w = 0; w < kW; ++w) {
-        const int sx = smem[w], sy = smem[kW + w];
-        if (w < warp) {
-            wx += sx;
-            wy += sy;
-        }
-        tx += sx;
-        ty += sy;
-    }
-    ex = wx + ix - x;
-    ey = wy + iy - y;
-    __syncthreads();
-}
-
-// Rows of one thread: offsets and per-row (bn, rn).  Rows at or beyond M (last tile only) count as
-// empty rows that start at the matrix' end.
-template <bool kPow2>
-__device__ __forceinline__ void load_rows(const Params &p, int M, const int *__restrict__ row_ptr, int row0,
-                                          int (&offs)[kRowsPerThread + 1], int (&bn)[kRowsPerThread],
-                                          int (&rn)[kRowsPerThread], int &bsum, int &rsum) {
-    bsum = 0;
-    rsum = 0;
-    const bool whole_tile = (static_cast<int>(blockIdx.x) + 1) * kTile <= M;  // CTA-uniform
-    if (whole_tile) {
-#pragma unroll
-        for (int i = 0; i <= kRowsPerThread; ++i) offs[i] = __ldg(row_ptr + row0 + i);  // all independent
-#pragma unroll
-        for (int i = 0; i < kRowsPerThread; ++i) {
-            row_counts<kPow2>(offs[i], offs[i + 1], p, bn[i], rn[i]);
-            bsum += bn[i];
-            rsum += rn[i];
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i <= kRowsPerThread; ++i) offs[i] = __ldg(row_ptr + min(row0 + i, M));
-#pragma unroll
-        for (int i = 0; i < kRowsPerThread; ++i) {
-            bn[i] = 0;
-            rn[i] = 0;
-            if (row0 + i < M) row_counts<kPow2>(offs[i], offs[i + 1], p, bn[i], rn[i]);
-            bsum += bn[i];
-            rsum += rn[i];
-        }
-    }
-}
-
-// Tile totals, then (in the CTA that finishes last) the scan over them.  `scratch` as laid out above;
-// the counter is zero when the grid starts and is left at zero.
-constexpr int kScanPerThread = 8;  // tiles per thread and pass of the last CTA's scan
-template <bool kPow2>
-__global__ void __launch_bounds__(kThreads, RODE_PRE_COUNT_MIN_CTAS)
-count_tiles(Params p, int M, const int *__restrict__ row_ptr, int2 *__restrict__ scratch, int *__restrict__ st_off,
-            int *__restrict__ n_blk, int *__restrict__ n_res, bool write_sentinel) {
-    __shared__ int smem[2 * kWarps];
-    __shared__ bool is_last;
-    int2 *tile_totals = scratch + kScratchHeader;
-    int *finished = reinterpret_cast<int *>(scratch);
-    {
-        const int row0 = blockIdx.x * kTile + threadIdx.x * kRowsPerThread;
-        int offs[kRowsPerThread + 1], bn[kRowsPerThread], rn[kRowsPerThread], bsum, rsum;
-        load_rows<kPow2>(p, M, row_ptr, row0, offs, bn, rn, bsum, rsum);
-        // only the totals are needed here: one warp reduction each, then the warps' sums
-        const int wb = __reduce_add_sync(0xffffffffu, bsum), wr = __reduce_add_sync(0xffffffffu, rsum);
-        if ((threadIdx.x & 31) == 0) {
-            smem[threadIdx.x >> 5] = wb;
-            smem[kWarps + (threadIdx.x >> 5)] = wr;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int tx = 0, ty = 0;
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) {
-                tx += smem[w];
-                ty += smem[kWarps + w];
-            }
-            tile_totals[blockIdx.x] = make_int2(tx, ty);
-            __threadfence();  // the total is visible before the count of finished CTAs moves
-            is_last = atomicAdd(finished, 1) == static_cast<int>(gridDim.x) - 1;
-        }
-    }
-    __syncthreads();
-    // The fill grid may be scheduled once every CTA of this grid has come this far: its CTAs then read
-    // and scan their rows while the last CTA scans the tile totals.  (Released at the START of the CTAs
-    // instead, the fill grid measured 30 us slower on R-MAT scale 23 with 32-long segments, 98 against
-    // 68 us, and 4 us slower on R-MAT scale 21; without the early launch at all every matrix lost 5 us.)
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (!is_last) return;
-    // Every other CTA has published its total.  Exclusive scan over the tiles, in place.
-    __threadfence();
-    const int n_tiles = static_cast<int>(gridDim.x);
-    int carry_b = 0, carry_r = 0;
-    for (int base = 0; base < n_tiles; base += kThreads * kScanPerThread) {
-        const int t0 = base + threadIdx.x * kScanPerThread;
-        int2 v[kScanPerThread];
-        int sum_b = 0, sum_r = 0;
-#pragma unroll
-        for (int i = 0; i < kScanPerThread; ++i) {
-            v[i] = make_int2(0, 0);
-            if (t0 + i < n_tiles) v[i] = __ldcg(tile_totals + t0 + i);  // written by other SMs: not through L1
-            sum_b += v[i].x;
-            sum_r += v[i].y;
-        }
-        int ex, ey, tx, ty;
-        block_exclusive_scan2(sum_b, sum_r, smem, ex, ey, tx, ty);
-        int run_b = carry_b + ex, run_r = carry_r + ey;
-#pragma unroll
-        for (int i = 0; i < kScanPerThread; ++i) {
-            if (t0 + i < n_tiles) tile_totals[t0 + i] = make_int2(run_b, run_r);
-            run_b += v[i].x;
-            run_r += v[i].y;
-        }
-        carry_b += tx;
-        carry_r += ty;
-    }
-    if (threadIdx.x == 0) {
-        n_blk[0] = carry_b;
-        n_res[0] = carry_r;
-        if (write_sentinel) st_off[carry_b] = __ldg(row_ptr + M);
-        *finished = 0;  // ready for the next call on this scratch
-    }
-}
-
 // M == 0: no tile, only the counts and the sentinel.
 __global__ void empty_matrix(const int *__restrict__ row_ptr, int *__restrict__ st_off, int *__restrict__ n_blk,
                              int *__restrict__ n_res, bool write_sentinel) {
@@ -242,15 +75,128 @@ __global__ void empty_matrix(const int *__restrict__ row_ptr, int *__restrict__ 
     if (write_sentinel) st_off[0] = row_ptr[0];
 }
 
-// Segments of one long row, written by the whole warp.  `row`, `off`, `cnt` are warp-uniform.
+// Segments of one row: j = first, first + step, ...
 template <bool kPow2>
-__device__ __forceinline__ void write_long_row(const Params &p, int lane, int row, int off, int cnt,
-                                               int *__restrict__ dst_row, int *__restrict__ dst_off) {
+__device__ __forceinline__ void write_row(const Params &p, int first, int step, int row, int off, int cnt,
+                                          int *__restrict__ dst_row, int *__restrict__ dst_off) {
     const int aligned = off - mod_vec<kPow2>(off, p);
-    for (int j = lane; j < cnt; j += 32) {
+    for (int j = first; j < cnt; j += step) {
         dst_row[j] = row;
         dst_off[j] = j == 0 ? off : aligned + j * p.seg_len;
     }
+}
+
+// The rows of one warp: kVecs x 128 of them, unit i of a lane being rows row0 + 128 i .. + 3, in registers
+// from 16-byte loads that are all in flight together.
+constexpr int kUnit = 128;
+constexpr int kVecs = kTile / kThreads / 4;
+constexpr int kWarpRows = kUnit * kVecs;
+template <bool kPow2>
+struct WarpRows {
+    int o[kVecs][4];
+    int after;  // offset of the row behind the last one
+    int row0;
+    bool wide;  // warp-uniform: all rows exist and the row pointer is 16-byte aligned
+
+    __device__ __forceinline__ void load(int M, const int *__restrict__ row_ptr, int warp_row0, int lane) {
+        row0 = warp_row0 + lane * 4;
+        wide = reinterpret_cast<size_t>(row_ptr) % 16 == 0 && warp_row0 + kWarpRows <= M;
+        if (wide) {
+#pragma unroll
+            for (int i = 0; i < kVecs; ++i) {
+                const int4 v = __ldg(reinterpret_cast<const int4 *>(row_ptr + row0 + kUnit * i));
+                o[i][0] = v.x;
+                o[i][1] = v.y;
+                o[i][2] = v.z;
+                o[i][3] = v.w;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < kVecs; ++i)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) o[i][k] = __ldg(row_ptr + min(row0 + kUnit * i + k, M));
+        }
+        after = __ldg(row_ptr + min(warp_row0 + kWarpRows, M));
+    }
+    int packed[kVecs][4];  // 2 * segments + residue flag of each row, set by sums()
+    // The four rows of unit i; rows at or beyond M count as nothing.
+    __device__ __forceinline__ void count(const Params &p, int M, int lane, int i) {
+        const int behind = i + 1 < kVecs ? o[i + 1 < kVecs ? i + 1 : i][0] : after;
+        const int next = __shfl_sync(0xffffffffu, lane == 0 ? behind : o[i][0], (lane + 1) & 31);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            int bn, rn;
+            row_counts<kPow2>(o[i][k], k < 3 ? o[i][k < 3 ? k + 1 : k] : next, p, bn, rn);
+            packed[i][k] = !wide && row0 + kUnit * i + k >= M ? 0 : 2 * bn + rn;
+        }
+    }
+    __device__ __forceinline__ void sums(const Params &p, int M, int lane, int &b, int &r) {  // of the warp
+        b = r = 0;
+#pragma unroll
+        for (int i = 0; i < kVecs; ++i) {
+            count(p, M, lane, i);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                b += packed[i][k] >> 1;
+                r += packed[i][k] & 1;
+            }
+        }
+        b = __reduce_add_sync(0xffffffffu, b);
+        r = __reduce_add_sync(0xffffffffu, r);
+    }
+};
+
+// Counts of `group` tiles (1, or a multiple of kGroup) per CTA: sums[t] = segments and residue rows from the first row
+// of the group to the end of tile t, so the last tile of a group holds the group's total.
+constexpr int kGroup = 8;
+template <bool kPow2>
+__global__ void __launch_bounds__(kThreads, 4)
+count_tiles(Params p, int M, int n_tiles, int group, const int *__restrict__ row_ptr, int2 *__restrict__ sums) {
+    __shared__ int2 s_warp[kGroup][kWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int carry_b = 0, carry_r = 0;
+    for (int t0 = 0; t0 < group; t0 += kGroup) {
+        const int tile0 = static_cast<int>(blockIdx.x) * group + t0;
+        if (tile0 >= n_tiles) break;
+#pragma unroll 4
+        for (int t = 0; t < kGroup; ++t) {
+            int b = 0, r = 0;
+            if (tile0 + t < n_tiles && t < group) {
+                WarpRows<kPow2> rows;
+                rows.load(M, row_ptr, (tile0 + t) * kTile + warp * kWarpRows, lane);
+                rows.sums(p, M, lane, b, r);
+            }
+            if (lane == 0) s_warp[t][warp] = make_int2(b, r);
+        }
+        __syncthreads();
+        if (warp == 0) {
+            int b = 0, r = 0;
+            if (lane < kGroup) {
+#pragma unroll
+                for (int w = 0; w < kWarps; ++w) {
+                    b += s_warp[lane][w].x;
+                    r += s_warp[lane][w].y;
+                }
+            }
+#pragma unroll
+            for (int d = 1; d < kGroup; d <<= 1) {
+                const int ub = __shfl_up_sync(0xffffffffu, b, d), ur = __shfl_up_sync(0xffffffffu, r, d);
+                if (lane >= d) {
+                    b += ub;
+                    r += ur;
+                }
+            }
+            b += carry_b;
+            r += carry_r;
+            if (lane < min(group, kGroup) && tile0 + lane < n_tiles) sums[tile0 + lane] = make_int2(b, r);
+            carry_b = __shfl_sync(0xffffffffu, b, kGroup - 1);
+            carry_r = __shfl_sync(0xffffffffu, r, kGroup - 1);
+        }
+        __syncthreads();
+    }
+    // the fill grid may start once every CTA of this grid has come this far (released at the start of the CTAs
+    // instead, its CTAs take slots from this grid)
+    chain_begin();
 }
 
 // The listed long rows, taken by the CTA's warps in turn.  The next row's list entry and bounds are
@@ -274,7 +220,7 @@ __device__ __forceinline__ void write_long_rows(const Params &p, int lane, int w
         }
         int cnt, unused;
         row_counts<kPow2>(off, next, p, cnt, unused);
-        write_long_row<kPow2>(p, lane, row, off, cnt, out_row + dst, out_off + dst);
+        write_row<kPow2>(p, lane, 32, row, off, cnt, out_row + dst, out_off + dst);
         if (s2 >= total) return;
         s = s2;
         row = row2;
@@ -284,92 +230,161 @@ __device__ __forceinline__ void write_long_rows(const Params &p, int lane, int w
     }
 }
 
+// The outputs of every tile.  Its place comes from the group totals before it, added up by the tile's own CTA, and
+// the places inside it from one warp scan per 128 rows over the thread's (segments, residue rows), packed into
+// one word.  A row's first segment is written by its thread, and so are a few further ones; rows of more than
+// kShortRow segments are listed and written by the CTA's warps in turn (on graphs they cluster in the first tile).
+//
+// What bounds the decomposition: the latency of its phases, the instructions per row (19 + 60 warp instructions
+// per 32 rows in the two kernels) and the tile with the longest rows; of the bytes 33 MB are read (the second time
+// from the L2) and 38 MB written at 8.4 M rows (11 us at the copy bandwidth).  us per call, segments of 512 / 32,
+// with a memset, a count kernel that scans in its last CTA and a fill kernel that orders through shared
+// memory -> now: R-MAT scale 23 41.2 / 67.6 -> 34.9 / 59.7, R-MAT 21 16.9 / 39.7 -> 14.2 / 34.8, Pareto 2^22 rows
+// 26.7 / 34.9 -> 22.6 / 32.7, 131,072 rows 10.1 / 10.6 -> 7.4 / 8.2, 1000 rows 8.3 / 9.6 -> 5.0 / 6.2.  Measured and dropped:
+// one kernel with a look-back over the tiles' states (the CTAs that poll the same few lines hold up those that
+// publish: 54 to 78 us), one row per lane with ballots (98 instructions per 32 rows), one segment per lane by a
+// search in the warp's prefix (a chain of shuffles, 5 us per CTA), larger tiles (4096 rows 50, 8192 96 us).
+//
+// in_cluster: no count grid; this grid is one cluster of at most kClusterTiles CTAs and the totals travel
+// through distributed shared memory.
+constexpr int kClusterTiles = 8;
 template <bool kPow2>
-__global__ void __launch_bounds__(kThreads, RODE_PRE_FILL_MIN_CTAS)
-fill_tiles(Params p, int M, const int *__restrict__ row_ptr, const int2 *__restrict__ scratch,
-           int *__restrict__ block_r_ind, int *__restrict__ st_off, int *__restrict__ residue_r_ind) {
-    __shared__ int smem[2 * kWarps];
-    // The tile's outputs in order: residue rows always, segments when the tile has at most kTile.
-    __shared__ int s_res[kTile];
-    __shared__ int s_seg_row[kTile];
-    __shared__ int s_seg_off[kTile];
-    // Rows with more than kLongRow segments are listed and then written by the CTA's warps in turn
-    // (on skewed matrices they cluster in the first lanes of a tile).  A staged tile has at most
-    // kTile / (kLongRow + 1) of them; a tile that is not staged keeps the list in the staging arrays.
-    constexpr int kLongCap = kTile / (kLongRow + 1) + 1;
-    __shared__ int s_long_row[kLongCap];
-    __shared__ int s_long_dst[kLongCap];
+__global__ void __launch_bounds__(kThreads, 4)
+fill_tiles(Params p, int M, int group, const int *__restrict__ row_ptr, const int2 *__restrict__ sums,
+           int *__restrict__ block_r_ind, int *__restrict__ st_off, int *__restrict__ residue_r_ind,
+           int *__restrict__ n_blk, int *__restrict__ n_res, bool write_sentinel, bool in_cluster) {
+    constexpr unsigned kFull = 0xffffffffu;
+    __shared__ int2 s_warp[kWarps], s_before[kWarps];
+    __shared__ int2 s_total;
+    __shared__ int s_long_row[kTile], s_long_dst[kTile];
     __shared__ int n_long;
-    if (threadIdx.x == 0) n_long = 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-
-    const int row0 = blockIdx.x * kTile + threadIdx.x * kRowsPerThread;
-    int offs[kRowsPerThread + 1], bn[kRowsPerThread], rn[kRowsPerThread], bsum, rsum;
-    load_rows<kPow2>(p, M, row_ptr, row0, offs, bn, rn, bsum, rsum);
-    int ex, ey, tx, ty;
-    block_exclusive_scan2(bsum, rsum, smem, ex, ey, tx, ty);  // also orders n_long = 0
-    const bool staged = tx <= kTile;  // CTA-uniform
-    int *list_row = staged ? s_long_row : s_seg_row;
-    int *list_dst = staged ? s_long_dst : s_seg_off;
-
-    // ---- residue rows, the list of long rows, and a staged tile's short rows ----------------------
-    int lr = ey, lb = ex;
-#pragma unroll
-    for (int i = 0; i < kRowsPerThread; ++i) {
-        if (rn[i]) s_res[lr] = row0 + i;
-        lr += rn[i];
-        if (bn[i] > kLongRow) {
-            const int slot = atomicAdd(&n_long, 1);  // shared-memory slot counter, order irrelevant
-            list_row[slot] = row0 + i;
-            list_dst[slot] = lb;
-        } else if (staged && bn[i] > 0) {
-            const int off = offs[i];
-            const int aligned = off - mod_vec<kPow2>(off, p);
-            s_seg_row[lb] = row0 + i;
-            s_seg_off[lb] = off;
-            for (int j = 1; j < bn[i]; ++j) {
-                s_seg_row[lb + j] = row0 + i;
-                s_seg_off[lb + j] = aligned + j * p.seg_len;
-            }
+    const int tile = static_cast<int>(blockIdx.x);
+    if (threadIdx.x == 0) n_long = 0;
+    const int warp_row0 = tile * kTile + warp * kWarpRows;
+    WarpRows<kPow2> rows;
+    rows.load(M, row_ptr, warp_row0, lane);
+    const int row0 = rows.row0;
+    const auto &o = rows.o;
+    if (!in_cluster) {
+        chain_wait();  // the count grid's sums
+        int b = 0, r = 0;
+        const int groups = tile / group;
+#pragma unroll 4
+        for (int g = threadIdx.x; g < groups; g += kThreads) {
+            const int2 v = __ldcg(sums + (static_cast<size_t>(g) + 1) * group - 1);
+            b += v.x;
+            r += v.y;
         }
-        lb += bn[i];
+        if (threadIdx.x == 0 && tile % group != 0) {
+            const int2 v = __ldcg(sums + tile - 1);
+            b += v.x;
+            r += v.y;
+        }
+        b = __reduce_add_sync(kFull, b);
+        r = __reduce_add_sync(kFull, r);
+        if (lane == 0) s_before[warp] = make_int2(b, r);
+    }
+    int bsum, rsum;
+    rows.sums(p, M, lane, bsum, rsum);
+    if (lane == 0) s_warp[warp] = make_int2(bsum, rsum);
+    __syncthreads();
+    // lane w < kWarps: warp w's sums; then the sums of the warps before this one
+    int2 mine = make_int2(0, 0);
+    if (lane < kWarps) mine = s_warp[lane];
+    int base_b = __reduce_add_sync(kFull, lane < warp ? mine.x : 0), base_r = __reduce_add_sync(kFull, lane < warp ? mine.y : 0);
+    const bool last = tile == static_cast<int>(gridDim.x) - 1;
+    int place_b = 0, place_r = 0;
+    if (in_cluster) {
+        const auto cluster = cooperative_groups::this_cluster();
+        const int total_b = __reduce_add_sync(kFull, mine.x), total_r = __reduce_add_sync(kFull, mine.y);
+        if (threadIdx.x == 0) s_total = make_int2(total_b, total_r);
+        cluster.sync();
+        for (int t = 0; t < tile; ++t) {
+            const int2 v = *cluster.map_shared_rank(&s_total, t);
+            place_b += v.x;
+            place_r += v.y;
+        }
+        cluster.sync();  // nobody leaves while its totals are being read
+    } else {
+        int2 before = make_int2(0, 0);
+        if (lane < kWarps) before = s_before[lane];
+        place_b = __reduce_add_sync(kFull, before.x);
+        place_r = __reduce_add_sync(kFull, before.y);
+    }
+    if (last && warp == 0) {  // the last rows of the matrix
+        const int n_b = place_b + __reduce_add_sync(kFull, mine.x), n_r = place_r + __reduce_add_sync(kFull, mine.y);
+        if (lane == 0) {
+            n_blk[0] = n_b;
+            n_res[0] = n_r;
+            if (write_sentinel) st_off[n_b] = __ldg(row_ptr + M);
+        }
+    }
+    base_b += place_b;
+    base_r += place_r;
+
+    // ---- outputs --------------------------------------------------------------------------------------
+    auto inclusive = [&](int x) {  // prefix sum over the lanes
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int up = __shfl_up_sync(kFull, x, d);
+            if (lane >= d) x += up;
+        }
+        return x;
+    };
+    constexpr int kResBits = 8;  // at most 128 residue rows per unit
+    const bool packs = bsum < (1 << (31 - kResBits));
+#pragma unroll
+    for (int i = 0; i < kVecs; ++i) {
+        int bn[4], rn[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            bn[k] = rows.packed[i][k] >> 1;
+            rn[k] = rows.packed[i][k] & 1;
+        }
+        const int b4 = bn[0] + bn[1] + bn[2] + bn[3], r4 = rn[0] + rn[1] + rn[2] + rn[3];
+        int b_incl, r_incl;
+        if (packs) {
+            const int x = inclusive((b4 << kResBits) | r4);
+            b_incl = x >> kResBits;
+            r_incl = x & ((1 << kResBits) - 1);
+        } else {
+            b_incl = inclusive(b4);
+            r_incl = inclusive(r4);
+        }
+        const int row = row0 + kUnit * i;
+        int at_r = base_r + r_incl - r4;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (rn[k]) residue_r_ind[at_r] = row + k;
+            at_r += rn[k];
+        }
+        base_r += __shfl_sync(kFull, r_incl, 31);
+        const int unit_b = __shfl_sync(kFull, b_incl, 31);
+        if (unit_b == 0) continue;
+        int at = base_b + b_incl - b4;
+        base_b += unit_b;
+        const bool several = __any_sync(kFull, (bn[0] > 1) | (bn[1] > 1) | (bn[2] > 1) | (bn[3] > 1));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (bn[k]) {
+                block_r_ind[at] = row + k;
+                st_off[at] = o[i][k];
+            }
+            if (several) {  // warp-uniform
+                if (bn[k] > 1 && bn[k] <= kShortRow)
+                    write_row<kPow2>(p, 1, 1, row + k, o[i][k], bn[k], block_r_ind + at, st_off + at);
+                if (bn[k] > kShortRow) {
+                    const int slot = atomicAdd(&n_long, 1);
+                    s_long_row[slot] = row + k;
+                    s_long_dst[slot] = at;
+                }
+            }
+            at += bn[k];
+        }
     }
     __syncthreads();
-    const int total_long = n_long;
-    if (staged) {
-        write_long_rows<kPow2>(p, lane, warp, total_long, list_row, list_dst, row_ptr, s_seg_row, s_seg_off);
-        __syncthreads();
-    }
-
-    // ---- the tile's place in the outputs: written by the count grid's last CTA --------------------
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int2 tile_off = __ldcg(scratch + kScratchHeader + blockIdx.x);
-    for (int i = threadIdx.x; i < ty; i += kThreads) residue_r_ind[tile_off.y + i] = s_res[i];
-    if (staged) {
-        for (int i = threadIdx.x; i < tx; i += kThreads) {
-            block_r_ind[tile_off.x + i] = s_seg_row[i];
-            st_off[tile_off.x + i] = s_seg_off[i];
-        }
-        return;
-    }
-    // A tile with more segments than the staging holds (very long rows): straight to the outputs.
-    int gb = tile_off.x + ex;
-#pragma unroll
-    for (int i = 0; i < kRowsPerThread; ++i) {
-        if (bn[i] > 0 && bn[i] <= kLongRow) {
-            const int off = offs[i];
-            const int aligned = off - mod_vec<kPow2>(off, p);
-            block_r_ind[gb] = row0 + i;
-            st_off[gb] = off;
-            for (int j = 1; j < bn[i]; ++j) {
-                block_r_ind[gb + j] = row0 + i;
-                st_off[gb + j] = aligned + j * p.seg_len;
-            }
-        }
-        gb += bn[i];
-    }
-    write_long_rows<kPow2>(p, lane, warp, total_long, list_row, list_dst, row_ptr, block_r_ind + tile_off.x,
-                           st_off + tile_off.x);
+    write_long_rows<kPow2>(p, lane, warp, n_long, s_long_row, s_long_dst, row_ptr, block_r_ind, st_off);
 }
 
 int check_params(int seg_len, int k_block, int vec_len, int M, const void *row_ptr) {
@@ -387,30 +402,43 @@ int check_params(int seg_len, int k_block, int vec_len, int M, const void *row_p
 
 }  // namespace
 
-// Launches the two kernels; `scratch` holds kScratchHeader + one int2 per tile.  write_sentinel: also
-// store st_off[n_blk] = row_ptr[M] (the C ABI's contract; the reference's device version does
-// not, and its callers size st_off without room for it).
+int preprocess_tiles(int M) { return (M + kTile - 1) / kTile; }
+constexpr int kMaxGroups = 2048;
+
+// `sums` holds one entry per tile.  write_sentinel: also store st_off[n_blk] = row_ptr[M] (the C ABI's
+// contract; the reference's device version does not, and its callers size st_off without room for it).
 template <bool kPow2>
-int launch_preprocess_kernels(const Params &p, int n_tiles, int M, const int *row_ptr, int *block_r_ind, int *st_off,
-                              int *residue_r_ind, int *n_blk, int *n_res, int2 *scratch, cudaStream_t stream,
+int launch_preprocess_kernels(const Params &p, int M, const int *row_ptr, int *block_r_ind, int *st_off,
+                              int *residue_r_ind, int *n_blk, int *n_res, int2 *sums, cudaStream_t stream,
                               bool write_sentinel) {
-    // the count of finished CTAs: the scratch may be a caller's buffer with any contents
-    RODE_CUDA_TRY(cudaMemsetAsync(scratch, 0, sizeof(int2), stream));
-    count_tiles<kPow2><<<n_tiles, kThreads, 0, stream>>>(p, M, row_ptr, scratch, st_off, n_blk, n_res, write_sentinel);
-    RODE_CHECK_LAUNCH("rode::count_tiles");
+    // What one portable cluster holds takes one launch; otherwise count, then fill as a programmatic dependent.
+    const int n_tiles = preprocess_tiles(M);
+    const bool in_cluster = n_tiles <= kClusterTiles;
+    // tiles per count CTA: one while a fill CTA can add up all of them quickly (131,072 rows 10.2 us with eight),
+    // then so many that it adds up at most kMaxGroups sums
+    int group = n_tiles <= 1024 ? 1 : kGroup;
+    while (n_tiles / group > kMaxGroups) group *= 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n_tiles);
     cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = 0;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const int2 *scratch_in = scratch;
-    RODE_CUDA_TRY(cudaLaunchKernelEx(&cfg, fill_tiles<kPow2>, p, M, row_ptr, scratch_in, block_r_ind, st_off,
-                                     residue_r_ind));
+    if (in_cluster) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = n_tiles;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+    } else {
+        count_tiles<kPow2><<<(n_tiles + group - 1) / group, kThreads, 0, stream>>>(p, M, n_tiles, group, row_ptr, sums);
+        RODE_CHECK_LAUNCH("rode::count_tiles");
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+    }
+    const int2 *sums_in = sums;
+    RODE_CUDA_TRY(cudaLaunchKernelEx(&cfg, fill_tiles<kPow2>, p, M, group, row_ptr, sums_in, block_r_ind, st_off,
+                                     residue_r_ind, n_blk, n_res, write_sentinel, in_cluster));
     RODE_CHECK_LAUNCH("rode::fill_tiles");
     return RODE_OK;
 }
@@ -418,24 +446,21 @@ int launch_preprocess_kernels(const Params &p, int n_tiles, int M, const int *ro
 int launch_preprocess(int seg_len, int k_block, int vec_len, int M, const int *row_ptr, int *block_r_ind,
                       int *st_off, int *residue_r_ind, int *n_blk, int *n_res, int2 *tile_scratch,
                       cudaStream_t stream, bool write_sentinel = true) {
-    const int n_tiles = (M + kTile - 1) / kTile;
     auto pow2 = [](int x) { return (x & (x - 1)) == 0; };
     const bool all_pow2 = pow2(seg_len) && pow2(k_block) && pow2(vec_len);
     Params p = {seg_len, k_block, vec_len, 0};
     while (all_pow2 && (1 << p.seg_shift) < seg_len) ++p.seg_shift;
-    if (n_tiles == 0) {
+    if (M == 0) {
         empty_matrix<<<1, 1, 0, stream>>>(row_ptr, st_off, n_blk, n_res, write_sentinel);
         RODE_CHECK_LAUNCH("rode::empty_matrix");
         return RODE_OK;
     }
     if (all_pow2)
-        return launch_preprocess_kernels<true>(p, n_tiles, M, row_ptr, block_r_ind, st_off, residue_r_ind, n_blk, n_res,
+        return launch_preprocess_kernels<true>(p, M, row_ptr, block_r_ind, st_off, residue_r_ind, n_blk, n_res,
                                                tile_scratch, stream, write_sentinel);
-    return launch_preprocess_kernels<false>(p, n_tiles, M, row_ptr, block_r_ind, st_off, residue_r_ind, n_blk, n_res,
+    return launch_preprocess_kernels<false>(p, M, row_ptr, block_r_ind, st_off, residue_r_ind, n_blk, n_res,
                                             tile_scratch, stream, write_sentinel);
 }
-
-int preprocess_tiles(int M) { return (M + kTile - 1) / kTile; }
 
 // Body of the reference-signature entry point RoDe_preprocess (Preprocess_opt/_preprocess.cu:323-339):
 // default stream, and nothing is written beyond the n_blk segments and n_res residue rows -- the
@@ -524,7 +549,6 @@ int rode_preprocess_noalloc(int seg_len, int k_block, int vec_len, int M, const 
                           M, rode::kNoAllocMaxRows);
     int2 *scratch = nullptr;
     if (int rc = rode::noalloc_scratch(&scratch)) return rc;
-    // count_tiles rewrites every tile total it later reads; the counter is cleared on the stream.
     return rode::launch_preprocess(seg_len, k_block, vec_len, M, row_ptr, block_r_ind, st_off, residue_r_ind,
                                    n_blk, n_res, scratch, stream);
 }

@@ -124,3 +124,16 @@ def test_reference_signature_entry_point(oracle_cpu):
         assert np.array_equal(res[:m2].cpu().numpy(), want[2])
         # nothing is written past the counts
         assert bool((blk[m1:] == -1).all()) and bool((st[m1:] == -1).all()) and bool((res[m2:] == -1).all())
+
+
+@pytest.mark.parametrize("seg,kb,vec", [(512, 32, 4), (32, 32, 4), (96, 48, 12)])
+@pytest.mark.parametrize("M", [1, 2047, 2049, 8 * 2048, 8 * 2048 + 1, 1025 * 2048 + 7])
+def test_gpu_preprocess_single_pass(oracle_cpu, M, seg, kb, vec):
+    """One tile, one cluster of tiles, the first grid with a look-back, one whose look-back takes a second
+    step; a tile with more long rows (over eight segments) than the CTA's list holds."""
+    rng = np.random.default_rng(M)
+    lens = rng.integers(0, 70, M)
+    lens[M // 2: M // 2 + 300] = 9 * seg + 5
+    lens[-1] = 40 * seg + kb
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    _same(_gpu(rp, seg, kb, vec), oracle_cpu.preprocess(rp, seg, kb, vec))
