@@ -226,14 +226,20 @@ __device__ __forceinline__ V gather(const V *lane_base, int c, unsigned row_byte
 // read the same address: one broadcast wavefront per load, against one per element with shuffles).
 template <int U>
 __device__ __forceinline__ void ld_shared_run(const int *p, int (&out)[U]) {
-    static_assert(U % 4 == 0, "runs of four");
+    static_assert(U == 2 || U % 4 == 0, "runs of two or four");
+    if constexpr (U == 2) {
+        const int2 x = *reinterpret_cast<const int2 *>(p);
+        out[0] = x.x;
+        out[1] = x.y;
+    } else {
 #pragma unroll
-    for (int u = 0; u < U; u += 4) {
-        const int4 x = *reinterpret_cast<const int4 *>(p + u);
-        out[u] = x.x;
-        out[u + 1] = x.y;
-        out[u + 2] = x.z;
-        out[u + 3] = x.w;
+        for (int u = 0; u < U; u += 4) {
+            const int4 x = *reinterpret_cast<const int4 *>(p + u);
+            out[u] = x.x;
+            out[u + 1] = x.y;
+            out[u + 2] = x.z;
+            out[u + 3] = x.w;
+        }
     }
 }
 template <int U>
@@ -260,9 +266,23 @@ __device__ __forceinline__ void ld_shared_run(const double *p, double (&out)[U])
 }
 
 // Streaming read of CSR data (touched once): do not let it displace dense rows in L1.
-__device__ __forceinline__ int ld_stream(const int *p) { return __ldcs(p); }
-__device__ __forceinline__ float ld_stream(const float *p) { return __ldcs(p); }
-__device__ __forceinline__ double ld_stream(const double *p) { return __ldcs(p); }
+// (Read-only loads: the compiler may then move them across the stores of results, which it cannot know to be
+// to another array once a kernel's body is a function of its own.)
+__device__ __forceinline__ int ld_stream(const int *p) {
+    int v;
+    asm("ld.global.cs.nc.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float ld_stream(const float *p) {
+    float v;
+    asm("ld.global.cs.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double ld_stream(const double *p) {
+    double v;
+    asm("ld.global.cs.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
 
 // Streaming store of results (written once, not read again by this kernel).
 template <typename V>

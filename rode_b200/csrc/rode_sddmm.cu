@@ -41,6 +41,7 @@
 // 4*K bytes of lhs per group that touches it.  No atomics, no workspace in global memory.
 #include <climits>
 #include <mutex>
+#include <type_traits>
 
 #include "rode_common.cuh"
 
@@ -56,9 +57,8 @@ namespace {
 #ifndef RODE_SDDMM_COLUMNS_IN_SMEM
 #define RODE_SDDMM_COLUMNS_IN_SMEM 1
 #endif
-// Lane-group sizes L of the stream kernel for which it stages (bit mask: 8 | 16 | 32).
-#ifndef RODE_SDDMM_ITEMS_SMEM_MASK
-#define RODE_SDDMM_ITEMS_SMEM_MASK (8 | 16 | 32)
+#ifndef RODE_SDDMM_ROW_MODE_MIN32
+#define RODE_SDDMM_ROW_MODE_MIN32 16
 #endif
 constexpr int kLoadsInFlight = 8;  // 16-byte loads per lane per batch
 constexpr unsigned kFull = 0xffffffffu;
@@ -96,14 +96,13 @@ __device__ __forceinline__ float reduce_batch(float (&p)[NB], int l, unsigned gm
 // buffer to use next; both are carried from row to row so that a group never stores into a
 // buffer that one of its lanes may still read.
 // kRagged: the dense rows hold row_vecs_arg <= L * VPL vectors, the rest of the lanes idle.
-template <int L, int VPL, bool kStageAllowed, bool kRagged>
+template <int L, int VPL, int kBatch, bool kRagged>
 __device__ __forceinline__ void sddmm_one_row(int row, int begin, int end, int lane, int row_vecs_arg,
                                               const int *__restrict__ column_indices,
                                               const float *__restrict__ values, const float *__restrict__ lhs,
                                               const float *__restrict__ rhs, float *__restrict__ out, int *stage,
                                               int &stage_buf) {
-    constexpr int kBatch = (kLoadsInFlight / VPL < L) ? kLoadsInFlight / VPL : L;
-    constexpr bool kStage = RODE_SDDMM_COLUMNS_IN_SMEM != 0 && kStageAllowed && (kBatch % 4 == 0);
+    constexpr bool kStage = RODE_SDDMM_COLUMNS_IN_SMEM != 0;
     const unsigned row_vecs = kRagged ? row_vecs_arg : L * VPL;
     const int l = lane % L;
     const unsigned gmask = group_mask<L>(lane);
@@ -172,6 +171,144 @@ __device__ __forceinline__ void sddmm_one_row(int row, int begin, int end, int l
     }
 }
 
+// ---------------------------------------------------------------------------------------
+// One warp per block segment (used where segments are long, K other than 128: up to 543
+// nonzeros).  Chunks of 32 nonzeros are plain coalesced loads without any search, the G groups take every G-th
+// nonzero of a chunk, and the lhs slice stays in registers.
+//
+// Few lanes per dense row with several loads each keep the instruction count low: the reduction over the
+// lanes, its selects and shuffles, is paid once per L lanes, the FMAs and loads are the same in every shape.
+// A full chunk takes a form without bounds (no predicate and no zero-fill per load).  (Block grids, us: Zipf
+// 100003 x 50021 K = 96, 32 lanes x 1 85, 8 x 3 54; Zipf 65536 K = 64, 16 x 1 27, 8 x 2 23; R-MAT 21 K = 96 900 and 700.)
+//
+// kClaim (grids of one resident wave): a warp starts with the segment of its own index and
+// claims further ones from *next_segment; the claim is issued before the segment's work and
+// read after it.  One-warp CTAs of one segment each live a few microseconds, and a fifth of the
+// warp slots stood empty waiting for the next CTA to be launched into them.
+template <int L, int VPL, int U, bool kClaim, bool kRagged>
+__device__ __forceinline__ void block_segments(int m1, const int *__restrict__ block_r_ind, const int *__restrict__ st_off,
+            const int *__restrict__ row_offsets, const int *__restrict__ column_indices,
+            const float *__restrict__ values, const float *__restrict__ lhs, const float *__restrict__ rhs,
+            float *__restrict__ out, int *__restrict__ next_segment, int row_vecs_arg) {
+    constexpr int G = 32 / L;
+    static_assert(L % U == 0 && U >= 2, "a chunk is a whole number of batches");
+    const unsigned row_vecs = kRagged ? static_cast<unsigned>(row_vecs_arg) : L * VPL;
+    const unsigned row_bytes = row_vecs * 16u;
+    __shared__ __align__(16) int s_col[2][32];  // column indices of the current chunk, two buffers
+    int stage_buf = 0;
+    const int lane = threadIdx.x;
+    const int g = lane / L, l = lane % L;
+    // (with four vectors per lane a second form only spills; L = 16 is the form of the large grids)
+    constexpr bool kFullPath = VPL <= 3 && L == 8;
+    const int pos = l * G + g;  // this lane's nonzero of a chunk: group g holds positions g, g + G, ...
+    int seg = blockIdx.x;
+    while (seg < m1) {
+    int claimed = INT_MAX;  // never used in arithmetic: the loop test compares it with m1 as it is
+    if constexpr (kClaim) {
+        if (lane == 0) claimed = static_cast<int>(gridDim.x) + atomicAdd(next_segment, 1);
+    }
+
+    const int row = __ldg(block_r_ind + seg);
+    const int off = __ldg(st_off + seg);
+    const int next = (seg + 1 < m1) ? __ldg(st_off + seg + 1) : INT_MAX;
+    const int end = min(__ldg(row_offsets + row + 1), next);
+
+    const float4 *rhs_lane = reinterpret_cast<const float4 *>(rhs) + l;
+    auto inside = [&](int v) { return !kRagged || static_cast<unsigned>(l + v * L) < row_vecs; };
+    float4 a[VPL];
+#pragma unroll
+    for (int v = 0; v < VPL; ++v)
+        a[v] = inside(v)
+                   ? __ldg(reinterpret_cast<const float4 *>(lhs) + static_cast<size_t>(row) * row_vecs + v * L + l)
+                   : make_float4(0.f, 0.f, 0.f, 0.f);
+
+    int c_cur = 0, c_nxt = 0;
+    float v_cur = 0.f, v_nxt = 0.f;
+    if (off + pos < end) {
+        c_cur = ld_stream(column_indices + off + pos);
+        v_cur = ld_stream(values + off + pos);
+    }
+    if (off + 32 + pos < end) {
+        c_nxt = ld_stream(column_indices + off + 32 + pos);
+        v_nxt = ld_stream(values + off + 32 + pos);
+    }
+    for (int base = off; base < end; base += 32) {
+        int c_pre = 0;
+        float v_pre = 0.f;
+        if (base + 64 + pos < end) {  // pairs of the chunk after next
+            c_pre = ld_stream(column_indices + base + 64 + pos);
+            v_pre = ld_stream(values + base + 64 + pos);
+        }
+        const int cnt = min(32, end - base);
+        float mine = 0.f;
+        s_col[stage_buf][lane] = c_cur;
+        __syncwarp();
+        const int *my_cols = &s_col[stage_buf][g * L];
+        auto chunk = [&](auto full_tag) {
+            constexpr bool kFullChunk = decltype(full_tag)::value;
+#pragma unroll
+            for (int b = 0; b < L / U; ++b) {
+                if (!kFullChunk && b * U * G >= cnt) break;  // warp-uniform
+                float4 bb[U][VPL];
+                int cc[U];
+                ld_shared_run<U>(my_cols + b * U, cc);
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const float4 *src = dense_row(rhs_lane, static_cast<unsigned>(cc[u]), row_bytes);
+#pragma unroll
+                    for (int v = 0; v < VPL; ++v) {
+                        if constexpr (kFullChunk && !kRagged) {
+                            bb[u][v] = ld_dense(src + v * L);
+                        } else {
+                            bb[u][v] = make_float4(0.f, 0.f, 0.f, 0.f);
+                            if ((kFullChunk || (b * U + u) * G + g < cnt) && inside(v)) bb[u][v] = ld_dense(src + v * L);
+                        }
+                    }
+                }
+                float p[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    float d = 0.f;
+#pragma unroll
+                    for (int v = 0; v < VPL; ++v) d = dot4(a[v], bb[u][v], d);
+                    p[u] = d;
+                }
+                const float r = reduce_batch<L, U>(p, l, kFull);
+                // nonzero u of the batch sits in lanes u * (L / U) ..; lane b * U + u of the group wants it
+                const float got = (L == U) ? r : __shfl_sync(kFull, r, (l & (U - 1)) * (L / U), L);
+                if ((l / U) == b) mine = got;
+            }
+        };
+        if (kFullPath && cnt == 32)
+            chunk(std::true_type{});
+        else
+            chunk(std::false_type{});
+        if (pos < cnt) st_stream(out + base + pos, v_cur * mine);
+        c_cur = c_nxt;
+        v_cur = v_nxt;
+        c_nxt = c_pre;
+        v_nxt = v_pre;
+        stage_buf ^= 1;
+    }
+    seg = kClaim ? __shfl_sync(kFull, claimed, 0) : INT_MAX;
+    }  // segments of this warp
+}
+// One-warp CTAs per SM: 64 registers while a lane holds two vectors per dense row, 72 beyond.
+constexpr int block_ctas(int vpl) { return vpl <= 2 ? 32 : 28; }
+template <int L, int VPL, int U, bool kClaim, bool kRagged>
+__global__ void __launch_bounds__(32, block_ctas(VPL))
+sddmm_block(int m1, const int *__restrict__ block_r_ind, const int *__restrict__ st_off,
+            const int *__restrict__ row_offsets, const int *__restrict__ column_indices,
+            const float *__restrict__ values, const float *__restrict__ lhs, const float *__restrict__ rhs,
+            float *__restrict__ out, int *__restrict__ next_segment, int row_vecs) {
+    chain_begin();
+    block_segments<L, VPL, U, kClaim, kRagged>(m1, block_r_ind, st_off, row_offsets, column_indices, values, lhs, rhs, out,
+                                               next_segment, row_vecs);
+}
+
+// ---------------------------------------------------------------------------------------
+// Items as an entry stream, or rows one by one.
+//
 // kSegments: items are block segments (block_r_ind / st_off); otherwise residue rows
 // (residue_r_ind) without a block part.
 //
@@ -185,18 +322,22 @@ __device__ __forceinline__ void sddmm_one_row(int row, int begin, int end, int l
 // and empty rows (graphs) are better served by the stream, which splits the warp's nonzeros
 // evenly.  The warp decides from the row lengths it has just loaded, so no statistic of the
 // matrix has to be passed in.
+//
+// BL > 0 (residue rows only): segments and rows in one launch, for grids so small that the second launch is
+// what costs: the first m1 CTAs take a segment each, the others a bundle of rows (Bernoulli 4096^2, K = 32,
+// back to back 10.6 -> 8.6 us).
 // One-warp CTAs per SM the register allocation must allow: 28 (72 registers).  Left to itself the
 // compiler takes 78-80 registers for K = 64 once the chunk staging is in, and the four warps per
 // SM that costs outweigh what the staging gains; 64 registers (32 CTAs) spill.
 #ifndef RODE_SDDMM_ITEMS_MIN_CTAS
 #define RODE_SDDMM_ITEMS_MIN_CTAS 28
 #endif
-template <int L, int VPL, bool kSegments, bool kRagged = false, int LB = 0, int VPLB = 1>
-__global__ void __launch_bounds__(32, VPL > 1 ? 24 : RODE_SDDMM_ITEMS_MIN_CTAS)
+template <int L, int VPL, bool kSegments, bool kRagged, int LB, int VPLB, int UB, int BL = 0, int BVPL = 1, int BU = 1>
+__global__ void __launch_bounds__(32, (VPL > 1 || BL > 0) ? 24 : RODE_SDDMM_ITEMS_MIN_CTAS)
 sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, const int *__restrict__ st_off,
             const int *__restrict__ row_offsets, const int *__restrict__ column_indices,
             const float *__restrict__ values, const float *__restrict__ lhs, const float *__restrict__ rhs,
-            float *__restrict__ out, int row_vecs_arg, int row_mode_min) {
+            float *__restrict__ out, int row_vecs_arg, int row_mode_min, int m1, const int *__restrict__ seg_rows) {
     constexpr int G = 32 / L;
     constexpr int kBatch = kLoadsInFlight / VPL;  // nonzeros per batch
     const size_t row_vecs = kRagged ? static_cast<unsigned>(row_vecs_arg) : L * VPL;  // float4 per dense row (K / 4)
@@ -209,8 +350,15 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
     const int lane = threadIdx.x;
     const int g = lane / L, l = lane % L;
     const unsigned gmask = group_mask<L>(lane);
-    const long long item0 = static_cast<long long>(blockIdx.x) * items_per_warp;
+    int bundle = blockIdx.x;
+    if constexpr (BL > 0) {
+        if (bundle < m1)
+            return block_segments<BL, BVPL, BU, false, kRagged>(m1, seg_rows, st_off, row_offsets, column_indices, values, lhs,
+                                                                rhs, out, nullptr, row_vecs_arg);
+        bundle -= m1;
+    }
     chain_begin();
+    const long long item0 = static_cast<long long>(bundle) * items_per_warp;
     if (item0 >= n_items) return chain_wait();  // the CTA behind the items
 
     // ---- descriptors: lane j owns item item0 + j --------------------------------------------
@@ -241,10 +389,10 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
     const unsigned nonempty = __ballot_sync(kFull, len > 0);
     if (total == 0) return;
     if constexpr (LB > 0 && !kSegments) {
-        static_assert(LB * VPLB == L * VPL, "both lane-group shapes must cover the same dense row");
+        static_assert(LB * VPLB == L * VPL || kRagged, "both lane-group shapes must cover the same dense row");
         // (full warps of 32 rows only: short lists give a warp fewer rows than it has groups, and
         // there the stream's even split of the nonzeros is what shortens the dependent chain)
-        if (items_per_warp == 32 && total >= row_mode_min * 32) {  // warp-uniform
+        if (BL > 0 || (items_per_warp == 32 && total >= row_mode_min * 32)) {  // warp-uniform
             constexpr int GB = 32 / LB;
             const int gb = lane / LB;
             for (int j0 = 0; j0 < items_per_warp; j0 += GB) {
@@ -253,7 +401,7 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
                 const int b0 = __shfl_sync(kFull, begin, j & 31);
                 const int n0 = __shfl_sync(kFull, len, j & 31);
                 if (j < items_per_warp && n0 > 0)
-                    sddmm_one_row<LB, VPLB, ((RODE_SDDMM_ITEMS_SMEM_MASK) & L) != 0, kRagged>(
+                    sddmm_one_row<LB, VPLB, UB, kRagged>(
                         r, b0, b0 + n0, lane, row_vecs_arg, column_indices, values, lhs, rhs, out, &s_col[0][0], stage_buf);
             }
             return;
@@ -330,7 +478,7 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
         fetch(p0 + (ch + 2) * L + l, e_pre, c_pre, v_pre);
         const int cnt = min(L, p1 - (p0 + ch * L));  // valid nonzeros of this chunk (may be <= 0)
         float mine = 0.f;
-        constexpr bool kStage = RODE_SDDMM_COLUMNS_IN_SMEM != 0 && ((RODE_SDDMM_ITEMS_SMEM_MASK) & L) != 0 && (kBatch % 4 == 0);
+        constexpr bool kStage = RODE_SDDMM_COLUMNS_IN_SMEM != 0 && (kBatch % 4 == 0);
         int *my_stage = &s_col[stage_buf][lane - l];  // this group's region of the chunk buffer
         if constexpr (kStage) {
             my_stage[l] = c_cur;
@@ -401,115 +549,6 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
 }
 
 // ---------------------------------------------------------------------------------------
-// One warp per block segment (used where segments are long, K = 32 and 64: up to 543
-// nonzeros): coalesced chunk loads without any search, the G groups take consecutive
-// L-nonzero pieces of each 32-nonzero chunk, the lhs slice stays in registers.
-//
-// kClaim (grids of one resident wave): a warp starts with the segment of its own index and
-// claims further ones from *next_segment; the claim is issued before the segment's work and
-// read after it.  One-warp CTAs of one segment each live a few microseconds, and a fifth of the
-// warp slots stood empty waiting for the next CTA to be launched into them.
-template <int L, int VPL, bool kClaim, bool kRagged = false>
-__global__ void __launch_bounds__(32, VPL == 1 ? 32 : 24)  // 64 registers: 32 one-warp CTAs per SM
-sddmm_block(int m1, const int *__restrict__ block_r_ind, const int *__restrict__ st_off,
-            const int *__restrict__ row_offsets, const int *__restrict__ column_indices,
-            const float *__restrict__ values, const float *__restrict__ lhs, const float *__restrict__ rhs,
-            float *__restrict__ out, int *__restrict__ next_segment, int row_vecs_arg) {
-    constexpr int kBatch = kLoadsInFlight / VPL;
-    const size_t row_vecs = kRagged ? static_cast<unsigned>(row_vecs_arg) : L * VPL;
-    constexpr bool kStage = RODE_SDDMM_COLUMNS_IN_SMEM != 0 && (kBatch % 4 == 0);
-    __shared__ __align__(16) int s_col[2][32];  // column indices of the current chunk, two buffers
-    int stage_buf = 0;
-    const int lane = threadIdx.x;
-    const int l = lane % L;
-    const int gbase = lane - l;  // first lane (= first nonzero of the chunk) of this group
-    const unsigned gmask = group_mask<L>(lane);
-    chain_begin();
-    int seg = blockIdx.x;
-    while (seg < m1) {
-    int claimed = INT_MAX;  // never used in arithmetic: the loop test compares it with m1 as it is
-    if constexpr (kClaim) {
-        if (lane == 0) claimed = static_cast<int>(gridDim.x) + atomicAdd(next_segment, 1);
-    }
-
-    const int row = __ldg(block_r_ind + seg);
-    const int off = __ldg(st_off + seg);
-    const int next = (seg + 1 < m1) ? __ldg(st_off + seg + 1) : INT_MAX;
-    const int end = min(__ldg(row_offsets + row + 1), next);
-
-    const float4 *rhs_lane = reinterpret_cast<const float4 *>(rhs) + l;
-    auto inside = [&](int v) { return !kRagged || static_cast<size_t>(l + v * L) < row_vecs; };
-    float4 a[VPL];
-#pragma unroll
-    for (int v = 0; v < VPL; ++v)
-        a[v] = inside(v) ? __ldg(reinterpret_cast<const float4 *>(lhs) + static_cast<size_t>(row) * row_vecs + v * L + l)
-                         : make_float4(0.f, 0.f, 0.f, 0.f);
-
-    int c_cur = 0, c_nxt = 0;
-    float v_cur = 0.f, v_nxt = 0.f;
-    if (off + lane < end) {
-        c_cur = ld_stream(column_indices + off + lane);
-        v_cur = ld_stream(values + off + lane);
-    }
-    if (off + 32 + lane < end) {
-        c_nxt = ld_stream(column_indices + off + 32 + lane);
-        v_nxt = ld_stream(values + off + 32 + lane);
-    }
-    for (int base = off; base < end; base += 32) {
-        int c_pre = 0;
-        float v_pre = 0.f;
-        if (base + 64 + lane < end) {  // pairs of the chunk after next
-            c_pre = ld_stream(column_indices + base + 64 + lane);
-            v_pre = ld_stream(values + base + 64 + lane);
-        }
-        const int cnt = min(32, end - base);
-        float mine = 0.f;
-        if constexpr (kStage) {
-            s_col[stage_buf][lane] = c_cur;
-            __syncwarp();
-        }
-#pragma unroll
-        for (int b = 0; b < L / kBatch; ++b) {
-            if (gbase + b * kBatch < cnt) {  // uniform inside the group
-                float4 bb[kBatch][VPL];
-                int cc[kBatch];
-                if constexpr (kStage) ld_shared_run<kBatch>(&s_col[stage_buf][gbase + b * kBatch], cc);
-#pragma unroll
-                for (int u = 0; u < kBatch; ++u) {
-                    const int t = b * kBatch + u;  // nonzero inside the group's part of the chunk
-                    if constexpr (!kStage) cc[u] = __shfl_sync(gmask, c_cur, t, L);
-#pragma unroll
-                    for (int v = 0; v < VPL; ++v) {
-                        bb[u][v] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (gbase + t < cnt && inside(v))
-                            bb[u][v] = ld_dense(rhs_lane + static_cast<size_t>(cc[u]) * row_vecs + v * L);
-                    }
-                }
-                float p[kBatch];
-#pragma unroll
-                for (int u = 0; u < kBatch; ++u) {
-                    float d = 0.f;
-#pragma unroll
-                    for (int v = 0; v < VPL; ++v) d = dot4(a[v], bb[u][v], d);
-                    p[u] = d;
-                }
-                const float r = reduce_batch<L, kBatch>(p, l, gmask);
-                const float got = (L == kBatch) ? r : __shfl_sync(gmask, r, (l & (kBatch - 1)) * (L / kBatch), L);
-                if ((l / kBatch) == b) mine = got;
-            }
-        }
-        if (base + lane < end) st_stream(out + base + lane, v_cur * mine);
-        c_cur = c_nxt;
-        v_cur = v_nxt;
-        c_nxt = c_pre;
-        v_nxt = v_pre;
-        stage_buf ^= 1;
-    }
-    seg = kClaim ? __shfl_sync(kFull, claimed, 0) : INT_MAX;
-    }  // segments of this warp
-}
-
-// ---------------------------------------------------------------------------------------
 // Claim counter of the persistent block grid.  The SDDMM entry points carry no workspace, so the
 // counters live in a fixed array of the library's device image: kClaimSlots slots of 64 ints
 // (32 KB on every GPU that loads the library).  A slot belongs to one (device, stream1, stream2)
@@ -565,39 +604,56 @@ int items_per_warp(int n_items, int cap) {
 
 // L lanes x VPL vectors for the segments and the streams, RL x RVPL (RL = 0: none) for the row mode of the
 // residue kernel.  kLongSegments: a warp per segment, else up to 32 segments per warp.
-template <int L, int VPL, int RL, int RVPL, bool kRagged, bool kLongSegments>
+template <int L, int VPL, int BL, int BVPL, int BU, int PL, int PVPL, int PU, int RL,
+          int RVPL, int RU, bool kRagged, bool kLongSegments>
 int launch_k(int m1, int m2, int k, const int *block_r_ind, const int *residue_r_ind,
              const int *st_off, const int *row_offsets, const int *col, const float *values, const float *lhs,
              const float *rhs, float *out, cudaStream_t s1, cudaStream_t s2) {
     const int row_vecs = k / 4;
+    // nonzeros per row from which a warp takes its rows one by one: where the stream form has one lane group only
+    // it balances nothing, but short rows still lose more to the idle lane groups of the row form (R-MAT 21,
+    // K = 96: 0.56 ms as a stream, 0.65 to 0.68 ms row by row; stencil, K = 128: 1.78 against 1.57 ms)
+    const int row_mode_min = L == 32 ? RODE_SDDMM_ROW_MODE_MIN32 : RODE_SDDMM_ROW_MODE_MIN;
+    if constexpr (kLongSegments) {
+        // (a row per lane group: on such matrices most residue rows have had their tail taken by a segment)
+        const int per = RL > 0 ? 32 / (RL > 0 ? RL : 1) : 1;
+        const long long ctas = static_cast<long long>(m1) + (m2 + per - 1) / per;
+        if (m1 > 0 && m2 > 0 && s1 == s2 && ctas <= 4LL * 24 * sm_count()) {
+            sddmm_items<L, VPL, false, kRagged, RL, RVPL, RU, BL, BVPL, BU><<<static_cast<unsigned>(ctas), 32, 0, s1>>>(
+                m2, per, residue_r_ind, st_off, row_offsets, col, values, lhs, rhs, out, row_vecs, row_mode_min, m1,
+                block_r_ind);
+            RODE_CHECK_LAUNCH("rode::sddmm_items<segments and rows>");
+            return RODE_OK;
+        }
+    }
     if (m1 > 0) {
         if constexpr (kLongSegments) {
-            const int resident = (VPL == 1 ? 32 : 24) * sm_count();
+            const int resident = block_ctas(BVPL) * sm_count();
             int *claim = nullptr;
-            if (RODE_SDDMM_PERSISTENT && m1 > 16 * resident) {  // from about 16 segments per warp on it pays
+            if (m1 > 16 * resident) {  // from about 16 segments per warp on it pays
                 if (int rc = claim_counters(s1, s2, &claim)) return rc;
             }
             if (claim != nullptr) {
                 RODE_CUDA_TRY(cudaMemsetAsync(claim, 0, sizeof(int), s1));
-                sddmm_block<L, VPL, true, kRagged><<<resident, 32, 0, s1>>>(m1, block_r_ind, st_off, row_offsets, col, values,
-                                                                            lhs, rhs, out, claim, row_vecs);
+                sddmm_block<PL, PVPL, PU, true, kRagged><<<resident, 32, 0, s1>>>(
+                    m1, block_r_ind, st_off, row_offsets, col, values, lhs, rhs, out, claim, row_vecs);
             } else {
-                sddmm_block<L, VPL, false, kRagged><<<m1, 32, 0, s1>>>(m1, block_r_ind, st_off, row_offsets, col, values, lhs,
-                                                                       rhs, out, nullptr, row_vecs);
+                sddmm_block<BL, BVPL, BU, false, kRagged><<<m1, 32, 0, s1>>>(m1, block_r_ind, st_off, row_offsets, col, values,
+                                                                            lhs, rhs, out, nullptr, row_vecs);
             }
             RODE_CHECK_LAUNCH("rode::sddmm_block");
         } else {
             const int per = items_per_warp(m1, 32);
-            sddmm_items<L, VPL, true, kRagged><<<(m1 + per - 1) / per, 32, 0, s1>>>(
-                m1, per, block_r_ind, st_off, row_offsets, col, values, lhs, rhs, out, row_vecs, 0);
+            sddmm_items<L, VPL, true, kRagged, 0, 1, 1><<<(m1 + per - 1) / per, 32, 0, s1>>>(
+                m1, per, block_r_ind, st_off, row_offsets, col, values, lhs, rhs, out, row_vecs, 0, 0, nullptr);
             RODE_CHECK_LAUNCH("rode::sddmm_items<segments>");
         }
     }
     if (m2 > 0) {
         const int per = items_per_warp(m2, 32);
-        RODE_CUDA_TRY(launch_chained(sddmm_items<L, VPL, false, kRagged, RL, RVPL>, dim3((m2 + per - 1) / per + 1), dim3(32), s2,
+        RODE_CUDA_TRY(launch_chained(sddmm_items<L, VPL, false, kRagged, RL, RVPL, RU>, dim3((m2 + per - 1) / per + 1), dim3(32), s2,
                                      m1 > 0 && s1 == s2, m2, per, residue_r_ind, nullptr, row_offsets, col, values, lhs,
-                                     rhs, out, row_vecs, RODE_SDDMM_ROW_MODE_MIN));
+                                     rhs, out, row_vecs, row_mode_min, 0, nullptr));
         RODE_CHECK_LAUNCH("rode::sddmm_items<rows>");
     }
     return RODE_OK;
@@ -622,20 +678,25 @@ extern "C" int rode_sddmm_f32(int m1, int m2, int n, int k, const int *block_r_i
     if (m2 > 0 && !residue_r_ind) return fail(RODE_ERR_INVALID_ARGUMENT, "sddmm: null residue metadata");
     if (!aligned_to(lhs, 16) || !aligned_to(rhs, 16))
         return fail(RODE_ERR_INVALID_ARGUMENT, "sddmm: lhs and rhs must be 16-byte aligned");
-#define RODE_SDDMM_LAUNCH(L, VPL, RL, RVPL, ragged, long_segments)                                                    \
-    launch_k<L, VPL, RL, RVPL, ragged, long_segments>(m1, m2, k, block_r_ind, residue_r_ind, st_off, row_offsets,    \
-                                       column_indices, values, lhs, rhs, out, stream1, stream2)
+#define RODE_SDDMM_LAUNCH(...)                                                                                   \
+    launch_k<__VA_ARGS__>(m1, m2, k, block_r_ind, residue_r_ind, st_off, row_offsets, column_indices, values, lhs, rhs, \
+                          out, stream1, stream2)
     // The narrowest lane group that covers the dense row; where it does not fit exactly the lanes beyond the
     // row's end idle (ragged).  (One form of 32 lanes x 2 vectors for all of those widths took 0.209 ms on
     // the 100003 x 50021 Zipf matrix at K = 96, the 32 x 1 form 0.117 ms.)  The decomposition that goes with
     // K = 128 has 32-long segments, all others 512-long ones.
     const int vecs = k / 4;
-    if (vecs == 8) return RODE_SDDMM_LAUNCH(8, 1, 8, 1, false, true);
-    if (vecs == 16) return RODE_SDDMM_LAUNCH(16, 1, 8, 2, false, true);
-    if (vecs == 32) return RODE_SDDMM_LAUNCH(32, 1, 0, 1, false, false);
-    if (vecs < 8) return RODE_SDDMM_LAUNCH(8, 1, 8, 1, true, true);
-    if (vecs < 16) return RODE_SDDMM_LAUNCH(16, 1, 8, 2, true, true);
-    if (vecs < 32) return RODE_SDDMM_LAUNCH(32, 1, 0, 1, true, true);
-    return RODE_SDDMM_LAUNCH(32, 2, 0, 1, true, true);
+    // (stream shape; block shape and nonzeros per batch, the same for persistent block grids; row-mode shape and
+    // nonzeros per batch.  K = 64: 8 x 2 takes fewer instructions, Pareto 2^18 block grid 119 -> 103 us, Zipf
+    // 65536 29 -> 23 us; matrices of millions of rows are bound by the L2 and DRAM and lose 4 % with it, R-MAT
+    // 23 3.16 -> 3.29 ms, so persistent grids keep 16 x 1 in the form without a separate full chunk.)
+    if (vecs == 8) return RODE_SDDMM_LAUNCH(8, 1, 8, 1, 8, 8, 1, 8, 8, 1, 8, false, true);
+    if (vecs == 16) return RODE_SDDMM_LAUNCH(16, 1, 8, 2, 4, 16, 1, 8, 8, 2, 4, false, true);
+    if (vecs == 32) return RODE_SDDMM_LAUNCH(32, 1, 8, 4, 2, 8, 4, 2, 8, 4, 2, false, false);
+    if (vecs < 8) return RODE_SDDMM_LAUNCH(8, 1, 8, 1, 8, 8, 1, 8, 8, 1, 8, true, true);
+    if (vecs < 16) return RODE_SDDMM_LAUNCH(16, 1, 8, 2, 4, 8, 2, 4, 8, 2, 4, true, true);
+    if (vecs <= 24) return RODE_SDDMM_LAUNCH(32, 1, 8, 3, 4, 8, 3, 4, 8, 3, 2, true, true);
+    if (vecs < 32) return RODE_SDDMM_LAUNCH(32, 1, 8, 4, 2, 8, 4, 2, 8, 4, 2, true, true);
+    return RODE_SDDMM_LAUNCH(32, 2, 16, 4, 2, 16, 4, 2, 16, 4, 2, true, true);
 #undef RODE_SDDMM_LAUNCH
 }
