@@ -6,7 +6,9 @@ path here: if the library is missing, loading fails loudly.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
+import functools
 import os
 from dataclasses import dataclass
 from typing import Optional
@@ -191,12 +193,19 @@ def preprocess(row_ptr: torch.Tensor, nnz: int, seg_len: int = 512, k_block: int
     return RodeMeta(blk, st, res, m1, m2, seg_len, k_block, vec_len)
 
 
-class _null:
-    def __enter__(self):
-        return self
+def _null():
+    return contextlib.nullcontext()
 
-    def __exit__(self, *a):
-        return False
+
+def _current(dev: torch.device) -> int:
+    """Handle of torch's current stream (torch.cuda.current_stream builds an object for it, 2 us)."""
+    return torch._C._cuda_getCurrentRawStream(dev.index)
+
+
+def _on(dev: torch.device):
+    """torch.cuda.device(dev), or nothing where dev is current already (entering and leaving the
+    context costs as much as a launch)."""
+    return _null() if torch.cuda.current_device() == dev.index else torch.cuda.device(dev)
 
 
 def preprocess_cpu(row_ptr: torch.Tensor, seg_len: int = 512, k_block: int = 32, vec_len: int = 4):
@@ -219,6 +228,7 @@ def preprocess_cpu(row_ptr: torch.Tensor, seg_len: int = 512, k_block: int = 32,
 
 
 # ---------------------------------------------------------------------------------------
+@functools.lru_cache(maxsize=256)
 def spmm_workspace_bytes(m1: int, n: int, elem_size: int = 4) -> int:
     out = ctypes.c_size_t(0)
     check(load().rode_spmm_workspace_bytes(m1, n, elem_size, ctypes.byref(out)))
@@ -289,8 +299,8 @@ def spmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torch
     if not (B.is_cuda and B.is_contiguous() and values.is_contiguous() and col.is_contiguous()):
         raise ValueError("contiguous CUDA tensors required")
     dev = B.device
-    with torch.cuda.device(dev):
-        cur = torch.cuda.current_stream(dev)
+    with _on(dev):
+        cur = _current(dev)
         s1 = cur if stream1 is None else stream1
         s2 = cur if stream2 is None else stream2
         whole = C is None and (meta.m1 > 0 or meta.m2 > 0)
@@ -302,9 +312,10 @@ def spmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torch
             # the buffer goes back to torch's allocator when this function returns: tell the
             # allocator which other streams still use it, or a call enqueued right afterwards
             # could be handed the same memory while this call's kernels run
-            for s in (s1, s2):
-                if isinstance(s, torch.cuda.Stream) and s != cur:
-                    workspace.record_stream(s)
+            if s1 is not cur or s2 is not cur:
+                for s in (s1, s2):
+                    if isinstance(s, torch.cuda.Stream) and s.cuda_stream != cur:
+                        workspace.record_stream(s)
         ws_bytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
         if whole:
             spmm_all_raw(B.dtype, M, meta.m1, k, n, values.data_ptr(), col.data_ptr(), row_ptr.data_ptr(),
@@ -331,8 +342,8 @@ def sddmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torc
     if rhs.shape[1] != k:
         raise ValueError("lhs and rhs must have the same number of columns")
     dev = lhs.device
-    with torch.cuda.device(dev):
-        cur = torch.cuda.current_stream(dev)
+    with _on(dev):
+        cur = _current(dev)
         s1 = cur if stream1 is None else stream1
         s2 = cur if stream2 is None else stream2
         if out is None:  # every stored entry lies in a block segment or a residue row, so all of it is written

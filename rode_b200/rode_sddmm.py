@@ -102,9 +102,9 @@ class RoDeCSR:
 
 
 def _check_dense(name: str, t: torch.Tensor, shape, sparse: RoDeCSR):
-    if tuple(t.shape) != tuple(shape):
-        raise ValueError(f"{name} shape must be {tuple(shape)}, got {tuple(t.shape)}")
-    assert t.is_cuda and t.device == sparse.device, f"{name} must be on {sparse.device}, got {t.device}"
+    if t.shape != shape:
+        raise ValueError(f"{name} shape must be {shape}, got {tuple(t.shape)}")
+    assert t.device == sparse.device, f"{name} must be on {sparse.device}, got {t.device}"
     assert t.dtype == torch.float32, f"{name} must be float32, got {t.dtype}"
 
 
@@ -121,21 +121,21 @@ def rode_sddmm(sparse_matrix: RoDeCSR, lhs: torch.Tensor, rhs: torch.Tensor) -> 
 
 
 def rode_spmm(sparse_matrix: RoDeCSR, dense: torch.Tensor, hints: bool = True) -> torch.Tensor:
-    """C = S @ dense for dense [n, width], width a multiple of 4.  Needs metadata from
-    seg_length 512 (k = 32 or 64 at construction); the reference has no Python SpMM.
+    """C = S @ dense for dense [n, width], width a multiple of 4.  Takes the metadata of any k (all of
+    them are decomposed with k_block 32; segments of 512, k other than 128 at construction, serve it
+    best); the reference has no Python SpMM.
 
     ``hints``: gather popular columns' rows with an L2 policy that keeps them resident
     (same results, fewer DRAM bytes on skewed matrices).  The popularity bitmap is built on
     the first call for a given width and cached on ``sparse_matrix``."""
-    if sparse_matrix.config_for(sparse_matrix.k)["k_block"] != 32:
-        raise ValueError("SpMM needs k_block = 32 metadata")
-    if dense.dim() != 2 or dense.shape[0] != sparse_matrix.n:
-        raise ValueError(f"dense must be ({sparse_matrix.n}, width), got {tuple(dense.shape)}")
-    assert dense.is_cuda and dense.device == sparse_matrix.device and dense.dtype == torch.float32
+    shape = dense.shape
+    if len(shape) != 2 or shape[0] != sparse_matrix.n:
+        raise ValueError(f"dense must be ({sparse_matrix.n}, width), got {tuple(shape)}")
+    assert dense.device == sparse_matrix.device and dense.dtype == torch.float32
     hot = None
-    if hints and dense.shape[1] % 128 == 0:
+    if hints and shape[1] % 128 == 0:
         cache = sparse_matrix.__dict__.setdefault("_hot_columns", {})
-        row_bytes = dense.shape[1] * dense.element_size()
+        row_bytes = shape[1] * dense.element_size()
         if row_bytes not in cache:
             cache[row_bytes] = rode_sddmm_cuda.hot_columns(sparse_matrix.column_indices, sparse_matrix.n, row_bytes)
         hot = cache[row_bytes]

@@ -16,6 +16,7 @@
 //   * k_version may also be 64.
 //   * spmm_forward and hot_columns are new: the reference has no Python entry for SpMM.
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
@@ -33,6 +34,12 @@ namespace {
     RODE_CHECK_CONTIGUOUS(x)
 #define RODE_CHECK_FLOAT(x) TORCH_CHECK((x).dtype() == torch::kFloat32, #x " must be float32")
 #define RODE_CHECK_INT(x) TORCH_CHECK((x).dtype() == torch::kInt32, #x " must be int32")
+
+// A fresh CUDA tensor straight from the allocator: a small call's time is host work, and the dispatcher's part
+// of torch::empty is a fifth of it.
+torch::Tensor empty_cuda(at::IntArrayRef sizes, at::ScalarType dtype, const c10::Device &device) {
+    return at::detail::empty_cuda(sizes, dtype, device, c10::nullopt);
+}
 
 void check_status(int status) { TORCH_CHECK(status == RODE_OK, "rode_b200: ", rode_last_error()); }
 
@@ -105,7 +112,7 @@ torch::Tensor py_sddmm_forward(torch::Tensor block_indices, torch::Tensor residu
     const c10::cuda::CUDAGuard guard(values.device());
     if (m1 == 0 && m2 == 0) return torch::zeros({values.size(0)}, values.options());
     // every stored entry lies in a block segment or a residue row, so every element is written
-    torch::Tensor out = torch::empty({values.size(0)}, values.options());
+    torch::Tensor out = empty_cuda({values.size(0)}, torch::kFloat32, values.device());
     const cudaStream_t s = at::cuda::getCurrentCUDAStream(values.device().index()).stream();
     check_status(rode_sddmm_f32(m1, m2, n, k, block_indices.data_ptr<int>(), residue_indices.data_ptr<int>(),
                                 st_offsets.data_ptr<int>(), row_offsets.data_ptr<int>(), column_indices.data_ptr<int>(),
@@ -163,11 +170,17 @@ torch::Tensor py_spmm_forward(torch::Tensor block_indices, torch::Tensor residue
 
     const c10::cuda::CUDAGuard guard(values.device());
     if (m1 == 0 && m2 == 0) return torch::zeros({m, n}, dense.options());
-    torch::Tensor out = torch::empty({m, n}, dense.options());  // every row is written
+    torch::Tensor out = empty_cuda({m, n}, dense.scalar_type(), dense.device());  // every row is written
+    // Without segments the workspace would hold the claim counters of the persistent residue kernel only, which
+    // lists of less than half a million rows do not use.
     size_t ws_bytes = 0;
-    check_status(rode_spmm_workspace_bytes(m1, n, static_cast<int>(dense.element_size()), &ws_bytes));
-    torch::Tensor ws = torch::empty({static_cast<long long>(std::max<size_t>(ws_bytes, 16))},
-                                    dense.options().dtype(torch::kUInt8));
+    torch::Tensor ws;
+    void *ws_ptr = nullptr;
+    if (m1 > 0 || m >= 1 << 19) {
+        check_status(rode_spmm_workspace_bytes(m1, n, static_cast<int>(dense.element_size()), &ws_bytes));
+        ws = empty_cuda({static_cast<long long>(ws_bytes)}, torch::kUInt8, dense.device());
+        ws_ptr = ws.data_ptr();
+    }
     const unsigned *hot = nullptr;
     if (hot_columns.has_value()) {
         RODE_CHECK_INPUT(*hot_columns);
@@ -181,12 +194,12 @@ torch::Tensor py_spmm_forward(torch::Tensor block_indices, torch::Tensor residue
         check_status(rode_spmm_f32_all(m, m1, k, n, values.data_ptr<float>(), column_indices.data_ptr<int>(),
                                        row_offsets.data_ptr<int>(), block_indices.data_ptr<int>(),
                                        st_offsets.data_ptr<int>(), dense.data_ptr<float>(), out.data_ptr<float>(),
-                                       ws.data_ptr(), ws_bytes, hot, s, s));
+                                       ws_ptr, ws_bytes, hot, s, s));
     else
         check_status(rode_spmm_f64_all(m, m1, k, n, values.data_ptr<double>(), column_indices.data_ptr<int>(),
                                        row_offsets.data_ptr<int>(), block_indices.data_ptr<int>(),
                                        st_offsets.data_ptr<int>(), dense.data_ptr<double>(), out.data_ptr<double>(),
-                                       ws.data_ptr(), ws_bytes, hot, s, s));
+                                       ws_ptr, ws_bytes, hot, s, s));
     return out;
 }
 
