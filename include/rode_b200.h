@@ -164,15 +164,16 @@ int rode_spmm_f64(int m1, int m2, int k, int n, const double *values, const int 
 /* SpMM into a C of any contents: the same product, and every one of the M rows of C is written, those
  * without a nonzero with zeros, so the caller does not zero-fill C first (for a result that is as
  * large as the dense operand that saves one of the passes over it).  Takes no residue list: the
- * residue kernel goes through the rows themselves.  hot_columns: null, or a bitmap of rode_hot_columns
+ * residue kernel goes through the rows themselves.  nnz: the number of nonzeros, from which the call picks
+ * kernels for short rows and small products, or -1 where the caller does not have it at hand.  hot_columns: null, or a bitmap of rode_hot_columns
  * (below).  With stream1 == stream2 the kernels run as a chain of programmatic dependents, side by
  * side as on two streams.  Everything else as for rode_spmm_f32 / _f64.  No counterpart in the reference. */
-int rode_spmm_f32_all(int M, int m1, int k, int n, const float *values, const int *column_indices,
+int rode_spmm_f32_all(int M, int m1, int k, int n, long long nnz, const float *values, const int *column_indices,
                       const int *row_offsets, const int *block_r_ind, const int *st_off, const float *B,
                       float *C, void *workspace, size_t workspace_bytes, const unsigned *hot_columns,
                       rode_stream_t stream1, rode_stream_t stream2);
 
-int rode_spmm_f64_all(int M, int m1, int k, int n, const double *values, const int *column_indices,
+int rode_spmm_f64_all(int M, int m1, int k, int n, long long nnz, const double *values, const int *column_indices,
                       const int *row_offsets, const int *block_r_ind, const int *st_off, const double *B,
                       double *C, void *workspace, size_t workspace_bytes, const unsigned *hot_columns,
                       rode_stream_t stream1, rode_stream_t stream2);

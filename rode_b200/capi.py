@@ -83,7 +83,7 @@ def load() -> ctypes.CDLL:
     lib.rode_hot_columns.argtypes = [ctypes.c_longlong, ci, vp, sz, sz, vp, vp, sz, vp]
     lib.rode_spmm_f32_hot.argtypes = [ci, ci, ci, ci, vp, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp, vp, vp]
     lib.rode_spmm_f64_hot.argtypes = lib.rode_spmm_f32_hot.argtypes
-    lib.rode_spmm_f32_all.argtypes = [ci, ci, ci, ci, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp, vp, vp]
+    lib.rode_spmm_f32_all.argtypes = [ci, ci, ci, ci, ctypes.c_longlong, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp, vp, vp]
     lib.rode_spmm_f64_all.argtypes = lib.rode_spmm_f32_all.argtypes
     for name in ("rode_preprocess_workspace_bytes", "rode_preprocess_capacity", "rode_preprocess",
                  "rode_preprocess_noalloc", "rode_preprocess_cpu", "rode_spmm_workspace_bytes", "rode_spmm_f32", "rode_spmm_f64",
@@ -250,10 +250,10 @@ def spmm_raw(dtype, m1, m2, k, n, values, col, row_ptr, blk, res, st, B, C, work
 
 
 def spmm_all_raw(dtype, M, m1, k, n, values, col, row_ptr, blk, st, B, C, workspace, workspace_bytes, stream1=None,
-                 stream2=None, hot=None) -> None:
+                 stream2=None, hot=None, nnz=-1) -> None:
     """rode_spmm_f32_all / _f64_all on raw device addresses: C may hold anything, every row is written."""
     fn = load().rode_spmm_f32_all if dtype == torch.float32 else load().rode_spmm_f64_all
-    check(fn(M, m1, k, n, values, col, row_ptr, blk, st, B, C, workspace, workspace_bytes, hot, _stream(stream1),
+    check(fn(M, m1, k, n, nnz, values, col, row_ptr, blk, st, B, C, workspace, workspace_bytes, hot, _stream(stream1),
              _stream(stream2)))
 
 
@@ -320,7 +320,7 @@ def spmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torch
         if whole:
             spmm_all_raw(B.dtype, M, meta.m1, k, n, values.data_ptr(), col.data_ptr(), row_ptr.data_ptr(),
                          meta.block_r_ind.data_ptr(), meta.st_off.data_ptr(), B.data_ptr(), C.data_ptr(),
-                         _ptr(workspace), ws_bytes, s1, s2, hot=_ptr(hot))
+                         _ptr(workspace), ws_bytes, s1, s2, hot=_ptr(hot), nnz=values.numel())
             return C
         spmm_raw(B.dtype, meta.m1, meta.m2, k, n, values.data_ptr(), col.data_ptr(), row_ptr.data_ptr(),
                  meta.block_r_ind.data_ptr(), meta.residue_r_ind.data_ptr(), meta.st_off.data_ptr(), B.data_ptr(),

@@ -266,23 +266,9 @@ __device__ __forceinline__ void ld_shared_run(const double *p, double (&out)[U])
 }
 
 // Streaming read of CSR data (touched once): do not let it displace dense rows in L1.
-// (Read-only loads: the compiler may then move them across the stores of results, which it cannot know to be
-// to another array once a kernel's body is a function of its own.)
-__device__ __forceinline__ int ld_stream(const int *p) {
-    int v;
-    asm("ld.global.cs.nc.b32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ float ld_stream(const float *p) {
-    float v;
-    asm("ld.global.cs.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ double ld_stream(const double *p) {
-    double v;
-    asm("ld.global.cs.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
-    return v;
-}
+__device__ __forceinline__ int ld_stream(const int *p) { return __ldcs(p); }
+__device__ __forceinline__ float ld_stream(const float *p) { return __ldcs(p); }
+__device__ __forceinline__ double ld_stream(const double *p) { return __ldcs(p); }
 
 // Streaming store of results (written once, not read again by this kernel).
 template <typename V>
@@ -309,9 +295,11 @@ __device__ __forceinline__ unsigned group_mask(int lane) {
 }
 
 // ---------------------------------------------------------------------------------------
-// The kernels of one call as a chain of programmatic dependents on one stream: each grid lets the next
+// The kernels of one call as a chain of programmatic dependents on one stream: the block grid lets the next
 // one start as soon as all its own CTAs have started (chain_begin), so the chain runs like grids on
-// several streams but costs one launch call per grid and no events.  A grid that completes lets the
+// several streams but costs one launch call per grid and no events.  (The row grids give no early start: the
+// fix-up's CTAs would wait in their slots, R-MAT 21 N = 64 0.96 ms instead of 0.74, Zipf 671,008 rows N = 64 0.27
+// instead of 0.21.)  A grid that completes lets the
 // stream move on, so one warp or CTA of every grid that has nothing (more) to do waits for the grid
 // before it (chain_wait): no grid of the chain completes before all earlier ones have completed and
 // flushed their stores.  In the kernels whose code generation suffers from a common exit (the per-row

@@ -357,7 +357,7 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
                                                                 rhs, out, nullptr, row_vecs_arg);
         bundle -= m1;
     }
-    chain_begin();
+    if constexpr (kSegments) chain_begin();
     const long long item0 = static_cast<long long>(bundle) * items_per_warp;
     if (item0 >= n_items) return chain_wait();  // the CTA behind the items
 

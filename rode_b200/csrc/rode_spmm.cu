@@ -465,7 +465,6 @@ spmm_rows(int m2, int rows_per_group, int n, const T *__restrict__ values,
     constexpr int NB = (L + U - 1) / U;  // batches per L-nonzero chunk
     constexpr int kAlign = 4;            // vec_len of the preprocessing
     constexpr int kBlockK = 32;          // k_block of the preprocessing
-    chain_begin();
     const int lane = threadIdx.x & 31;
     const int l = lane % L;
     const unsigned gmask = group_mask<L>(lane);
@@ -619,7 +618,7 @@ spmm_rows(int m2, int rows_per_group, int n, const T *__restrict__ values,
 }
 
 // ---------------------------------------------------------------------------------------
-// Residue rows without a block part, one lane group (L lanes x VPL vectors) per row.  Used
+// Residue rows without a block part, one lane group (L lanes x VPL vectors) per R neighbouring rows.  Used
 // where a warp holds several groups: there the groups would run different entry streams in
 // spmm_rows and diverge, which measured slower (stencil N = 64: 1.43 ms against 0.93 ms),
 // while for 32-lane groups the batched kernel wins (R-MAT N = 128: 327 us against 770 us).
@@ -632,7 +631,7 @@ constexpr int kRowsCtaThreads = RODE_SPMM_ROWS_CTA;
 #define RODE_SPMM_WIDE_ROWS_WAVES 2
 #endif
 
-template <typename T, int VB, int L, int VPL, bool kRagged>
+template <typename T, int VB, int L, int VPL, int R, bool kRagged>
 __global__ void __launch_bounds__(kRowsCtaThreads, 1024 / kRowsCtaThreads)  // 64 registers: 32 warps per SM
 spmm_rows_simple(int m2, int n, const T *__restrict__ values, const int *__restrict__ column_indices,
                  const int *__restrict__ row_offsets, const int *__restrict__ residue_r_ind,
@@ -643,40 +642,46 @@ spmm_rows_simple(int m2, int n, const T *__restrict__ values, const int *__restr
     constexpr int U = (kInFlight < L) ? kInFlight : L;
     constexpr int kAlign = 4;    // vec_len of the preprocessing
     constexpr int kBlockK = 32;  // k_block of the preprocessing
-    chain_begin();
     if (blockIdx.x == gridDim.x - 1) return chain_wait();  // the CTA behind the rows
-    const long long item_ll = (static_cast<long long>(blockIdx.x) * kRowsCtaThreads + threadIdx.x) / L;
-    if (item_ll >= m2) return;
-    const int item = static_cast<int>(item_ll);
     const int lane = threadIdx.x & 31;
     const int l = lane % L;
     const unsigned gmask = group_mask<L>(lane);
-
-    const int row = residue_r_ind != nullptr ? __ldg(residue_r_ind + item) : item;
-    const int begin = __ldg(row_offsets + row);
-    const int end = __ldg(row_offsets + row + 1);
-    // aligned length >= k_block: a block part exists and its last segment took the tail;
-    // list form, no nonzero: the row stays as the caller zero-filled it (all rows: zeros are stored below)
-    if (end - begin + (begin % kAlign) >= kBlockK || (end == begin && residue_r_ind != nullptr)) return;
-
+    const long long item0 = ((static_cast<long long>(blockIdx.x) * kRowsCtaThreads + threadIdx.x) / L) * R;
+    int row[R], begin[R], end[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        row[r] = -1;
+        begin[r] = end[r] = 0;
+        if (item0 + r < m2) row[r] = residue_r_ind != nullptr ? __ldg(residue_r_ind + item0 + r) : static_cast<int>(item0 + r);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        if (row[r] >= 0) {
+            begin[r] = __ldg(row_offsets + row[r]);
+            end[r] = __ldg(row_offsets + row[r] + 1);
+        }
+    // Lane l keeps nonzero l of a chunk of L; the pair is fetched one chunk ahead, so that the
+    // fetch overlaps the gathers of the current chunk.
+    int c_first[R];
+    T v_first[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        // aligned length >= k_block: a block part exists and its last segment took the tail;
+        // list form, no nonzero: the row stays as the caller zero-filled it (all rows: zeros are stored below)
+        if (end[r] - begin[r] + (begin[r] % kAlign) >= kBlockK || (end[r] == begin[r] && residue_r_ind != nullptr)) row[r] = -1;
+        c_first[r] = 0;
+        v_first[r] = T(0);
+        if (row[r] >= 0 && begin[r] + l < end[r]) {
+            c_first[r] = ld_stream(column_indices + begin[r] + l);
+            v_first[r] = ld_stream(values + begin[r] + l);
+        }
+    }
     // (this kernel keeps the 64-bit index form of the dense-row address: the 32 x 32 -> 64 bit form of
     // the other kernels measured 2.7 % slower here, stencil N = 64 0.692 -> 0.711 ms)
     const size_t row_vecs = static_cast<size_t>(n) / kLen;
     const size_t col_vec = static_cast<size_t>(blockIdx.y) * L * VPL + l;
     const V *b_lane = reinterpret_cast<const V *>(B) + col_vec;
     auto inside = [&](int v) { return !kRagged || col_vec + v * L < row_vecs; };
-
-    V acc[VPL];
-#pragma unroll
-    for (int v = 0; v < VPL; ++v) acc[v] = vzero(static_cast<V *>(nullptr));
-    // Lane l keeps nonzero l of a chunk of L; the pair is fetched one chunk ahead, so that the
-    // fetch overlaps the gathers of the current chunk.
-    int c_nxt = 0;
-    T v_nxt = T(0);
-    if (begin + l < end) {
-        c_nxt = ld_stream(column_indices + begin + l);
-        v_nxt = ld_stream(values + begin + l);
-    }
     // chunk staging in shared memory as in spmm_block (one region of L pairs per lane group; the
     // groups of a warp run rows of different lengths, so they synchronise by group)
     constexpr bool kStage = RODE_SPMM_PAIRS_IN_SMEM != 0 && (L % U == 0) && (U % 4 == 0);
@@ -684,56 +689,66 @@ spmm_rows_simple(int m2, int n, const T *__restrict__ values, const int *__restr
     __shared__ __align__(16) T s_val[2][kStage ? kRowsCtaThreads : 1];
     const int stage_base = (threadIdx.x / L) * L;
     int stage_buf = 0;
-    for (int base = begin; base < end; base += L) {
-        const int c = c_nxt;
-        const T val = v_nxt;
-        const int e = base + L + l;
-        c_nxt = 0;
-        v_nxt = T(0);
-        if (e < end) {
-            c_nxt = ld_stream(column_indices + e);
-            v_nxt = ld_stream(values + e);
-        }
-        const int cnt = min(L, end - base);
-        if constexpr (kStage) {
-            s_col[stage_buf][stage_base + l] = c;
-            s_val[stage_buf][stage_base + l] = val;
-            __syncwarp(gmask);
-        }
 #pragma unroll
-        for (int t0 = 0; t0 < L; t0 += U) {
-            if (t0 >= cnt) break;
-            int cc[U];
-            T vv[U];
-            V bb[U][VPL];
+    for (int r = 0; r < R; ++r) {
+        if (row[r] < 0) continue;
+        V acc[VPL];
+#pragma unroll
+        for (int v = 0; v < VPL; ++v) acc[v] = vzero(static_cast<V *>(nullptr));
+        int c_nxt = c_first[r];
+        T v_nxt = v_first[r];
+        for (int base = begin[r]; base < end[r]; base += L) {
+            const int c = c_nxt;
+            const T val = v_nxt;
+            const int e = base + L + l;
+            c_nxt = 0;
+            v_nxt = T(0);
+            if (e < end[r]) {
+                c_nxt = ld_stream(column_indices + e);
+                v_nxt = ld_stream(values + e);
+            }
+            const int cnt = min(L, end[r] - base);
             if constexpr (kStage) {
-                ld_shared_run<U>(&s_col[stage_buf][stage_base + t0], cc);
-                ld_shared_run<U>(&s_val[stage_buf][stage_base + t0], vv);
-            } else {
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    cc[u] = __shfl_sync(gmask, c, t0 + u, L);
-                    vv[u] = __shfl_sync(gmask, val, t0 + u, L);
-                }
+                s_col[stage_buf][stage_base + l] = c;
+                s_val[stage_buf][stage_base + l] = val;
+                __syncwarp(gmask);
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u)
+            for (int t0 = 0; t0 < L; t0 += U) {
+                if (t0 >= cnt) break;
+                int cc[U];
+                T vv[U];
+                V bb[U][VPL];
+                if constexpr (kStage) {
+                    ld_shared_run<U>(&s_col[stage_buf][stage_base + t0], cc);
+                    ld_shared_run<U>(&s_val[stage_buf][stage_base + t0], vv);
+                } else {
 #pragma unroll
-                for (int v = 0; v < VPL; ++v) {
-                    bb[u][v] = vzero(static_cast<V *>(nullptr));
-                    if (t0 + u < cnt && inside(v))
-                        bb[u][v] = ld_dense(b_lane + static_cast<size_t>(cc[u]) * row_vecs + v * L);
+                    for (int u = 0; u < U; ++u) {
+                        cc[u] = __shfl_sync(gmask, c, t0 + u, L);
+                        vv[u] = __shfl_sync(gmask, val, t0 + u, L);
+                    }
                 }
 #pragma unroll
-            for (int u = 0; u < U; ++u)
+                for (int u = 0; u < U; ++u)
 #pragma unroll
-                for (int v = 0; v < VPL; ++v) vfma(acc[v], vv[u], bb[u][v]);
+                    for (int v = 0; v < VPL; ++v) {
+                        bb[u][v] = vzero(static_cast<V *>(nullptr));
+                        if (t0 + u < cnt && inside(v))
+                            bb[u][v] = ld_dense(b_lane + static_cast<size_t>(cc[u]) * row_vecs + v * L);
+                    }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int v = 0; v < VPL; ++v) vfma(acc[v], vv[u], bb[u][v]);
+            }
+            stage_buf ^= 1;
         }
-        stage_buf ^= 1;
-    }
 #pragma unroll
-    for (int v = 0; v < VPL; ++v)
-        if (inside(v)) st_stream(reinterpret_cast<V *>(C) + static_cast<size_t>(row) * row_vecs + col_vec + v * L, acc[v]);
+        for (int v = 0; v < VPL; ++v)
+            if (inside(v))
+                st_stream(reinterpret_cast<V *>(C) + static_cast<size_t>(row[r]) * row_vecs + col_vec + v * L, acc[v]);
+    }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -754,7 +769,6 @@ spmm_rows_wide(int m2, int n, const T *__restrict__ values, const int *__restric
     constexpr int kAlign = 4;    // vec_len of the preprocessing
     constexpr int kBlockK = 32;  // k_block of the preprocessing
     constexpr unsigned kFull = 0xffffffffu;
-    chain_begin();
     if (blockIdx.x == gridDim.x - 1) return chain_wait();  // the CTA behind the rows
     const int item = blockIdx.x * kSmallGridWarps + (threadIdx.x >> 5);
     if (item >= m2) return;
@@ -823,14 +837,15 @@ spmm_rows_wide(int m2, int n, const T *__restrict__ values, const int *__restric
 
 template <typename T, int VB, int L, int VPL, bool kRagged>
 int launch_rows(int m2, int n, const T *values, const int *col, const int *row_offsets, const int *residue_r_ind,
-                const T *B, T *C, int *counters, bool chained, bool counters_clear, cudaStream_t s2);
+                const T *B, T *C, int *counters, bool chained, bool counters_clear, long long nnz,
+                cudaStream_t s2);
 
 // Block kernel of shape (VB bytes per load, L lanes, VPL loads per lane) and residue-row kernel
 // of shape (RVB, RL, RVPL); both cover the same column tile.
 template <typename T, int VB, int L, int VPL, int RVB, int RL, int RVPL, bool kRagged>
 int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, const int *row_offsets,
                  const int *block_r_ind, const int *residue_r_ind, const int *st_off, const T *B, T *C,
-                 T *partial, int *counters, const unsigned *hot, cudaStream_t s1, cudaStream_t s2) {
+                 T *partial, int *counters, const unsigned *hot, long long nnz, cudaStream_t s1, cudaStream_t s2) {
     static_assert(L * VPL * VB == RL * RVPL * RVB, "block and residue kernels must cover the same tile");
     constexpr int kTileWidth = L * VPL * VecB<T, VB>::kLen;
     constexpr int U = kLoadsInFlight * 16 / VB / VPL;            // rows per batch, large grids
@@ -888,7 +903,7 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
     // they are a plain launch.
     if (m2 > 0) {
         if (int rc = launch_rows<T, RVB, RL, RVPL, kRagged>(m2, n, values, col, row_offsets, residue_r_ind, B, C, counters,
-                                                            chained, counters_clear, s2))
+                                                            chained, counters_clear, nnz, s2))
             return rc;
     }
     if (m1 > 0) {
@@ -906,7 +921,8 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
 
 template <typename T, int VB, int L, int VPL, bool kRagged>
 int launch_rows(int m2, int n, const T *values, const int *col, const int *row_offsets, const int *residue_r_ind,
-                const T *B, T *C, int *counters, bool chained, bool counters_clear, cudaStream_t s2) {
+                const T *B, T *C, int *counters, bool chained, bool counters_clear, long long nnz,
+                cudaStream_t s2) {
     constexpr int kTileWidth = L * VPL * VecB<T, VB>::kLen;
     const unsigned tiles = static_cast<unsigned>(kRagged ? (n + kTileWidth - 1) / kTileWidth : n / kTileWidth);
     if constexpr (VB == 16 && L == 32 && VPL == 1) {
@@ -935,10 +951,21 @@ int launch_rows(int m2, int n, const T *values, const int *col, const int *row_o
         RODE_CUDA_TRY(launch_chained(spmm_rows_wide<T, VB, L, VPL, kRagged>, grid, dim3(32 * kSmallGridWarps), s2, chained, m2,
                                      n, values, col, row_offsets, residue_r_ind, B, C));
     } else {
-        constexpr int kRowsPerCta = kRowsCtaThreads / L;
-        const dim3 grid((m2 + kRowsPerCta - 1) / kRowsPerCta + 1, tiles);
-        RODE_CUDA_TRY(launch_chained(spmm_rows_simple<T, VB, L, VPL, kRagged>, grid, dim3(kRowsCtaThreads), s2, chained, m2, n,
-                                     values, col, row_offsets, residue_r_ind, B, C));
+        // Two rows per lane group where rows are short on average (and their number is known): both rows' bounds and
+        // first columns are then fetched together, and a short row's life is that chain of loads.  Zipf 671,008
+        // rows N = 64 206 -> 191 us, 3.2 M rows N = 32 646 -> 610, R-MAT 21 N = 64 741 -> 694; long even rows lose it again
+        // to the longer life of a warp (stencil N = 96 1.33 -> 1.50 ms, 27 per row; Pareto 2^20, 32 per row, 5 %).
+        auto launch = [&](auto two) {
+            constexpr int R = decltype(two)::value ? 2 : 1;
+            constexpr int kRowsPerCta = R * kRowsCtaThreads / L;
+            const dim3 grid(static_cast<unsigned>((static_cast<long long>(m2) + kRowsPerCta - 1) / kRowsPerCta + 1), tiles);
+            return launch_chained(spmm_rows_simple<T, VB, L, VPL, R, kRagged>, grid, dim3(kRowsCtaThreads), s2, chained, m2, n,
+                                  values, col, row_offsets, residue_r_ind, B, C);
+        };
+        if (nnz >= 0 && nnz < 20LL * m2)
+            RODE_CUDA_TRY(launch(std::true_type{}));
+        else
+            RODE_CUDA_TRY(launch(std::false_type{}));
     }
     RODE_CHECK_LAUNCH("rode::spmm_rows");
     return RODE_OK;
@@ -953,7 +980,7 @@ template <typename T>
 int spmm(int m1, int m2, int k, int n, const T *values, const int *col, const int *row_offsets,
          const int *block_r_ind, const int *residue_r_ind, const int *st_off, const T *B, T *C, void *workspace,
          size_t workspace_bytes, const unsigned *hot, rode_stream_t stream1, rode_stream_t stream2,
-         bool all_rows = false) {
+         bool all_rows = false, long long nnz = -1) {
     constexpr int kLen = Vec16<T>::kLen;
     if (m1 < 0 || m2 < 0 || n <= 0) return fail(RODE_ERR_INVALID_ARGUMENT, "spmm: m1, m2 >= 0 and n > 0 required");
     if (hot != nullptr && k <= 0)
@@ -989,14 +1016,14 @@ int spmm(int m1, int m2, int k, int n, const T *values, const int *col, const in
 #define RODE_LAUNCH16(shape, rows_shape) RODE_LAUNCH16R(shape, rows_shape, false)
 #define RODE_LAUNCH16R(shape, rows_shape, ragged)                                                               \
     launch_shape<T, 16, (shape) / 100, (shape) % 100, 16, (rows_shape) / 100, (rows_shape) % 100, ragged>(      \
-        m1, m2, k, n, values, col, row_offsets, block_r_ind, residue_r_ind, st_off, B, C, partial, counters, hot, stream1, \
-        stream2)
+        m1, m2, k, n, values, col, row_offsets, block_r_ind, residue_r_ind, st_off, B, C, partial, counters, hot, nnz,     \
+        stream1, stream2)
 #define RODE_LAUNCH32(shape, rows_shape, rows_bytes)                                                             \
     launch_shape<T, 32, wide_lanes(shape), wide_vpl(shape), rows_bytes,                                          \
                  (rows_bytes) == 32 ? wide_lanes(rows_shape) : (rows_shape) / 100,                               \
                  (rows_bytes) == 32 ? wide_vpl(rows_shape) : (rows_shape) % 100, false>(                         \
-        m1, m2, k, n, values, col, row_offsets, block_r_ind, residue_r_ind, st_off, B, C, partial, counters, hot, stream1, \
-        stream2)
+        m1, m2, k, n, values, col, row_offsets, block_r_ind, residue_r_ind, st_off, B, C, partial, counters, hot, nnz,     \
+        stream1, stream2)
     const int vecs = n / kLen;
     // Widths the tiles do not divide (any other multiple of 4 columns; the reference has none of
     // them): the narrowest shape that covers the row, or 512-byte tiles with a partly empty last
@@ -1027,7 +1054,7 @@ int spmm(int m1, int m2, int k, int n, const T *values, const int *col, const in
     if constexpr (RODE_SPMM_TILE8_WIDE_LOADS != 0) {
         if (aligned_to(B, 32) && aligned_to(C, 32) && aligned_to(workspace, 32))
             return launch_shape<T, 32, 4, 1, 32, 4, 1, false>(m1, m2, k, n, values, col, row_offsets, block_r_ind,
-                                                              residue_r_ind, st_off, B, C, partial, counters, hot,
+                                                              residue_r_ind, st_off, B, C, partial, counters, hot, nnz,
                                                               stream1, stream2);
     }
     return RODE_LAUNCH16(RODE_SPMM_SHAPE_8, RODE_SPMM_ROWS_SHAPE_8);
@@ -1083,20 +1110,20 @@ int rode_spmm_f64_hot(int m1, int m2, int k, int n, const double *values, const 
                               st_off, B, C, workspace, workspace_bytes, hot_columns, stream1, stream2);
 }
 
-int rode_spmm_f32_all(int M, int m1, int k, int n, const float *values, const int *column_indices,
+int rode_spmm_f32_all(int M, int m1, int k, int n, long long nnz, const float *values, const int *column_indices,
                       const int *row_offsets, const int *block_r_ind, const int *st_off, const float *B, float *C,
                       void *workspace, size_t workspace_bytes, const unsigned *hot_columns, rode_stream_t stream1,
                       rode_stream_t stream2) {
     return rode::spmm<float>(m1, M, k, n, values, column_indices, row_offsets, block_r_ind, nullptr, st_off, B, C,
-                             workspace, workspace_bytes, hot_columns, stream1, stream2, /*all_rows=*/true);
+                             workspace, workspace_bytes, hot_columns, stream1, stream2, /*all_rows=*/true, nnz);
 }
 
-int rode_spmm_f64_all(int M, int m1, int k, int n, const double *values, const int *column_indices,
+int rode_spmm_f64_all(int M, int m1, int k, int n, long long nnz, const double *values, const int *column_indices,
                       const int *row_offsets, const int *block_r_ind, const int *st_off, const double *B, double *C,
                       void *workspace, size_t workspace_bytes, const unsigned *hot_columns, rode_stream_t stream1,
                       rode_stream_t stream2) {
     return rode::spmm<double>(m1, M, k, n, values, column_indices, row_offsets, block_r_ind, nullptr, st_off, B, C,
-                              workspace, workspace_bytes, hot_columns, stream1, stream2, /*all_rows=*/true);
+                              workspace, workspace_bytes, hot_columns, stream1, stream2, /*all_rows=*/true, nnz);
 }
 
 }  // extern "C"

@@ -191,12 +191,12 @@ torch::Tensor py_spmm_forward(torch::Tensor block_indices, torch::Tensor residue
     }
     const cudaStream_t s = at::cuda::getCurrentCUDAStream(values.device().index()).stream();
     if (dense.dtype() == torch::kFloat32)
-        check_status(rode_spmm_f32_all(m, m1, k, n, values.data_ptr<float>(), column_indices.data_ptr<int>(),
+        check_status(rode_spmm_f32_all(m, m1, k, n, values.size(0), values.data_ptr<float>(), column_indices.data_ptr<int>(),
                                        row_offsets.data_ptr<int>(), block_indices.data_ptr<int>(),
                                        st_offsets.data_ptr<int>(), dense.data_ptr<float>(), out.data_ptr<float>(),
                                        ws_ptr, ws_bytes, hot, s, s));
     else
-        check_status(rode_spmm_f64_all(m, m1, k, n, values.data_ptr<double>(), column_indices.data_ptr<int>(),
+        check_status(rode_spmm_f64_all(m, m1, k, n, values.size(0), values.data_ptr<double>(), column_indices.data_ptr<int>(),
                                        row_offsets.data_ptr<int>(), block_indices.data_ptr<int>(),
                                        st_offsets.data_ptr<int>(), dense.data_ptr<double>(), out.data_ptr<double>(),
                                        ws_ptr, ws_bytes, hot, s, s));

@@ -41,18 +41,20 @@ def test_every_row_is_written(oracle_cpu, n, rows, dtype):
         ws = torch.empty(capi.spmm_workspace_bytes(meta.m1, n, Bd.element_size()), dtype=torch.uint8, device="cuda")
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
-        for streams in ((None, None), (None, side)):    # one chain; two streams
+        # one chain; two streams; the kernels for a known number of nonzeros
+        for streams, nnz in (((None, None), -1), ((None, side), -1), ((None, None), A.nnz)):
             buf = torch.full((A.m + 2, n), float("nan"), dtype=dtype, device="cuda")
             torch.cuda.synchronize()
             C = buf[1:-1]
             capi.spmm_all_raw(dtype, A.m, meta.m1, A.n, n, vd.data_ptr(), d.col.data_ptr(), d.row_ptr.data_ptr(),
                               meta.block_r_ind.data_ptr(), meta.st_off.data_ptr(), Bd.data_ptr(), C.data_ptr(),
-                              ws.data_ptr(), ws.numel(), *streams)
+                              ws.data_ptr(), ws.numel(), *streams, nnz=nnz)
             torch.cuda.synchronize()
             assert_close_to_truth(C.cpu().numpy(), truth, scale, f"n={n} rows={rows} seg={seg}")
             assert torch.isnan(buf[0]).all() and torch.isnan(buf[-1]).all()
             assert bool((C[torch.from_numpy(np.diff(rp) == 0).cuda()] == 0).all())
             # the list form, into a zero-filled C, gives the same bits
-            Z = torch.zeros_like(C)
-            capi.spmm(meta, d.row_ptr, d.col, vd, Bd, C=Z, workspace=ws)
-            assert torch.equal(Z, C)
+            if nnz < 0:
+                Z = torch.zeros_like(C)
+                capi.spmm(meta, d.row_ptr, d.col, vd, Bd, C=Z, workspace=ws)
+                assert torch.equal(Z, C)
