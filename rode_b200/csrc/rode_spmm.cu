@@ -308,6 +308,197 @@ spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ 
 }
 
 // ---------------------------------------------------------------------------------------
+// Segments and rows of a small matrix in one launch: its kernels take a few microseconds each, less than the
+// host needs to launch them.  A CTA of four warps takes four segments, far apart in the list (neighbours are
+// often pieces of one long row), and splits their chunks of 32 nonzeros evenly over the warps, whatever the
+// segments' lengths; a warp writes its partial row of every segment it touched to shared memory, and warp s adds
+// those of segment s in a fixed order.  The CTAs behind the segments take the rows without a block part (list or
+// all rows, as in the residue kernels), a warp per row: fewer than 32 nonzeros, so one chunk.
+// SpMM calls through the C ABI, back to back, us: Bernoulli 4096^2 N = 32 15.3 -> 11.9, 2000^2 11.3 -> 8.2, R-MAT 12 11.4
+// -> 8.9.  As the kernel of larger grids it is slower than one warp per segment with the whole chunk in flight
+// (Zipf 65536 N = 128 45 -> 51 us, R-MAT 19 as long as the persistent grids' threshold 262 -> 306).
+constexpr int kOneLaunchWarps = 4;
+template <typename T, int VB, int L, int VPL, int U, bool kRagged>
+__global__ void __launch_bounds__(32 * kOneLaunchWarps, 5)  // 96 registers
+spmm_one_launch(int m1, int seg_ctas, int rows, int n, const T *__restrict__ values, const int *__restrict__ column_indices,
+                const int *__restrict__ row_offsets, const int *__restrict__ block_r_ind, const int *__restrict__ st_off,
+                const int *__restrict__ residue_r_ind, const T *__restrict__ B, T *__restrict__ C, T *__restrict__ partial) {
+    using V = typename VecB<T, VB>::type;
+    constexpr int kLen = VecB<T, VB>::kLen;
+    constexpr int W = kOneLaunchWarps;
+    constexpr int G = 32 / L;   // lane groups, each takes every G-th nonzero of a chunk
+    constexpr int NB = L / U;   // batches per chunk
+    static_assert(L % U == 0, "a chunk is a whole number of batches");
+    constexpr unsigned kFull = 0xffffffffu;
+    constexpr int kAlign = 4;    // vec_len of the preprocessing
+    constexpr int kBlockK = 32;  // k_block of the preprocessing
+    __shared__ __align__(16) int s_col[W][2][32];
+    __shared__ __align__(16) T s_val[W][2][32];
+    __shared__ __align__(32) V s_acc[W][W][L * VPL];  // [warp][segment]
+    chain_begin();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane / L, l = lane % L;
+    const int stage_slot = (lane % G) * L + lane / G;
+    int stage_buf = 0;
+    const size_t row_vecs = static_cast<size_t>(n) / kLen;
+    const unsigned row_bytes = static_cast<unsigned>(n) * static_cast<unsigned>(sizeof(T));  // n < 2^21 elements
+    const size_t tile_vec = static_cast<size_t>(blockIdx.y) * L * VPL;
+    const V *b_lane = reinterpret_cast<const V *>(B) + tile_vec + l;
+    auto inside = [&](int v) { return !kRagged || tile_vec + l + v * L < row_vecs; };
+    V acc[VPL];
+    auto clear = [&]() {
+#pragma unroll
+        for (int v = 0; v < VPL; ++v) acc[v] = vzero(static_cast<V *>(nullptr));
+    };
+    // one chunk: lane t holds nonzero t < cnt
+    auto chunk = [&](int c, T val, int cnt) {
+        s_col[warp][stage_buf][stage_slot] = c;
+        s_val[warp][stage_buf][stage_slot] = val;
+        __syncwarp();
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            if (b * U * G >= cnt) break;  // warp-uniform
+            V buf[U][VPL];
+            T vv[U];
+            int cc[U];
+            ld_shared_run<U>(&s_col[warp][stage_buf][g * L + b * U], cc);
+            ld_shared_run<U>(&s_val[warp][stage_buf][g * L + b * U], vv);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int v = 0; v < VPL; ++v) {
+                    buf[u][v] = vzero(static_cast<V *>(nullptr));
+                    if ((b * U + u) * G + g < cnt && inside(v))
+                        buf[u][v] = ld_dense(dense_row(b_lane + v * L, static_cast<unsigned>(cc[u]), row_bytes));
+                }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int v = 0; v < VPL; ++v) vfma(acc[v], vv[u], buf[u][v]);
+        }
+        stage_buf ^= 1;
+    };
+    auto add_groups = [&]() {
+#pragma unroll
+        for (int v = 0; v < VPL; ++v)
+#pragma unroll
+            for (int w = L; w < 32; w <<= 1) vadd(acc[v], vshfl_xor(kFull, acc[v], w));
+    };
+
+    if (static_cast<int>(blockIdx.x) >= seg_ctas) {  // ---- a row per warp -----------------------------------
+        const int item = (static_cast<int>(blockIdx.x) - seg_ctas) * W + warp;
+        if (item >= rows) return;
+        const int row = residue_r_ind != nullptr ? __ldg(residue_r_ind + item) : item;
+        const int begin = __ldg(row_offsets + row), end = __ldg(row_offsets + row + 1);
+        // aligned length >= k_block: a block part exists and its last segment took the tail; list form, no
+        // nonzero: the row stays as the caller zero-filled it
+        if (end - begin + (begin % kAlign) >= kBlockK || (end == begin && residue_r_ind != nullptr)) return;
+        int c = 0;
+        T val = T(0);
+        if (begin + lane < end) {
+            c = ld_stream(column_indices + begin + lane);
+            val = ld_stream(values + begin + lane);
+        }
+        clear();
+        chunk(c, val, end - begin);
+        add_groups();
+        if (g == 0) {
+#pragma unroll
+            for (int v = 0; v < VPL; ++v)
+                if (inside(v))
+                    st_stream(reinterpret_cast<V *>(C) + static_cast<size_t>(row) * row_vecs + tile_vec + l + v * L, acc[v]);
+        }
+        return;
+    }
+
+    // ---- four segments, far apart: lane j < W of every warp holds segment j ---------------------------------
+    const int my_seg = static_cast<int>(blockIdx.x) + lane * seg_ctas;
+    int row = 0, off = 0, end = 0;
+    bool whole = false;
+    if (lane < W && my_seg < m1) {
+        row = __ldg(block_r_ind + my_seg);
+        off = __ldg(st_off + my_seg);
+        const int next = (my_seg + 1 < m1) ? __ldg(st_off + my_seg + 1) : INT_MAX;
+        const int row_begin = __ldg(row_offsets + row), row_end = __ldg(row_offsets + row + 1);
+        end = min(row_end, next);
+        whole = off == row_begin && next >= row_end;
+    }
+    const int chunks = (end - off + 31) / 32;
+    int incl = chunks;  // prefix sum over the segments
+#pragma unroll
+    for (int d = 1; d < W; d <<= 1) {
+        const int up = __shfl_up_sync(kFull, incl, d);
+        if (lane >= d) incl += up;
+    }
+    const int total = __shfl_sync(kFull, incl, W - 1);
+    const int per = (total + W - 1) / W;
+    const int q_end = min((warp + 1) * per, total);
+    struct Chunk {
+        int seg, base, end;
+    };
+    auto locate = [&](int q) {  // chunk q of the CTA
+        Chunk k;
+        k.seg = min(__popc(__ballot_sync(kFull, lane < W && incl <= q)), W - 1);
+        k.base = __shfl_sync(kFull, off - (incl - chunks) * 32, k.seg) + q * 32;
+        const int seg_end = __shfl_sync(kFull, end, k.seg);
+        k.end = q < q_end ? seg_end : 0;
+        return k;
+    };
+    auto fetch = [&](const Chunk &k, int &c, T &val) {
+        c = 0;
+        val = T(0);
+        if (k.base + lane < k.end) {
+            c = ld_stream(column_indices + k.base + lane);
+            val = ld_stream(values + k.base + lane);
+        }
+    };
+    auto flush = [&](int s) {
+        add_groups();
+        if (g == 0) {
+#pragma unroll
+            for (int v = 0; v < VPL; ++v) s_acc[warp][s][l + v * L] = acc[v];
+        }
+        clear();
+    };
+    int q = warp * per;
+    Chunk cur = locate(q), nxt = locate(q + 1);
+    int c_cur, c_nxt;
+    T v_cur, v_nxt;
+    fetch(cur, c_cur, v_cur);
+    fetch(nxt, c_nxt, v_nxt);
+    clear();
+    for (; q < q_end; ++q) {
+        const Chunk pre = locate(q + 2);
+        int c_pre;
+        T v_pre;
+        fetch(pre, c_pre, v_pre);
+        chunk(c_cur, v_cur, min(32, cur.end - cur.base));
+        if (q + 1 == q_end || nxt.seg != cur.seg) flush(cur.seg);  // warp-uniform
+        cur = nxt;
+        nxt = pre;
+        c_cur = c_nxt;
+        v_cur = v_nxt;
+        c_nxt = c_pre;
+        v_nxt = v_pre;
+    }
+    __syncthreads();
+    // warp s adds the partial rows of segment s, in the order of the warps
+    const int seg = static_cast<int>(blockIdx.x) + warp * seg_ctas;
+    if (seg >= m1) return;
+    const int first = __shfl_sync(kFull, incl - chunks, warp) / per, last = (__shfl_sync(kFull, incl, warp) - 1) / per;
+    const int out_row = __shfl_sync(kFull, row, warp);
+    const bool out_whole = __shfl_sync(kFull, static_cast<int>(whole), warp) != 0;
+    if (lane < L * VPL && (!kRagged || tile_vec + lane < row_vecs)) {
+        V sum = s_acc[first][warp][lane];
+        for (int w = first + 1; w <= last; ++w) vadd(sum, s_acc[w][warp][lane]);
+        if (out_whole)
+            st_stream(reinterpret_cast<V *>(C) + static_cast<size_t>(out_row) * row_vecs + tile_vec + lane, sum);
+        else
+            reinterpret_cast<V *>(partial)[static_cast<size_t>(seg) * row_vecs + tile_vec + lane] = sum;
+    }
+}
+
+// ---------------------------------------------------------------------------------------
 // Sums the workspace slots of every row that was cut into several segments, with fp64
 // accumulation and in an order that the code fixes, so the result is deterministic.
 //
@@ -855,6 +1046,7 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
     // ragged widths: the last tile is partly empty
     const unsigned tiles = static_cast<unsigned>(kRagged ? (n + kTileWidth - 1) / kTileWidth : n / kTileWidth);
     const bool chained = s1 == s2 && m1 > 0;
+    bool rows_done = false;
     bool counters_clear = false;  // the residue kernel's claim counters have been zeroed already
     if (m1 > 0) {
         // Fewer warps than two full waves of 32 per SM: the latency of the longest segment
@@ -889,6 +1081,18 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
                 launched = true;
             }
         }
+        // Up to 40 MB of gathers the host's launches are what a call waits for: one for segments and rows.  (Beyond
+        // that the separate kernels win back their launch: R-MAT 13 N = 128, 64 MB, 16.7 us with them, 18.7 in one.)
+        const bool one_launch = chained && nnz >= 0 && nnz * n * static_cast<long long>(sizeof(T)) <= 40LL << 20 &&
+                                small_grid && static_cast<long long>(m2) * tiles <= 2LL * 32 * sm_count();
+        if (one_launch) {
+            constexpr int UOne = 2 * U <= L ? 2 * U : L;
+            const int seg_ctas = (m1 + kOneLaunchWarps - 1) / kOneLaunchWarps;
+            const int row_ctas = (m2 + kOneLaunchWarps - 1) / kOneLaunchWarps;
+            spmm_one_launch<T, VB, L, VPL, UOne, kRagged><<<dim3(seg_ctas + row_ctas, tiles), 32 * kOneLaunchWarps, 0, s1>>>(
+                m1, seg_ctas, m2, n, values, col, row_offsets, block_r_ind, st_off, residue_r_ind, B, C, partial);
+            rows_done = launched = true;
+        }
         if (launched) {
         } else if (small_grid && USmall > U) {
             spmm_block<T, VB, L, VPL, USmall, kCtaWarps, false, false, kRagged><<<grid, kCtaThreads, 0, s1>>>(
@@ -901,7 +1105,7 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
     }
     // Rows: on the block kernel's own stream they are chained behind it (see chain_begin), on another one
     // they are a plain launch.
-    if (m2 > 0) {
+    if (m2 > 0 && !rows_done) {
         if (int rc = launch_rows<T, RVB, RL, RVPL, kRagged>(m2, n, values, col, row_offsets, residue_r_ind, B, C, counters,
                                                             chained, counters_clear, nnz, s2))
             return rc;
