@@ -614,11 +614,13 @@ int launch_k(int m1, int m2, int k, const int *block_r_ind, const int *residue_r
     // it balances nothing, but short rows still lose more to the idle lane groups of the row form (R-MAT 21,
     // K = 96: 0.56 ms as a stream, 0.65 to 0.68 ms row by row; stencil, K = 128: 1.78 against 1.57 ms)
     const int row_mode_min = L == 32 ? RODE_SDDMM_ROW_MODE_MIN32 : RODE_SDDMM_ROW_MODE_MIN;
-    if constexpr (kLongSegments) {
+    {
         // (a row per lane group: on such matrices most residue rows have had their tail taken by a segment)
         const int per = RL > 0 ? 32 / (RL > 0 ? RL : 1) : 1;
         const long long ctas = static_cast<long long>(m1) + (m2 + per - 1) / per;
-        if (m1 > 0 && m2 > 0 && s1 == s2 && ctas <= 4LL * 24 * sm_count()) {
+        // (a warp per 32-long segment, K = 128, pays while they all fit at once: Bernoulli 4096^2 13.5 us with the two
+        // kernels, 14.7 in one; 2000^2 12.3 and 10.3)
+        if (m1 > 0 && m2 > 0 && s1 == s2 && ctas <= (kLongSegments ? 4LL : 1LL) * 24 * sm_count()) {
             sddmm_items<L, VPL, false, kRagged, RL, RVPL, RU, BL, BVPL, BU><<<static_cast<unsigned>(ctas), 32, 0, s1>>>(
                 m2, per, residue_r_ind, st_off, row_offsets, col, values, lhs, rhs, out, row_vecs, row_mode_min, m1,
                 block_r_ind);
