@@ -193,8 +193,11 @@ def preprocess(row_ptr: torch.Tensor, nnz: int, seg_len: int = 512, k_block: int
     return RodeMeta(blk, st, res, m1, m2, seg_len, k_block, vec_len)
 
 
+_NULL = contextlib.nullcontext()
+
+
 def _null():
-    return contextlib.nullcontext()
+    return _NULL
 
 
 def _current(dev: torch.device) -> int:
@@ -305,10 +308,10 @@ def spmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torch
         s2 = cur if stream2 is None else stream2
         whole = C is None and (meta.m1 > 0 or meta.m2 > 0)
         if C is None:
-            C = (torch.empty if whole else torch.zeros)((M, n), dtype=B.dtype, device=dev)
+            C = B.new_empty((M, n)) if whole else B.new_zeros((M, n))
         need = spmm_workspace_bytes(meta.m1, n, B.element_size())
         if workspace is None and need:
-            workspace = torch.empty(need, dtype=torch.uint8, device=dev)
+            workspace = B.new_empty(need, dtype=torch.uint8)
             # the buffer goes back to torch's allocator when this function returns: tell the
             # allocator which other streams still use it, or a call enqueued right afterwards
             # could be handed the same memory while this call's kernels run
@@ -347,7 +350,7 @@ def sddmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torc
         s1 = cur if stream1 is None else stream1
         s2 = cur if stream2 is None else stream2
         if out is None:  # every stored entry lies in a block segment or a residue row, so all of it is written
-            out = torch.empty(values.numel(), dtype=torch.float32, device=dev)
+            out = values.new_empty(values.numel())
         sddmm_raw(meta.m1, meta.m2, rhs.shape[0], k, meta.block_r_ind.data_ptr(), meta.residue_r_ind.data_ptr(),
                   meta.st_off.data_ptr(), row_ptr.data_ptr(), col.data_ptr(), values.data_ptr(), lhs.data_ptr(),
                   rhs.data_ptr(), out.data_ptr(), s1, s2)

@@ -1110,7 +1110,7 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
                                                             chained, counters_clear, nnz, s2))
             return rc;
     }
-    if (m1 > 0) {
+    if (m1 > 1) {  // (a row that was cut has two segments at least)
         // fix-up last, chained behind the block grid (and the rows): its launch latency and its
         // metadata prologue overlap the tail of those grids
         int per = (m1 / (4 * sm_count()) + 31) / 32 * 32;  // segments per CTA: about four CTAs per SM
