@@ -390,9 +390,12 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
     if (total == 0) return;
     if constexpr (LB > 0 && !kSegments) {
         static_assert(LB * VPLB == L * VPL || kRagged, "both lane-group shapes must cover the same dense row");
-        // (full warps of 32 rows only: short lists give a warp fewer rows than it has groups, and
-        // there the stream's even split of the nonzeros is what shortens the dependent chain)
-        if (BL > 0 || (items_per_warp == 32 && total >= row_mode_min * 32)) {  // warp-uniform
+        // Short lists give a warp few rows, and there the stream's even split of the nonzeros shortens the dependent
+        // chain: then only rows of about equal length are taken one by one (none longer than twice the mean; 27-point
+        // stencil of 48^3 rows, us: K = 32 42 -> 33, K = 64 66 -> 50, K = 96 136 -> 80; Zipf 100003 x 50021 K = 64 would go 40 ->
+        // 43, R-MAT 17 K = 64 46 -> 48).
+        const bool even = items_per_warp == 32 || (items_per_warp >= 32 / LB && __reduce_max_sync(kFull, len) * items_per_warp <= 2 * total);
+        if (BL > 0 || (even && total >= row_mode_min * items_per_warp)) {  // warp-uniform
             constexpr int GB = 32 / LB;
             const int gb = lane / LB;
             for (int j0 = 0; j0 < items_per_warp; j0 += GB) {
@@ -594,9 +597,12 @@ int claim_counters(cudaStream_t s1, cudaStream_t s2, int **out) {
     return RODE_OK;
 }
 
-// Items per warp: 32 when that still gives every SM several waves of warps, fewer otherwise.
-int items_per_warp(int n_items, int cap) {
-    const long long slots = 4LL * 24 * sm_count();
+// Items per warp: up to `cap` when that still gives every SM `waves` waves of warps, fewer otherwise.  Rows whose warp
+// holds several lane groups want two waves, because a warp then brings its own balance (us with four waves -> two: Zipf 65536
+// K = 32 22.8 -> 18.8, K = 64 28.9 -> 25.6, Zipf 100003 x 50021 K = 64 42.5 -> 39.7);
+// a warp of one group wants four (R-MAT 17 K = 96 95 us with two, 92 with four; K = 128 90 and 85).
+int items_per_warp(int n_items, int cap, int waves) {
+    const long long slots = waves * 24LL * sm_count();
     long long per = (n_items + slots - 1) / slots;
     per = per < 1 ? 1 : (per > cap ? cap : per);
     return static_cast<int>(per);
@@ -645,14 +651,14 @@ int launch_k(int m1, int m2, int k, const int *block_r_ind, const int *residue_r
             }
             RODE_CHECK_LAUNCH("rode::sddmm_block");
         } else {
-            const int per = items_per_warp(m1, 32);
+            const int per = items_per_warp(m1, 32, 4);
             sddmm_items<L, VPL, true, kRagged, 0, 1, 1><<<(m1 + per - 1) / per, 32, 0, s1>>>(
                 m1, per, block_r_ind, st_off, row_offsets, col, values, lhs, rhs, out, row_vecs, 0, 0, nullptr);
             RODE_CHECK_LAUNCH("rode::sddmm_items<segments>");
         }
     }
     if (m2 > 0) {
-        const int per = items_per_warp(m2, 32);
+        const int per = items_per_warp(m2, 32, L < 32 ? 2 : 4);
         RODE_CUDA_TRY(launch_chained(sddmm_items<L, VPL, false, kRagged, RL, RVPL, RU>, dim3((m2 + per - 1) / per + 1), dim3(32), s2,
                                      m1 > 0 && s1 == s2, m2, per, residue_r_ind, nullptr, row_offsets, col, values, lhs,
                                      rhs, out, row_vecs, row_mode_min, 0, nullptr));

@@ -132,6 +132,11 @@ constexpr int kPersistentMinWaves = 16;
 #ifndef RODE_SPMM_PERSISTENT_CTAS_PER_SM
 #define RODE_SPMM_PERSISTENT_CTAS_PER_SM 32
 #endif
+// Block grids of at most this many warps per SM keep a whole chunk in flight per warp: 163 registers, 12 warps at a time,
+// so less than two waves.  The time of such a grid is the chain of batches of its longest segment; beyond, its
+// throughput (us, whole chunk against 8 rows in flight: 2949 segments of Pareto 2^14 N = 128 31 and 35, 3269 of a Zipf matrix
+// 43 and 39, 3706 of Zipf 65536 45 and 41, 3911 of Bernoulli 4096^2 16.5 and 14.5).
+constexpr int kWholeChunkWarpsPerSm = 22;
 // 16-byte units a lane keeps in flight per batch (dense rows per batch = this * 16 / bytes per load / VPL).
 constexpr int kLoadsInFlight = 8;
 
@@ -1094,7 +1099,7 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
             rows_done = launched = true;
         }
         if (launched) {
-        } else if (small_grid && USmall > U) {
+        } else if (USmall > U && static_cast<long long>(m1) * tiles <= kWholeChunkWarpsPerSm * sm_count()) {
             spmm_block<T, VB, L, VPL, USmall, kCtaWarps, false, false, kRagged><<<grid, kCtaThreads, 0, s1>>>(
                 m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0, claim);
         } else {
