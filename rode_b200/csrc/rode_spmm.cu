@@ -132,27 +132,26 @@ constexpr int kPersistentMinWaves = 16;
 #ifndef RODE_SPMM_PERSISTENT_CTAS_PER_SM
 #define RODE_SPMM_PERSISTENT_CTAS_PER_SM 32
 #endif
-// Block grids of at most this many warps per SM keep a whole chunk in flight per warp: 163 registers, 12 warps at a time,
-// so less than two waves.  The time of such a grid is the chain of batches of its longest segment; beyond, its
-// throughput (us, whole chunk against 8 rows in flight: 2949 segments of Pareto 2^14 N = 128 31 and 35, 3269 of a Zipf matrix
-// 43 and 39, 3706 of Zipf 65536 45 and 41, 3911 of Bernoulli 4096^2 16.5 and 14.5).
-constexpr int kWholeChunkWarpsPerSm = 22;
+// Block grids of at most so many segments per SM give a segment four or two warps, which take its chunks in turn and add
+// their rows through shared memory: the time of such a grid is the chain of batches of its longest segment, beyond that
+// it is its throughput.  us, one warp with 8 rows in flight / one warp with a whole chunk in flight (163 registers, which
+// these two forms replace) / two warps / four: R-MAT 14 N = 128 (1508 segments) 27 / 21 / 19 / 17, R-MAT 15 (1981) 31 / 25 / 22 /
+// 21, Zipf 50000 (2800) 37 / 39 / 33 / 35, Pareto 2^14 (2949) 35 / 31 / 29 / 28, Zipf 65536 (3706) 41 / 45 / 41 / 42, Bernoulli
+// 4096^2 (3911) 14.5 / 16.5 / 15 / 17.
+constexpr int kSplit4WarpsPerSm = 16;
+constexpr int kSplit2WarpsPerSm = 22;
 // 16-byte units a lane keeps in flight per batch (dense rows per batch = this * 16 / bytes per load / VPL).
 constexpr int kLoadsInFlight = 8;
 
 // ---------------------------------------------------------------------------------------
-// One warp per block segment; grid.y walks the column tiles of L * VPL vectors.  U = dense
-// rows per batch: kLoadsInFlight / VPL for grids that fill the GPU (64 registers keep 32
-// warps per SM resident); the whole chunk for small grids, where the time is the
-// dependent-batch chain of the longest segment and registers are free.
-// One-warp CTAs per SM that the register budget must allow, by 16-byte loads in flight per
-// lane: 8 -> 32 CTAs (64 registers), 12 -> 25 (80), 16 -> 20 (96), more -> no limit.
-constexpr int min_ctas_per_sm(int loads) { return loads <= 8 ? 32 : loads <= 12 ? 25 : loads <= 16 ? 20 : 1; }
-
+// One warp per block segment, or S warps (a CTA) that take its chunks in turn; grid.y walks the column tiles of
+// L * VPL vectors.  U = dense rows per batch: 8 loads of 16 bytes per lane, with which 64 registers keep 32 warps
+// per SM resident.
+//
 // kRagged: the width is not a multiple of the tile; the last tile's lanes beyond the row's end neither
 // load nor store (widths the reference's tiles do not serve: any multiple of 4 columns).
-template <typename T, int VB, int L, int VPL, int U, int W, bool kHints, bool kClaim, bool kRagged>
-__global__ void __launch_bounds__(32 * W, min_ctas_per_sm(U * VPL * VB / 16) / W)
+template <typename T, int VB, int L, int VPL, int U, int W, int S, bool kHints, bool kClaim, bool kRagged>
+__global__ void __launch_bounds__(32 * W, 32 / W)
 spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ column_indices,
            const int *__restrict__ row_offsets, const int *__restrict__ block_r_ind,
            const int *__restrict__ st_off, const T *__restrict__ B, T *__restrict__ C, T *__restrict__ partial,
@@ -164,6 +163,8 @@ spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ 
     constexpr int NB = (kSteps + U - 1) / U;
     constexpr unsigned kFull = 0xffffffffu;
     chain_begin();
+    static_assert(W % S == 0 && (S == 1 || (W == S && !kClaim && RODE_SPMM_PAIRS_IN_SMEM != 0)), "a CTA per split segment");
+    const int part = S == 1 ? 0 : threadIdx.x >> 5;  // this warp takes every S-th chunk of its segment
     const int lane = threadIdx.x & 31;
     const int g = lane / L, l = lane % L;
     // Chunk staging (two buffers, so one __syncwarp per chunk orders both the reads after the
@@ -189,7 +190,7 @@ spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ 
     // warp slot waits for a new CTA to be launched into it (one-warp CTAs of a few microseconds
     // each left a fifth of the slots empty at any time).  The claim is issued before the segment's
     // work and read after it, so its latency is hidden.  Otherwise one segment per warp.
-    int seg = blockIdx.x * W + (threadIdx.x >> 5);
+    int seg = S == 1 ? blockIdx.x * W + (threadIdx.x >> 5) : blockIdx.x;
     while (seg < m1) {
     int claimed = INT_MAX;
     if constexpr (kClaim) {
@@ -197,12 +198,13 @@ spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ 
             claimed = static_cast<int>(gridDim.x) * W + atomicAdd(next_segment + blockIdx.y, 1);
     }
     const int row = __ldg(block_r_ind + seg);
-    const int off = __ldg(st_off + seg);
+    const int seg_off = __ldg(st_off + seg);
+    const int off = seg_off + part * 32;
     const int next = (seg + 1 < m1) ? __ldg(st_off + seg + 1) : INT_MAX;
     const int row_begin = __ldg(row_offsets + row);
     const int row_end = __ldg(row_offsets + row + 1);
     const int end = min(row_end, next);
-    const bool whole_row = (off == row_begin) && (next >= row_end);
+    const bool whole_row = (seg_off == row_begin) && (next >= row_end);
 
     // (column, value) of this lane's nonzero in the current and in the next chunk
     int c_cur = 0, c_nxt = 0;
@@ -211,9 +213,9 @@ spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ 
         c_cur = ld_stream(column_indices + off + lane);
         v_cur = ld_stream(values + off + lane);
     }
-    if (off + 32 + lane < end) {
-        c_nxt = ld_stream(column_indices + off + 32 + lane);
-        v_nxt = ld_stream(values + off + 32 + lane);
+    if (off + 32 * S + lane < end) {
+        c_nxt = ld_stream(column_indices + off + 32 * S + lane);
+        v_nxt = ld_stream(values + off + 32 * S + lane);
     }
     // With popularity hints a column index carries its mark in bit 31.  The bitmap word of a
     // column is fetched one chunk after the column itself (which has arrived by then) and one
@@ -223,13 +225,13 @@ spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ 
     V acc[VPL];
 #pragma unroll
     for (int v = 0; v < VPL; ++v) acc[v] = vzero(static_cast<V *>(nullptr));
-    for (int base = off; base < end; base += 32) {
+    for (int base = off; base < end; base += 32 * S) {
         const int cnt = min(32, end - base);
         int c_pre = 0;
         T v_pre = T(0);
-        if (base + 64 + lane < end) {  // pairs of the chunk after next
-            c_pre = ld_stream(column_indices + base + 64 + lane);
-            v_pre = ld_stream(values + base + 64 + lane);
+        if (base + 64 * S + lane < end) {  // pairs of the chunk after next
+            c_pre = ld_stream(column_indices + base + 64 * S + lane);
+            v_pre = ld_stream(values + base + 64 * S + lane);
         }
         unsigned w_nxt = 0;
         if constexpr (kHints) w_nxt = hot_word(hot, c_nxt);
@@ -281,8 +283,8 @@ spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ 
             }
         };
         // (only the 512-byte tile of large grids: R-MAT 21 N = 128 block kernel 0.818 -> 0.787 ms, R-MAT 23
-        // step 4.76 -> 4.62 ms; the narrower shapes and the small-grid form measured 1-2 % slower with it)
-        constexpr bool kFullChunkPath = RODE_SPMM_FULL_CHUNK_PATH != 0 && L == 32 && U == kLoadsInFlight / VPL;
+        // step 4.76 -> 4.62 ms; the narrower shapes measured 1-2 % slower with it)
+        constexpr bool kFullChunkPath = RODE_SPMM_FULL_CHUNK_PATH != 0 && L == 32;
         if (kFullChunkPath && cnt == 32)
             chunk(std::true_type{});
         else
@@ -298,6 +300,21 @@ spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ 
 #pragma unroll
         for (int w = L; w < 32; w <<= 1) vadd(acc[v], vshfl_xor(kFull, acc[v], w));
 
+    if constexpr (S > 1) {  // the parts are added in order
+        __shared__ __align__(32) V s_part[S - 1][L * VPL];
+        if (part > 0 && g == 0) {
+#pragma unroll
+            for (int v = 0; v < VPL; ++v) s_part[part - 1][l + v * L] = acc[v];
+        }
+        __syncthreads();
+        if (part > 0) return;
+        if (g == 0) {
+#pragma unroll
+            for (int w = 0; w < S - 1; ++w)
+#pragma unroll
+                for (int v = 0; v < VPL; ++v) vadd(acc[v], s_part[w][l + v * L]);
+        }
+    }
     if (g == 0) {
 #pragma unroll
         for (int v = 0; v < VPL; ++v) {
@@ -1044,20 +1061,14 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
                  T *partial, int *counters, const unsigned *hot, long long nnz, cudaStream_t s1, cudaStream_t s2) {
     static_assert(L * VPL * VB == RL * RVPL * RVB, "block and residue kernels must cover the same tile");
     constexpr int kTileWidth = L * VPL * VecB<T, VB>::kLen;
-    constexpr int U = kLoadsInFlight * 16 / VB / VPL;            // rows per batch, large grids
-    constexpr int kChunkSteps = L;                               // nonzeros per group per chunk
-    constexpr int kSmallCap = 32 * 16 / VB;                      // small grids: at most 512 bytes per lane in flight
-    constexpr int USmall = (kChunkSteps * VPL <= kSmallCap) ? kChunkSteps : kSmallCap / VPL;
+    constexpr int U = kLoadsInFlight * 16 / VB / VPL;            // rows per batch
     // ragged widths: the last tile is partly empty
     const unsigned tiles = static_cast<unsigned>(kRagged ? (n + kTileWidth - 1) / kTileWidth : n / kTileWidth);
     const bool chained = s1 == s2 && m1 > 0;
     bool rows_done = false;
     bool counters_clear = false;  // the residue kernel's claim counters have been zeroed already
     if (m1 > 0) {
-        // Fewer warps than two full waves of 32 per SM: the latency of the longest segment
-        // rules, so batches are larger.  CTAs stay one warp: with 4-warp CTAs the Zipf matrix
-        // (segments of 32 to 512 nonzeros side by side) ran 0.035 ms instead of 0.029 ms at
-        // N = 32 and 0.27 ms instead of 0.06 ms at N = 128.
+        // fewer warps than two full waves of 32 per SM: no hints, no claims
         const bool small_grid = static_cast<long long>(m1) * tiles <= 2LL * 32 * sm_count();
         // large grids: one resident wave of CTAs whose warps claim segments from counters (one per
         // column tile) at the end of the workspace, zeroed on the stream before the launch
@@ -1081,7 +1092,7 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
         // cost more time than that returned (1.41 -> 1.52 ms).
         if constexpr (L * VPL * VB == 512 && !kRagged) {
             if (hot && !small_grid) {
-                spmm_block<T, VB, L, VPL, U, kCtaWarps, true, true, false><<<grid, kCtaThreads, 0, s1>>>(
+                spmm_block<T, VB, L, VPL, U, kCtaWarps, 1, true, true, false><<<grid, kCtaThreads, 0, s1>>>(
                     m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, hot, (k + 31) / 32, claim);
                 launched = true;
             }
@@ -1099,11 +1110,14 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
             rows_done = launched = true;
         }
         if (launched) {
-        } else if (USmall > U && static_cast<long long>(m1) * tiles <= kWholeChunkWarpsPerSm * sm_count()) {
-            spmm_block<T, VB, L, VPL, USmall, kCtaWarps, false, false, kRagged><<<grid, kCtaThreads, 0, s1>>>(
-                m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0, claim);
+        } else if (static_cast<long long>(m1) * tiles <= kSplit4WarpsPerSm * sm_count()) {
+            spmm_block<T, VB, L, VPL, U, 4, 4, false, false, kRagged><<<dim3(m1, tiles), 4 * 32, 0, s1>>>(
+                m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0, nullptr);
+        } else if (static_cast<long long>(m1) * tiles <= kSplit2WarpsPerSm * sm_count()) {
+            spmm_block<T, VB, L, VPL, U, 2, 2, false, false, kRagged><<<dim3(m1, tiles), 2 * 32, 0, s1>>>(
+                m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0, nullptr);
         } else {
-            spmm_block<T, VB, L, VPL, U, kCtaWarps, false, true, kRagged><<<grid, kCtaThreads, 0, s1>>>(
+            spmm_block<T, VB, L, VPL, U, kCtaWarps, 1, false, true, kRagged><<<grid, kCtaThreads, 0, s1>>>(
                 m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0, claim);
         }
         RODE_CHECK_LAUNCH("rode::spmm_block");
