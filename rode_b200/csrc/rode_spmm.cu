@@ -140,6 +140,8 @@ constexpr int kPersistentMinWaves = 16;
 // 4096^2 (3911) 14.5 / 16.5 / 15 / 17.
 constexpr int kSplit4WarpsPerSm = 16;
 constexpr int kSplit2WarpsPerSm = 22;
+// The mean row is short (and the number of nonzeros known).
+constexpr bool short_rows(long long nnz, long long rows) { return nnz >= 0 && nnz < 20 * rows; }
 // 16-byte units a lane keeps in flight per batch (dense rows per batch = this * 16 / bytes per load / VPL).
 constexpr int kLoadsInFlight = 8;
 
@@ -1053,13 +1055,12 @@ int launch_rows(int m2, int n, const T *values, const int *col, const int *row_o
                 const T *B, T *C, int *counters, bool chained, bool counters_clear, long long nnz,
                 cudaStream_t s2);
 
-// Block kernel of shape (VB bytes per load, L lanes, VPL loads per lane) and residue-row kernel
-// of shape (RVB, RL, RVPL); both cover the same column tile.
-template <typename T, int VB, int L, int VPL, int RVB, int RL, int RVPL, bool kRagged>
+// Block kernel of shape (VB bytes per load, L lanes, VPL loads per lane) and residue-row kernel of shape (RVB, RL, RVPL);
+// each walks the columns in tiles of its own.
+template <typename T, int VB, int L, int VPL, int RVB, int RL, int RVPL, bool kRagged, bool kRowsRagged = kRagged>
 int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, const int *row_offsets,
                  const int *block_r_ind, const int *residue_r_ind, const int *st_off, const T *B, T *C,
                  T *partial, int *counters, const unsigned *hot, long long nnz, cudaStream_t s1, cudaStream_t s2) {
-    static_assert(L * VPL * VB == RL * RVPL * RVB, "block and residue kernels must cover the same tile");
     constexpr int kTileWidth = L * VPL * VecB<T, VB>::kLen;
     constexpr int U = kLoadsInFlight * 16 / VB / VPL;            // rows per batch
     // ragged widths: the last tile is partly empty
@@ -1125,7 +1126,7 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
     // Rows: on the block kernel's own stream they are chained behind it (see chain_begin), on another one
     // they are a plain launch.
     if (m2 > 0 && !rows_done) {
-        if (int rc = launch_rows<T, RVB, RL, RVPL, kRagged>(m2, n, values, col, row_offsets, residue_r_ind, B, C, counters,
+        if (int rc = launch_rows<T, RVB, RL, RVPL, kRowsRagged>(m2, n, values, col, row_offsets, residue_r_ind, B, C, counters,
                                                             chained, counters_clear, nnz, s2))
             return rc;
     }
@@ -1185,7 +1186,7 @@ int launch_rows(int m2, int n, const T *values, const int *col, const int *row_o
             return launch_chained(spmm_rows_simple<T, VB, L, VPL, R, kRagged>, grid, dim3(kRowsCtaThreads), s2, chained, m2, n,
                                   values, col, row_offsets, residue_r_ind, B, C);
         };
-        if (nnz >= 0 && nnz < 20LL * m2)
+        if (short_rows(nnz, m2))
             RODE_CUDA_TRY(launch(std::true_type{}));
         else
             RODE_CUDA_TRY(launch(std::false_type{}));
@@ -1251,6 +1252,25 @@ int spmm(int m1, int m2, int k, int n, const T *values, const int *col, const in
     // Widths the tiles do not divide (any other multiple of 4 columns; the reference has none of
     // them): the narrowest shape that covers the row, or 512-byte tiles with a partly empty last
     // one.  Always 16-byte loads, no popularity hints.
+    // Widths of whole lines that the 512-byte tile does not divide (N = 96, 160, 192, 224 ...; fp64: N = 48): 512-byte tiles with a
+    // partly idle last one all the same, instead of up to seven passes over the sparse matrix with narrow ones.  The
+    // residue rows follow where they are short on average; long even rows (27-point stencil) keep the narrow per-row
+    // kernel, which neighbouring rows' L1 hits favour (N = 96 1.18 against 1.48 ms).  us, narrow -> wide: R-MAT 21 N = 96 1411
+    // -> 954, N = 160 2627 -> 1948, N = 224 3701 -> 2449; Pareto 2^20 N = 96 2309 -> 1756, N = 224 5897 -> 4493; Bernoulli 4096^2 N = 96
+    // 20.7 -> 12.5; Zipf 65536 N = 160 70 -> 74.  fp64, wider: 497 -> 568 on Pareto (300,007 rows, N = 80).
+    if (vecs % 8 == 0 && vecs > 16 && vecs % 32 != 0 && (sizeof(T) == 4 || vecs == 24)) {
+#define RODE_WIDE_BLOCK(rows_shape, rows_ragged)                                                                  \
+    launch_shape<T, 16, RODE_SPMM_SHAPE_32 / 100, RODE_SPMM_SHAPE_32 % 100, 16, (rows_shape) / 100, (rows_shape) % 100, true, \
+                 rows_ragged>(m1, m2, k, n, values, col, row_offsets, block_r_ind, residue_r_ind, st_off, B, C, partial,     \
+                              counters, nullptr, nnz, stream1, stream2)
+        if (short_rows(nnz, m2)) return RODE_WIDE_BLOCK(RODE_SPMM_ROWS_SHAPE_32, true);
+        if (vecs % 16 == 0) return RODE_WIDE_BLOCK(RODE_SPMM_SHAPE_16, false);
+        if (aligned_to(B, 32) && aligned_to(C, 32))
+            return launch_shape<T, 16, RODE_SPMM_SHAPE_32 / 100, RODE_SPMM_SHAPE_32 % 100, 32, 4, 1, true, false>(
+                m1, m2, k, n, values, col, row_offsets, block_r_ind, residue_r_ind, st_off, B, C, partial, counters, nullptr, nnz,
+                stream1, stream2);
+        return RODE_WIDE_BLOCK(RODE_SPMM_ROWS_SHAPE_8, false);
+    }
     if (vecs % 8 != 0) {
         if (vecs < 8) return RODE_LAUNCH16R(RODE_SPMM_SHAPE_8, RODE_SPMM_ROWS_SHAPE_8, true);
         if (vecs < 16) return RODE_LAUNCH16R(RODE_SPMM_SHAPE_16, RODE_SPMM_SHAPE_16, true);
@@ -1281,6 +1301,7 @@ int spmm(int m1, int m2, int k, int n, const T *values, const int *col, const in
                                                               stream1, stream2);
     }
     return RODE_LAUNCH16(RODE_SPMM_SHAPE_8, RODE_SPMM_ROWS_SHAPE_8);
+#undef RODE_WIDE_BLOCK
 #undef RODE_LAUNCH16
 #undef RODE_LAUNCH16R
 #undef RODE_LAUNCH32

@@ -27,7 +27,7 @@ def _matrix(rows, seed=0):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
 @pytest.mark.parametrize("rows", [37, 5000, 70001])     # one warp per row; between; a lane group or bundle per row
-@pytest.mark.parametrize("n", [4, 32, 64, 100, 128, 256])
+@pytest.mark.parametrize("n", [4, 32, 48, 64, 96, 100, 128, 160, 224, 256])
 def test_every_row_is_written(oracle_cpu, n, rows, dtype):
     A = _matrix(rows)
     d = A.to("cuda")
