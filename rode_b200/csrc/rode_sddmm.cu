@@ -557,45 +557,58 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
 // (32 KB on every GPU that loads the library).  A slot belongs to one (device, stream1, stream2)
 // for the life of the process: calls on the same streams are ordered by them and may share
 // their counter, calls on other streams get other slots; when all slots are taken a call simply
-// runs one CTA per segment.  Nothing is allocated.  (Two host threads that enqueue calls on the
-// SAME pair of streams at the same time could interleave one call's counter reset with the
-// other's kernel; like the reference, the entry points expect one enqueueing thread per stream.)
-#ifndef RODE_SDDMM_PERSISTENT
-#define RODE_SDDMM_PERSISTENT 1
-#endif
+// runs one CTA per segment.  Nothing is allocated.  What keeps two kernels off one counter:
+//   * streams are told apart by cudaStreamGetId, not by handle: cudaStreamPerThread is one handle for a stream per
+//     thread, and a destroyed stream's handle is given to a new one while its last kernels may still run;
+//   * the reset and the kernel that follows it are enqueued under one lock (ClaimCounter holds it), so that host
+//     threads that share a stream cannot come between them;
+//   * a call that is being captured gets no counter: its graph may be replayed on any stream, next to graphs
+//     captured on the same one.
 constexpr int kClaimSlots = 128;
 constexpr int kClaimInts = 64;
 static __device__ __align__(256) int g_claim_counters[kClaimSlots * kClaimInts];
+std::mutex g_claim_mutex;
 
-int claim_counters(cudaStream_t s1, cudaStream_t s2, int **out) {
-    struct Key {
-        int dev;
-        cudaStream_t s1, s2;
-    };
-    static Key keys[kClaimSlots];
-    static int n_keys = 0;
-    static int *base[64] = {nullptr};  // device address of the array, per device
-    static std::mutex lock;
-    *out = nullptr;
-    int dev = 0;
-    RODE_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64) return RODE_OK;
-    std::lock_guard<std::mutex> guard(lock);
-    if (base[dev] == nullptr) {
-        void *p = nullptr;
-        RODE_CUDA_TRY(cudaGetSymbolAddress(&p, g_claim_counters));
-        base[dev] = static_cast<int *>(p);
+struct ClaimCounter {
+    int *ptr = nullptr;  // null: run one CTA per segment
+    std::unique_lock<std::mutex> enqueue;
+
+    int acquire(cudaStream_t s1, cudaStream_t s2) {
+        struct Key {
+            int dev;
+            unsigned long long id1, id2;
+        };
+        static Key keys[kClaimSlots];
+        static int n_keys = 0;
+        static int *base[64] = {nullptr};  // device address of the array, per device
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s1, &capture) != cudaSuccess) {
+            (void)cudaGetLastError();  // the legacy stream while another one is being captured: the launch itself reports it
+            return RODE_OK;
+        }
+        if (capture != cudaStreamCaptureStatusNone) return RODE_OK;
+        Key key = {0, 0, 0};
+        RODE_CUDA_TRY(cudaGetDevice(&key.dev));
+        if (key.dev < 0 || key.dev >= 64) return RODE_OK;
+        RODE_CUDA_TRY(cudaStreamGetId(s1, &key.id1));
+        RODE_CUDA_TRY(cudaStreamGetId(s2, &key.id2));
+        enqueue = std::unique_lock<std::mutex>(g_claim_mutex);
+        if (base[key.dev] == nullptr) {
+            void *p = nullptr;
+            RODE_CUDA_TRY(cudaGetSymbolAddress(&p, g_claim_counters));
+            base[key.dev] = static_cast<int *>(p);
+        }
+        int slot = -1;
+        for (int i = 0; i < n_keys; ++i)
+            if (keys[i].dev == key.dev && keys[i].id1 == key.id1 && keys[i].id2 == key.id2) slot = i;
+        if (slot < 0 && n_keys < kClaimSlots) {
+            slot = n_keys++;
+            keys[slot] = key;
+        }
+        if (slot >= 0) ptr = base[key.dev] + slot * kClaimInts;
+        return RODE_OK;
     }
-    int slot = -1;
-    for (int i = 0; i < n_keys; ++i)
-        if (keys[i].dev == dev && keys[i].s1 == s1 && keys[i].s2 == s2) slot = i;
-    if (slot < 0 && n_keys < kClaimSlots) {
-        slot = n_keys++;
-        keys[slot] = {dev, s1, s2};
-    }
-    if (slot >= 0) *out = base[dev] + slot * kClaimInts;
-    return RODE_OK;
-}
+};
 
 // Items per warp: up to `cap` when that still gives every SM `waves` waves of warps, fewer otherwise.  Rows whose warp
 // holds several lane groups want two waves, because a warp then brings its own balance (us with four waves -> two: Zipf 65536
@@ -637,14 +650,14 @@ int launch_k(int m1, int m2, int k, const int *block_r_ind, const int *residue_r
     if (m1 > 0) {
         if constexpr (kLongSegments) {
             const int resident = block_ctas(BVPL) * sm_count();
-            int *claim = nullptr;
+            ClaimCounter claim;  // holds its lock until the kernel is enqueued
             if (m1 > 16 * resident) {  // from about 16 segments per warp on it pays
-                if (int rc = claim_counters(s1, s2, &claim)) return rc;
+                if (int rc = claim.acquire(s1, s2)) return rc;
             }
-            if (claim != nullptr) {
-                RODE_CUDA_TRY(cudaMemsetAsync(claim, 0, sizeof(int), s1));
+            if (claim.ptr != nullptr) {
+                RODE_CUDA_TRY(cudaMemsetAsync(claim.ptr, 0, sizeof(int), s1));
                 sddmm_block<PL, PVPL, PU, true, kRagged><<<resident, 32, 0, s1>>>(
-                    m1, block_r_ind, st_off, row_offsets, col, values, lhs, rhs, out, claim, row_vecs);
+                    m1, block_r_ind, st_off, row_offsets, col, values, lhs, rhs, out, claim.ptr, row_vecs);
             } else {
                 sddmm_block<BL, BVPL, BU, false, kRagged><<<m1, 32, 0, s1>>>(m1, block_r_ind, st_off, row_offsets, col, values,
                                                                             lhs, rhs, out, nullptr, row_vecs);

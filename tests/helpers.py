@@ -113,3 +113,38 @@ def sample_rows_csr(A, rows):
     idx = torch.repeat_interleave(lo - new_rp[:-1], lens) + torch.arange(int(new_rp[-1]), device=rp.device)
     return (new_rp.to(torch.int32).cpu().numpy(), A.col[idx].cpu().numpy(), A.val[idx].cpu().numpy(),
             idx.cpu().numpy())
+
+
+def graph_nodes(call):
+    """What one run of ``call`` puts on the current stream, captured: a list of kernel names (mangled) and, for
+    other nodes, "memset" or "node type <n>".  Shows which kernels a call takes without timing anything."""
+    import ctypes
+
+    import torch
+
+    cu = ctypes.CDLL("libcuda.so.1")
+
+    def ok(status):
+        assert status == 0, f"driver API status {status}"
+
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+    handle = ctypes.c_void_p(graph.raw_cuda_graph())
+    count = ctypes.c_size_t(0)
+    ok(cu.cuGraphGetNodes(handle, None, ctypes.byref(count)))
+    nodes = (ctypes.c_void_p * max(count.value, 1))()
+    ok(cu.cuGraphGetNodes(handle, nodes, ctypes.byref(count)))
+    out = []
+    for node in nodes[: count.value]:
+        kind = ctypes.c_int(-1)
+        ok(cu.cuGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(kind)))
+        if kind.value != 0:  # CU_GRAPH_NODE_TYPE_KERNEL
+            out.append("memset" if kind.value == 2 else f"node type {kind.value}")
+            continue
+        params = (ctypes.c_uint64 * 16)()  # CUDA_KERNEL_NODE_PARAMS begins with the function's handle
+        ok(cu.cuGraphKernelNodeGetParams_v2(ctypes.c_void_p(node), params))
+        name = ctypes.c_char_p()
+        ok(cu.cuFuncGetName(ctypes.byref(name), ctypes.c_void_p(params[0])))
+        out.append(name.value.decode())
+    return out

@@ -10,7 +10,7 @@ import torch
 from oracle import ref
 from rode_b200 import capi
 from rode_b200 import workloads as W
-from tests.helpers import assert_close_to_truth, run_reference_sddmm, sample_rows_csr, sddmm_abs_scale
+from tests.helpers import assert_close_to_truth, graph_nodes, run_reference_sddmm, sample_rows_csr, sddmm_abs_scale
 
 pytestmark = pytest.mark.gpu
 SEG_FOR_K = {32: 512, 64: 512, 128: 32}   # RoDe_SDDMM/rode_sddmm.py:35-38 (K = 64 follows K = 32)
@@ -249,3 +249,70 @@ def test_sddmm_widths_that_leave_lanes_idle(oracle_cpu, family, k):
     assert_close_to_truth(out[1:-1].cpu().numpy(), truth, sddmm_abs_scale(rp, col, val, lhs.numpy(), rhs.numpy()),
                           f"{family} k={k}")
     assert bool(torch.isnan(out[0])) and bool(torch.isnan(out[-1]))
+
+
+def _persistent_grid_case(k):
+    """80,000 rows of 40 nonzeros: enough segments for the block kernel to run as a persistent grid."""
+    m, n = 80_000, 5_000
+    rp = torch.arange(m + 1, dtype=torch.int32, device="cuda") * 40
+    col = (torch.arange(m * 40, device="cuda") * 7919 % n).to(torch.int32)
+    A = W.CSR(m, n, rp, col, W.dense(m, 40, device="cuda", seed=4).flatten())
+    meta = capi.preprocess(A.row_ptr, A.nnz, 512, 32, 4)
+    assert meta.m1 > 16 * 32 * 148
+    return A, meta, W.dense(m, k, device="cuda", seed=5), W.dense(n, k, device="cuda", seed=6)
+
+
+@pytest.mark.parametrize("k", [32, 64])
+def test_sddmm_graphs_captured_on_one_stream_share_no_counter(k):
+    """Two graphs captured on the same stream and replayed side by side on two others: a captured call uses no claim
+    counter (its reset would be a memset node), so neither replay can take the other's segments."""
+    A, meta, lhs, rhs = _persistent_grid_case(k)
+    want = capi.sddmm(meta, A.row_ptr, A.col, A.val, lhs, rhs)
+    outs = [torch.empty_like(A.val) for _ in range(2)]
+    nodes = graph_nodes(lambda: capi.sddmm(meta, A.row_ptr, A.col, A.val, lhs, rhs, out=outs[0]))
+    assert nodes and all("sddmm" in name for name in nodes), nodes
+    capture, replay = torch.cuda.Stream(), [torch.cuda.Stream() for _ in outs]
+    graphs = []
+    for out in outs:
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1], stream=capture):
+            capi.sddmm(meta, A.row_ptr, A.col, A.val, lhs, rhs, out=out)
+    for _ in range(4):
+        for out in outs:
+            out.fill_(float("nan"))
+        torch.cuda.synchronize()
+        for graph, stream in zip(graphs, replay):
+            with torch.cuda.stream(stream):
+                graph.replay()
+        torch.cuda.synchronize()
+        for out in outs:
+            assert torch.allclose(out, want, rtol=1e-5, atol=1e-6 * k)
+    del graphs
+
+
+def test_sddmm_threads_that_share_a_stream():
+    """Host threads whose calls interleave on one stream (the ctypes calls run without the GIL): the reset of the claim
+    counter and the kernel that uses it stay together."""
+    import threading
+
+    A, meta, lhs, rhs = _persistent_grid_case(32)
+    want = capi.sddmm(meta, A.row_ptr, A.col, A.val, lhs, rhs)
+    outs = [[torch.full_like(A.val, float("nan")) for _ in range(12)] for _ in range(4)]
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    start = threading.Barrier(len(outs))
+
+    def work(mine):
+        start.wait()
+        for out in mine:
+            capi.sddmm(meta, A.row_ptr, A.col, A.val, lhs, rhs, out=out, stream1=stream, stream2=stream)
+
+    threads = [threading.Thread(target=work, args=(mine,)) for mine in outs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for mine in outs:
+        for out in mine:
+            assert torch.equal(out, want)
