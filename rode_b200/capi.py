@@ -338,7 +338,8 @@ def sddmm_raw(m1, m2, n, k, blk, res, st, row_ptr, col, values, lhs, rhs, out, s
 
 def sddmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torch.Tensor, lhs: torch.Tensor,
           rhs: torch.Tensor, out: Optional[torch.Tensor] = None, stream1=None, stream2=None) -> torch.Tensor:
-    """out[e] = values[e] * <lhs[row(e)], rhs[col(e)]> through rode_sddmm_f32."""
+    """out[e] = values[e] * <lhs[row(e)], rhs[col(e)]> through rode_sddmm_f32.  A given ``out`` keeps what it holds in the
+    entries outside [row_ptr[0], row_ptr[M]); by default they are zero."""
     k = lhs.shape[1]
     if lhs.dtype != torch.float32 or rhs.dtype != torch.float32 or values.dtype != torch.float32:
         raise ValueError("float32 tensors required")
@@ -349,8 +350,8 @@ def sddmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torc
         cur = _current(dev)
         s1 = cur if stream1 is None else stream1
         s2 = cur if stream2 is None else stream2
-        if out is None:  # every stored entry lies in a block segment or a residue row, so all of it is written
-            out = values.new_empty(values.numel())
+        if out is None:  # (entries that belong to no row of row_ptr are not written)
+            out = values.new_zeros(values.numel())
         sddmm_raw(meta.m1, meta.m2, rhs.shape[0], k, meta.block_r_ind.data_ptr(), meta.residue_r_ind.data_ptr(),
                   meta.st_off.data_ptr(), row_ptr.data_ptr(), col.data_ptr(), values.data_ptr(), lhs.data_ptr(),
                   rhs.data_ptr(), out.data_ptr(), s1, s2)

@@ -35,6 +35,7 @@ class RoDeCSR:
         128: {"seg_length": 32, "k_block": 32, "vec_len": 4},
     }
     MAX_K = 256
+    _entry_range = None  # (row_offsets[0], row_offsets[m]) as of construction
 
     @classmethod
     def config_for(cls, k: int) -> dict:
@@ -58,6 +59,9 @@ class RoDeCSR:
         self.row_offsets_cpu = row_offsets.to(dtype=torch.int32, device="cpu").contiguous()
         self.column_indices = column_indices.to(dtype=torch.int32, device=self.device).contiguous()
         self.values = values.to(dtype=torch.float32, device=self.device).contiguous()
+        # entries in front of the first and behind the last row (a row pointer cut out of a larger one) are allowed
+        ends = self.row_offsets_cpu[[0, -1]].tolist() if self.row_offsets_cpu.numel() else [0, 0]
+        self._entry_range = (ends[0], ends[1])
         self._preprocess()
 
     def _preprocess(self):
@@ -109,15 +113,15 @@ def _check_dense(name: str, t: torch.Tensor, shape, sparse: RoDeCSR):
 
 
 def rode_sddmm(sparse_matrix: RoDeCSR, lhs: torch.Tensor, rhs: torch.Tensor) -> torch.Tensor:
-    """out = S ⊙ (lhs @ rhs^T) sampled at the stored entries of S; returns values [nnz]
-    (mirrors ``rode_sddmm.py:194-248``)."""
+    """out = S ⊙ (lhs @ rhs^T) sampled at the stored entries of S; returns values [nnz], zero for entries that
+    belong to no row (mirrors ``rode_sddmm.py:194-248``)."""
     m, n, k = sparse_matrix.m, sparse_matrix.n, sparse_matrix.k
     _check_dense("lhs_matrix", lhs, (m, k), sparse_matrix)
     _check_dense("rhs_matrix", rhs, (n, k), sparse_matrix)
     return rode_sddmm_cuda.sddmm_forward(
         sparse_matrix.block_indices, sparse_matrix.residue_indices, sparse_matrix.st_offsets, sparse_matrix.m1,
         sparse_matrix.m2, sparse_matrix.row_offsets, sparse_matrix.column_indices, sparse_matrix.values, m, n,
-        lhs.contiguous(), rhs.contiguous(), k)
+        lhs.contiguous(), rhs.contiguous(), k, sparse_matrix._entry_range == (0, sparse_matrix.values.numel()))
 
 
 def rode_spmm(sparse_matrix: RoDeCSR, dense: torch.Tensor, hints: bool = True) -> torch.Tensor:

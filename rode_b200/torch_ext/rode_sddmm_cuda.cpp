@@ -13,7 +13,9 @@
 //   * sddmm_forward launches on torch's current stream, where block and residue part run side by
 //     side as programmatic dependents, instead of creating, synchronising and destroying two
 //     streams per call (RoDe_SDDMM/rode_sddmm_cuda.cu:203-246); it does not block the host.
-//   * k_version may also be 64.
+//   * k_version may be any multiple of 4 up to 256.
+//   * covers_values (default false) says that row_offsets runs from 0 to the number of values, so that the result
+//     need not be zero-filled first.
 //   * spmm_forward and hot_columns are new: the reference has no Python entry for SpMM.
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
@@ -82,7 +84,7 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, int, int> py_preprocess(
 torch::Tensor py_sddmm_forward(torch::Tensor block_indices, torch::Tensor residue_indices, torch::Tensor st_offsets,
                                  int m1, int m2, torch::Tensor row_offsets, torch::Tensor column_indices,
                                  torch::Tensor values, int m, int n, torch::Tensor lhs_matrix,
-                                 torch::Tensor rhs_matrix, int k_version) {
+                                 torch::Tensor rhs_matrix, int k_version, bool covers_values) {
     RODE_CHECK_INPUT(block_indices);
     RODE_CHECK_INPUT(residue_indices);
     RODE_CHECK_INPUT(st_offsets);
@@ -111,8 +113,10 @@ torch::Tensor py_sddmm_forward(torch::Tensor block_indices, torch::Tensor residu
 
     const c10::cuda::CUDAGuard guard(values.device());
     if (m1 == 0 && m2 == 0) return torch::zeros({values.size(0)}, values.options());
-    // every stored entry lies in a block segment or a residue row, so every element is written
-    torch::Tensor out = empty_cuda({values.size(0)}, torch::kFloat32, values.device());
+    // Entries outside [row_offsets[0], row_offsets[m]) belong to no row (a row pointer cut out of a larger one, padding
+    // behind the last row) and are zero, as the reference returns them; the kernels write all others.
+    torch::Tensor out = covers_values ? empty_cuda({values.size(0)}, torch::kFloat32, values.device())
+                                      : torch::zeros({values.size(0)}, values.options());
     const cudaStream_t s = at::cuda::getCurrentCUDAStream(values.device().index()).stream();
     check_status(rode_sddmm_f32(m1, m2, n, k, block_indices.data_ptr<int>(), residue_indices.data_ptr<int>(),
                                 st_offsets.data_ptr<int>(), row_offsets.data_ptr<int>(), column_indices.data_ptr<int>(),
@@ -211,7 +215,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("sddmm_forward", &py_sddmm_forward, "RoDe SDDMM forward (CUDA)", py::arg("block_indices"),
           py::arg("residue_indices"), py::arg("st_offsets"), py::arg("m1"), py::arg("m2"), py::arg("row_offsets"),
           py::arg("column_indices"), py::arg("values"), py::arg("m"), py::arg("n"), py::arg("lhs_matrix"),
-          py::arg("rhs_matrix"), py::arg("k_version"));
+          py::arg("rhs_matrix"), py::arg("k_version"), py::arg("covers_values") = false);
     m.def("spmm_forward", &py_spmm_forward, "RoDe SpMM forward (CUDA)", py::arg("block_indices"),
           py::arg("residue_indices"), py::arg("st_offsets"), py::arg("m1"), py::arg("m2"), py::arg("row_offsets"),
           py::arg("column_indices"), py::arg("values"), py::arg("m"), py::arg("k"), py::arg("dense"),

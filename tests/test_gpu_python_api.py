@@ -123,3 +123,36 @@ def test_launches_on_the_current_stream_without_blocking(api):
         total = scaled.sum()
     s.synchronize()
     assert torch.allclose(total, 2 * base.sum(), rtol=1e-4)
+
+
+@pytest.mark.parametrize("k", [32, 64, 128, 100])
+def test_entries_that_belong_to_no_row_are_zero(api, oracle_cpu, k):
+    """A row pointer cut out of a larger one, with the larger one's columns and values: the entries in front of the first
+    and behind the last row are zero in the SDDMM's result, whatever the allocator's memory held before; SpMM ignores them."""
+    from rode_b200 import capi
+    from rode_b200 import workloads as W
+
+    A = W.zipf_rows(m=4096, n=3000, cap=1500, mean=20)
+    first, last = 1001, 3003
+    rp = A.row_ptr[first: last + 1].contiguous()
+    lo, hi = int(rp[0]), int(rp[-1])
+    assert 0 < lo < hi < A.nnz
+    S = api.RoDeCSR(rp, A.col, A.val, torch.device("cuda"), last - first, A.n, k=k)
+    lhs, rhs = W.dense(last - first, k, seed=5), W.dense(A.n, k, seed=6)
+    part = A.rows(first, last)
+    truth = oracle_cpu.sddmm_f64acc(part.row_ptr.numpy(), part.col.numpy(), part.val.numpy(), lhs.numpy(), rhs.numpy())
+    meta = capi.RodeMeta(S.block_indices, S.st_offsets, S.residue_indices, S.m1, S.m2, 0, 32, 4)
+    calls = (lambda: api.rode_sddmm(S, lhs.cuda(), rhs.cuda()),
+             lambda: capi.sddmm(meta, S.row_offsets, S.column_indices, S.values, lhs.cuda(), rhs.cuda()),
+             lambda: api.rode_sddmm_cuda.sddmm_forward(S.block_indices, S.residue_indices, S.st_offsets, S.m1, S.m2,
+                                                       S.row_offsets, S.column_indices, S.values, S.m, S.n, lhs.cuda(),
+                                                       rhs.cuda(), k))
+    for call in calls:
+        dirty = [torch.full((A.nnz,), float("nan"), device="cuda") for _ in range(4)]  # what a fresh result may be made of
+        del dirty
+        out = call()
+        assert bool((out[:lo] == 0).all()) and bool((out[hi:] == 0).all())
+        assert np.allclose(out[lo:hi].cpu().numpy(), truth, rtol=1e-5, atol=2e-6 * (k / 32))
+    X = W.dense(A.n, 32, seed=7)
+    want = oracle_cpu.spmm_f64acc(part.row_ptr.numpy(), part.col.numpy(), part.val.numpy(), X.numpy())
+    assert np.allclose(api.rode_spmm(S, X.cuda()).cpu().numpy(), want, rtol=1e-5, atol=1e-4)
