@@ -175,15 +175,12 @@ torch::Tensor py_spmm_forward(torch::Tensor block_indices, torch::Tensor residue
     const c10::cuda::CUDAGuard guard(values.device());
     if (m1 == 0 && m2 == 0) return torch::zeros({m, n}, dense.options());
     torch::Tensor out = empty_cuda({m, n}, dense.scalar_type(), dense.device());  // every row is written
-    // Without segments the workspace holds the claim counters of the persistent residue kernel only.  That form starts at
-    // 16 waves of 32 warps per SM with 32 rows each, counted over the column tiles of 512 bytes: 2.4 million row tiles on
-    // 148 SMs (and no fewer than half a million on a part of 32).  Smaller products, whose time is host work, do
-    // without the allocation.
+    // Without segments the workspace would hold the claim counters of the persistent residue kernel only, which
+    // lists of less than half a million rows do not use.
     size_t ws_bytes = 0;
     torch::Tensor ws;
     void *ws_ptr = nullptr;
-    const long long column_tiles = (static_cast<long long>(n) * dense.element_size() + 511) / 512;
-    if (m1 > 0 || m * column_tiles >= 1 << 19) {
+    if (m1 > 0 || m >= 1 << 19) {
         check_status(rode_spmm_workspace_bytes(m1, n, static_cast<int>(dense.element_size()), &ws_bytes));
         ws = empty_cuda({static_cast<long long>(ws_bytes)}, torch::kUInt8, dense.device());
         ws_ptr = ws.data_ptr();

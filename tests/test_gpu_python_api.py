@@ -156,28 +156,3 @@ def test_entries_that_belong_to_no_row_are_zero(api, oracle_cpu, k):
     X = W.dense(A.n, 32, seed=7)
     want = oracle_cpu.spmm_f64acc(part.row_ptr.numpy(), part.col.numpy(), part.val.numpy(), X.numpy())
     assert np.allclose(api.rode_spmm(S, X.cuda()).cpu().numpy(), want, rtol=1e-5, atol=1e-4)
-
-
-@pytest.mark.parametrize("m,width,claims", [(310_000, 1024, True), (490_000, 640, True), (300_000, 1024, False)])
-def test_wide_products_of_short_rows_claim_their_rows(api, oracle_cpu, m, width, claims):
-    """Without segments the residue kernel still becomes a persistent grid from 16 waves of work on, counted over the
-    column tiles; its claim counters (a memset node in front of it) need a workspace from the binding."""
-    from rode_b200 import workloads as W
-    from tests.helpers import graph_nodes
-
-    lens = torch.arange(m, device="cuda") % 4
-    rp = torch.zeros(m + 1, dtype=torch.int64, device="cuda")
-    torch.cumsum(lens, 0, out=rp[1:])
-    nnz = int(rp[-1])
-    col = (torch.arange(nnz, device="cuda") * 37 % 500).to(torch.int32)
-    S = api.RoDeCSR(rp.to(torch.int32), col, W.dense(nnz, 1, device="cuda", seed=1).flatten(), torch.device("cuda"), m, 500, k=32)
-    X = W.dense(500, width, device="cuda", seed=2)
-    assert S.m1 == 0
-    C = api.rode_spmm(S, X, hints=False)
-    nodes = graph_nodes(lambda: api.rode_spmm(S, X, hints=False))
-    assert ("memset" in nodes) == claims and sum("spmm_rows" in name for name in nodes) == 1, nodes
-    rows = torch.randint(0, m, (200,), device="cuda")
-    for r in rows.tolist() + [0, m - 1]:
-        lo, hi = int(rp[r]), int(rp[r + 1])
-        want = (S.values[lo:hi].double()[:, None] * X[col[lo:hi].long()].double()).sum(0)
-        assert torch.allclose(C[r].double(), want, rtol=1e-5, atol=1e-6)
