@@ -116,22 +116,26 @@ constexpr int kSmallGridWarps = RODE_SPMM_WIDE_ROWS_CTA_WARPS;  // rows (warps) 
 #ifndef RODE_SPMM_FULL_CHUNK_PATH
 #define RODE_SPMM_FULL_CHUNK_PATH 1
 #endif
-// Claim counters of the persistent block kernel: one int per column tile, at the end of the workspace.
+// Claim counters of the persistent kernels, at the end of the workspace: one int per column tile for the block kernel, then
+// as many for the rows.
 constexpr size_t kCounterBytes = 256;
-constexpr unsigned kMaxCounterTiles = kCounterBytes / sizeof(int);
-// Residue-row kernel of the 512-byte tile as a persistent grid too (1) or one CTA per bundle of rows (0).
-#ifndef RODE_SPMM_PERSISTENT_ROWS
-#define RODE_SPMM_PERSISTENT_ROWS 1
-#endif
-// A grid becomes persistent from this many resident waves of work on: with fewer segments per warp
-// the claimed order's tail (one long segment claimed last) costs more than the launch gaps it
-// saves (measured: gain from about 20 segments per warp, loss below 10).
+constexpr int kClaimTiles = 2;
+// A grid becomes persistent (one resident wave of so many CTAs per SM, whose warps claim segments or bundles of rows)
+// from so many resident waves of work on: with fewer segments per warp the claimed order's tail (one long segment claimed
+// last) costs more than the launch gaps it saves (measured: gain from about 20 segments per warp, loss below 10).  Dense
+// rows of more than one and a half column tiles keep one CTA per segment or bundle: such a grid walks its tiles one after
+// the other, and the slice of the dense operand that a tile gathers from stays in the L2, where one resident wave over all
+// tiles works on all slices at once (ms, persistent / not: Zipf 671,008 rows of mean 40, N = 224 3.53 / 3.12, N = 512
+// 7.91 / 6.56; R-MAT 21 N = 224 2.40 / 2.29, N = 384 4.74 / 3.88; 1,000,000 rows of 0 to 12 and 100,000 columns, N = 512 1.55 /
+// 0.94).  Below that the second tile is the smaller part of the row, and gathering a row's two parts close together pays
+// (N = 132 and 160: Zipf 2.37 / 2.61 and 2.42 / 2.46, R-MAT 21 1.91 / 2.09 and 1.87 / 1.97; N = 192: Zipf 2.84 / 2.59, R-MAT
+// 20 of 40 per row 2.20 / 2.33).
 constexpr int kPersistentMinWaves = 16;
-// Block kernel as a persistent grid: CTAs per SM of the one wave that is launched (0 = one CTA per
-// segment instead).
-#ifndef RODE_SPMM_PERSISTENT_CTAS_PER_SM
-#define RODE_SPMM_PERSISTENT_CTAS_PER_SM 32
-#endif
+constexpr int kPersistentCtasPerSm = 32;
+template <typename T>
+constexpr bool claims_work(int n, unsigned tiles) {  // (fp64, bound by DRAM on twice the bytes, measured 5 % slower with it)
+    return sizeof(T) == 4 && tiles <= kClaimTiles && static_cast<long long>(n) * sizeof(T) <= 768;
+}
 // Block grids of at most so many segments per SM give a segment four or two warps, which take its chunks in turn and add
 // their rows through shared memory: the time of such a grid is the chain of batches of its longest segment, beyond that
 // it is its throughput.  us, one warp with 8 rows in flight / one warp with a whole chunk in flight (163 registers, which
@@ -1071,21 +1075,17 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
     if (m1 > 0) {
         // fewer warps than two full waves of 32 per SM: no hints, no claims
         const bool small_grid = static_cast<long long>(m1) * tiles <= 2LL * 32 * sm_count();
-        // large grids: one resident wave of CTAs whose warps claim segments from counters (one per
-        // column tile) at the end of the workspace, zeroed on the stream before the launch
+        // large grids: one resident wave of CTAs whose warps claim segments from counters at the end of the workspace,
+        // zeroed on the stream before the launch
         const int ctas_needed = (m1 + kCtaWarps - 1) / kCtaWarps;
-        const int resident = RODE_SPMM_PERSISTENT_CTAS_PER_SM * sm_count();
-        // (fp32 only: the fp64 kernels, bound by DRAM on twice the bytes, measured 5 % slower with it)
-        const bool persistent = RODE_SPMM_PERSISTENT_CTAS_PER_SM > 0 && sizeof(T) == 4 && !small_grid &&
-                                counters != nullptr &&
-                                tiles <= kMaxCounterTiles / 2 &&
-                                ctas_needed > kPersistentMinWaves * (resident / static_cast<int>(tiles));
-        int *claim = nullptr;
+        const int resident = kPersistentCtasPerSm * sm_count();
+        const int resident_per_tile = resident / static_cast<int>(tiles <= kClaimTiles ? tiles : 1);
+        const bool claims = counters != nullptr && claims_work<T>(n, tiles);
+        const bool persistent = claims && !small_grid && ctas_needed > kPersistentMinWaves * resident_per_tile;
         // in a chain the residue kernel's counters are zeroed here too: nothing may stand between two of its grids
-        counters_clear = chained && counters != nullptr && m2 > 32LL * kPersistentMinWaves * (resident / static_cast<int>(tiles));
-        if (persistent || counters_clear)
-            RODE_CUDA_TRY(cudaMemsetAsync(counters, 0, counters_clear ? kCounterBytes : sizeof(int) * tiles, s1));
-        if (persistent) claim = counters;
+        counters_clear = claims && chained && m2 > 32LL * kPersistentMinWaves * resident_per_tile;
+        if (persistent || counters_clear) RODE_CUDA_TRY(cudaMemsetAsync(counters, 0, 2 * kClaimTiles * sizeof(int), s1));
+        int *claim = persistent ? counters : nullptr;
         dim3 grid(persistent ? (resident + tiles - 1) / tiles : ctas_needed, tiles);
         bool launched = false;
         // Popularity hints: block kernel of the 512-byte tile only.  In the residue-row kernel
@@ -1158,14 +1158,13 @@ int launch_rows(int m2, int n, const T *values, const int *col, const int *row_o
         const long long groups = (static_cast<long long>(m2) + per_group - 1) / per_group;
         constexpr int kGroupsPerCta = kCtaThreads / 32;
         const long long ctas_needed = (groups + kGroupsPerCta - 1) / kGroupsPerCta;
-        const long long resident = static_cast<long long>(RODE_SPMM_PERSISTENT_CTAS_PER_SM) * sm_count();
-        const bool persistent = RODE_SPMM_PERSISTENT_ROWS != 0 && sizeof(T) == 4 && counters != nullptr &&
-                                tiles <= kMaxCounterTiles / 2 && (!chained || counters_clear) &&
+        const long long resident = static_cast<long long>(kPersistentCtasPerSm) * sm_count();
+        const bool persistent = counters != nullptr && claims_work<T>(n, tiles) && (!chained || counters_clear) &&
                                 ctas_needed > kPersistentMinWaves * (resident / tiles);
         int *claim = nullptr;
         if (persistent) {
-            claim = counters + kMaxCounterTiles / 2;  // second half: the residue kernel's counters
-            if (!counters_clear) RODE_CUDA_TRY(cudaMemsetAsync(claim, 0, sizeof(int) * tiles, s2));
+            claim = counters + kClaimTiles;
+            if (!counters_clear) RODE_CUDA_TRY(cudaMemsetAsync(claim, 0, kClaimTiles * sizeof(int), s2));
         }
         const dim3 grid(static_cast<unsigned>(persistent ? (resident + tiles - 1) / tiles : ctas_needed), tiles);
         RODE_CUDA_TRY(launch_chained(spmm_rows<T, 32, kRagged>, grid, dim3(kCtaThreads), s2, chained, m2, per_group, n, values,

@@ -175,8 +175,8 @@ torch::Tensor py_spmm_forward(torch::Tensor block_indices, torch::Tensor residue
     const c10::cuda::CUDAGuard guard(values.device());
     if (m1 == 0 && m2 == 0) return torch::zeros({m, n}, dense.options());
     torch::Tensor out = empty_cuda({m, n}, dense.scalar_type(), dense.device());  // every row is written
-    // Without segments the workspace would hold the claim counters of the persistent residue kernel only, which
-    // lists of less than half a million rows do not use.
+    // Without segments the workspace holds the claim counters of the persistent residue kernel only, which starts at 16
+    // waves of 32 warps per SM with 32 rows each over at most two column tiles: 1.2 million rows on 148 SMs.
     size_t ws_bytes = 0;
     torch::Tensor ws;
     void *ws_ptr = nullptr;

@@ -9,7 +9,8 @@ import torch
 from oracle import ref
 from rode_b200 import capi
 from rode_b200 import workloads as W
-from tests.helpers import (assert_close_to_truth, gpu_inputs, run_reference_spmm, sample_rows_csr, spmm_abs_scale)
+from tests.helpers import (assert_close_to_truth, gpu_inputs, graph_nodes, run_reference_spmm, sample_rows_csr,
+                           spmm_abs_scale)
 
 pytestmark = pytest.mark.gpu
 
@@ -362,3 +363,27 @@ def test_spmm_persistent_grids_on_stream_pairs_in_flight_together():
         torch.cuda.synchronize()
         for out in outs:
             assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("n,claims", [(100, True), (128, True), (132, True), (192, True), (196, False), (256, False), (1024, False)])
+@pytest.mark.parametrize("rows_only", [False, True])    # many segments; many short rows
+def test_which_large_grids_claim_their_work(n, claims, rows_only):
+    """Large grids claim segments or rows from counters (a memset node in front of them), but not for dense rows of more
+    than one and a half column tiles, whose tiles would then all be worked on at once."""
+    per_row, m, cols = (1, 2_500_000, 300) if rows_only else (40, 80_000, 300)
+    m = m if n <= 256 else m // 16                          # (the result of 2.5 million rows: at most 2.6 GB)
+    rp = torch.arange(m + 1, dtype=torch.int32, device="cuda") * per_row
+    col = (torch.arange(m * per_row, device="cuda") * 7 % cols).to(torch.int32)
+    val = W.dense(m, per_row, device="cuda", seed=1).flatten()
+    meta = capi.preprocess(rp, m * per_row)
+    assert meta.m1 == (0 if rows_only else m)
+    B = W.dense(cols, n, device="cuda", seed=2)
+    out = []
+    nodes = graph_nodes(lambda: out.append(capi.spmm(meta, rp, col, val, B)))
+    assert ("memset" in nodes) == claims, nodes
+    del out
+    C = capi.spmm(meta, rp, col, val, B)
+    rows = torch.randint(0, m, (500,), device="cuda")
+    picked = rows[:, None] * per_row + torch.arange(per_row, device="cuda")
+    want = (val[picked].double()[..., None] * B[col[picked].long()].double()).sum(1)
+    assert torch.allclose(C[rows].double(), want, rtol=1e-5, atol=1e-5)
