@@ -67,6 +67,18 @@ __device__ __forceinline__ float dot4(const float4 &a, const float4 &b, float ac
     return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc))));
 }
 
+// Where the dense row of a column starts, seen from a lane's base pointer.  Widths known at compile time: shifts and adds.
+// Ragged ones: one 32 x 32 -> 64 bit multiply by the row's bytes.  (A signed column times an unsigned row length was a
+// 64-bit multiply per gather: R-MAT 21 residue rows K = 96 540 -> 433 us, Pareto 131,072 rows K = 200 297 -> 195.  With four vectors
+// per lane, one multiply per four loads, the row mode is faster with the 64-bit form: stencil 64^3 K = 256 400 against 439 us.)
+template <bool kMultiply>
+__device__ __forceinline__ const float4 *rhs_row(const float4 *lane_base, int c, size_t row_vecs) {
+    if constexpr (kMultiply)
+        return dense_row(lane_base, static_cast<unsigned>(c), static_cast<unsigned>(row_vecs) * 16u);
+    else
+        return lane_base + static_cast<size_t>(c) * row_vecs;
+}
+
 // p[u] = this lane's share of the dot product of nonzero u of the batch (u = 0..NB-1).
 // Returns the complete dot product of nonzero l / (L / NB) - the same value in the L / NB
 // lanes that share those bits.  All L lanes of the group named by gmask take part.
@@ -103,11 +115,11 @@ __device__ __forceinline__ void sddmm_one_row(int row, int begin, int end, int l
                                               const float *__restrict__ rhs, float *__restrict__ out, int *stage,
                                               int &stage_buf) {
     constexpr bool kStage = RODE_SDDMM_COLUMNS_IN_SMEM != 0;
-    const unsigned row_vecs = kRagged ? row_vecs_arg : L * VPL;
+    const size_t row_vecs = kRagged ? static_cast<unsigned>(row_vecs_arg) : L * VPL;
     const int l = lane % L;
     const unsigned gmask = group_mask<L>(lane);
     const float4 *rhs_lane = reinterpret_cast<const float4 *>(rhs) + l;
-    auto inside = [&](int v) { return !kRagged || static_cast<unsigned>(l + v * L) < row_vecs; };
+    auto inside = [&](int v) { return !kRagged || static_cast<size_t>(l + v * L) < row_vecs; };
     float4 a[VPL];
 #pragma unroll
     for (int v = 0; v < VPL; ++v)
@@ -151,7 +163,7 @@ __device__ __forceinline__ void sddmm_one_row(int row, int begin, int end, int l
                     for (int v = 0; v < VPL; ++v) {
                         bb[u][v] = make_float4(0.f, 0.f, 0.f, 0.f);
                         if (t < cnt && inside(v))
-                            bb[u][v] = ld_dense(rhs_lane + static_cast<size_t>(cc[u]) * row_vecs + v * L);
+                            bb[u][v] = ld_dense(rhs_row<kRagged && VPL < 4>(rhs_lane, cc[u], row_vecs) + v * L);
                     }
                 }
                 float p[kBatch];
@@ -340,7 +352,7 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
             float *__restrict__ out, int row_vecs_arg, int row_mode_min, int m1, const int *__restrict__ seg_rows) {
     constexpr int G = 32 / L;
     constexpr int kBatch = kLoadsInFlight / VPL;  // nonzeros per batch
-    const size_t row_vecs = kRagged ? static_cast<unsigned>(row_vecs_arg) : L * VPL;  // float4 per dense row (K / 4)
+    const size_t row_vecs = kRagged ? static_cast<size_t>(row_vecs_arg) : L * VPL;  // float4 per dense row (K / 4)
     constexpr int kAlign = 4;             // vec_len of the preprocessing
     constexpr int kBlockK = 32;           // k_block of the preprocessing
     __shared__ int s_end[32];             // stream position where item j ends
@@ -502,7 +514,7 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
                     for (int v = 0; v < VPL; ++v) {
                         bb[u][v] = make_float4(0.f, 0.f, 0.f, 0.f);
                         if (t < cnt && inside(v))
-                            bb[u][v] = ld_dense(rhs_lane + static_cast<size_t>(cc[u]) * row_vecs + v * L);
+                            bb[u][v] = ld_dense(rhs_row<kRagged>(rhs_lane, cc[u], row_vecs) + v * L);
                     }
                 }
                 float p[kBatch];
