@@ -402,12 +402,28 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
     if (total == 0) return;
     if constexpr (LB > 0 && !kSegments) {
         static_assert(LB * VPLB == L * VPL || kRagged, "both lane-group shapes must cover the same dense row");
-        // Short lists give a warp few rows, and there the stream's even split of the nonzeros shortens the dependent
-        // chain: then only rows of about equal length are taken one by one (none longer than twice the mean; 27-point
-        // stencil of 48^3 rows, us: K = 32 42 -> 33, K = 64 66 -> 50, K = 96 136 -> 80; Zipf 100003 x 50021 K = 64 would go 40 ->
-        // 43, R-MAT 17 K = 64 46 -> 48).
-        const bool even = items_per_warp == 32 || (items_per_warp >= 32 / LB && __reduce_max_sync(kFull, len) * items_per_warp <= 2 * total);
-        if (BL > 0 || (even && total >= row_mode_min * items_per_warp)) {  // warp-uniform
+        bool one_by_one = BL > 0;
+        if (BL == 0 && total >= row_mode_min * items_per_warp) {  // warp-uniform
+            if constexpr (L == 32) {
+                // The stream has one lane group and leaves no lane idle.  Row by row a round lasts as long as its longest row
+                // (in batches of UB nonzeros), and the lane groups of shorter rows, or of none, wait: taken where the lanes'
+                // time stays within a quarter of the stream's.  us, rows only, without / with this test (and 16 x 2 lanes
+                // for 8 x 4, which spilled): R-MAT 16 of 43 per row K = 128 26 / 21, Pareto 131,072 rows 80 / 72, 300,000 rows of 0 to 31
+                // 296 / 254, stencil 64^3 227 / 203.
+                int longest = (len + UB - 1) & ~(UB - 1);
+#pragma unroll
+                for (int d = 1; d < 32 / LB; d <<= 1) longest = max(longest, __shfl_xor_sync(kFull, longest, d));
+                one_by_one = __reduce_add_sync(kFull, longest) * (4 * LB * VPLB) <= total * (5 * L * VPL);
+            } else {
+                // Short lists give a warp few rows, and there the stream's even split of the nonzeros shortens the
+                // dependent chain: then only rows of about equal length are taken one by one (none longer than twice the
+                // mean; 27-point stencil of 48^3 rows, us: K = 32 42 -> 33, K = 64 66 -> 50; Zipf 100003 x 50021 K = 64 would go
+                // 40 -> 43, R-MAT 17 K = 64 46 -> 48).
+                one_by_one = items_per_warp == 32 ||
+                             (items_per_warp >= 32 / LB && __reduce_max_sync(kFull, len) * items_per_warp <= 2 * total);
+            }
+        }
+        if (one_by_one) {
             constexpr int GB = 32 / LB;
             const int gb = lane / LB;
             for (int j0 = 0; j0 < items_per_warp; j0 += GB) {
@@ -633,7 +649,7 @@ int items_per_warp(int n_items, int cap, int waves) {
     return static_cast<int>(per);
 }
 
-// L lanes x VPL vectors for the segments and the streams, RL x RVPL (RL = 0: none) for the row mode of the
+// L lanes x VPL vectors for the segments and the streams, RL x RVPL for the row mode of the
 // residue kernel.  kLongSegments: a warp per segment, else up to 32 segments per warp.
 template <int L, int VPL, int BL, int BVPL, int BU, int PL, int PVPL, int PU, int RL,
           int RVPL, int RU, bool kRagged, bool kLongSegments>
@@ -646,13 +662,16 @@ int launch_k(int m1, int m2, int k, const int *block_r_ind, const int *residue_r
     // K = 96: 0.56 ms as a stream, 0.65 to 0.68 ms row by row; stencil, K = 128: 1.78 against 1.57 ms)
     const int row_mode_min = L == 32 ? RODE_SDDMM_ROW_MODE_MIN32 : RODE_SDDMM_ROW_MODE_MIN;
     {
-        // (a row per lane group: on such matrices most residue rows have had their tail taken by a segment)
-        const int per = RL > 0 ? 32 / (RL > 0 ? RL : 1) : 1;
+        // (a row per lane group of the segments' shape: on such matrices most residue rows have had their tail taken by a
+        // segment.  16 x 2 lanes for the rows of K = 100: Zipf 16384 28.0 -> 28.8 us, R-MAT 15, which then takes two launches,
+        // 32.8 -> 39.1)
+        constexpr int kRowU = BL == RL && BVPL == RVPL ? RU : BU;
+        const int per = 32 / BL;
         const long long ctas = static_cast<long long>(m1) + (m2 + per - 1) / per;
         // (a warp per 32-long segment, K = 128, pays while they all fit at once: Bernoulli 4096^2 13.5 us with the two
         // kernels, 14.7 in one; 2000^2 12.3 and 10.3)
         if (m1 > 0 && m2 > 0 && s1 == s2 && ctas <= (kLongSegments ? 4LL : 1LL) * 24 * sm_count()) {
-            sddmm_items<L, VPL, false, kRagged, RL, RVPL, RU, BL, BVPL, BU><<<static_cast<unsigned>(ctas), 32, 0, s1>>>(
+            sddmm_items<L, VPL, false, kRagged, BL, BVPL, kRowU, BL, BVPL, BU><<<static_cast<unsigned>(ctas), 32, 0, s1>>>(
                 m2, per, residue_r_ind, st_off, row_offsets, col, values, lhs, rhs, out, row_vecs, row_mode_min, m1,
                 block_r_ind);
             RODE_CHECK_LAUNCH("rode::sddmm_items<segments and rows>");
@@ -683,7 +702,9 @@ int launch_k(int m1, int m2, int k, const int *block_r_ind, const int *residue_r
         }
     }
     if (m2 > 0) {
-        const int per = items_per_warp(m2, 32, L < 32 ? 2 : 4);
+        int per = items_per_warp(m2, 32, L < 32 ? 2 : 4);
+        // whole rounds of the row mode (30,000 rows of 25, 3 -> 4 rows per warp: K = 128 28.6 -> 25.3 us, K = 96 28.8 -> 22.6)
+        if (L == 32 && per > 1) per = (per + 32 / RL - 1) / (32 / RL) * (32 / RL);
         RODE_CUDA_TRY(launch_chained(sddmm_items<L, VPL, false, kRagged, RL, RVPL, RU>, dim3((m2 + per - 1) / per + 1), dim3(32), s2,
                                      m1 > 0 && s1 == s2, m2, per, residue_r_ind, nullptr, row_offsets, col, values, lhs,
                                      rhs, out, row_vecs, row_mode_min, 0, nullptr));
@@ -725,11 +746,11 @@ extern "C" int rode_sddmm_f32(int m1, int m2, int n, int k, const int *block_r_i
     // 23 3.16 -> 3.29 ms, so persistent grids keep 16 x 1 in the form without a separate full chunk.)
     if (vecs == 8) return RODE_SDDMM_LAUNCH(8, 1, 8, 1, 8, 8, 1, 8, 8, 1, 8, false, true);
     if (vecs == 16) return RODE_SDDMM_LAUNCH(16, 1, 8, 2, 4, 16, 1, 8, 8, 2, 4, false, true);
-    if (vecs == 32) return RODE_SDDMM_LAUNCH(32, 1, 8, 4, 2, 8, 4, 2, 8, 4, 2, false, false);
+    if (vecs == 32) return RODE_SDDMM_LAUNCH(32, 1, 8, 4, 2, 8, 4, 2, 16, 2, 4, false, false);
     if (vecs < 8) return RODE_SDDMM_LAUNCH(8, 1, 8, 1, 8, 8, 1, 8, 8, 1, 8, true, true);
     if (vecs < 16) return RODE_SDDMM_LAUNCH(16, 1, 8, 2, 4, 8, 2, 4, 8, 2, 4, true, true);
     if (vecs <= 24) return RODE_SDDMM_LAUNCH(32, 1, 8, 3, 4, 8, 3, 4, 8, 3, 2, true, true);
-    if (vecs < 32) return RODE_SDDMM_LAUNCH(32, 1, 8, 4, 2, 8, 4, 2, 8, 4, 2, true, true);
+    if (vecs < 32) return RODE_SDDMM_LAUNCH(32, 1, 8, 4, 2, 8, 4, 2, 16, 2, 4, true, true);
     return RODE_SDDMM_LAUNCH(32, 2, 16, 4, 2, 16, 4, 2, 16, 4, 2, true, true);
 #undef RODE_SDDMM_LAUNCH
 }

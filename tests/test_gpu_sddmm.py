@@ -316,3 +316,41 @@ def test_sddmm_threads_that_share_a_stream():
     for mine in outs:
         for out in mine:
             assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("k", [96, 100, 128, 132, 256])
+@pytest.mark.parametrize("rows", [14_000, 28_000, 31_001, 110_000, 440_001])   # 1, 2, 3 (made 4), 8 and 32 rows per warp on 148 SMs
+def test_sddmm_row_mode_of_wide_rows(oracle_cpu, rows, k):
+    """The residue rows of K above 64, where a warp's rows go one by one only if they are about equally long: rows of 26,
+    rows of 0 to 31, rows that alternate between 31 and 16, and a short stretch, so that both forms and warps just on
+    either side of the line occur; every entry is checked in a result filled with NaN."""
+    g = torch.Generator().manual_seed(rows)
+    lens = torch.full((rows,), 26)
+    part = rows // 4
+    lens[part: 2 * part] = torch.randint(0, 32, (part,), generator=g)
+    lens[2 * part: 3 * part] = torch.where(torch.arange(part) % 2 == 0, 28, 16)
+    lens[3 * part: 3 * part + part // 2] = torch.randint(0, 4, (part // 2,), generator=g)
+    rp = torch.zeros(rows + 1, dtype=torch.int64)
+    torch.cumsum(lens, 0, out=rp[1:])
+    nnz, n = int(rp[-1]), 2003
+    col = torch.randint(0, n, (nnz,), generator=g).to(torch.int32)
+    A = W.CSR(rows, n, rp.to(torch.int32), col, torch.rand(nnz, generator=g) * 2 - 1)
+    lhs, rhs = W.dense(rows, k, seed=5), W.dense(n, k, seed=6)
+    d = A.to("cuda")
+    lhs_d, rhs_d = lhs.cuda(), rhs.cuda()
+    for seg in ((32,) if k == 128 else (512,)):
+        meta = capi.preprocess(d.row_ptr, d.nnz, seg, 32, 4)
+        out = torch.full((nnz + 2,), float("nan"), device="cuda")
+        capi.sddmm_raw(0, meta.m2, n, k, meta.block_r_ind.data_ptr(), meta.residue_r_ind.data_ptr(), meta.st_off.data_ptr(),
+                       d.row_ptr.data_ptr(), d.col.data_ptr(), d.val.data_ptr(), lhs_d.data_ptr(),
+                       rhs_d.data_ptr(), out[1:-1].data_ptr())
+        torch.cuda.synchronize()
+        # rows of an aligned length of 32 and more belong to the segments, which were left out
+        short = lens + (rp[:-1] % 4) < 32
+        mine = torch.repeat_interleave(short, lens).numpy()
+        truth = oracle_cpu.sddmm_f64acc(A.row_ptr.numpy(), col.numpy(), A.val.numpy(), lhs.numpy(), rhs.numpy(),
+                                        threads=oracle_cpu.max_threads())
+        got = out[1:-1].cpu().numpy()
+        scale = sddmm_abs_scale(A.row_ptr.numpy(), col.numpy(), A.val.numpy(), lhs.numpy(), rhs.numpy())
+        assert_close_to_truth(got[mine], truth[mine], scale[mine], f"rows={rows} k={k}")
+        assert np.isnan(got[~mine]).all() and bool(torch.isnan(out[0])) and bool(torch.isnan(out[-1]))
