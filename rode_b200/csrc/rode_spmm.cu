@@ -123,18 +123,18 @@ constexpr int kClaimTiles = 2;
 // A grid becomes persistent (one resident wave of so many CTAs per SM, whose warps claim segments or bundles of rows)
 // from so many resident waves of work on: with fewer segments per warp the claimed order's tail (one long segment claimed
 // last) costs more than the launch gaps it saves (measured: gain from about 20 segments per warp, loss below 10).  Dense
-// rows of more than one and a half column tiles keep one CTA per segment or bundle: such a grid walks its tiles one after
-// the other, and the slice of the dense operand that a tile gathers from stays in the L2, where one resident wave over all
-// tiles works on all slices at once (ms, persistent / not: Zipf 671,008 rows of mean 40, N = 224 3.53 / 3.12, N = 512
-// 7.91 / 6.56; R-MAT 21 N = 224 2.40 / 2.29, N = 384 4.74 / 3.88; 1,000,000 rows of 0 to 12 and 100,000 columns, N = 512 1.55 /
-// 0.94).  Below that the second tile is the smaller part of the row, and gathering a row's two parts close together pays
-// (N = 132 and 160: Zipf 2.37 / 2.61 and 2.42 / 2.46, R-MAT 21 1.91 / 2.09 and 1.87 / 1.97; N = 192: Zipf 2.84 / 2.59, R-MAT
-// 20 of 40 per row 2.20 / 2.33).
+// rows of 1.75 column tiles and more keep one CTA per segment or bundle: such a grid walks its tiles one after the other, and
+// the slice of the dense operand that a tile gathers from stays in the L2, where one resident wave over all tiles works
+// on all slices at once (ms, persistent / not: Zipf 671,008 rows of mean 40, N = 224 3.53 / 3.12, N = 512 7.91 / 6.56; R-MAT 21
+// N = 224 2.40 / 2.29, N = 384 4.74 / 3.88; 1,000,000 rows of 0 to 12 and 100,000 columns, N = 512 1.55 / 0.94).  Below that the
+// second tile is the smaller part of the row, and gathering a row's two parts close together pays on graphs (N = 132 and
+// 160: Zipf 2.37 / 2.61 and 2.42 / 2.46, R-MAT 21 1.91 / 2.09 and 1.87 / 1.97; N = 192 and 196: Zipf 2.84 / 2.59, Pareto 200,000 of
+// mean 60 0.97 / 0.88, R-MAT 20 of 40 per row 2.20 / 2.33, R-MAT 18 of 64 0.71 / 0.75).
 constexpr int kPersistentMinWaves = 16;
 constexpr int kPersistentCtasPerSm = 32;
 template <typename T>
 constexpr bool claims_work(int n, unsigned tiles) {  // (fp64, bound by DRAM on twice the bytes, measured 5 % slower with it)
-    return sizeof(T) == 4 && tiles <= kClaimTiles && static_cast<long long>(n) * sizeof(T) <= 768;
+    return sizeof(T) == 4 && tiles <= kClaimTiles && static_cast<long long>(n) * sizeof(T) < 896;
 }
 // Block grids of at most so many segments per SM give a segment four or two warps, which take its chunks in turn and add
 // their rows through shared memory: the time of such a grid is the chain of batches of its longest segment, beyond that

@@ -365,11 +365,11 @@ def test_spmm_persistent_grids_on_stream_pairs_in_flight_together():
             assert torch.equal(out, want)
 
 
-@pytest.mark.parametrize("n,claims", [(100, True), (128, True), (132, True), (192, True), (196, False), (256, False), (1024, False)])
+@pytest.mark.parametrize("n,claims", [(100, True), (128, True), (132, True), (220, True), (224, False), (256, False), (1024, False)])
 @pytest.mark.parametrize("rows_only", [False, True])    # many segments; many short rows
 def test_which_large_grids_claim_their_work(n, claims, rows_only):
     """Large grids claim segments or rows from counters (a memset node in front of them), but not for dense rows of more
-    than one and a half column tiles, whose tiles would then all be worked on at once."""
+    than one and three quarters of a column tile, whose tiles would then all be worked on at once."""
     per_row, m, cols = (1, 2_500_000, 300) if rows_only else (40, 80_000, 300)
     m = m if n <= 256 else m // 16                          # (the result of 2.5 million rows: at most 2.6 GB)
     rp = torch.arange(m + 1, dtype=torch.int32, device="cuda") * per_row
