@@ -144,8 +144,20 @@ constexpr bool claims_work(int n, unsigned tiles) {  // (fp64, bound by DRAM on 
 // 4096^2 (3911) 14.5 / 16.5 / 15 / 17.
 constexpr int kSplit4WarpsPerSm = 16;
 constexpr int kSplit2WarpsPerSm = 22;
-// The mean row is short (and the number of nonzeros known).
-constexpr bool short_rows(long long nnz, long long rows) { return nnz >= 0 && nnz < 20 * rows; }
+// What a call knows of the rows that the residue kernels work on, those of fewer than 32 nonzeros: the number of nonzeros of
+// the matrix (not always, nnz < 0 then) and of segments, which hold at most 543 each.  Their mean is therefore
+// at least (nnz - 543 m1) / rows, and it is no larger than that of all rows.  Matrices with heavier tails than the
+// lower bound can tell apart (Zipf of mean 40: short rows of 2.0; Pareto of mean 32: 11.8) are known by neither.
+constexpr bool rows_hold(long long nnz, long long m1, long long rows, int mean) {  // at least so many on average, surely
+    return nnz >= 0 && nnz - 543 * m1 >= mean * rows;
+}
+// Two rows per lane group in spmm_rows_simple.  us, one / two: rows of 1.6 (Zipf 671,008 N = 64) 353 / 341, of 5.2 (R-MAT 21)
+// 752 / 704, of 7 (2 to 12) 72 / 70, of 27 (stencil) 700 / 724.  In the 128-byte tile long rows lose more: of 9.8 (Pareto
+// 300,007 N = 32) 91.3 / 92.5, of 12 and 16 (Bernoulli 30,000) 8.3 / 10.3 and 11.4 / 13.2, of 19.5 (15 to 24) 62 / 66, of 27 401 / 444;
+// in the wider ones not (of 16 N = 64 16.1 / 15.3, fp64 N = 32 16.0 / 14.4).
+constexpr bool short_rows(long long nnz, long long m1, long long rows, int tile_bytes) {
+    return nnz >= 0 && nnz < 20 * rows && !(tile_bytes == 128 && rows_hold(nnz, m1, rows, 10));
+}
 // 16-byte units a lane keeps in flight per batch (dense rows per batch = this * 16 / bytes per load / VPL).
 constexpr int kLoadsInFlight = 8;
 
@@ -1056,7 +1068,7 @@ spmm_rows_wide(int m2, int n, const T *__restrict__ values, const int *__restric
 
 template <typename T, int VB, int L, int VPL, bool kRagged>
 int launch_rows(int m2, int n, const T *values, const int *col, const int *row_offsets, const int *residue_r_ind,
-                const T *B, T *C, int *counters, bool chained, bool counters_clear, long long nnz,
+                const T *B, T *C, int *counters, bool chained, bool counters_clear, bool two_rows,
                 cudaStream_t s2);
 
 // Block kernel of shape (VB bytes per load, L lanes, VPL loads per lane) and residue-row kernel of shape (RVB, RL, RVPL);
@@ -1127,7 +1139,7 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
     // they are a plain launch.
     if (m2 > 0 && !rows_done) {
         if (int rc = launch_rows<T, RVB, RL, RVPL, kRowsRagged>(m2, n, values, col, row_offsets, residue_r_ind, B, C, counters,
-                                                            chained, counters_clear, nnz, s2))
+                                                            chained, counters_clear, short_rows(nnz, m1, m2, RVB * RL * RVPL), s2))
             return rc;
     }
     if (m1 > 1) {  // (a row that was cut has two segments at least)
@@ -1145,7 +1157,7 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
 
 template <typename T, int VB, int L, int VPL, bool kRagged>
 int launch_rows(int m2, int n, const T *values, const int *col, const int *row_offsets, const int *residue_r_ind,
-                const T *B, T *C, int *counters, bool chained, bool counters_clear, long long nnz,
+                const T *B, T *C, int *counters, bool chained, bool counters_clear, bool two_rows,
                 cudaStream_t s2) {
     constexpr int kTileWidth = L * VPL * VecB<T, VB>::kLen;
     const unsigned tiles = static_cast<unsigned>(kRagged ? (n + kTileWidth - 1) / kTileWidth : n / kTileWidth);
@@ -1174,10 +1186,8 @@ int launch_rows(int m2, int n, const T *values, const int *col, const int *row_o
         RODE_CUDA_TRY(launch_chained(spmm_rows_wide<T, VB, L, VPL, kRagged>, grid, dim3(32 * kSmallGridWarps), s2, chained, m2,
                                      n, values, col, row_offsets, residue_r_ind, B, C));
     } else {
-        // Two rows per lane group where rows are short on average (and their number is known): both rows' bounds and
-        // first columns are then fetched together, and a short row's life is that chain of loads.  Zipf 671,008
-        // rows N = 64 206 -> 191 us, 3.2 M rows N = 32 646 -> 610, R-MAT 21 N = 64 741 -> 694; long even rows lose it again
-        // to the longer life of a warp (stencil N = 96 1.33 -> 1.50 ms, 27 per row; Pareto 2^20, 32 per row, 5 %).
+        // Two rows per lane group where rows are short: both rows' bounds and first columns are then fetched together, and a
+        // short row's life is that chain of loads; long even rows lose it again to the longer life of a warp.
         auto launch = [&](auto two) {
             constexpr int R = decltype(two)::value ? 2 : 1;
             constexpr int kRowsPerCta = R * kRowsCtaThreads / L;
@@ -1185,7 +1195,7 @@ int launch_rows(int m2, int n, const T *values, const int *col, const int *row_o
             return launch_chained(spmm_rows_simple<T, VB, L, VPL, R, kRagged>, grid, dim3(kRowsCtaThreads), s2, chained, m2, n,
                                   values, col, row_offsets, residue_r_ind, B, C);
         };
-        if (short_rows(nnz, m2))
+        if (two_rows)
             RODE_CUDA_TRY(launch(std::true_type{}));
         else
             RODE_CUDA_TRY(launch(std::false_type{}));
@@ -1251,18 +1261,31 @@ int spmm(int m1, int m2, int k, int n, const T *values, const int *col, const in
     // Widths the tiles do not divide (any other multiple of 4 columns; the reference has none of
     // them): the narrowest shape that covers the row, or 512-byte tiles with a partly empty last
     // one.  Always 16-byte loads, no popularity hints.
-    // Widths of whole lines that the 512-byte tile does not divide (N = 96, 160, 192, 224 ...; fp64: N = 48): 512-byte tiles with a
-    // partly idle last one all the same, instead of up to seven passes over the sparse matrix with narrow ones.  The
-    // residue rows follow where they are short on average; long even rows (27-point stencil) keep the narrow per-row
-    // kernel, which neighbouring rows' L1 hits favour (N = 96 1.18 against 1.48 ms).  us, narrow -> wide: R-MAT 21 N = 96 1411
-    // -> 954, N = 160 2627 -> 1948, N = 224 3701 -> 2449; Pareto 2^20 N = 96 2309 -> 1756, N = 224 5897 -> 4493; Bernoulli 4096^2 N = 96
-    // 20.7 -> 12.5; Zipf 65536 N = 160 70 -> 74.  fp64, wider: 497 -> 568 on Pareto (300,007 rows, N = 80).
-    if (vecs % 8 == 0 && vecs > 16 && vecs % 32 != 0 && (sizeof(T) == 4 || vecs == 24)) {
+    // Widths of whole lines that the 512-byte tile does not divide (N = 96, 160, 192, 224 ...): 512-byte tiles with a
+    // partly idle last one all the same, instead of up to seven passes over the sparse matrix with narrow ones.  us, narrow ->
+    // wide: R-MAT 21 N = 96 1411 -> 954, N = 160 2627 -> 1948, N = 224 3701 -> 2449; Pareto 2^20 N = 96 2309 -> 1756, N = 224
+    // 5897 -> 4493; Bernoulli 4096^2 N = 96 20.7 -> 12.5; Zipf 65536 N = 160 70 -> 74.  fp64 only where it is one tile instead
+    // of three passes (R-MAT 20 692 -> 517, 30,000 rows of 25 41 -> 31, Zipf 300,007 of mean 40 369 -> 373): several tiles lose what
+    // the narrow ones' passes over a slice of the operand keep in the L2 (Zipf of mean 40 N = 112 848 -> 917, N = 144 1092 ->
+    // 1356, Pareto 300,007 N = 80 496 -> 566).
+    //
+    // The residue rows take wide tiles too unless they are long (narrow / wide, us): of 2 (0 to 4) N = 96 61 / 52, N = 160 100 /
+    // 100, N = 224 138 / 117; of 4 82 / 72, 133 / 143, 184 / 163; of 7 102 / 101, 166 / 197, 233 / 226; of 10 (8 to 12) 112 / 123,
+    // 183 / 250, 259 / 286; of 19.5 190 / 210, 312 / 422, 455 / 489; uneven ones of 5.9 (R-MAT 18) 152 / 138, 280 / 253, 330 / 266, of
+    // 11.5 (Pareto 2^20) 1806 / 1718, 3218 / 3211, 4611 / 4286.  So the line lies at 6 where the tiles are three quarters full or
+    // more, and at 2 for N = 160.  Beyond a mean of 20 over all rows the narrow form is taken, which loses less on even rows
+    // (30,000 rows of 25 N = 96 27 / 31, N = 160 44 / 53) than it gives away on uneven ones (Zipf of mean 40 412 / 376);
+    // in fp64, where it gives away more, only if there are fewer segments than one for 20 rows (30,000 rows of 21 27 / 30) or
+    // more than one for 8 (rows of 25 31 / 33), else not (Zipf of mean 40 415 / 373, Pareto 300,007 306 / 294).
+    if (vecs % 8 == 0 && vecs > 16 && vecs % 32 != 0 && (sizeof(T) == 4 || vecs < 32)) {
+        const int full = 4 * vecs >= 3 * 32 * ((vecs + 31) / 32) ? 6 : 2;
+        const bool wide_rows = nnz >= 0 && !rows_hold(nnz, m1, m2, full) &&
+                               (nnz < 20LL * m2 || (sizeof(T) == 8 && 20LL * m1 >= m2 && 8LL * m1 <= m2));
 #define RODE_WIDE_BLOCK(rows_shape, rows_ragged)                                                                  \
     launch_shape<T, 16, RODE_SPMM_SHAPE_32 / 100, RODE_SPMM_SHAPE_32 % 100, 16, (rows_shape) / 100, (rows_shape) % 100, true, \
                  rows_ragged>(m1, m2, k, n, values, col, row_offsets, block_r_ind, residue_r_ind, st_off, B, C, partial,     \
                               counters, nullptr, nnz, stream1, stream2)
-        if (short_rows(nnz, m2)) return RODE_WIDE_BLOCK(RODE_SPMM_ROWS_SHAPE_32, true);
+        if (wide_rows) return RODE_WIDE_BLOCK(RODE_SPMM_ROWS_SHAPE_32, true);
         if (vecs % 16 == 0) return RODE_WIDE_BLOCK(RODE_SPMM_SHAPE_16, false);
         if (aligned_to(B, 32) && aligned_to(C, 32))
             return launch_shape<T, 16, RODE_SPMM_SHAPE_32 / 100, RODE_SPMM_SHAPE_32 % 100, 32, 4, 1, true, false>(

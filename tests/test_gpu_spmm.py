@@ -387,3 +387,51 @@ def test_which_large_grids_claim_their_work(n, claims, rows_only):
     picked = rows[:, None] * per_row + torch.arange(per_row, device="cuda")
     want = (val[picked].double()[..., None] * B[col[picked].long()].double()).sum(1)
     assert torch.allclose(C[rows].double(), want, rtol=1e-5, atol=1e-5)
+
+
+def _rows_of(lengths, n_cols, seed=3):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    rp = torch.zeros(lengths.numel() + 1, dtype=torch.int64, device="cuda")
+    torch.cumsum(lengths, 0, out=rp[1:])
+    nnz = int(rp[-1])
+    return W.CSR(lengths.numel(), n_cols, rp.to(torch.int32),
+                 torch.randint(0, n_cols, (nnz,), device="cuda", generator=g).to(torch.int32),
+                 torch.rand(nnz, device="cuda", generator=g) * 2 - 1)
+
+
+@pytest.mark.parametrize("lo,hi,heavy,two_rows,wide96,wide160", [
+    (1, 2, 0, True, True, True),           # mean 1.5
+    (2, 3, 0, True, True, False),          # 2.5
+    (4, 6, 0, True, True, False),          # 5
+    (5, 8, 0, True, False, False),         # 6.5
+    (9, 10, 0, True, False, False),        # 9.5
+    (10, 11, 0, False, False, False),      # 10.5
+    (15, 24, 0, False, False, False),      # long and even, with fewer than 20 per row
+    (1, 3, 3000, True, True, True),        # 3000 rows of 600 that the bounds cannot rule out as the bulk
+])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_row_kernels_follow_what_is_known_of_the_short_rows(lo, hi, heavy, two_rows, wide96, wide160, dtype):
+    """Two rows per lane group, and wide tiles for the rows of widths that the 512-byte tile does not divide, only where
+    the rows without a block part are not long for sure: by the kernels in a captured call, and the results at both."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    lens = torch.randint(lo, hi + 1, (100_000,), device="cuda", generator=g)
+    if heavy:
+        lens[torch.randperm(100_000, device="cuda", generator=g)[:heavy]] = 600
+    A = _rows_of(lens, 4001)
+    meta = capi.preprocess(A.row_ptr, A.nnz)
+    val = A.val.to(dtype)
+    size = val.element_size()
+    rows = torch.cat([torch.topk(lens, 5).indices, torch.randint(0, A.m, (300,), device="cuda", generator=g)])
+    for n, check in ((128 // size, lambda k: ("spmm_rows_simple" in k and "ELi2ELb" in k) == two_rows),
+                     (384 // size, lambda k: ("spmm_rows_simple" not in k) == wide96),
+                     (640 // size, lambda k: ("spmm_rows_simple" not in k) == (wide160 and size == 4))):
+        B = W.dense(A.n, n, device="cuda", seed=n, dtype=dtype)
+        out = []
+        nodes = [k for k in graph_nodes(lambda: out.append(capi.spmm(meta, A.row_ptr, A.col, val, B))) if "spmm_rows" in k]
+        assert len(nodes) == 1 and check(nodes[0]), (n, nodes)
+        del out
+        C = capi.spmm(meta, A.row_ptr, A.col, val, B)
+        for r in rows.tolist():
+            a, b = int(A.row_ptr[r]), int(A.row_ptr[r + 1])
+            want = (val[a:b].double()[:, None] * B[A.col[a:b].long()].double()).sum(0)
+            assert torch.allclose(C[r].double(), want, rtol=1e-5, atol=2e-5 if size == 4 else 1e-12)
