@@ -25,8 +25,7 @@ constexpr int kThreads = 256;
 constexpr int kTile = 2048;    // rows per CTA
 constexpr int kWarps = kThreads / 32;
 constexpr int kShortRow = 8;   // rows of up to so many segments are written by one thread, others by a warp
-// Scratch: running sums of the tiles, one int2 each (callers provide for one more).
-constexpr int kScratchHeader = 1;
+// Scratch: running sums of the tiles, one int2 each.
 
 // The three parameters of the decomposition.  kPow2 = all of them are powers of two (every
 // parameter set the reference uses: (512, 32, 4) and (32, 32, 4)): quotients and remainders
@@ -482,7 +481,7 @@ int preprocess_reference_signature(int seg_len, int k_block, int vec_len, int M,
 // code this name is only a handle; the device address comes from cudaGetSymbolAddress.
 constexpr int kNoAllocMaxRows = 1 << 24;
 constexpr int kNoAllocTiles = kNoAllocMaxRows / kTile;
-static __device__ __align__(256) int2 g_noalloc_tile_scratch[kScratchHeader + kNoAllocTiles];
+static __device__ __align__(256) int2 g_noalloc_tile_scratch[kNoAllocTiles];
 
 // Device address of the scratch array on the current device, looked up once per device.
 int noalloc_scratch(int2 **out) {
@@ -509,7 +508,7 @@ int rode_preprocess_workspace_bytes(int M, size_t *bytes) {
     if (bytes == nullptr || M < 0)
         return rode::fail(RODE_ERR_INVALID_ARGUMENT, "preprocess_workspace_bytes: bad argument");
     const size_t tiles = static_cast<size_t>(rode::preprocess_tiles(M));
-    *bytes = (tiles + rode::kScratchHeader) * sizeof(int2);
+    *bytes = (tiles + 1) * sizeof(int2);  // one entry spare, so that no matrix needs an empty buffer
     return RODE_OK;
 }
 

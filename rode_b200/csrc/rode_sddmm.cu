@@ -48,18 +48,10 @@
 namespace rode {
 namespace {
 
-// Mean number of nonzeros per row from which a warp of the residue-row kernel takes its rows one by one.
-#ifndef RODE_SDDMM_ROW_MODE_MIN
-#define RODE_SDDMM_ROW_MODE_MIN 6
-#endif
-// 1: the column indices of a chunk reach the lanes of a group through shared memory (stored
-// once, read as 16-byte broadcast runs); 0: by one shuffle per nonzero.
-#ifndef RODE_SDDMM_COLUMNS_IN_SMEM
-#define RODE_SDDMM_COLUMNS_IN_SMEM 1
-#endif
-#ifndef RODE_SDDMM_ROW_MODE_MIN32
-#define RODE_SDDMM_ROW_MODE_MIN32 16
-#endif
+// Mean number of nonzeros per row from which a warp of the residue-row kernel takes its rows one by one, where the stream
+// has several lane groups and where it has one.
+constexpr int kRowModeMin = 6;
+constexpr int kRowModeMin32 = 16;
 constexpr int kLoadsInFlight = 8;  // 16-byte loads per lane per batch
 constexpr unsigned kFull = 0xffffffffu;
 
@@ -114,7 +106,6 @@ __device__ __forceinline__ void sddmm_one_row(int row, int begin, int end, int l
                                               const float *__restrict__ values, const float *__restrict__ lhs,
                                               const float *__restrict__ rhs, float *__restrict__ out, int *stage,
                                               int &stage_buf) {
-    constexpr bool kStage = RODE_SDDMM_COLUMNS_IN_SMEM != 0;
     const size_t row_vecs = kRagged ? static_cast<unsigned>(row_vecs_arg) : L * VPL;
     const int l = lane % L;
     const unsigned gmask = group_mask<L>(lane);
@@ -144,21 +135,18 @@ __device__ __forceinline__ void sddmm_one_row(int row, int begin, int end, int l
         const int cnt = min(L, end - base);
         float mine = 0.f;
         int *my_stage = stage + stage_buf * 32 + (lane - l);  // this group's region of the buffer
-        if constexpr (kStage) {
-            my_stage[l] = c;
-            __syncwarp(gmask);
-            stage_buf ^= 1;
-        }
+        my_stage[l] = c;
+        __syncwarp(gmask);
+        stage_buf ^= 1;
 #pragma unroll
         for (int b = 0; b < L / kBatch; ++b) {
             if (b * kBatch < cnt) {  // uniform inside the group
                 float4 bb[kBatch][VPL];
                 int cc[kBatch];
-                if constexpr (kStage) ld_shared_run<kBatch>(my_stage + b * kBatch, cc);
+                ld_shared_run<kBatch>(my_stage + b * kBatch, cc);
 #pragma unroll
                 for (int u = 0; u < kBatch; ++u) {
                     const int t = b * kBatch + u;
-                    if constexpr (!kStage) cc[u] = __shfl_sync(gmask, c, t, L);
 #pragma unroll
                     for (int v = 0; v < VPL; ++v) {
                         bb[u][v] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -341,11 +329,9 @@ sddmm_block(int m1, const int *__restrict__ block_r_ind, const int *__restrict__
 // One-warp CTAs per SM the register allocation must allow: 28 (72 registers).  Left to itself the
 // compiler takes 78-80 registers for K = 64 once the chunk staging is in, and the four warps per
 // SM that costs outweigh what the staging gains; 64 registers (32 CTAs) spill.
-#ifndef RODE_SDDMM_ITEMS_MIN_CTAS
-#define RODE_SDDMM_ITEMS_MIN_CTAS 28
-#endif
+constexpr int kItemsCtas = 28;
 template <int L, int VPL, bool kSegments, bool kRagged, int LB, int VPLB, int UB, int BL = 0, int BVPL = 1, int BU = 1>
-__global__ void __launch_bounds__(32, (VPL > 1 || BL > 0) ? 24 : RODE_SDDMM_ITEMS_MIN_CTAS)
+__global__ void __launch_bounds__(32, (VPL > 1 || BL > 0) ? 24 : kItemsCtas)
 sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, const int *__restrict__ st_off,
             const int *__restrict__ row_offsets, const int *__restrict__ column_indices,
             const float *__restrict__ values, const float *__restrict__ lhs, const float *__restrict__ rhs,
@@ -509,23 +495,19 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
         fetch(p0 + (ch + 2) * L + l, e_pre, c_pre, v_pre);
         const int cnt = min(L, p1 - (p0 + ch * L));  // valid nonzeros of this chunk (may be <= 0)
         float mine = 0.f;
-        constexpr bool kStage = RODE_SDDMM_COLUMNS_IN_SMEM != 0 && (kBatch % 4 == 0);
         int *my_stage = &s_col[stage_buf][lane - l];  // this group's region of the chunk buffer
-        if constexpr (kStage) {
-            my_stage[l] = c_cur;
-            __syncwarp();  // every group runs the same number of chunks
-            stage_buf ^= 1;
-        }
+        my_stage[l] = c_cur;
+        __syncwarp();  // every group runs the same number of chunks
+        stage_buf ^= 1;
 #pragma unroll
         for (int b = 0; b < L / kBatch; ++b) {
             if (b * kBatch < cnt) {  // uniform inside the group; no warp-wide shuffles inside
                 float4 bb[kBatch][VPL];
                 int cc[kBatch];
-                if constexpr (kStage) ld_shared_run<kBatch>(my_stage + b * kBatch, cc);
+                ld_shared_run<kBatch>(my_stage + b * kBatch, cc);
 #pragma unroll
                 for (int u = 0; u < kBatch; ++u) {
                     const int t = b * kBatch + u;
-                    if constexpr (!kStage) cc[u] = __shfl_sync(gmask, c_cur, t, L);
 #pragma unroll
                     for (int v = 0; v < VPL; ++v) {
                         bb[u][v] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -649,18 +631,25 @@ int items_per_warp(int n_items, int cap, int waves) {
     return static_cast<int>(per);
 }
 
-// L lanes x VPL vectors for the segments and the streams, RL x RVPL for the row mode of the
-// residue kernel.  kLongSegments: a warp per segment, else up to 32 segments per warp.
-template <int L, int VPL, int BL, int BVPL, int BU, int PL, int PVPL, int PU, int RL,
-          int RVPL, int RU, bool kRagged, bool kLongSegments>
+// A lane group of L lanes x VPL vectors, with U nonzeros per batch.
+template <int L_, int VPL_, int U_>
+struct Shape {
+    static constexpr int L = L_, VPL = VPL_, U = U_;
+};
+// L lanes x VPL vectors for the streams; shapes of the segments (a warp each: kLongSegments, else up to 32 segments per warp
+// run as a stream, and Block serves the small grids) and of the row mode of the residue kernel; Claimed: of the persistent
+// grids of segments.
+template <int L, int VPL, typename Block, typename Rows, bool kRagged, bool kLongSegments, typename Claimed = Block>
 int launch_k(int m1, int m2, int k, const int *block_r_ind, const int *residue_r_ind,
              const int *st_off, const int *row_offsets, const int *col, const float *values, const float *lhs,
              const float *rhs, float *out, cudaStream_t s1, cudaStream_t s2) {
+    constexpr int BL = Block::L, BVPL = Block::VPL, BU = Block::U;
+    constexpr int RL = Rows::L, RVPL = Rows::VPL, RU = Rows::U;
     const int row_vecs = k / 4;
     // nonzeros per row from which a warp takes its rows one by one: where the stream form has one lane group only
     // it balances nothing, but short rows still lose more to the idle lane groups of the row form (R-MAT 21,
     // K = 96: 0.56 ms as a stream, 0.65 to 0.68 ms row by row; stencil, K = 128: 1.78 against 1.57 ms)
-    const int row_mode_min = L == 32 ? RODE_SDDMM_ROW_MODE_MIN32 : RODE_SDDMM_ROW_MODE_MIN;
+    const int row_mode_min = L == 32 ? kRowModeMin32 : kRowModeMin;
     {
         // (a row per lane group of the segments' shape: on such matrices most residue rows have had their tail taken by a
         // segment.  16 x 2 lanes for the rows of K = 100: Zipf 16384 28.0 -> 28.8 us, R-MAT 15, which then takes two launches,
@@ -680,14 +669,14 @@ int launch_k(int m1, int m2, int k, const int *block_r_ind, const int *residue_r
     }
     if (m1 > 0) {
         if constexpr (kLongSegments) {
-            const int resident = block_ctas(BVPL) * sm_count();
+            const int resident = block_ctas(Claimed::VPL) * sm_count();
             ClaimCounter claim;  // holds its lock until the kernel is enqueued
             if (m1 > 16 * resident) {  // from about 16 segments per warp on it pays
                 if (int rc = claim.acquire(s1, s2)) return rc;
             }
             if (claim.ptr != nullptr) {
                 RODE_CUDA_TRY(cudaMemsetAsync(claim.ptr, 0, sizeof(int), s1));
-                sddmm_block<PL, PVPL, PU, true, kRagged><<<resident, 32, 0, s1>>>(
+                sddmm_block<Claimed::L, Claimed::VPL, Claimed::U, true, kRagged><<<resident, 32, 0, s1>>>(
                     m1, block_r_ind, st_off, row_offsets, col, values, lhs, rhs, out, claim.ptr, row_vecs);
             } else {
                 sddmm_block<BL, BVPL, BU, false, kRagged><<<m1, 32, 0, s1>>>(m1, block_r_ind, st_off, row_offsets, col, values,
@@ -740,17 +729,16 @@ extern "C" int rode_sddmm_f32(int m1, int m2, int n, int k, const int *block_r_i
     // the 100003 x 50021 Zipf matrix at K = 96, the 32 x 1 form 0.117 ms.)  The decomposition that goes with
     // K = 128 has 32-long segments, all others 512-long ones.
     const int vecs = k / 4;
-    // (stream shape; block shape and nonzeros per batch, the same for persistent block grids; row-mode shape and
-    // nonzeros per batch.  K = 64: 8 x 2 takes fewer instructions, Pareto 2^18 block grid 119 -> 103 us, Zipf
-    // 65536 29 -> 23 us; matrices of millions of rows are bound by the L2 and DRAM and lose 4 % with it, R-MAT
-    // 23 3.16 -> 3.29 ms, so persistent grids keep 16 x 1 in the form without a separate full chunk.)
-    if (vecs == 8) return RODE_SDDMM_LAUNCH(8, 1, 8, 1, 8, 8, 1, 8, 8, 1, 8, false, true);
-    if (vecs == 16) return RODE_SDDMM_LAUNCH(16, 1, 8, 2, 4, 16, 1, 8, 8, 2, 4, false, true);
-    if (vecs == 32) return RODE_SDDMM_LAUNCH(32, 1, 8, 4, 2, 8, 4, 2, 16, 2, 4, false, false);
-    if (vecs < 8) return RODE_SDDMM_LAUNCH(8, 1, 8, 1, 8, 8, 1, 8, 8, 1, 8, true, true);
-    if (vecs < 16) return RODE_SDDMM_LAUNCH(16, 1, 8, 2, 4, 8, 2, 4, 8, 2, 4, true, true);
-    if (vecs <= 24) return RODE_SDDMM_LAUNCH(32, 1, 8, 3, 4, 8, 3, 4, 8, 3, 2, true, true);
-    if (vecs < 32) return RODE_SDDMM_LAUNCH(32, 1, 8, 4, 2, 8, 4, 2, 16, 2, 4, true, true);
-    return RODE_SDDMM_LAUNCH(32, 2, 16, 4, 2, 16, 4, 2, 16, 4, 2, true, true);
+    // (K = 64: 8 x 2 takes fewer instructions, Pareto 2^18 block grid 119 -> 103 us, Zipf 65536 29 -> 23 us; matrices of
+    // millions of rows lose 4 % with it, each of its loads asking for half of the row, R-MAT 23 3.16 -> 3.29 ms: persistent
+    // grids keep 16 x 1 in the form without a separate full chunk.)
+    if (vecs == 8) return RODE_SDDMM_LAUNCH(8, 1, Shape<8, 1, 8>, Shape<8, 1, 8>, false, true);
+    if (vecs == 16) return RODE_SDDMM_LAUNCH(16, 1, Shape<8, 2, 4>, Shape<8, 2, 4>, false, true, Shape<16, 1, 8>);
+    if (vecs == 32) return RODE_SDDMM_LAUNCH(32, 1, Shape<8, 4, 2>, Shape<16, 2, 4>, false, false);
+    if (vecs < 8) return RODE_SDDMM_LAUNCH(8, 1, Shape<8, 1, 8>, Shape<8, 1, 8>, true, true);
+    if (vecs < 16) return RODE_SDDMM_LAUNCH(16, 1, Shape<8, 2, 4>, Shape<8, 2, 4>, true, true);
+    if (vecs <= 24) return RODE_SDDMM_LAUNCH(32, 1, Shape<8, 3, 4>, Shape<8, 3, 2>, true, true);
+    if (vecs < 32) return RODE_SDDMM_LAUNCH(32, 1, Shape<8, 4, 2>, Shape<16, 2, 4>, true, true);
+    return RODE_SDDMM_LAUNCH(32, 2, Shape<16, 4, 2>, Shape<16, 4, 2>, true, true);
 #undef RODE_SDDMM_LAUNCH
 }

@@ -50,72 +50,30 @@
 namespace rode {
 namespace {
 
-#ifndef RODE_SPMM_CTA_WARPS
-#define RODE_SPMM_CTA_WARPS 1
-#endif
 // Small CTAs: a CTA's slot is held until its slowest warp is done, and segments differ in
 // length by more than 10x, so fewer warps per CTA keep more warps resident on average.
-constexpr int kCtaWarps = RODE_SPMM_CTA_WARPS;
+constexpr int kCtaWarps = 1;
 constexpr int kCtaThreads = 32 * kCtaWarps;
-#ifndef RODE_SPMM_WIDE_ROWS_CTA_WARPS
-#define RODE_SPMM_WIDE_ROWS_CTA_WARPS 4
-#endif
-constexpr int kSmallGridWarps = RODE_SPMM_WIDE_ROWS_CTA_WARPS;  // rows (warps) per CTA of spmm_rows_wide
+constexpr int kSmallGridWarps = 4;  // rows (warps) per CTA of spmm_rows_wide
 
-// Shape of a lane group per tile width (in 16-byte vectors: 8, 16 or 32 per dense-row slice):
-// L lanes x VPL vectors per lane, encoded as L * 100 + VPL.
+// A lane group: L lanes with VPL vectors of VB bytes each (LDG.128, or the 256-bit loads of sm_100) cover a tile of a
+// dense row.  16-byte shapes of the tiles of 128, 256 and 512 bytes:
 // (8 x 1 in the block kernel of the 128-byte tile: a load instruction then covers whole 128-byte lines, 4
 // rows per warp, where 4 x 2 covers 8 half lines.  R-MAT 23 N = 32 block kernel 2.19 -> 1.20 ms, R-MAT 21
 // N = 96 1.43 -> 0.92 ms, Zipf N = 32 -7 %; uniformly random columns lose 3 %: Pareto 2^20 N = 32 0.354 ->
 // 0.365 ms.  The per-row residue kernels measured faster with 4 x 2: R-MAT 23 N = 32 0.756 against 1.079 ms.)
-#ifndef RODE_SPMM_SHAPE_8
-#define RODE_SPMM_SHAPE_8 801
-#endif
-// Residue rows of 8-vector tiles (spmm_rows_simple, spmm_rows_wide) may use another shape than the block kernel.
-#ifndef RODE_SPMM_ROWS_SHAPE_8
-#define RODE_SPMM_ROWS_SHAPE_8 402
-#endif
-#ifndef RODE_SPMM_SHAPE_16
-#define RODE_SPMM_SHAPE_16 802
-#endif
-#ifndef RODE_SPMM_SHAPE_32
-#define RODE_SPMM_SHAPE_32 3201
-#endif
-// Residue rows of 32-vector tiles may use another shape than the block kernel (3201 selects
-// the batched spmm_rows kernel).
-#ifndef RODE_SPMM_ROWS_SHAPE_32
-#define RODE_SPMM_ROWS_SHAPE_32 3201
-#endif
-// Widest column tile (in 16-byte vectors) a launch covers; narrower tiles walk the columns
-// in several passes over the sparse matrix (grid.y), which shrinks the dense working set of
-// each pass.
-#ifndef RODE_SPMM_MAX_TILE_VECS
-#define RODE_SPMM_MAX_TILE_VECS 32
-#endif
-// 128-byte tile (N = 32 floats, 16 doubles) with one 32-byte load per lane and 4 lanes per dense row (1) or
-// with the 16-byte shapes above (0).  Stencil 128^3 N = 32 0.510 -> 0.401 ms (a load instruction of the
-// per-row kernel covers whole lines of 8 rows instead of half lines); the other matrices measure the same
-// as with the 8 x 1 block shape.
-#ifndef RODE_SPMM_TILE8_WIDE_LOADS
-#define RODE_SPMM_TILE8_WIDE_LOADS 1
-#endif
-// Bytes per load instruction of a lane in the block kernel and the per-row residue kernels:
-// 16 (LDG.128) or 32 (the 256-bit loads of sm_100).  The shapes above are given in 16-byte
-// vectors; with 32-byte loads a lane group has half as many lanes.
-#ifndef RODE_SPMM_VEC_BYTES
-#define RODE_SPMM_VEC_BYTES 16
-#endif
-// How the (column, value) pairs of a chunk reach the lanes that gather with them: 1 = through
-// shared memory (the chunk is stored once, every lane group reads its run with 16-byte broadcast
-// loads), 0 = by one shuffle per pair and element.  Shuffles and loads share the SM's load/store
-// data path, where a shuffle costs as much as 128 bytes of gathered data.
-#ifndef RODE_SPMM_PAIRS_IN_SMEM
-#define RODE_SPMM_PAIRS_IN_SMEM 1
-#endif
-// Block kernel: a separate unpredicated form for full chunks of 32 nonzeros (1) or one predicated form (0).
-#ifndef RODE_SPMM_FULL_CHUNK_PATH
-#define RODE_SPMM_FULL_CHUNK_PATH 1
-#endif
+template <int VB_, int L_, int VPL_>
+struct Shape {
+    static constexpr int VB = VB_, L = L_, VPL = VPL_;
+};
+using Block128 = Shape<16, 8, 1>;
+using Rows128 = Shape<16, 4, 2>;
+using Tile256 = Shape<16, 8, 2>;
+using Tile512 = Shape<16, 32, 1>;  // (its rows: the batched kernel spmm_rows)
+// 128-byte tile with one 32-byte load per lane and 4 lanes per dense row, where the operands are aligned to 32 bytes.
+// Stencil 128^3 N = 32 0.510 -> 0.401 ms (a load instruction of the per-row kernel covers whole lines of 8 rows instead of
+// half lines); the other matrices measure the same as with the 8 x 1 block shape.
+using Aligned128 = Shape<32, 4, 1>;
 // Claim counters of the persistent kernels, at the end of the workspace: one int per column tile for the block kernel, then
 // as many for the rows.
 constexpr size_t kCounterBytes = 256;
@@ -181,17 +139,17 @@ spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ 
     constexpr int NB = (kSteps + U - 1) / U;
     constexpr unsigned kFull = 0xffffffffu;
     chain_begin();
-    static_assert(W % S == 0 && (S == 1 || (W == S && !kClaim && RODE_SPMM_PAIRS_IN_SMEM != 0)), "a CTA per split segment");
+    static_assert(W % S == 0 && (S == 1 || (W == S && !kClaim)), "a CTA per split segment");
     const int part = S == 1 ? 0 : threadIdx.x >> 5;  // this warp takes every S-th chunk of its segment
     const int lane = threadIdx.x & 31;
     const int g = lane / L, l = lane % L;
     // Chunk staging (two buffers, so one __syncwarp per chunk orders both the reads after the
     // writes and the next-but-one chunk's writes after these reads).  The pair of position t
     // sits at (t % G) * kSteps + t / G: the run of a lane group is contiguous.
-    constexpr bool kStage = RODE_SPMM_PAIRS_IN_SMEM != 0 && (kSteps % U == 0) && (U % 4 == 0);
-    __shared__ __align__(16) int s_col[kStage ? W : 1][2][32];
-    __shared__ __align__(16) T s_val[kStage ? W : 1][2][32];
-    const int warp_in_cta = kStage ? (threadIdx.x >> 5) : 0;
+    static_assert(kSteps % U == 0 && U % 4 == 0, "whole batches, read as runs of four");
+    __shared__ __align__(16) int s_col[W][2][32];
+    __shared__ __align__(16) T s_val[W][2][32];
+    const int warp_in_cta = threadIdx.x >> 5;
     const int stage_slot = (lane % G) * kSteps + lane / G;
     int stage_buf = 0;
     const size_t row_vecs = static_cast<size_t>(n) / kLen;
@@ -253,11 +211,9 @@ spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ 
         }
         unsigned w_nxt = 0;
         if constexpr (kHints) w_nxt = hot_word(hot, c_nxt);
-        if constexpr (kStage) {
-            s_col[warp_in_cta][stage_buf][stage_slot] = c_cur;
-            s_val[warp_in_cta][stage_buf][stage_slot] = v_cur;
-            __syncwarp();
-        }
+        s_col[warp_in_cta][stage_buf][stage_slot] = c_cur;
+        s_val[warp_in_cta][stage_buf][stage_slot] = v_cur;
+        __syncwarp();
         // One chunk of the batched gather.  A full chunk (every chunk of a segment but its last) can take
         // a form without bounds: no predicate per gather and no zero-fill of the row buffers (ncu counted
         // 23 warp instructions per gathered row in the predicated form: 4 FMA, 1 load, the rest address,
@@ -272,17 +228,11 @@ spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ 
                 V buf[U][VPL];
                 T vv[U];
                 int cc[U];
-                if constexpr (kStage) {
-                    ld_shared_run<U>(&s_col[warp_in_cta][stage_buf][g * kSteps + b * U], cc);
-                    ld_shared_run<U>(&s_val[warp_in_cta][stage_buf][g * kSteps + b * U], vv);
-                }
+                ld_shared_run<U>(&s_col[warp_in_cta][stage_buf][g * kSteps + b * U], cc);
+                ld_shared_run<U>(&s_val[warp_in_cta][stage_buf][g * kSteps + b * U], vv);
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     const int t = (b * U + u) * G + g;  // position inside the chunk
-                    if constexpr (!kStage) {
-                        cc[u] = __shfl_sync(kFull, c_cur, t & 31);
-                        vv[u] = __shfl_sync(kFull, v_cur, t & 31);
-                    }
 #pragma unroll
                     for (int v = 0; v < VPL; ++v) {
                         if constexpr (kFullChunk && !kRagged) {
@@ -302,8 +252,7 @@ spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ 
         };
         // (only the 512-byte tile of large grids: R-MAT 21 N = 128 block kernel 0.818 -> 0.787 ms, R-MAT 23
         // step 4.76 -> 4.62 ms; the narrower shapes measured 1-2 % slower with it)
-        constexpr bool kFullChunkPath = RODE_SPMM_FULL_CHUNK_PATH != 0 && L == 32;
-        if (kFullChunkPath && cnt == 32)
+        if (L == 32 && cnt == 32)
             chunk(std::true_type{});
         else
             chunk(std::false_type{});
@@ -701,9 +650,9 @@ spmm_rows(int m2, int rows_per_group, int n, const T *__restrict__ values,
     const unsigned gmask = group_mask<L>(lane);
     const int gshift = lane & ~(L - 1);
     // chunk staging in shared memory as in spmm_block (one region of L pairs per lane group)
-    constexpr bool kStage = RODE_SPMM_PAIRS_IN_SMEM != 0 && (L % U == 0) && (U % 4 == 0);
-    __shared__ __align__(16) int s_col[2][kStage ? kCtaThreads : 1];
-    __shared__ __align__(16) T s_val[2][kStage ? kCtaThreads : 1];
+    static_assert(L % U == 0 && U % 4 == 0, "whole batches, read as runs of four");
+    __shared__ __align__(16) int s_col[2][kCtaThreads];
+    __shared__ __align__(16) T s_val[2][kCtaThreads];
     const int stage_base = (threadIdx.x / L) * L;  // first slot of this group's region
     int stage_buf = 0;
     // Persistent form (next_group != null, a grid of one resident wave): a lane group starts with
@@ -793,28 +742,20 @@ spmm_rows(int m2, int rows_per_group, int n, const T *__restrict__ values,
         int c_pre;
         T v_pre;
         fetch(base + 2 * L + l, c_pre, v_pre);
-        if constexpr (kStage) {
-            s_col[stage_buf][stage_base + l] = c_cur;
-            s_val[stage_buf][stage_base + l] = v_cur;
-            __syncwarp(gmask);
-        }
+        s_col[stage_buf][stage_base + l] = c_cur;
+        s_val[stage_buf][stage_base + l] = v_cur;
+        __syncwarp(gmask);
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
             if (b * U >= cnt) break;  // group-uniform
             V buf[U];
             T vv[U];
             int cc[U];
-            if constexpr (kStage) {
-                ld_shared_run<U>(&s_col[stage_buf][stage_base + b * U], cc);
-                ld_shared_run<U>(&s_val[stage_buf][stage_base + b * U], vv);
-            }
+            ld_shared_run<U>(&s_col[stage_buf][stage_base + b * U], cc);
+            ld_shared_run<U>(&s_val[stage_buf][stage_base + b * U], vv);
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int t = b * U + u;  // position inside the chunk
-                if constexpr (!kStage) {
-                    cc[u] = __shfl_sync(gmask, c_cur, t, L);
-                    vv[u] = __shfl_sync(gmask, v_cur, t, L);
-                }
                 buf[u] = vzero(static_cast<V *>(nullptr));
                 if (t < cnt && inside) buf[u] = ld_dense(dense_row(b_lane, static_cast<unsigned>(cc[u]), row_bytes));
             }
@@ -853,14 +794,8 @@ spmm_rows(int m2, int rows_per_group, int n, const T *__restrict__ values,
 // where a warp holds several groups: there the groups would run different entry streams in
 // spmm_rows and diverge, which measured slower (stencil N = 64: 1.43 ms against 0.93 ms),
 // while for 32-lane groups the batched kernel wins (R-MAT N = 128: 327 us against 770 us).
-#ifndef RODE_SPMM_ROWS_CTA
-#define RODE_SPMM_ROWS_CTA 32
-#endif
-constexpr int kRowsCtaThreads = RODE_SPMM_ROWS_CTA;
-// spmm_rows_wide (a warp per row) serves lists of at most this many full waves of warps
-#ifndef RODE_SPMM_WIDE_ROWS_WAVES
-#define RODE_SPMM_WIDE_ROWS_WAVES 2
-#endif
+constexpr int kRowsCtaThreads = 32;
+constexpr long long kWideRowsWaves = 2;  // spmm_rows_wide (a warp per row) serves lists of at most so many waves of 32 warps per SM
 
 template <typename T, int VB, int L, int VPL, int R, bool kRagged>
 __global__ void __launch_bounds__(kRowsCtaThreads, 1024 / kRowsCtaThreads)  // 64 registers: 32 warps per SM
@@ -915,9 +850,9 @@ spmm_rows_simple(int m2, int n, const T *__restrict__ values, const int *__restr
     auto inside = [&](int v) { return !kRagged || col_vec + v * L < row_vecs; };
     // chunk staging in shared memory as in spmm_block (one region of L pairs per lane group; the
     // groups of a warp run rows of different lengths, so they synchronise by group)
-    constexpr bool kStage = RODE_SPMM_PAIRS_IN_SMEM != 0 && (L % U == 0) && (U % 4 == 0);
-    __shared__ __align__(16) int s_col[2][kStage ? kRowsCtaThreads : 1];
-    __shared__ __align__(16) T s_val[2][kStage ? kRowsCtaThreads : 1];
+    static_assert(L % U == 0 && U % 4 == 0, "whole batches, read as runs of four");
+    __shared__ __align__(16) int s_col[2][kRowsCtaThreads];
+    __shared__ __align__(16) T s_val[2][kRowsCtaThreads];
     const int stage_base = (threadIdx.x / L) * L;
     int stage_buf = 0;
 #pragma unroll
@@ -939,27 +874,17 @@ spmm_rows_simple(int m2, int n, const T *__restrict__ values, const int *__restr
                 v_nxt = ld_stream(values + e);
             }
             const int cnt = min(L, end[r] - base);
-            if constexpr (kStage) {
-                s_col[stage_buf][stage_base + l] = c;
-                s_val[stage_buf][stage_base + l] = val;
-                __syncwarp(gmask);
-            }
+            s_col[stage_buf][stage_base + l] = c;
+            s_val[stage_buf][stage_base + l] = val;
+            __syncwarp(gmask);
 #pragma unroll
             for (int t0 = 0; t0 < L; t0 += U) {
                 if (t0 >= cnt) break;
                 int cc[U];
                 T vv[U];
                 V bb[U][VPL];
-                if constexpr (kStage) {
-                    ld_shared_run<U>(&s_col[stage_buf][stage_base + t0], cc);
-                    ld_shared_run<U>(&s_val[stage_buf][stage_base + t0], vv);
-                } else {
-#pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        cc[u] = __shfl_sync(gmask, c, t0 + u, L);
-                        vv[u] = __shfl_sync(gmask, val, t0 + u, L);
-                    }
-                }
+                ld_shared_run<U>(&s_col[stage_buf][stage_base + t0], cc);
+                ld_shared_run<U>(&s_val[stage_buf][stage_base + t0], vv);
 #pragma unroll
                 for (int u = 0; u < U; ++u)
 #pragma unroll
@@ -1071,12 +996,12 @@ int launch_rows(int m2, int n, const T *values, const int *col, const int *row_o
                 const T *B, T *C, int *counters, bool chained, bool counters_clear, bool two_rows,
                 cudaStream_t s2);
 
-// Block kernel of shape (VB bytes per load, L lanes, VPL loads per lane) and residue-row kernel of shape (RVB, RL, RVPL);
-// each walks the columns in tiles of its own.
-template <typename T, int VB, int L, int VPL, int RVB, int RL, int RVPL, bool kRagged, bool kRowsRagged = kRagged>
+// Block kernel of one shape and residue-row kernel of another; each walks the columns in tiles of its own.
+template <typename T, typename Block, typename Rows, bool kRagged = false, bool kRowsRagged = kRagged>
 int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, const int *row_offsets,
                  const int *block_r_ind, const int *residue_r_ind, const int *st_off, const T *B, T *C,
                  T *partial, int *counters, const unsigned *hot, long long nnz, cudaStream_t s1, cudaStream_t s2) {
+    constexpr int VB = Block::VB, L = Block::L, VPL = Block::VPL;
     constexpr int kTileWidth = L * VPL * VecB<T, VB>::kLen;
     constexpr int U = kLoadsInFlight * 16 / VB / VPL;            // rows per batch
     // ragged widths: the last tile is partly empty
@@ -1099,7 +1024,7 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
         if (persistent || counters_clear) RODE_CUDA_TRY(cudaMemsetAsync(counters, 0, 2 * kClaimTiles * sizeof(int), s1));
         int *claim = persistent ? counters : nullptr;
         dim3 grid(persistent ? (resident + tiles - 1) / tiles : ctas_needed, tiles);
-        bool launched = false;
+        bool launched = false;  // one of the two special forms
         // Popularity hints: block kernel of the 512-byte tile only.  In the residue-row kernel
         // the marks saved DRAM bytes (5.36 -> 4.79 GB on R-MAT scale 23) but the extra registers
         // cost more time than that returned (1.41 -> 1.52 ms).
@@ -1122,14 +1047,14 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
                 m1, seg_ctas, m2, n, values, col, row_offsets, block_r_ind, st_off, residue_r_ind, B, C, partial);
             rows_done = launched = true;
         }
-        if (launched) {
-        } else if (static_cast<long long>(m1) * tiles <= kSplit4WarpsPerSm * sm_count()) {
+        const long long warps = static_cast<long long>(m1) * tiles;
+        if (!launched && warps <= kSplit4WarpsPerSm * sm_count()) {
             spmm_block<T, VB, L, VPL, U, 4, 4, false, false, kRagged><<<dim3(m1, tiles), 4 * 32, 0, s1>>>(
                 m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0, nullptr);
-        } else if (static_cast<long long>(m1) * tiles <= kSplit2WarpsPerSm * sm_count()) {
+        } else if (!launched && warps <= kSplit2WarpsPerSm * sm_count()) {
             spmm_block<T, VB, L, VPL, U, 2, 2, false, false, kRagged><<<dim3(m1, tiles), 2 * 32, 0, s1>>>(
                 m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0, nullptr);
-        } else {
+        } else if (!launched) {
             spmm_block<T, VB, L, VPL, U, kCtaWarps, 1, false, true, kRagged><<<grid, kCtaThreads, 0, s1>>>(
                 m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0, claim);
         }
@@ -1138,8 +1063,8 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
     // Rows: on the block kernel's own stream they are chained behind it (see chain_begin), on another one
     // they are a plain launch.
     if (m2 > 0 && !rows_done) {
-        if (int rc = launch_rows<T, RVB, RL, RVPL, kRowsRagged>(m2, n, values, col, row_offsets, residue_r_ind, B, C, counters,
-                                                            chained, counters_clear, short_rows(nnz, m1, m2, RVB * RL * RVPL), s2))
+        if (int rc = launch_rows<T, Rows::VB, Rows::L, Rows::VPL, kRowsRagged>(m2, n, values, col, row_offsets, residue_r_ind, B, C, counters,
+                                                            chained, counters_clear, short_rows(nnz, m1, m2, Rows::VB * Rows::L * Rows::VPL), s2))
             return rc;
     }
     if (m1 > 1) {  // (a row that was cut has two segments at least)
@@ -1181,7 +1106,7 @@ int launch_rows(int m2, int n, const T *values, const int *col, const int *row_o
         const dim3 grid(static_cast<unsigned>(persistent ? (resident + tiles - 1) / tiles : ctas_needed), tiles);
         RODE_CUDA_TRY(launch_chained(spmm_rows<T, 32, kRagged>, grid, dim3(kCtaThreads), s2, chained, m2, per_group, n, values,
                                      col, row_offsets, residue_r_ind, B, C, claim));
-    } else if (static_cast<long long>(m2) * tiles <= RODE_SPMM_WIDE_ROWS_WAVES * 32LL * sm_count()) {
+    } else if (static_cast<long long>(m2) * tiles <= kWideRowsWaves * 32 * sm_count()) {
         const dim3 grid((m2 + kSmallGridWarps - 1) / kSmallGridWarps + 1, tiles);
         RODE_CUDA_TRY(launch_chained(spmm_rows_wide<T, VB, L, VPL, kRagged>, grid, dim3(32 * kSmallGridWarps), s2, chained, m2,
                                      n, values, col, row_offsets, residue_r_ind, B, C));
@@ -1203,11 +1128,6 @@ int launch_rows(int m2, int n, const T *values, const int *col, const int *row_o
     RODE_CHECK_LAUNCH("rode::spmm_rows");
     return RODE_OK;
 }
-
-// A shape given in 16-byte vectors (L * 100 + VPL), re-expressed for 32-byte loads: half the
-// loads per lane where that number is even, else half the lanes.
-constexpr int wide_lanes(int shape) { return (shape % 100) % 2 == 0 ? shape / 100 : shape / 200; }
-constexpr int wide_vpl(int shape) { return (shape % 100) % 2 == 0 ? (shape % 100) / 2 : shape % 100; }
 
 template <typename T>
 int spmm(int m1, int m2, int k, int n, const T *values, const int *col, const int *row_offsets,
@@ -1243,24 +1163,12 @@ int spmm(int m1, int m2, int k, int n, const T *values, const int *col, const in
     // the claim counters of the persistent block kernel sit behind the partial rows
     int *counters = workspace != nullptr
                         ? reinterpret_cast<int *>(static_cast<char *>(workspace) + need - kCounterBytes) : nullptr;
-    // Widest tile (32, 16 or 8 vectors of 16 bytes) that divides the row.  Shapes are given in
-    // 16-byte vectors; with 32-byte loads (operands 32-byte aligned) a group has half the lanes.
-    // The batched residue kernel of the widest tile (shape 3201) always loads 16 bytes per lane.
-#define RODE_LAUNCH16(shape, rows_shape) RODE_LAUNCH16R(shape, rows_shape, false)
-#define RODE_LAUNCH16R(shape, rows_shape, ragged)                                                               \
-    launch_shape<T, 16, (shape) / 100, (shape) % 100, 16, (rows_shape) / 100, (rows_shape) % 100, ragged>(      \
-        m1, m2, k, n, values, col, row_offsets, block_r_ind, residue_r_ind, st_off, B, C, partial, counters, hot, nnz,     \
-        stream1, stream2)
-#define RODE_LAUNCH32(shape, rows_shape, rows_bytes)                                                             \
-    launch_shape<T, 32, wide_lanes(shape), wide_vpl(shape), rows_bytes,                                          \
-                 (rows_bytes) == 32 ? wide_lanes(rows_shape) : (rows_shape) / 100,                               \
-                 (rows_bytes) == 32 ? wide_vpl(rows_shape) : (rows_shape) % 100, false>(                         \
-        m1, m2, k, n, values, col, row_offsets, block_r_ind, residue_r_ind, st_off, B, C, partial, counters, hot, nnz,     \
-        stream1, stream2)
+    // Widest tile (32, 16 or 8 vectors of 16 bytes) that divides the row.
+#define RODE_LAUNCH(...)                                                                                             \
+    launch_shape<T, __VA_ARGS__>(m1, m2, k, n, values, col, row_offsets, block_r_ind, residue_r_ind, st_off, B, C, partial, \
+                                 counters, hot, nnz, stream1, stream2)
+    const bool aligned32 = aligned_to(B, 32) && aligned_to(C, 32) && aligned_to(workspace, 32);
     const int vecs = n / kLen;
-    // Widths the tiles do not divide (any other multiple of 4 columns; the reference has none of
-    // them): the narrowest shape that covers the row, or 512-byte tiles with a partly empty last
-    // one.  Always 16-byte loads, no popularity hints.
     // Widths of whole lines that the 512-byte tile does not divide (N = 96, 160, 192, 224 ...): 512-byte tiles with a
     // partly idle last one all the same, instead of up to seven passes over the sparse matrix with narrow ones.  us, narrow ->
     // wide: R-MAT 21 N = 96 1411 -> 954, N = 160 2627 -> 1948, N = 224 3701 -> 2449; Pareto 2^20 N = 96 2309 -> 1756, N = 224
@@ -1281,52 +1189,25 @@ int spmm(int m1, int m2, int k, int n, const T *values, const int *col, const in
         const int full = 4 * vecs >= 3 * 32 * ((vecs + 31) / 32) ? 6 : 2;
         const bool wide_rows = nnz >= 0 && !rows_hold(nnz, m1, m2, full) &&
                                (nnz < 20LL * m2 || (sizeof(T) == 8 && 20LL * m1 >= m2 && 8LL * m1 <= m2));
-#define RODE_WIDE_BLOCK(rows_shape, rows_ragged)                                                                  \
-    launch_shape<T, 16, RODE_SPMM_SHAPE_32 / 100, RODE_SPMM_SHAPE_32 % 100, 16, (rows_shape) / 100, (rows_shape) % 100, true, \
-                 rows_ragged>(m1, m2, k, n, values, col, row_offsets, block_r_ind, residue_r_ind, st_off, B, C, partial,     \
-                              counters, nullptr, nnz, stream1, stream2)
-        if (wide_rows) return RODE_WIDE_BLOCK(RODE_SPMM_ROWS_SHAPE_32, true);
-        if (vecs % 16 == 0) return RODE_WIDE_BLOCK(RODE_SPMM_SHAPE_16, false);
-        if (aligned_to(B, 32) && aligned_to(C, 32))
-            return launch_shape<T, 16, RODE_SPMM_SHAPE_32 / 100, RODE_SPMM_SHAPE_32 % 100, 32, 4, 1, true, false>(
-                m1, m2, k, n, values, col, row_offsets, block_r_ind, residue_r_ind, st_off, B, C, partial, counters, nullptr, nnz,
-                stream1, stream2);
-        return RODE_WIDE_BLOCK(RODE_SPMM_ROWS_SHAPE_8, false);
+        hot = nullptr;  // (no popularity hints here)
+        if (wide_rows) return RODE_LAUNCH(Tile512, Tile512, true, true);
+        if (vecs % 16 == 0) return RODE_LAUNCH(Tile512, Tile256, true, false);
+        if (aligned_to(B, 32) && aligned_to(C, 32)) return RODE_LAUNCH(Tile512, Aligned128, true, false);
+        return RODE_LAUNCH(Tile512, Rows128, true, false);
     }
+    // Widths the tiles do not divide (any other multiple of 4 columns; the reference has none of them): the narrowest
+    // shape that covers the row, or 512-byte tiles with a partly empty last one.  No popularity hints.
     if (vecs % 8 != 0) {
-        if (vecs < 8) return RODE_LAUNCH16R(RODE_SPMM_SHAPE_8, RODE_SPMM_ROWS_SHAPE_8, true);
-        if (vecs < 16) return RODE_LAUNCH16R(RODE_SPMM_SHAPE_16, RODE_SPMM_SHAPE_16, true);
-        return RODE_LAUNCH16R(RODE_SPMM_SHAPE_32, RODE_SPMM_ROWS_SHAPE_32, true);
+        if (vecs < 8) return RODE_LAUNCH(Block128, Rows128, true);
+        if (vecs < 16) return RODE_LAUNCH(Tile256, Tile256, true);
+        return RODE_LAUNCH(Tile512, Tile512, true);
     }
-    // 32-byte loads measured no faster than 16-byte ones on any benchmark matrix (the gathers are
-    // bound by bytes through L1/L2, not by load instructions), so the default build does not
-    // instantiate them.
-    if constexpr (RODE_SPMM_VEC_BYTES == 32) {
-        if (aligned_to(B, 32) && aligned_to(C, 32) && aligned_to(workspace, 32)) {
-            if (vecs % 32 == 0 && RODE_SPMM_MAX_TILE_VECS >= 32) {
-                if (RODE_SPMM_ROWS_SHAPE_32 == 3201)
-                    return RODE_LAUNCH32(RODE_SPMM_SHAPE_32, RODE_SPMM_ROWS_SHAPE_32, 16);
-                return RODE_LAUNCH32(RODE_SPMM_SHAPE_32, RODE_SPMM_ROWS_SHAPE_32, 32);
-            }
-            if (vecs % 16 == 0) return RODE_LAUNCH32(RODE_SPMM_SHAPE_16, RODE_SPMM_SHAPE_16, 32);
-            return RODE_LAUNCH32(RODE_SPMM_SHAPE_8, RODE_SPMM_ROWS_SHAPE_8, 32);
-        }
-    }
-    if (vecs % 32 == 0 && RODE_SPMM_MAX_TILE_VECS >= 32) return RODE_LAUNCH16(RODE_SPMM_SHAPE_32, RODE_SPMM_ROWS_SHAPE_32);
-    if (vecs % 16 == 0) return RODE_LAUNCH16(RODE_SPMM_SHAPE_16, RODE_SPMM_SHAPE_16);
-    // 128-byte tile: 4 lanes x one 32-byte load cover a whole line per dense row and 8 rows per warp, in
-    // the block and the per-row residue kernels alike (operands 32-byte aligned; else the 16-byte shapes)
-    if constexpr (RODE_SPMM_TILE8_WIDE_LOADS != 0) {
-        if (aligned_to(B, 32) && aligned_to(C, 32) && aligned_to(workspace, 32))
-            return launch_shape<T, 32, 4, 1, 32, 4, 1, false>(m1, m2, k, n, values, col, row_offsets, block_r_ind,
-                                                              residue_r_ind, st_off, B, C, partial, counters, hot, nnz,
-                                                              stream1, stream2);
-    }
-    return RODE_LAUNCH16(RODE_SPMM_SHAPE_8, RODE_SPMM_ROWS_SHAPE_8);
-#undef RODE_WIDE_BLOCK
-#undef RODE_LAUNCH16
-#undef RODE_LAUNCH16R
-#undef RODE_LAUNCH32
+    // (32-byte loads measured no faster than 16-byte ones in the wider tiles: the gathers are bound by bytes through L1 and L2)
+    if (vecs % 32 == 0) return RODE_LAUNCH(Tile512, Tile512);
+    if (vecs % 16 == 0) return RODE_LAUNCH(Tile256, Tile256);
+    if (aligned32) return RODE_LAUNCH(Aligned128, Aligned128);
+    return RODE_LAUNCH(Block128, Rows128);
+#undef RODE_LAUNCH
 }
 
 }  // namespace
