@@ -19,7 +19,9 @@
  * the first call on that pair of streams (cudaMalloc) and re-used afterwards.  Calls on the same
  * streams are ordered by them and share the buffer; calls on other streams get buffers of
  * their own and may overlap on the GPU, as with the reference.  Callers that must not
- * allocate at call time pass their own workspace to rode_spmm_f32 / rode_spmm_f64.
+ * allocate at call time pass their own workspace to rode_spmm_f32 / rode_spmm_f64.  A call that is
+ * captured into a graph needs its buffer beforehand (one earlier call of the size on the same streams);
+ * the graph keeps using that buffer, so graphs captured on one pair of streams must not be replayed side by side.
  */
 #ifndef RODE_B200_RODESPMM_H_
 #define RODE_B200_RODESPMM_H_

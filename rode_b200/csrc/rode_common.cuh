@@ -328,6 +328,23 @@ cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, cudaStre
 }
 #endif
 
+// The stream's own number: unlike its handle it is never given to another stream, and cudaStreamPerThread, one handle, has
+// one number per thread.  Not for a stream that is being captured.
+inline unsigned long long stream_id(cudaStream_t s) {
+    unsigned long long id = 0;
+    if (cudaStreamGetId(s, &id) == cudaSuccess) return id;
+    (void)cudaGetLastError();
+    return reinterpret_cast<unsigned long long>(s);
+}
+// Work enqueued on the stream now is being recorded into a graph.  (The query fails on the legacy stream while another
+// stream is captured, where the launch itself will report it.)
+inline bool is_capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
+    (void)cudaGetLastError();
+    return true;
+}
+
 // Number of SMs of the current device (looked up once per device; 148 if the query fails).
 inline int sm_count() {
     static int cached[64] = {0};

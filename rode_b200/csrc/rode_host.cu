@@ -31,16 +31,20 @@ namespace {
 // calls on the same streams are ordered by them, so they may share a buffer (the SpMM workspace
 // is used by the block kernel on stream1 and, for its claim counters, by the residue kernel on
 // stream2, hence both streams are part of the key); calls on other streams may overlap on the GPU
-// and get buffers of their own, which keeps the entry points re-entrant like the reference's.  At most kMaxScratch buffers are kept; the least recently
-// used one is released when a new key arrives.  Growing or releasing calls cudaFree, which
-// waits for work that may still use the buffer.
+// and get buffers of their own, which keeps the entry points re-entrant like the reference's.  At most
+// kMaxScratch buffers are kept; the least recently used one is released when a new key arrives.  Growing or
+// releasing calls cudaFree, which waits for work that may still use the buffer.
+//
+// A buffer that a captured call uses is in a graph from then on, which may be replayed at any time: it is never
+// released, a larger one takes its place beside it.
 struct Scratch {
     int kind = 0;
     int dev = -1;
-    cudaStream_t stream = nullptr;
-    cudaStream_t stream2 = nullptr;
+    cudaStream_t stream = nullptr, stream2 = nullptr;
+    unsigned long long id = 0, id2 = 0;  // stream_id
     void *ptr = nullptr;
     size_t bytes = 0;
+    bool captured = false;
     unsigned long long last_use = 0;
 };
 constexpr int kMaxScratch = 32;
@@ -56,19 +60,21 @@ int scratch_for(ScratchKind kind, cudaStream_t stream, cudaStream_t stream2, siz
     if (bytes == 0) return RODE_OK;
     int dev = 0;
     RODE_CUDA_TRY(cudaGetDevice(&dev));
+    // (a stream that is being captured must not be asked for its number: the handles say which buffer, the last one if several)
+    const bool capturing = is_capturing(stream) || is_capturing(stream2);
+    const unsigned long long id = capturing ? 0 : stream_id(stream), id2 = capturing ? 0 : stream_id(stream2);
     std::lock_guard<std::mutex> lock(g_scratch_mutex);
     Scratch *slot = nullptr, *oldest = &g_scratch[0];
     for (Scratch &s : g_scratch) {
-        if (s.ptr && s.kind == kind && s.dev == dev && s.stream == stream && s.stream2 == stream2) {
+        if (s.ptr && s.kind == kind && s.dev == dev && s.stream == stream && s.stream2 == stream2 &&
+            (capturing ? slot == nullptr || s.last_use > slot->last_use : s.id == id && s.id2 == id2))
             slot = &s;
-            break;
-        }
         if (s.ptr == nullptr ? oldest->ptr != nullptr : (oldest->ptr != nullptr && s.last_use < oldest->last_use))
             oldest = &s;  // a free slot wins over any used one; among used ones the oldest
     }
     if (slot == nullptr) {
         slot = oldest;
-        if (slot->ptr) {  // evict: the buffer belongs to another device if slot->dev != dev
+        if (slot->ptr && !slot->captured) {  // evict: the buffer belongs to another device if slot->dev != dev
             int err = cudaSuccess;
             if (slot->dev != dev) err = cudaSetDevice(slot->dev);
             if (err == cudaSuccess) err = cudaFree(slot->ptr);
@@ -81,15 +87,19 @@ int scratch_for(ScratchKind kind, cudaStream_t stream, cudaStream_t stream2, siz
         slot->dev = dev;
         slot->stream = stream;
         slot->stream2 = stream2;
+        slot->id = id;
+        slot->id2 = id2;
     }
     if (slot->bytes < bytes) {
-        if (slot->ptr) RODE_CUDA_TRY(cudaFree(slot->ptr));
+        if (slot->ptr && !slot->captured) RODE_CUDA_TRY(cudaFree(slot->ptr));
         slot->ptr = nullptr;
         slot->bytes = 0;
+        slot->captured = false;
         const size_t grown = bytes + bytes / 4;  // head-room against repeated regrowth
         RODE_CUDA_TRY(cudaMalloc(&slot->ptr, grown));
         slot->bytes = grown;
     }
+    slot->captured = slot->captured || capturing;
     slot->last_use = ++g_scratch_clock;
     *out = slot->ptr;
     return RODE_OK;

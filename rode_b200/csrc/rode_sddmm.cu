@@ -568,8 +568,8 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
 // for the life of the process: calls on the same streams are ordered by them and may share
 // their counter, calls on other streams get other slots; when all slots are taken a call simply
 // runs one CTA per segment.  Nothing is allocated.  What keeps two kernels off one counter:
-//   * streams are told apart by cudaStreamGetId, not by handle: cudaStreamPerThread is one handle for a stream per
-//     thread, and a destroyed stream's handle is given to a new one while its last kernels may still run;
+//   * streams are told apart by number, not by handle (stream_id): a destroyed stream's handle is given to a new one
+//     while its last kernels may still run;
 //   * the reset and the kernel that follows it are enqueued under one lock (ClaimCounter holds it), so that host
 //     threads that share a stream cannot come between them;
 //   * a call that is being captured gets no counter: its graph may be replayed on any stream, next to graphs
@@ -591,17 +591,10 @@ struct ClaimCounter {
         static Key keys[kClaimSlots];
         static int n_keys = 0;
         static int *base[64] = {nullptr};  // device address of the array, per device
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s1, &capture) != cudaSuccess) {
-            (void)cudaGetLastError();  // the legacy stream while another one is being captured: the launch itself reports it
-            return RODE_OK;
-        }
-        if (capture != cudaStreamCaptureStatusNone) return RODE_OK;
-        Key key = {0, 0, 0};
+        if (is_capturing(s1) || is_capturing(s2)) return RODE_OK;
+        Key key = {0, stream_id(s1), stream_id(s2)};
         RODE_CUDA_TRY(cudaGetDevice(&key.dev));
         if (key.dev < 0 || key.dev >= 64) return RODE_OK;
-        RODE_CUDA_TRY(cudaStreamGetId(s1, &key.id1));
-        RODE_CUDA_TRY(cudaStreamGetId(s2, &key.id2));
         enqueue = std::unique_lock<std::mutex>(g_claim_mutex);
         if (base[key.dev] == nullptr) {
             void *p = nullptr;

@@ -435,3 +435,49 @@ def test_row_kernels_follow_what_is_known_of_the_short_rows(lo, hi, heavy, two_r
             a, b = int(A.row_ptr[r]), int(A.row_ptr[r + 1])
             want = (val[a:b].double()[:, None] * B[A.col[a:b].long()].double()).sum(0)
             assert torch.allclose(C[r].double(), want, rtol=1e-5, atol=2e-5 if size == 4 else 1e-12)
+
+
+def test_captured_reference_signature_call_keeps_its_workspace():
+    """A graph of a RoDeSpmm call holds the library's workspace for its streams: a later, larger call on the same streams,
+    which needs a larger buffer, must leave the old one alive."""
+    lib = capi.load()
+    fn = getattr(lib, capi.CPP_SYMBOLS["RoDeSpmm_n128_f32"])
+    fn.restype = None
+    vp = ctypes.c_void_p
+    stream = torch.cuda.Stream()
+    cases = []
+    for m, per_row in ((300, 1500), (6000, 1500)):          # rows of three segments: partial rows in the workspace
+        A = _rows_of(torch.full((m,), per_row, device="cuda"), 4001, seed=m)
+        meta = capi.preprocess(A.row_ptr, A.nnz)
+        B = W.dense(A.n, 128, device="cuda", seed=m)
+        cases.append((A, meta, B, torch.zeros((m, 128), device="cuda")))
+
+    def call(i):
+        A, meta, B, C = cases[i]
+        fn(meta.m1, meta.m2, A.n, 128, vp(A.val.data_ptr()), vp(A.col.data_ptr()), vp(A.row_ptr.data_ptr()),
+           vp(meta.block_r_ind.data_ptr()), vp(meta.residue_r_ind.data_ptr()), vp(meta.st_off.data_ptr()),
+           vp(B.data_ptr()), vp(C.data_ptr()), vp(stream.cuda_stream), vp(stream.cuda_stream))
+
+    torch.cuda.synchronize()
+    call(0)
+    torch.cuda.synchronize()
+    want = cases[0][3].clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        call(0)
+    free_before, _ = torch.cuda.mem_get_info()
+    call(1)
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] < free_before       # a larger buffer, beside the captured one
+    filler = torch.full((1 << 22,), float("nan"), device="cuda")
+    for _ in range(2):
+        cases[0][3].fill_(float("nan"))
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            graph.replay()
+        call(1)
+        torch.cuda.synchronize()
+        assert torch.equal(cases[0][3], want)
+    big = capi.spmm(cases[1][1], cases[1][0].row_ptr, cases[1][0].col, cases[1][0].val, cases[1][2])
+    assert torch.equal(cases[1][3], big)
+    del filler, graph
