@@ -175,9 +175,8 @@ def preprocess(row_ptr: torch.Tensor, nnz: int, seg_len: int = 512, k_block: int
     dev = row_ptr.device
     cap = preprocess_capacity(seg_len, vec_len, M, int(nnz))
     with torch.cuda.device(dev):
-        if stream is None:
-            stream = torch.cuda.current_stream(dev)
-        with torch.cuda.stream(stream) if isinstance(stream, torch.cuda.Stream) else _null():
+        stream = _stream_object(stream, dev)
+        with torch.cuda.stream(stream):
             blk = torch.empty(max(cap, 1), dtype=torch.int32, device=dev)
             st = torch.empty(cap + 1, dtype=torch.int32, device=dev)
             res = torch.empty(max(M, 1), dtype=torch.int32, device=dev)
@@ -196,8 +195,11 @@ def preprocess(row_ptr: torch.Tensor, nnz: int, seg_len: int = 512, k_block: int
 _NULL = contextlib.nullcontext()
 
 
-def _null():
-    return _NULL
+def _stream_object(s, dev: torch.device) -> torch.cuda.Stream:
+    """The stream of a torch stream, a raw handle, or None (torch's current one)."""
+    if s is None:
+        return torch.cuda.current_stream(dev)
+    return s if isinstance(s, torch.cuda.Stream) else torch.cuda.ExternalStream(int(s), device=dev)
 
 
 def _current(dev: torch.device) -> int:
@@ -208,7 +210,21 @@ def _current(dev: torch.device) -> int:
 def _on(dev: torch.device):
     """torch.cuda.device(dev), or nothing where dev is current already (entering and leaving the
     context costs as much as a launch)."""
-    return _null() if torch.cuda.current_device() == dev.index else torch.cuda.device(dev)
+    return _NULL if torch.cuda.current_device() == dev.index else torch.cuda.device(dev)
+
+
+def _used_on(streams, cur: int, dev: torch.device, *tensors) -> None:
+    """Tensors just made on the current stream for kernels on others: these wait for it (for a fill, and for earlier
+    work on memory that came back to the allocator), and the allocator learns who uses them, so that they are not
+    handed out again while those streams still work on them."""
+    for s in streams:
+        if s is cur:
+            continue
+        s = _stream_object(s, dev)
+        if s.cuda_stream != cur:
+            s.wait_stream(torch.cuda.current_stream(dev))
+            for t in tensors:
+                t.record_stream(s)
 
 
 def preprocess_cpu(row_ptr: torch.Tensor, seg_len: int = 512, k_block: int = 32, vec_len: int = 4):
@@ -277,9 +293,8 @@ def hot_columns(col: torch.Tensor, n_cols: int, dense_row_bytes: int, budget_byt
     check(load().rode_hot_columns_words(n_cols, ctypes.byref(words)))
     check(load().rode_hot_columns_workspace_bytes(n_cols, ctypes.byref(need)))
     with torch.cuda.device(dev):
-        if stream is None:
-            stream = torch.cuda.current_stream(dev)
-        with torch.cuda.stream(stream) if isinstance(stream, torch.cuda.Stream) else _null():
+        stream = _stream_object(stream, dev)
+        with torch.cuda.stream(stream):
             bitmap = torch.empty(words.value, dtype=torch.int32, device=dev)
             ws = torch.empty(need.value, dtype=torch.uint8, device=dev)
             hot_columns_raw(col.numel(), n_cols, col.data_ptr(), dense_row_bytes, budget_bytes, bitmap.data_ptr(),
@@ -292,8 +307,9 @@ def spmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torch
          C: Optional[torch.Tensor] = None, workspace: Optional[torch.Tensor] = None, stream1=None,
          stream2=None, hot: Optional[torch.Tensor] = None) -> torch.Tensor:
     """C = S @ B through rode_spmm_f32 / rode_spmm_f64.  Asynchronous on the two streams
-    (default: torch's current stream for both).  A given ``C`` must be zero in the rows without a
-    nonzero, which are not written; by default C is a fresh tensor of which every row is written.
+    (default: torch's current stream for both; other ones wait for it where ``C`` or ``workspace`` is
+    made here).  A given ``C`` must be zero in the rows without a nonzero, which are not written; by
+    default C is a fresh tensor of which every row is written.
     ``hot``: popularity bitmap from ``hot_columns`` (same results, fewer DRAM bytes)."""
     M = row_ptr.numel() - 1
     k, n = B.shape
@@ -309,16 +325,11 @@ def spmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torch
         whole = C is None and (meta.m1 > 0 or meta.m2 > 0)
         if C is None:
             C = B.new_empty((M, n)) if whole else B.new_zeros((M, n))
+            _used_on((s1, s2), cur, dev, C)
         need = spmm_workspace_bytes(meta.m1, n, B.element_size())
         if workspace is None and need:
             workspace = B.new_empty(need, dtype=torch.uint8)
-            # the buffer goes back to torch's allocator when this function returns: tell the
-            # allocator which other streams still use it, or a call enqueued right afterwards
-            # could be handed the same memory while this call's kernels run
-            if s1 is not cur or s2 is not cur:
-                for s in (s1, s2):
-                    if isinstance(s, torch.cuda.Stream) and s.cuda_stream != cur:
-                        workspace.record_stream(s)
+            _used_on((s1, s2), cur, dev, workspace)
         ws_bytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
         if whole:
             spmm_all_raw(B.dtype, M, meta.m1, k, n, values.data_ptr(), col.data_ptr(), row_ptr.data_ptr(),
@@ -352,6 +363,7 @@ def sddmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torc
         s2 = cur if stream2 is None else stream2
         if out is None:  # (entries that belong to no row of row_ptr are not written)
             out = values.new_zeros(values.numel())
+            _used_on((s1, s2), cur, dev, out)
         sddmm_raw(meta.m1, meta.m2, rhs.shape[0], k, meta.block_r_ind.data_ptr(), meta.residue_r_ind.data_ptr(),
                   meta.st_off.data_ptr(), row_ptr.data_ptr(), col.data_ptr(), values.data_ptr(), lhs.data_ptr(),
                   rhs.data_ptr(), out.data_ptr(), s1, s2)

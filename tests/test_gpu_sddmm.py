@@ -354,3 +354,34 @@ def test_sddmm_row_mode_of_wide_rows(oracle_cpu, rows, k):
         scale = sddmm_abs_scale(A.row_ptr.numpy(), col.numpy(), A.val.numpy(), lhs.numpy(), rhs.numpy())
         assert_close_to_truth(got[mine], truth[mine], scale[mine], f"rows={rows} k={k}")
         assert np.isnan(got[~mine]).all() and bool(torch.isnan(out[0])) and bool(torch.isnan(out[-1]))
+
+
+@pytest.mark.parametrize("as_int", [False, True])
+def test_results_made_for_other_streams(as_int):
+    """Results and workspaces that capi makes for calls on streams other than the current one: the zero-fill of an SDDMM
+    result comes before the kernels, and memory that such a stream still uses is not handed out again."""
+    A = W.zipf_rows(m=60000, n=60000, cap=4096, mean=16, device="cuda")
+    meta = capi.preprocess(A.row_ptr, A.nnz)
+    lhs, rhs = W.dense(A.m, 64, device="cuda", seed=5), W.dense(A.n, 64, device="cuda", seed=6)
+    want, want_c = capi.sddmm(meta, A.row_ptr, A.col, A.val, lhs, rhs), capi.spmm(meta, A.row_ptr, A.col, A.val, rhs)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    handle = side.cuda_stream if as_int else side
+    counts = (meta.m1, meta.m2)
+    for _ in range(5):
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(5_000_000)       # the counts are read behind the kernels, not before
+        late = capi.preprocess(A.row_ptr, A.nnz, stream=handle)
+        assert (late.m1, late.m2) == counts
+        torch.cuda._sleep(20_000_000)          # the current stream is late: a fill on it comes after the kernels unless they wait
+        out = capi.sddmm(meta, A.row_ptr, A.col, A.val, lhs, rhs, stream1=handle, stream2=handle)
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(20_000_000)      # the side stream is late: its workspace is still to be used
+        C = capi.spmm(meta, A.row_ptr, A.col, A.val, rhs, stream1=handle, stream2=handle)
+        for size in {capi.spmm_workspace_bytes(meta.m1, 64, 4), C.numel() * 4}:
+            for _ in range(3):
+                torch.full((size // 4 + 1,), float("nan"), device="cuda")
+        torch.cuda.synchronize()
+        assert torch.equal(C, want_c)
