@@ -221,9 +221,10 @@ int rode_spmm_f64_hot(int m1, int m2, int k, int n, const double *values, const 
  *
  * Replaces RoDeSDDMM_n32 / RoDeSDDMM_n128 (RoDe_SDDMM/RoDeSddmm.h:4-9, launchers
  * RoDe_SDDMM/RoDeSddmm.cu:496-545).  k: any multiple of 4 up to 256 (the reference has 32
- * and 128; here 32, 64 and 128 have kernels of their own shape, every other k runs a
- * 32-lane x 2-vector form with the vectors beyond the row's end masked);
- * lhs is [M x k], rhs is [n x k], both row-major; out is fp32[nnz] aligned with values.
+ * and 128; here 32, 64 and 128 have kernels of their own shape, every other k runs the
+ * narrowest lane group that covers the row, with the vectors beyond its end masked);
+ * lhs is [M x k], rhs is [n x k], both row-major; out is fp32[nnz] aligned with values; entries outside
+ * [row_offsets[0], row_offsets[M]) are not written.
  * Block segments run on stream1, pure-residue rows on stream2.  A null stream is the
  * default stream (the reference silently skips a kernel whose stream handle is null,
  * RoDeSddmm.cu:503,509; this library does not).  Needs no workspace: the one counter the

@@ -2,8 +2,8 @@
 //
 // Stands in for the reference's SDDMMKernel4Block / SDDMMKernel4Residue
 // (RoDe_SDDMM/RoDeSddmm.cu:15-203, :206-494) and their launchers (:496-545).  The work
-// split follows the reference's metadata (block segments, residue rows); one kernel,
-// sddmm_items, serves both lists and every K:
+// split follows the reference's metadata (block segments, residue rows).  sddmm_items serves the residue rows of
+// every K and the 32-long segments that go with K = 128; sddmm_block the long segments:
 //
 //  * A warp takes up to 32 consecutive ITEMS (block segments, or residue rows that have no
 //    block part): lane j reads the descriptor of item j, so the dependent chain row index ->
@@ -17,14 +17,15 @@
 //    its current item in registers and prefetches the next item's.
 //  * Nonzeros are handled in chunks of L per group (lane l fetches column and value of
 //    nonzero l, two chunks ahead) and, inside a chunk, in batches of 8: 8 * VPL independent
-//    LDG.128 per lane, one partial dot product per nonzero, then a shuffle reduce that halves
+//    LDG.128 per lane (8 loads in all: fewer nonzeros where a lane has several), one partial dot product per
+//    nonzero, then a shuffle reduce that halves
 //    the number of live partials at every step (4 + 2 + 1 exchanges, then a butterfly over
 //    the remaining lanes).  The finished dot products land in the lanes that hold the
 //    matching values, so results are stored coalesced.
-//  * Row mode of the residue-row kernel: a warp whose 32 rows hold at least 6 nonzeros on average
-//    does not form a stream; its lane groups (8 lanes x 2 loads for K = 64) take the rows one
-//    each, neighbouring rows side by side, each row by the plain per-row loop sddmm_one_row.
-//    The warp decides from the row lengths it has just loaded (27-point stencil, K = 64:
+//  * Row mode of the residue-row kernel: a warp whose rows are long enough (6 nonzeros on average, 16 where the stream has
+//    one lane group) and, in short lists and wide rows, about equally long does not form a stream; its lane groups
+//    take the rows one each, neighbouring rows side by side, each row by the plain per-row loop
+//    sddmm_one_row.  The warp decides from the row lengths it has just loaded (27-point stencil, K = 64:
 //    1.26 -> 0.81 ms, rhs rows shared by neighbouring rows now hit in L1; power-law rows,
 //    K = 64: 0.51 -> 0.44 ms; graphs with many empty rows keep the stream).
 //  * The column indices of a chunk reach the lanes that gather with them through a small
@@ -32,9 +33,10 @@
 //    instead of one shuffle per nonzero: shuffles share the SM's load/store data path with the
 //    gathers (block kernel K = 64 on an R-MAT graph 2.29 -> 2.16 ms, power-law residue rows
 //    K = 32 0.33 -> 0.26 ms).
-//  * sddmm_block: where segments are long (K = 32, 64: up to 543 nonzeros) a segment gets a
+//  * sddmm_block: where segments are long (every K but 128: up to 543 nonzeros) a segment gets a
 //    warp of its own; chunk loads are then plain coalesced loads without any search and the
 //    lhs slice never changes (power-law K = 32: 370 us against 744 us through sddmm_items).
+//    Small grids run segments and rows in one launch.
 //  * One-warp CTAs: a CTA's slot is held until its slowest warp finishes.
 //
 // Per nonzero: 12 B of CSR data/output plus 4*K bytes of rhs (L1/L2/HBM by reuse); per item
@@ -315,9 +317,9 @@ sddmm_block(int m1, const int *__restrict__ block_r_ind, const int *__restrict__
 // kRagged: the dense rows hold row_vecs_arg <= L * VPL vectors (any K that is a multiple of 4
 // up to 4 * L * VPL); vectors beyond the row's end are not loaded and count as zeros.
 //
-// LB > 0 (residue rows only): a warp whose rows hold at least row_mode_min nonzeros on average
+// LB > 0 (residue rows only): a warp whose rows hold at least row_mode_min nonzeros on average, and are even enough (below),
 // does not form a stream; its 32 / LB lane groups (LB lanes x VPLB loads) take the rows one
-// each, neighbouring rows side by side.  Long residue rows need no balancing over the groups,
+// each, neighbouring rows side by side.  Long even rows need no balancing over the groups,
 // and rows that share columns (stencils, meshes) then find each other's rhs rows in L1; short
 // and empty rows (graphs) are better served by the stream, which splits the warp's nonzeros
 // evenly.  The warp decides from the row lengths it has just loaded, so no statistic of the

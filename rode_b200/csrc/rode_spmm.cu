@@ -6,7 +6,8 @@
 //
 //  * A dense-row slice of the column tile (8, 16 or 32 vectors of 16 bytes) is covered by a
 //    lane group of L lanes with VPL vectors per lane (LDG.128 each): 4 x 2 for 8 vectors (8 x 1 in
-//    the block kernel), 8 x 2 for 16, 32 x 1 for 32.  Two vectors per lane halve the shuffles and the address
+//    the block kernel; 4 lanes with one 32-byte load in both where the operands are aligned to 32 bytes), 8 x 2 for 16,
+//    32 x 1 for 32.  Two vectors per lane halve the address
 //    arithmetic per byte (measured: N = 32 power-law 0.68 -> 0.58 ms, N = 64 R-MAT-21
 //    0.99 -> 0.75 ms, N = 64 stencil 0.97 -> 0.75 ms; for 32 vectors no shape beat 32 x 1).
 //    A warp holds G = 32/L lane groups.
@@ -23,8 +24,10 @@
 //    consumes the row's tail (the part shorter than 32 that the reference leaves to its
 //    residue kernel), so a row that fits one segment is finished by a single warp and
 //    stored with plain vector stores.
+//    Grids of a few segments per SM give a segment two or four warps; small products run segments and rows in
+//    one launch (spmm_one_launch).
 //  * Rows cut into several segments: every segment writes its partial row to a workspace
-//    slot (slot = segment index); spmm_fixup, ordered after spmm_block on the same stream,
+//    slot (slot = segment index); spmm_fixup, the last grid of the call,
 //    sums the slots of each such row in a fixed order (fp64 accumulation) and stores the
 //    row.  No floating-point atomics anywhere: results are deterministic.
 //  * spmm_rows (L = 32): residue rows that have no block part (aligned length < 32).  A warp
@@ -32,12 +35,13 @@
 //    dependent chain row index -> row pointer -> column -> dense row is paid once per 32
 //    rows, not per row.  The nonzeros of the 32 rows form one entry stream that runs through
 //    the same batched gather; a row is stored when the stream passes its end.
-//    spmm_rows_simple (L < 32): one lane group per residue row; spmm_rows_wide: one warp per
-//    row, for lists too short to fill the GPU.
+//    spmm_rows_simple (L < 32): one lane group per residue row, or per two short ones; spmm_rows_wide: one warp per
+//    row, for lists too short to fill the GPU.  All of them also take the rows of the whole matrix in the place of
+//    a list, and then store zeros in those without a nonzero.
 //    Rows of the list without a nonzero are not touched (the reference stores zeros there,
 //    RoDeSpmm.cu:185-194, into a C that its contract already wants zero-filled); rows with a
 //    block part are skipped (spmm_block finished them).
-//  * CTAs are one warp (four in spmm_rows_wide, whose rows are all shorter than 32): a CTA's
+//  * CTAs are one warp (four in spmm_rows_wide, whose rows are all shorter than 32, and in small grids): a CTA's
 //    slot is held until its slowest warp finishes, and segment lengths differ by more than 10x.
 //
 // Per nonzero the kernels move 8 B of CSR data and 16*L bytes of the dense operand (from

@@ -8,7 +8,7 @@ torch binding of ``librode_b200.so``).
 What differs from the reference wrapper:
   * the row decomposition runs on the GPU (the reference loops on the CPU at every
     construction and uploads three arrays, ``rode_sddmm.py:82-98``);
-  * ``k`` may also be 64, and ``rode_spmm`` is added (the reference exposes no SpMM in Python);
+  * ``k`` may be any multiple of 4 up to 256, and ``rode_spmm`` is added (the reference exposes no SpMM in Python);
   * ``rode_sddmm`` does not block the host: it launches on torch's current stream.
 """
 from __future__ import annotations

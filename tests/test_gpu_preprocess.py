@@ -129,8 +129,9 @@ def test_reference_signature_entry_point(oracle_cpu):
 @pytest.mark.parametrize("seg,kb,vec", [(512, 32, 4), (32, 32, 4), (96, 48, 12)])
 @pytest.mark.parametrize("M", [1, 2047, 2049, 8 * 2048, 8 * 2048 + 1, 1025 * 2048 + 7])
 def test_gpu_preprocess_single_pass(oracle_cpu, M, seg, kb, vec):
-    """One tile, one cluster of tiles, the first grid with a look-back, one whose look-back takes a second
-    step; a tile with more long rows (over eight segments) than the CTA's list holds."""
+    """One tile; the last grid that is one cluster and the first with a count grid before it; the first whose count CTAs take
+    eight tiles each.  300 rows of more than eight segments side by side, which a CTA's warps write, and a longer one at the
+    end."""
     rng = np.random.default_rng(M)
     lens = rng.integers(0, 70, M)
     lens[M // 2: M // 2 + 300] = 9 * seg + 5
