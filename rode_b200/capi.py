@@ -322,14 +322,17 @@ def spmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torch
         cur = _current(dev)
         s1 = cur if stream1 is None else stream1
         s2 = cur if stream2 is None else stream2
+        elsewhere = s1 is not cur or s2 is not cur
         whole = C is None and (meta.m1 > 0 or meta.m2 > 0)
         if C is None:
             C = B.new_empty((M, n)) if whole else B.new_zeros((M, n))
-            _used_on((s1, s2), cur, dev, C)
+            if elsewhere:
+                _used_on((s1, s2), cur, dev, C)
         need = spmm_workspace_bytes(meta.m1, n, B.element_size())
         if workspace is None and need:
             workspace = B.new_empty(need, dtype=torch.uint8)
-            _used_on((s1, s2), cur, dev, workspace)
+            if elsewhere:
+                _used_on((s1, s2), cur, dev, workspace)
         ws_bytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
         if whole:
             spmm_all_raw(B.dtype, M, meta.m1, k, n, values.data_ptr(), col.data_ptr(), row_ptr.data_ptr(),
