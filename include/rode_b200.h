@@ -240,6 +240,29 @@ int rode_sddmm_f32(int m1, int m2, int n, int k, const int *block_r_ind, const i
                    const float *values, const float *lhs, const float *rhs, float *out,
                    rode_stream_t stream1, rode_stream_t stream2);
 
+/* The same with scratch memory, in which the call puts the segments, cut into pieces of about 64 nonzeros (32 for k above
+ * 64), into the order of the columns that they gather from: with an rhs larger than the L2 most of the gathers then
+ * find their rows there.  Same results as rode_sddmm_f32 up to the rounding of the dot products.
+ *   M, nnz     rows of the matrix, length of values and column_indices
+ *   workspace  rode_sddmm_workspace_bytes() bytes, 16-byte aligned, contents don't-care before and after, not shared by
+ *              calls that may overlap in time; null: the call is rode_sddmm_f32.  From 2^26 rows on it is not used.
+ * The ordering runs on stream1.
+ *
+ * Whether that pays on a matrix: rode_sddmm_order_verdict sets *in_range (host) to 1 where the sizes are such that it can, and
+ * then, unless verdict (device, one int) is null, enqueues a kernel that looks at samples of the columns and writes its verdict;
+ * rode_sddmm_order_pays turns that number, read back, into yes or no for a width. */
+int rode_sddmm_order_verdict(int M, int m1, int n, int k, long long nnz, const int *row_offsets,
+                             const int *column_indices, const int *block_r_ind, int *in_range, int *verdict,
+                             rode_stream_t stream);
+int rode_sddmm_order_pays(int verdict, int k);
+int rode_sddmm_workspace_bytes(int m1, int k, long long nnz, size_t *bytes);
+
+int rode_sddmm_f32_ordered(int M, int m1, int m2, int n, int k, long long nnz, const int *block_r_ind,
+                           const int *residue_r_ind, const int *st_off, const int *row_offsets,
+                           const int *column_indices, const float *values, const float *lhs, const float *rhs,
+                           float *out, void *workspace, size_t workspace_bytes, rode_stream_t stream1,
+                           rode_stream_t stream2);
+
 #ifdef __cplusplus
 }
 #endif

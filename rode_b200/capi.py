@@ -30,6 +30,7 @@ C_ABI_SYMBOLS = (
     "rode_preprocess", "rode_preprocess_noalloc", "rode_preprocess_cpu", "rode_spmm_workspace_bytes", "rode_spmm_f32", "rode_spmm_f64",
     "rode_sddmm_f32", "rode_hot_columns_workspace_bytes", "rode_hot_columns_words", "rode_hot_columns",
     "rode_spmm_f32_hot", "rode_spmm_f64_hot", "rode_spmm_f32_all", "rode_spmm_f64_all",
+    "rode_sddmm_order_verdict", "rode_sddmm_order_pays", "rode_sddmm_workspace_bytes", "rode_sddmm_f32_ordered",
 )
 # Itanium-ABI names of the C++ entry points declared in RoDeSpmm.h / RoDeSddmm.h /
 # RoDePreprocess.h; identical to the names the reference's own objects export.
@@ -85,10 +86,15 @@ def load() -> ctypes.CDLL:
     lib.rode_spmm_f64_hot.argtypes = lib.rode_spmm_f32_hot.argtypes
     lib.rode_spmm_f32_all.argtypes = [ci, ci, ci, ci, ctypes.c_longlong, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp, vp, vp]
     lib.rode_spmm_f64_all.argtypes = lib.rode_spmm_f32_all.argtypes
+    lib.rode_sddmm_order_verdict.argtypes = [ci, ci, ci, ci, ctypes.c_longlong, vp, vp, vp, ctypes.POINTER(ci), vp, vp]
+    lib.rode_sddmm_order_pays.argtypes = [ci, ci]
+    lib.rode_sddmm_workspace_bytes.argtypes = [ci, ci, ctypes.c_longlong, ctypes.POINTER(sz)]
+    lib.rode_sddmm_f32_ordered.argtypes = [ci, ci, ci, ci, ci, ctypes.c_longlong] + [vp] * 10 + [sz, vp, vp]
     for name in ("rode_preprocess_workspace_bytes", "rode_preprocess_capacity", "rode_preprocess",
                  "rode_preprocess_noalloc", "rode_preprocess_cpu", "rode_spmm_workspace_bytes", "rode_spmm_f32", "rode_spmm_f64",
                  "rode_sddmm_f32", "rode_hot_columns_workspace_bytes", "rode_hot_columns_words", "rode_hot_columns",
-                 "rode_spmm_f32_hot", "rode_spmm_f64_hot", "rode_spmm_f32_all", "rode_spmm_f64_all"):
+                 "rode_spmm_f32_hot", "rode_spmm_f64_hot", "rode_spmm_f32_all", "rode_spmm_f64_all",
+                 "rode_sddmm_order_verdict", "rode_sddmm_order_pays", "rode_sddmm_workspace_bytes", "rode_sddmm_f32_ordered"):
         getattr(lib, name).restype = ci
     _lib = lib
     return lib
@@ -350,10 +356,43 @@ def sddmm_raw(m1, m2, n, k, blk, res, st, row_ptr, col, values, lhs, rhs, out, s
                                 _stream(stream2)))
 
 
+def sddmm_order_pays(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, n: int, k: int) -> bool:
+    """Whether ``sddmm(..., ordered=True)`` is the faster form for this matrix with an rhs of n rows and k columns
+    (rode_sddmm_order_verdict).  Reads the verdict back where the sizes are in range (4-byte D2H copy, synchronises
+    torch's current stream)."""
+    M, in_range = row_ptr.numel() - 1, ctypes.c_int(0)
+    lib = load()
+    check(lib.rode_sddmm_order_verdict(M, meta.m1, n, k, col.numel(), None, None, None, ctypes.byref(in_range), None, None))
+    if not in_range.value:
+        return False
+    with torch.cuda.device(col.device):
+        verdict = torch.empty(1, dtype=torch.int32, device=col.device)
+        check(lib.rode_sddmm_order_verdict(M, meta.m1, n, k, col.numel(), row_ptr.data_ptr(), col.data_ptr(),
+                                           meta.block_r_ind.data_ptr(), ctypes.byref(in_range), verdict.data_ptr(),
+                                           _current(col.device) or None))
+        return bool(lib.rode_sddmm_order_pays(int(verdict.item()), k))
+
+
+def sddmm_workspace_bytes(m1: int, k: int, nnz: int) -> int:
+    """Scratch of ``sddmm_ordered_raw``."""
+    out = ctypes.c_size_t(0)
+    check(load().rode_sddmm_workspace_bytes(m1, k, nnz, ctypes.byref(out)))
+    return out.value
+
+
+def sddmm_ordered_raw(M, m1, m2, n, k, nnz, blk, res, st, row_ptr, col, values, lhs, rhs, out, workspace, workspace_bytes,
+                      stream1=None, stream2=None) -> None:
+    """rode_sddmm_f32_ordered on raw device addresses."""
+    check(load().rode_sddmm_f32_ordered(M, m1, m2, n, k, nnz, blk, res, st, row_ptr, col, values, lhs, rhs, out, workspace,
+                                        workspace_bytes, _stream(stream1), _stream(stream2)))
+
+
 def sddmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torch.Tensor, lhs: torch.Tensor,
-          rhs: torch.Tensor, out: Optional[torch.Tensor] = None, stream1=None, stream2=None) -> torch.Tensor:
+          rhs: torch.Tensor, out: Optional[torch.Tensor] = None, stream1=None, stream2=None,
+          ordered: bool = False) -> torch.Tensor:
     """out[e] = values[e] * <lhs[row(e)], rhs[col(e)]> through rode_sddmm_f32.  A given ``out`` keeps what it holds in the
-    entries outside [row_ptr[0], row_ptr[M]); by default they are zero."""
+    entries outside [row_ptr[0], row_ptr[M]); by default they are zero.  ``ordered``: through rode_sddmm_f32_ordered, with
+    scratch made here (``sddmm_order_pays`` says where that is faster)."""
     k = lhs.shape[1]
     if lhs.dtype != torch.float32 or rhs.dtype != torch.float32 or values.dtype != torch.float32:
         raise ValueError("float32 tensors required")
@@ -367,7 +406,15 @@ def sddmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torc
         if out is None:  # (entries that belong to no row of row_ptr are not written)
             out = values.new_zeros(values.numel())
             _used_on((s1, s2), cur, dev, out)
-        sddmm_raw(meta.m1, meta.m2, rhs.shape[0], k, meta.block_r_ind.data_ptr(), meta.residue_r_ind.data_ptr(),
-                  meta.st_off.data_ptr(), row_ptr.data_ptr(), col.data_ptr(), values.data_ptr(), lhs.data_ptr(),
-                  rhs.data_ptr(), out.data_ptr(), s1, s2)
+        if not ordered:
+            sddmm_raw(meta.m1, meta.m2, rhs.shape[0], k, meta.block_r_ind.data_ptr(), meta.residue_r_ind.data_ptr(),
+                      meta.st_off.data_ptr(), row_ptr.data_ptr(), col.data_ptr(), values.data_ptr(), lhs.data_ptr(),
+                      rhs.data_ptr(), out.data_ptr(), s1, s2)
+            return out
+        need = sddmm_workspace_bytes(meta.m1, k, values.numel())
+        workspace = values.new_empty(need, dtype=torch.uint8)
+        _used_on((s1, s2), cur, dev, workspace)
+        sddmm_ordered_raw(row_ptr.numel() - 1, meta.m1, meta.m2, rhs.shape[0], k, values.numel(), meta.block_r_ind.data_ptr(),
+                          meta.residue_r_ind.data_ptr(), meta.st_off.data_ptr(), row_ptr.data_ptr(), col.data_ptr(),
+                          values.data_ptr(), lhs.data_ptr(), rhs.data_ptr(), out.data_ptr(), workspace.data_ptr(), need, s1, s2)
     return out

@@ -46,6 +46,7 @@
 #include <type_traits>
 
 #include "rode_common.cuh"
+#include "rode_order.cuh"
 
 namespace rode {
 namespace {
@@ -564,6 +565,130 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
 }
 
 // ---------------------------------------------------------------------------------------
+// The pieces of the block segments in the order of their columns (rode_order.cuh), a warp per piece, its G lane groups taking
+// every G-th nonzero.  One resident wave; a warp claims kPieceRounds pieces at a time, so that the pieces on the GPU are
+// neighbours in the list, and has the next piece's first columns and the one after's list entry on their way.
+//
+// What bounds it: latency (28 to 32 warps of 4 KB in flight each, every batch of 8 loads waiting for its slowest), and from 16 TB/s on the L2.
+// Pieces of 64 up to K = 64, of 32 beyond: Pareto 2^20 K = 128, order and pieces, us: P = 16 986, 32 959, against 1612 row by row; K = 64
+// P = 32 513, 64 513, 128 564, against 702; R-MAT 23 K = 64 32 2106, 64 1934, 128 2008, against 1972.  (A lane group per
+// piece: K = 128 P = 16 929 and R-MAT 21 959 against 876; spilled registers cost 10 to 40 %, so no shape here spills.)
+constexpr int kPieceRounds = 4;
+constexpr int piece_ctas(int vpl) { return vpl == 1 ? 32 : 28; }
+template <int L, int VPL, int U, bool kRagged>
+__global__ void __launch_bounds__(32, piece_ctas(VPL))
+sddmm_pieces(OrderHead *head, const unsigned long long *__restrict__ list, int capacity,
+             const int *__restrict__ column_indices, const float *__restrict__ values, const float *__restrict__ lhs,
+             const float *__restrict__ rhs, float *__restrict__ out, int row_vecs_arg) {
+    constexpr int G = 32 / L;
+    const unsigned row_vecs = kRagged ? static_cast<unsigned>(row_vecs_arg) : L * VPL;
+    const unsigned row_bytes = row_vecs * 16u;
+    const int lane = threadIdx.x;
+    const int g = lane / L, l = lane % L;
+    const int pos = l * G + g;  // this lane's nonzero of a chunk
+    __shared__ __align__(16) int s_col[2][32];
+    int stage_buf = 0;
+    chain_begin();
+    chain_wait();
+    int total = 0;
+#pragma unroll
+    for (int i = 0; i < kOrderBuckets / 32; ++i) total += __ldcg(&head->counts[lane + 32 * i]);
+    total = min(__reduce_add_sync(kFull, total), capacity);
+    const int bundles = (total + kPieceRounds - 1) / kPieceRounds;
+    const float4 *lhs_lane = reinterpret_cast<const float4 *>(lhs) + l;
+    const float4 *rhs_lane = reinterpret_cast<const float4 *>(rhs) + l;
+    auto inside = [&](int v) { return !kRagged || static_cast<unsigned>(l + v * L) < row_vecs; };
+    auto entry = [&](int bundle, int round) {
+        const long long i = static_cast<long long>(bundle) * kPieceRounds + round;
+        return bundle < bundles && i < total ? __ldcg(list + i) : 0ull;
+    };
+    // Position of the piece two ahead: round `r2` of bundle `b2`.
+    int b2 = blockIdx.x, r2 = 0;
+    if (b2 >= bundles) return;
+    int claimed = INT_MAX;
+    auto claim = [&]() {
+        if (lane == 0) claimed = static_cast<int>(gridDim.x) + atomicAdd(&head->claim[0], 1);
+    };
+    claim();
+    auto next_entry = [&]() {
+        const unsigned long long e = entry(b2, r2);
+        if (++r2 == kPieceRounds) {
+            r2 = 0;
+            b2 = __shfl_sync(kFull, claimed, 0);
+            claim();
+        }
+        return e;
+    };
+    auto fetch = [&](const Piece &p, int at, int &c, float &v) {
+        c = 0;
+        v = 0.f;
+        if (at < p.len) {
+            c = ld_stream(column_indices + p.off + at);
+            v = ld_stream(values + p.off + at);
+        }
+    };
+    Piece p = unpack_piece(next_entry());
+    unsigned long long e1 = next_entry();
+    int c_nxt;
+    float v_nxt;
+    fetch(p, pos, c_nxt, v_nxt);
+    while (true) {
+        if (p.len == 0) return;  // behind the end of the list
+        float4 a[VPL];
+#pragma unroll
+        for (int v = 0; v < VPL; ++v)
+            a[v] = inside(v) ? __ldg(lhs_lane + static_cast<size_t>(p.row) * row_vecs + v * L) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const Piece q = unpack_piece(e1);
+        int c_q;
+        float v_q;
+        fetch(q, pos, c_q, v_q);
+        e1 = next_entry();
+        for (int base = 0; base < p.len; base += 32) {
+            const int c = c_nxt;
+            const float val = v_nxt;
+            fetch(p, base + 32 + pos, c_nxt, v_nxt);
+            const int cnt = p.len - base;  // of this chunk, at most 32 count
+            float mine = 0.f;
+            s_col[stage_buf][lane] = c;
+            __syncwarp();
+            const int *my_cols = &s_col[stage_buf][g * L];
+            stage_buf ^= 1;
+#pragma unroll
+            for (int b = 0; b < L / U; ++b) {
+                if (b * U * G >= cnt) break;  // warp-uniform
+                float4 bb[U][VPL];
+                int cc[U];
+                ld_shared_run<U>(my_cols + b * U, cc);
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const float4 *src = dense_row(rhs_lane, static_cast<unsigned>(cc[u]), row_bytes);
+#pragma unroll
+                    for (int v = 0; v < VPL; ++v) {
+                        bb[u][v] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if ((b * U + u) * G + g < cnt && inside(v)) bb[u][v] = ld_dense(src + v * L);
+                    }
+                }
+                float d[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    // (two vectors per lane are added as two lanes with one each would: the same bits as the kernel without order)
+                    d[u] = dot4(a[0], bb[u][0], 0.f);
+#pragma unroll
+                    for (int v = 1; v < VPL; ++v) d[u] += dot4(a[v], bb[u][v], 0.f);
+                }
+                const float r = reduce_batch<L, U>(d, l, kFull);
+                const float got = (L == U) ? r : __shfl_sync(kFull, r, (l & (U - 1)) * (L / U), L);
+                if ((l / U) == b) mine = got;
+            }
+            if (pos < cnt) st_stream(out + p.off + base + pos, val * mine);
+        }
+        p = q;
+        c_nxt = c_q;
+        v_nxt = v_q;
+    }
+}
+
+// ---------------------------------------------------------------------------------------
 // Claim counter of the persistent block grid.  The SDDMM entry points carry no workspace, so the
 // counters live in a fixed array of the library's device image: kClaimSlots slots of 64 ints
 // (32 KB on every GPU that loads the library).  A slot belongs to one (device, stream1, stream2)
@@ -631,13 +756,36 @@ template <int L_, int VPL_, int U_>
 struct Shape {
     static constexpr int L = L_, VPL = VPL_, U = U_;
 };
+// Lengths of the pieces (rode_order.cuh) by the number of vectors of a dense row.
+constexpr int piece_len(int row_vecs) { return row_vecs <= 16 ? 64 : 32; }
+// When an order pays: an rhs beyond the L2, enough segments to pay for it, and columns that it helps (rode_order.cuh).  With wide
+// rows the pieces are also the better form for the segments of skewed matrices (whole calls, row by row / ordered, us: R-MAT 21
+// K = 128 1240 / 1189, K = 256 3106 / 2760, R-MAT 20 of 64 per row K = 128 1961 / 1910; K = 64 671 / 720, K = 96 1088 / 1229).
+// Uniform columns, us: K = 32 512 MB Pareto of mean 16 1912 / 1495, 128 MB 347 / 345 and of mean 8 228 / 241; K = 64 256 MB 1090 / 919
+// (mean 32), 364 / 368 (mean 8, 31,336 segments); Zipf 671,008 x 929,297 of mean 40 K = 64 800 / 517, K = 128 1797 / 942; K = 128 128 MB
+// Pareto 394 / 355.  Bands: 1M rows of 60 in 3000 columns K = 128 1775 / 1921.
+bool order_in_range(long long M, long long m1, long long n, int k) {
+    return M < kPieceMaxRows && m1 >= 1 << 15 && n * k * 4 >= (k > 96 ? 128ll << 20 : 160ll << 20);
+}
+bool order_pays(int verdict, int k) { return verdict == kOrderHelps || (verdict == kOrderSkewed && k > 96); }
+// The block segments through sddmm_pieces.
+template <int L, int VPL, int U>
+int launch_pieces(const Ordering &ord, int row_vecs, const int *col, const float *values, const float *lhs,
+                  const float *rhs, float *out, cudaStream_t s) {
+    const dim3 resident(piece_ctas(VPL) * sm_count());
+    const auto kernel = row_vecs == L * VPL ? sddmm_pieces<L, VPL, U, false> : sddmm_pieces<L, VPL, U, true>;
+    RODE_CUDA_TRY(launch_chained(kernel, resident, dim3(32), s, true, ord.head, ord.list, ord.capacity, col, values, lhs, rhs,
+                                 out, row_vecs));
+    RODE_CHECK_LAUNCH("rode::sddmm_pieces");
+    return RODE_OK;
+}
 // L lanes x VPL vectors for the streams; shapes of the segments (a warp each: kLongSegments, else up to 32 segments per warp
 // run as a stream, and Block serves the small grids) and of the row mode of the residue kernel; Claimed: of the persistent
 // grids of segments.
 template <int L, int VPL, typename Block, typename Rows, bool kRagged, bool kLongSegments, typename Claimed = Block>
 int launch_k(int m1, int m2, int k, const int *block_r_ind, const int *residue_r_ind,
              const int *st_off, const int *row_offsets, const int *col, const float *values, const float *lhs,
-             const float *rhs, float *out, cudaStream_t s1, cudaStream_t s2) {
+             const float *rhs, float *out, cudaStream_t s1, cudaStream_t s2, const Ordering *ord) {
     constexpr int BL = Block::L, BVPL = Block::VPL, BU = Block::U;
     constexpr int RL = Rows::L, RVPL = Rows::VPL, RU = Rows::U;
     const int row_vecs = k / 4;
@@ -654,7 +802,7 @@ int launch_k(int m1, int m2, int k, const int *block_r_ind, const int *residue_r
         const long long ctas = static_cast<long long>(m1) + (m2 + per - 1) / per;
         // (a warp per 32-long segment, K = 128, pays while they all fit at once: Bernoulli 4096^2 13.5 us with the two
         // kernels, 14.7 in one; 2000^2 12.3 and 10.3)
-        if (m1 > 0 && m2 > 0 && s1 == s2 && ctas <= (kLongSegments ? 4LL : 1LL) * 24 * sm_count()) {
+        if (ord == nullptr && m1 > 0 && m2 > 0 && s1 == s2 && ctas <= (kLongSegments ? 4LL : 1LL) * 24 * sm_count()) {
             sddmm_items<L, VPL, false, kRagged, BL, BVPL, kRowU, BL, BVPL, BU><<<static_cast<unsigned>(ctas), 32, 0, s1>>>(
                 m2, per, residue_r_ind, st_off, row_offsets, col, values, lhs, rhs, out, row_vecs, row_mode_min, m1,
                 block_r_ind);
@@ -662,7 +810,14 @@ int launch_k(int m1, int m2, int k, const int *block_r_ind, const int *residue_r
             return RODE_OK;
         }
     }
-    if (m1 > 0) {
+    if (ord != nullptr) {
+        const auto order = piece_len(row_vecs) == 64 ? launch_order<64> : launch_order<32>;
+        if (int rc = order(*ord, m1, row_offsets, col, block_r_ind, st_off, s1)) return rc;
+        const auto pieces = row_vecs <= 8 ? launch_pieces<8, 1, 8> : row_vecs <= 16 ? launch_pieces<16, 1, 8>
+                            : row_vecs <= 24 ? launch_pieces<8, 3, 2> : row_vecs <= 32 ? launch_pieces<16, 2, 4>
+                                                                                       : launch_pieces<32, 2, 4>;
+        if (int rc = pieces(*ord, row_vecs, col, values, lhs, rhs, out, s1)) return rc;
+    } else if (m1 > 0) {
         if constexpr (kLongSegments) {
             const int resident = block_ctas(Claimed::VPL) * sm_count();
             ClaimCounter claim;  // holds its lock until the kernel is enqueued
@@ -697,15 +852,9 @@ int launch_k(int m1, int m2, int k, const int *block_r_ind, const int *residue_r
     return RODE_OK;
 }
 
-}  // namespace
-}  // namespace rode
-
-extern "C" int rode_sddmm_f32(int m1, int m2, int n, int k, const int *block_r_ind, const int *residue_r_ind,
-                              const int *st_off, const int *row_offsets, const int *column_indices,
-                              const float *values, const float *lhs, const float *rhs, float *out,
-                              rode_stream_t stream1, rode_stream_t stream2) {
-    using namespace rode;
-    (void)n;
+int sddmm(int m1, int m2, int k, const int *block_r_ind, const int *residue_r_ind, const int *st_off, const int *row_offsets,
+          const int *column_indices, const float *values, const float *lhs, const float *rhs, float *out, cudaStream_t stream1,
+          cudaStream_t stream2, const Ordering *ord) {
     if (m1 < 0 || m2 < 0) return fail(RODE_ERR_INVALID_ARGUMENT, "sddmm: m1, m2 must be >= 0");
     if (k <= 0 || k % 4 != 0 || k > 256)
         return fail(RODE_ERR_INVALID_ARGUMENT, "sddmm: k = %d unsupported (a multiple of 4, at most 256)", k);
@@ -718,7 +867,7 @@ extern "C" int rode_sddmm_f32(int m1, int m2, int n, int k, const int *block_r_i
         return fail(RODE_ERR_INVALID_ARGUMENT, "sddmm: lhs and rhs must be 16-byte aligned");
 #define RODE_SDDMM_LAUNCH(...)                                                                                   \
     launch_k<__VA_ARGS__>(m1, m2, k, block_r_ind, residue_r_ind, st_off, row_offsets, column_indices, values, lhs, rhs, \
-                          out, stream1, stream2)
+                          out, stream1, stream2, ord)
     // The narrowest lane group that covers the dense row; where it does not fit exactly the lanes beyond the
     // row's end idle (ragged).  (One form of 32 lanes x 2 vectors for all of those widths took 0.209 ms on
     // the 100003 x 50021 Zipf matrix at K = 96, the 32 x 1 form 0.117 ms.)  The decomposition that goes with
@@ -737,3 +886,68 @@ extern "C" int rode_sddmm_f32(int m1, int m2, int n, int k, const int *block_r_i
     return RODE_SDDMM_LAUNCH(32, 2, Shape<16, 4, 2>, Shape<16, 4, 2>, true, true);
 #undef RODE_SDDMM_LAUNCH
 }
+
+// Bytes of an ordering workspace for pieces of at least P nonzeros on average.
+size_t ordering_bytes(long long m1, long long nnz, int P) {
+    return sizeof(OrderHead) + static_cast<size_t>(max_pieces(m1, nnz, P)) * sizeof(unsigned long long);
+}
+
+}  // namespace
+}  // namespace rode
+
+extern "C" {
+
+int rode_sddmm_f32(int m1, int m2, int n, int k, const int *block_r_ind, const int *residue_r_ind, const int *st_off,
+                   const int *row_offsets, const int *column_indices, const float *values, const float *lhs, const float *rhs,
+                   float *out, rode_stream_t stream1, rode_stream_t stream2) {
+    (void)n;
+    return rode::sddmm(m1, m2, k, block_r_ind, residue_r_ind, st_off, row_offsets, column_indices, values, lhs, rhs, out, stream1,
+                       stream2, nullptr);
+}
+
+int rode_sddmm_order_verdict(int M, int m1, int n, int k, long long nnz, const int *row_offsets, const int *column_indices,
+                             const int *block_r_ind, int *in_range, int *verdict, rode_stream_t stream) {
+    using namespace rode;
+    if (in_range == nullptr || M < 0 || m1 < 0 || n < 0 || k <= 0 || nnz < 0)
+        return fail(RODE_ERR_INVALID_ARGUMENT, "sddmm_order_verdict: bad argument");
+    *in_range = nnz > 0 && order_in_range(M, m1, n, k) ? 1 : 0;
+    if (*in_range == 0 || verdict == nullptr) return RODE_OK;
+    if (!row_offsets || !column_indices || !block_r_ind) return fail(RODE_ERR_INVALID_ARGUMENT, "sddmm_order_verdict: null array");
+    judge_columns<<<1, kJudgeThreads, 0, stream>>>(m1, n, nnz, row_offsets, column_indices, block_r_ind, verdict);
+    RODE_CHECK_LAUNCH("rode::judge_columns");
+    return RODE_OK;
+}
+
+int rode_sddmm_order_pays(int verdict, int k) { return rode::order_pays(verdict, k) ? 1 : 0; }
+
+int rode_sddmm_workspace_bytes(int m1, int k, long long nnz, size_t *bytes) {
+    using namespace rode;
+    if (bytes == nullptr || m1 < 0 || k <= 0 || nnz < 0)
+        return fail(RODE_ERR_INVALID_ARGUMENT, "sddmm_workspace_bytes: bad argument");
+    *bytes = ordering_bytes(m1, nnz, piece_len((k + 3) / 4));
+    return RODE_OK;
+}
+
+int rode_sddmm_f32_ordered(int M, int m1, int m2, int n, int k, long long nnz, const int *block_r_ind, const int *residue_r_ind,
+                           const int *st_off, const int *row_offsets, const int *column_indices, const float *values,
+                           const float *lhs, const float *rhs, float *out, void *workspace, size_t workspace_bytes,
+                           rode_stream_t stream1, rode_stream_t stream2) {
+    using namespace rode;
+    if (M < 0 || nnz < 0) return fail(RODE_ERR_INVALID_ARGUMENT, "sddmm: M, nnz must be >= 0");
+    Ordering ord = {};
+    const bool ordered = workspace != nullptr && m1 > 0 && n > 0 && k > 0 && nnz > 0 && M < kPieceMaxRows;
+    if (ordered) {
+        const size_t need = ordering_bytes(m1, nnz, piece_len((k + 3) / 4));
+        if (workspace_bytes < need)
+            return fail(RODE_ERR_WORKSPACE, "sddmm: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
+        if (!aligned_to(workspace, 16)) return fail(RODE_ERR_WORKSPACE, "sddmm: workspace must be 16-byte aligned");
+        ord.head = static_cast<OrderHead *>(workspace);
+        ord.list = reinterpret_cast<unsigned long long *>(ord.head + 1);
+        ord.capacity = static_cast<int>(max_pieces(m1, nnz, piece_len((k + 3) / 4)));
+        ord.n_cols = n;
+    }
+    return rode::sddmm(m1, m2, k, block_r_ind, residue_r_ind, st_off, row_offsets, column_indices, values, lhs, rhs, out, stream1,
+                       stream2, ordered ? &ord : nullptr);
+}
+
+}  // extern "C"

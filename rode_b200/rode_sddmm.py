@@ -36,6 +36,7 @@ class RoDeCSR:
     }
     MAX_K = 256
     _entry_range = None  # (row_offsets[0], row_offsets[m]) as of construction
+    _ordered = False     # rode_sddmm orders the segments by their columns
 
     @classmethod
     def config_for(cls, k: int) -> dict:
@@ -74,6 +75,9 @@ class RoDeCSR:
         self.residue_indices = res
         self.m1 = m1
         self.m2 = m2
+        if self.column_indices.numel() == self.nnz:
+            with torch.cuda.device(self.device):
+                self._ordered = rode_sddmm_cuda.order_pays(blk, m1, self.row_offsets, self.column_indices, self.m, self.n, self.k)
 
     @classmethod
     def from_random(cls, m: int, n: int, nnz_per_row: int, device: torch.device, k: int = 128) -> "RoDeCSR":
@@ -121,7 +125,8 @@ def rode_sddmm(sparse_matrix: RoDeCSR, lhs: torch.Tensor, rhs: torch.Tensor) -> 
     return rode_sddmm_cuda.sddmm_forward(
         sparse_matrix.block_indices, sparse_matrix.residue_indices, sparse_matrix.st_offsets, sparse_matrix.m1,
         sparse_matrix.m2, sparse_matrix.row_offsets, sparse_matrix.column_indices, sparse_matrix.values, m, n,
-        lhs.contiguous(), rhs.contiguous(), k, sparse_matrix._entry_range == (0, sparse_matrix.values.numel()))
+        lhs.contiguous(), rhs.contiguous(), k, sparse_matrix._entry_range == (0, sparse_matrix.values.numel()),
+        sparse_matrix._ordered)
 
 
 def rode_spmm(sparse_matrix: RoDeCSR, dense: torch.Tensor, hints: bool = True) -> torch.Tensor:

@@ -16,6 +16,8 @@
 //   * k_version may be any multiple of 4 up to 256.
 //   * covers_values (default false) says that row_offsets runs from 0 to the number of values, so that the result
 //     need not be zero-filled first.
+//   * ordered (default false) gives the call scratch memory in which it orders the segments by their columns; order_pays
+//     says whether that helps.
 //   * spmm_forward and hot_columns are new: the reference has no Python entry for SpMM.
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
@@ -84,7 +86,7 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, int, int> py_preprocess(
 torch::Tensor py_sddmm_forward(torch::Tensor block_indices, torch::Tensor residue_indices, torch::Tensor st_offsets,
                                  int m1, int m2, torch::Tensor row_offsets, torch::Tensor column_indices,
                                  torch::Tensor values, int m, int n, torch::Tensor lhs_matrix,
-                                 torch::Tensor rhs_matrix, int k_version, bool covers_values) {
+                                 torch::Tensor rhs_matrix, int k_version, bool covers_values, bool ordered) {
     RODE_CHECK_INPUT(block_indices);
     RODE_CHECK_INPUT(residue_indices);
     RODE_CHECK_INPUT(st_offsets);
@@ -118,11 +120,41 @@ torch::Tensor py_sddmm_forward(torch::Tensor block_indices, torch::Tensor residu
     torch::Tensor out = covers_values ? empty_cuda({values.size(0)}, torch::kFloat32, values.device())
                                       : torch::zeros({values.size(0)}, values.options());
     const cudaStream_t s = at::cuda::getCurrentCUDAStream(values.device().index()).stream();
-    check_status(rode_sddmm_f32(m1, m2, n, k, block_indices.data_ptr<int>(), residue_indices.data_ptr<int>(),
-                                st_offsets.data_ptr<int>(), row_offsets.data_ptr<int>(), column_indices.data_ptr<int>(),
-                                values.data_ptr<float>(), lhs_matrix.data_ptr<float>(), rhs_matrix.data_ptr<float>(),
-                                out.data_ptr<float>(), s, s));
+    size_t ws_bytes = 0;
+    torch::Tensor ws;
+    if (ordered) {
+        check_status(rode_sddmm_workspace_bytes(m1, k, values.size(0), &ws_bytes));
+        ws = empty_cuda({static_cast<long long>(ws_bytes)}, torch::kUInt8, values.device());
+    }
+    check_status(rode_sddmm_f32_ordered(m, m1, m2, n, k, values.size(0), block_indices.data_ptr<int>(),
+                                        residue_indices.data_ptr<int>(), st_offsets.data_ptr<int>(), row_offsets.data_ptr<int>(),
+                                        column_indices.data_ptr<int>(), values.data_ptr<float>(), lhs_matrix.data_ptr<float>(),
+                                        rhs_matrix.data_ptr<float>(), out.data_ptr<float>(), ordered ? ws.data_ptr() : nullptr,
+                                        ws_bytes, s, s));
     return out;
+}
+
+// Whether sddmm_forward should order the segments of this matrix by their columns (rode_sddmm_order_verdict).  Reads the verdict
+// back where the sizes are in range.
+bool py_order_pays(torch::Tensor block_indices, int m1, torch::Tensor row_offsets, torch::Tensor column_indices, int m, int n,
+                   int k) {
+    RODE_CHECK_INPUT(block_indices);
+    RODE_CHECK_INPUT(row_offsets);
+    RODE_CHECK_INPUT(column_indices);
+    RODE_CHECK_INT(block_indices);
+    RODE_CHECK_INT(row_offsets);
+    RODE_CHECK_INT(column_indices);
+    TORCH_CHECK(row_offsets.size(0) == static_cast<long long>(m) + 1, "row_offsets must have m + 1 entries");
+    const c10::cuda::CUDAGuard guard(column_indices.device());
+    const long long nnz = column_indices.numel();
+    int in_range = 0;
+    check_status(rode_sddmm_order_verdict(m, m1, n, k, nnz, nullptr, nullptr, nullptr, &in_range, nullptr, nullptr));
+    if (!in_range) return false;
+    torch::Tensor verdict = torch::empty({1}, column_indices.options());
+    check_status(rode_sddmm_order_verdict(m, m1, n, k, nnz, row_offsets.data_ptr<int>(), column_indices.data_ptr<int>(),
+                                          block_indices.data_ptr<int>(), &in_range, verdict.data_ptr<int>(),
+                                          at::cuda::getCurrentCUDAStream(column_indices.device().index()).stream()));
+    return rode_sddmm_order_pays(verdict.item<int>(), k) != 0;
 }
 
 // Popularity bitmap of the columns for spmm_forward's `hot_columns` argument (rode_hot_columns),
@@ -215,7 +247,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("sddmm_forward", &py_sddmm_forward, "RoDe SDDMM forward (CUDA)", py::arg("block_indices"),
           py::arg("residue_indices"), py::arg("st_offsets"), py::arg("m1"), py::arg("m2"), py::arg("row_offsets"),
           py::arg("column_indices"), py::arg("values"), py::arg("m"), py::arg("n"), py::arg("lhs_matrix"),
-          py::arg("rhs_matrix"), py::arg("k_version"), py::arg("covers_values") = false);
+          py::arg("rhs_matrix"), py::arg("k_version"), py::arg("covers_values") = false, py::arg("ordered") = false);
+    m.def("order_pays", &py_order_pays, "Whether ordered=True pays in sddmm_forward (CUDA)", py::arg("block_indices"),
+          py::arg("m1"), py::arg("row_offsets"), py::arg("column_indices"), py::arg("m"), py::arg("n"), py::arg("k"));
     m.def("spmm_forward", &py_spmm_forward, "RoDe SpMM forward (CUDA)", py::arg("block_indices"),
           py::arg("residue_indices"), py::arg("st_offsets"), py::arg("m1"), py::arg("m2"), py::arg("row_offsets"),
           py::arg("column_indices"), py::arg("values"), py::arg("m"), py::arg("k"), py::arg("dense"),
