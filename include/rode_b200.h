@@ -179,6 +179,37 @@ int rode_spmm_f64_all(int M, int m1, int k, int n, long long nnz, const double *
                       rode_stream_t stream1, rode_stream_t stream2);
 
 /* ------------------------------------------------------------------------------------
+ * Segments in the order of the columns that they gather from.  No counterpart in the reference.
+ *
+ * Columns ascend within a row, so a segment of a long row gathers from a narrow band of the dense operand.  With an operand
+ * larger than the L2, working through the segments row by row reads a dense row from DRAM almost once per gather; sorted by
+ * their first columns, segments that need the same rows run at about the same time.  rode_spmm_f32_ordered / _f64_ordered and
+ * rode_sddmm_f32_ordered sort them (into 256 bands of columns) on stream1 in every call; rows with columns in any order
+ * give the same results.
+ *
+ * Whether it helps on a matrix: rode_order_verdict sets *in_range (host) to 1 where the number of segments and columns is such
+ * that it can, and then, unless verdict (device, one int) is null, enqueues a kernel that looks at samples of the columns and
+ * writes its verdict (narrow bands anyway, a few columns with most of the references, neither).  rode_spmm_order_pays and
+ * rode_sddmm_order_pays turn that number, read back, into yes or no for one width.
+ *
+ * SpMM: everything as for rode_spmm_f32_all / _f64_all without hot_columns, bit for bit; the workspace is
+ * rode_spmm_ordered_workspace_bytes() large, 16-byte aligned. */
+int rode_order_verdict(int m1, int n_cols, long long nnz, const int *row_offsets, const int *column_indices,
+                       const int *block_r_ind, int *in_range, int *verdict, rode_stream_t stream);
+int rode_spmm_order_pays(int verdict, int m1, int k, int n, long long nnz, int elem_size);
+int rode_spmm_ordered_workspace_bytes(int m1, int n, int elem_size, size_t *bytes);
+
+int rode_spmm_f32_ordered(int M, int m1, int k, int n, long long nnz, const float *values, const int *column_indices,
+                          const int *row_offsets, const int *block_r_ind, const int *st_off, const float *B,
+                          float *C, void *workspace, size_t workspace_bytes, rode_stream_t stream1,
+                          rode_stream_t stream2);
+
+int rode_spmm_f64_ordered(int M, int m1, int k, int n, long long nnz, const double *values, const int *column_indices,
+                          const int *row_offsets, const int *block_r_ind, const int *st_off, const double *B,
+                          double *C, void *workspace, size_t workspace_bytes, rode_stream_t stream1,
+                          rode_stream_t stream2);
+
+/* ------------------------------------------------------------------------------------
  * Column popularity hints for the gathers.  No counterpart in the reference.
  *
  * When the dense operand is many times larger than the L2 and a few columns receive most of
@@ -240,21 +271,15 @@ int rode_sddmm_f32(int m1, int m2, int n, int k, const int *block_r_ind, const i
                    const float *values, const float *lhs, const float *rhs, float *out,
                    rode_stream_t stream1, rode_stream_t stream2);
 
-/* The same with scratch memory, in which the call puts the segments, cut into pieces of about 64 nonzeros (32 for k above
- * 64), into the order of the columns that they gather from: with an rhs larger than the L2 most of the gathers then
- * find their rows there.  Same results as rode_sddmm_f32 up to the rounding of the dot products.
+/* The same with the segments, cut into pieces of about 64 nonzeros (32 for k above 64), in the order of the columns that they
+ * gather from (see above).  Same results as rode_sddmm_f32 up to the rounding of the dot products.
  *   M, nnz     rows of the matrix, length of values and column_indices
  *   workspace  rode_sddmm_workspace_bytes() bytes, 16-byte aligned, contents don't-care before and after, not shared by
  *              calls that may overlap in time; null: the call is rode_sddmm_f32.  From 2^26 rows on it is not used.
  * The ordering runs on stream1.
  *
- * Whether that pays on a matrix: rode_sddmm_order_verdict sets *in_range (host) to 1 where the sizes are such that it can, and
- * then, unless verdict (device, one int) is null, enqueues a kernel that looks at samples of the columns and writes its verdict;
- * rode_sddmm_order_pays turns that number, read back, into yes or no for a width. */
-int rode_sddmm_order_verdict(int M, int m1, int n, int k, long long nnz, const int *row_offsets,
-                             const int *column_indices, const int *block_r_ind, int *in_range, int *verdict,
-                             rode_stream_t stream);
-int rode_sddmm_order_pays(int verdict, int k);
+ * Whether that pays: rode_sddmm_order_pays, with the verdict of rode_order_verdict on the matrix. */
+int rode_sddmm_order_pays(int verdict, int M, int m1, int n, int k, long long nnz);
 int rode_sddmm_workspace_bytes(int m1, int k, long long nnz, size_t *bytes);
 
 int rode_sddmm_f32_ordered(int M, int m1, int m2, int n, int k, long long nnz, const int *block_r_ind,

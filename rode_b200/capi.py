@@ -30,7 +30,8 @@ C_ABI_SYMBOLS = (
     "rode_preprocess", "rode_preprocess_noalloc", "rode_preprocess_cpu", "rode_spmm_workspace_bytes", "rode_spmm_f32", "rode_spmm_f64",
     "rode_sddmm_f32", "rode_hot_columns_workspace_bytes", "rode_hot_columns_words", "rode_hot_columns",
     "rode_spmm_f32_hot", "rode_spmm_f64_hot", "rode_spmm_f32_all", "rode_spmm_f64_all",
-    "rode_sddmm_order_verdict", "rode_sddmm_order_pays", "rode_sddmm_workspace_bytes", "rode_sddmm_f32_ordered",
+    "rode_order_verdict", "rode_sddmm_order_pays", "rode_sddmm_workspace_bytes", "rode_sddmm_f32_ordered",
+    "rode_spmm_order_pays", "rode_spmm_ordered_workspace_bytes", "rode_spmm_f32_ordered", "rode_spmm_f64_ordered",
 )
 # Itanium-ABI names of the C++ entry points declared in RoDeSpmm.h / RoDeSddmm.h /
 # RoDePreprocess.h; identical to the names the reference's own objects export.
@@ -86,15 +87,20 @@ def load() -> ctypes.CDLL:
     lib.rode_spmm_f64_hot.argtypes = lib.rode_spmm_f32_hot.argtypes
     lib.rode_spmm_f32_all.argtypes = [ci, ci, ci, ci, ctypes.c_longlong, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp, vp, vp]
     lib.rode_spmm_f64_all.argtypes = lib.rode_spmm_f32_all.argtypes
-    lib.rode_sddmm_order_verdict.argtypes = [ci, ci, ci, ci, ctypes.c_longlong, vp, vp, vp, ctypes.POINTER(ci), vp, vp]
-    lib.rode_sddmm_order_pays.argtypes = [ci, ci]
+    lib.rode_order_verdict.argtypes = [ci, ci, ctypes.c_longlong, vp, vp, vp, ctypes.POINTER(ci), vp, vp]
+    lib.rode_sddmm_order_pays.argtypes = [ci] * 5 + [ctypes.c_longlong]
+    lib.rode_spmm_order_pays.argtypes = [ci] * 4 + [ctypes.c_longlong, ci]
+    lib.rode_spmm_ordered_workspace_bytes.argtypes = [ci, ci, ci, ctypes.POINTER(sz)]
+    lib.rode_spmm_f32_ordered.argtypes = [ci, ci, ci, ci, ctypes.c_longlong, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp, vp]
+    lib.rode_spmm_f64_ordered.argtypes = lib.rode_spmm_f32_ordered.argtypes
     lib.rode_sddmm_workspace_bytes.argtypes = [ci, ci, ctypes.c_longlong, ctypes.POINTER(sz)]
     lib.rode_sddmm_f32_ordered.argtypes = [ci, ci, ci, ci, ci, ctypes.c_longlong] + [vp] * 10 + [sz, vp, vp]
     for name in ("rode_preprocess_workspace_bytes", "rode_preprocess_capacity", "rode_preprocess",
                  "rode_preprocess_noalloc", "rode_preprocess_cpu", "rode_spmm_workspace_bytes", "rode_spmm_f32", "rode_spmm_f64",
                  "rode_sddmm_f32", "rode_hot_columns_workspace_bytes", "rode_hot_columns_words", "rode_hot_columns",
                  "rode_spmm_f32_hot", "rode_spmm_f64_hot", "rode_spmm_f32_all", "rode_spmm_f64_all",
-                 "rode_sddmm_order_verdict", "rode_sddmm_order_pays", "rode_sddmm_workspace_bytes", "rode_sddmm_f32_ordered"):
+                 "rode_order_verdict", "rode_sddmm_order_pays", "rode_sddmm_workspace_bytes", "rode_sddmm_f32_ordered",
+                 "rode_spmm_order_pays", "rode_spmm_ordered_workspace_bytes", "rode_spmm_f32_ordered", "rode_spmm_f64_ordered"):
         getattr(lib, name).restype = ci
     _lib = lib
     return lib
@@ -282,6 +288,42 @@ def spmm_all_raw(dtype, M, m1, k, n, values, col, row_ptr, blk, st, B, C, worksp
              _stream(stream2)))
 
 
+def order_verdict(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, n_cols: int) -> int:
+    """What rode_order_verdict says of the columns, for ``spmm_order_pays`` and ``sddmm_order_pays``; -1 where the sizes are out
+    of its range.  Reads the verdict back where they are not (4-byte D2H copy, synchronises torch's current stream)."""
+    in_range, lib = ctypes.c_int(0), load()
+    check(lib.rode_order_verdict(meta.m1, n_cols, col.numel(), None, None, None, ctypes.byref(in_range), None, None))
+    if not in_range.value:
+        return -1
+    with torch.cuda.device(col.device):
+        verdict = torch.empty(1, dtype=torch.int32, device=col.device)
+        check(lib.rode_order_verdict(meta.m1, n_cols, col.numel(), row_ptr.data_ptr(), col.data_ptr(), meta.block_r_ind.data_ptr(),
+                                     ctypes.byref(in_range), verdict.data_ptr(), _current(col.device) or None))
+        return int(verdict.item())
+
+
+def spmm_order_pays(verdict: int, m1: int, n_cols: int, width: int, nnz: int, elem_size: int = 4) -> bool:
+    return bool(load().rode_spmm_order_pays(verdict, m1, n_cols, width, nnz, elem_size))
+
+
+def sddmm_order_pays(verdict: int, M: int, m1: int, n_cols: int, k: int, nnz: int) -> bool:
+    return bool(load().rode_sddmm_order_pays(verdict, M, m1, n_cols, k, nnz))
+
+
+def spmm_ordered_workspace_bytes(m1: int, n: int, elem_size: int = 4) -> int:
+    out = ctypes.c_size_t(0)
+    check(load().rode_spmm_ordered_workspace_bytes(m1, n, elem_size, ctypes.byref(out)))
+    return out.value
+
+
+def spmm_ordered_raw(dtype, M, m1, k, n, nnz, values, col, row_ptr, blk, st, B, C, workspace, workspace_bytes, stream1=None,
+                     stream2=None) -> None:
+    """rode_spmm_f32_ordered / _f64_ordered on raw device addresses."""
+    fn = load().rode_spmm_f32_ordered if dtype == torch.float32 else load().rode_spmm_f64_ordered
+    check(fn(M, m1, k, n, nnz, values, col, row_ptr, blk, st, B, C, workspace, workspace_bytes, _stream(stream1),
+             _stream(stream2)))
+
+
 def hot_columns_raw(nnz, n_cols, col, dense_row_bytes, budget_bytes, bitmap, workspace, workspace_bytes,
                     stream=None) -> None:
     check(load().rode_hot_columns(nnz, n_cols, col, dense_row_bytes, budget_bytes, bitmap, workspace,
@@ -354,23 +396,6 @@ def spmm(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, values: torch
 def sddmm_raw(m1, m2, n, k, blk, res, st, row_ptr, col, values, lhs, rhs, out, stream1=None, stream2=None) -> None:
     check(load().rode_sddmm_f32(m1, m2, n, k, blk, res, st, row_ptr, col, values, lhs, rhs, out, _stream(stream1),
                                 _stream(stream2)))
-
-
-def sddmm_order_pays(meta: RodeMeta, row_ptr: torch.Tensor, col: torch.Tensor, n: int, k: int) -> bool:
-    """Whether ``sddmm(..., ordered=True)`` is the faster form for this matrix with an rhs of n rows and k columns
-    (rode_sddmm_order_verdict).  Reads the verdict back where the sizes are in range (4-byte D2H copy, synchronises
-    torch's current stream)."""
-    M, in_range = row_ptr.numel() - 1, ctypes.c_int(0)
-    lib = load()
-    check(lib.rode_sddmm_order_verdict(M, meta.m1, n, k, col.numel(), None, None, None, ctypes.byref(in_range), None, None))
-    if not in_range.value:
-        return False
-    with torch.cuda.device(col.device):
-        verdict = torch.empty(1, dtype=torch.int32, device=col.device)
-        check(lib.rode_sddmm_order_verdict(M, meta.m1, n, k, col.numel(), row_ptr.data_ptr(), col.data_ptr(),
-                                           meta.block_r_ind.data_ptr(), ctypes.byref(in_range), verdict.data_ptr(),
-                                           _current(col.device) or None))
-        return bool(lib.rode_sddmm_order_pays(int(verdict.item()), k))
 
 
 def sddmm_workspace_bytes(m1: int, k: int, nnz: int) -> int:

@@ -17,9 +17,14 @@
 
 namespace rode {
 
+// Below so many segments an order does not pay for itself, below so many columns the dense operand fits the L2 at any width in
+// use (1 KB per row: 160 MB).
+constexpr int kOrderMinSegments = 1 << 13;
+constexpr int kOrderLongRows = 330;  // nonzeros of the matrix per segment: most are in rows of many (512-long) segments
+constexpr int kOrderMinColumns = 160 << 10;
 constexpr int kOrderBuckets = 256;   // one per thread of an ordering CTA
 constexpr int kOrderThreads = kOrderBuckets;
-constexpr int kOrderPerThread = 8;   // pieces a thread holds per round
+constexpr int kOrderPerThread = 8;   // pieces a thread holds per round (1 where a segment is one)
 // Head of the ordering's part of a workspace, zeroed before the call's first kernel; the list follows it.
 struct OrderHead {
     int counts[kOrderBuckets];  // pieces per bucket
@@ -59,6 +64,28 @@ struct Cuts {
 };
 // At most so many pieces in m1 segments that hold nnz nonzeros together.
 inline long long max_pieces(long long m1, long long nnz, int P) { return nnz / P + m1; }
+
+// P = 0: whole segments.  number: of the segment; last bit of `bits`: it is all of its row.
+struct __align__(16) WholeSegment {
+    int row, off, end, bits;
+    __host__ __device__ int number() const { return bits >> 1; }
+    __host__ __device__ bool whole_row() const { return (bits & 1) != 0; }
+};
+constexpr int kWholeMaxSegments = 1 << 30;
+template <int P>
+struct Entry {
+    using type = unsigned long long;
+};
+template <>
+struct Entry<0> {
+    using type = WholeSegment;
+};
+
+// Bytes of an ordering workspace.
+template <int P>
+size_t ordering_bytes(long long m1, long long nnz) {
+    return sizeof(OrderHead) + static_cast<size_t>(P > 0 ? max_pieces(m1, nnz, P > 0 ? P : 1) : m1) * sizeof(typename Entry<P>::type);
+}
 
 #ifdef __CUDACC__
 // What keeps an order by columns from helping, judged from samples at even distances.  kOrderLocal: rows are narrow bands already
@@ -127,9 +154,11 @@ template <int P, bool kPlace>
 __global__ void __launch_bounds__(kOrderThreads)
 order_pieces(int m1, int n_cols, const int *__restrict__ row_offsets, const int *__restrict__ column_indices,
              const int *__restrict__ block_r_ind, const int *__restrict__ st_off, OrderHead *head,
-             unsigned long long *__restrict__ list, int capacity) {
+             typename Entry<P>::type *__restrict__ list, int capacity) {
+    using E = typename Entry<P>::type;
     constexpr unsigned kFull = 0xffffffffu;
     __shared__ int s_row[kOrderThreads], s_off[kOrderThreads], s_end[kOrderThreads], s_stop[kOrderThreads];
+    __shared__ int s_whole[P == 0 ? kOrderThreads : 1];
     __shared__ int s_warp[kOrderThreads / 32], s_hist[kOrderBuckets], s_base[kOrderBuckets];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     chain_begin();
@@ -138,8 +167,14 @@ order_pieces(int m1, int n_cols, const int *__restrict__ row_offsets, const int 
     if (seg < m1) {
         row = __ldg(block_r_ind + seg);
         off = __ldg(st_off + seg);
-        end = min(__ldg(row_offsets + row + 1), seg + 1 < m1 ? __ldg(st_off + seg + 1) : INT_MAX);
-        n = Cuts<P>(off, end).count();
+        const int next = seg + 1 < m1 ? __ldg(st_off + seg + 1) : INT_MAX;
+        const int row_end = __ldg(row_offsets + row + 1);
+        end = min(row_end, next);
+        if constexpr (P == 0) s_whole[t] = off == __ldg(row_offsets + row) && next >= row_end ? 1 : 0;
+        if constexpr (P > 0)
+            n = Cuts<P>(off, end).count();
+        else
+            n = 1;
     }
     // exclusive prefix sum over the CTA
     auto scan = [&](int x, int &total) {
@@ -174,11 +209,12 @@ order_pieces(int m1, int n_cols, const int *__restrict__ row_offsets, const int 
         my_start = scan(__ldcg(&head->counts[t]), unused);
     }
     __syncthreads();
-    for (int base = 0; base < total; base += kOrderThreads * kOrderPerThread) {
-        unsigned long long piece[kOrderPerThread];
-        int key[kOrderPerThread], rank[kOrderPerThread];
+    constexpr int N = P > 0 ? kOrderPerThread : 1;
+    for (int base = 0; base < total; base += kOrderThreads * N) {
+        E piece[N];
+        int key[N], rank[N];
 #pragma unroll
-        for (int i = 0; i < kOrderPerThread; ++i) {
+        for (int i = 0; i < N; ++i) {
             const int q = base + i * kOrderThreads + t;
             key[i] = -1;
             if (q < total) {
@@ -186,17 +222,23 @@ order_pieces(int m1, int n_cols, const int *__restrict__ row_offsets, const int 
 #pragma unroll
                 for (int step = kOrderThreads / 2; step >= 1; step >>= 1)
                     if (s_stop[lo + step - 1] <= q) lo += step;
-                const Cuts<P> cuts(s_off[lo], s_end[lo]);
-                const int j = q - (lo > 0 ? s_stop[lo - 1] : 0);
-                const int b = cuts.begin(j);
-                piece[i] = pack_piece(s_row[lo], b, cuts.stop(j) - b);
+                int b;
+                if constexpr (P > 0) {
+                    const Cuts<P> cuts(s_off[lo], s_end[lo]);
+                    const int j = q - (lo > 0 ? s_stop[lo - 1] : 0);
+                    b = cuts.begin(j);
+                    piece[i] = pack_piece(s_row[lo], b, cuts.stop(j) - b);
+                } else {
+                    b = s_off[lo];
+                    piece[i] = {s_row[lo], b, s_end[lo], (static_cast<int>(blockIdx.x) * kOrderThreads + lo) << 1 | s_whole[lo]};
+                }
                 const unsigned c = static_cast<unsigned>(__ldg(column_indices + b));
                 key[i] = static_cast<int>(min(static_cast<unsigned long long>(c) * kOrderBuckets / static_cast<unsigned>(n_cols),
                                               kOrderBuckets - 1ull));
             }
         }
 #pragma unroll
-        for (int i = 0; i < kOrderPerThread; ++i)
+        for (int i = 0; i < N; ++i)
             if (key[i] >= 0) rank[i] = atomicAdd(&s_hist[key[i]], 1);
         if constexpr (kPlace) {
             __syncthreads();
@@ -205,7 +247,7 @@ order_pieces(int m1, int n_cols, const int *__restrict__ row_offsets, const int 
             s_hist[t] = 0;
             __syncthreads();
 #pragma unroll
-            for (int i = 0; i < kOrderPerThread; ++i)
+            for (int i = 0; i < N; ++i)
                 if (key[i] >= 0 && s_base[key[i]] + rank[i] < capacity) list[s_base[key[i]] + rank[i]] = piece[i];
             __syncthreads();
         }
@@ -218,8 +260,11 @@ order_pieces(int m1, int n_cols, const int *__restrict__ row_offsets, const int 
 // What a call with an ordering workspace has: the head, the list behind it, and the number of columns.
 struct Ordering {
     OrderHead *head;
-    unsigned long long *list;
     int capacity, n_cols;
+    template <int P>
+    typename Entry<P>::type *list() const {
+        return reinterpret_cast<typename Entry<P>::type *>(head + 1);
+    }
 };
 // The order of the segments' pieces, on s.  The kernel that works through the list is launched chained behind it.
 template <int P>
@@ -227,10 +272,10 @@ int launch_order(const Ordering &ord, int m1, const int *row_offsets, const int 
                  cudaStream_t s) {
     const dim3 grid((m1 + kOrderThreads - 1) / kOrderThreads), block(kOrderThreads);
     RODE_CUDA_TRY(cudaMemsetAsync(ord.head, 0, sizeof(OrderHead), s));
-    order_pieces<P, false><<<grid, block, 0, s>>>(m1, ord.n_cols, row_offsets, col, block_r_ind, st_off, ord.head, ord.list,
+    order_pieces<P, false><<<grid, block, 0, s>>>(m1, ord.n_cols, row_offsets, col, block_r_ind, st_off, ord.head, ord.list<P>(),
                                                   ord.capacity);
     RODE_CUDA_TRY(launch_chained(order_pieces<P, true>, grid, block, s, true, m1, ord.n_cols, row_offsets, col, block_r_ind,
-                                 st_off, ord.head, ord.list, ord.capacity));
+                                 st_off, ord.head, ord.list<P>(), ord.capacity));
     RODE_CHECK_LAUNCH("rode::order_pieces");
     return RODE_OK;
 }

@@ -763,18 +763,19 @@ constexpr int piece_len(int row_vecs) { return row_vecs <= 16 ? 64 : 32; }
 // K = 128 1240 / 1189, K = 256 3106 / 2760, R-MAT 20 of 64 per row K = 128 1961 / 1910; K = 64 671 / 720, K = 96 1088 / 1229).
 // Uniform columns, us: K = 32 512 MB Pareto of mean 16 1912 / 1495, 128 MB 347 / 345 and of mean 8 228 / 241; K = 64 256 MB 1090 / 919
 // (mean 32), 364 / 368 (mean 8, 31,336 segments); Zipf 671,008 x 929,297 of mean 40 K = 64 800 / 517, K = 128 1797 / 942; K = 128 128 MB
-// Pareto 394 / 355.  Bands: 1M rows of 60 in 3000 columns K = 128 1775 / 1921.
-bool order_in_range(long long M, long long m1, long long n, int k) {
-    return M < kPieceMaxRows && m1 >= 1 << 15 && n * k * 4 >= (k > 96 ? 128ll << 20 : 160ll << 20);
+// Pareto 394 / 355; 10,953 segments Zipf of mean 16 K = 64 159 / 156, K = 96 265 / 241.  Bands: 1M rows of 60 in 3000 columns K = 128 1775 / 1921.
+bool order_pays(int verdict, long long M, long long m1, long long n, int k, long long nnz) {
+    const bool enough = m1 >= 1 << 15 || (k > 64 && m1 >= kOrderMinSegments && nnz >= kOrderLongRows * m1);
+    return M < kPieceMaxRows && enough && n * k * 4 >= (k > 96 ? 128ll << 20 : 160ll << 20) &&
+           (verdict == kOrderHelps || (verdict == kOrderSkewed && k > 96));
 }
-bool order_pays(int verdict, int k) { return verdict == kOrderHelps || (verdict == kOrderSkewed && k > 96); }
 // The block segments through sddmm_pieces.
 template <int L, int VPL, int U>
 int launch_pieces(const Ordering &ord, int row_vecs, const int *col, const float *values, const float *lhs,
                   const float *rhs, float *out, cudaStream_t s) {
     const dim3 resident(piece_ctas(VPL) * sm_count());
     const auto kernel = row_vecs == L * VPL ? sddmm_pieces<L, VPL, U, false> : sddmm_pieces<L, VPL, U, true>;
-    RODE_CUDA_TRY(launch_chained(kernel, resident, dim3(32), s, true, ord.head, ord.list, ord.capacity, col, values, lhs, rhs,
+    RODE_CUDA_TRY(launch_chained(kernel, resident, dim3(32), s, true, ord.head, ord.list<64>(), ord.capacity, col, values, lhs, rhs,
                                  out, row_vecs));
     RODE_CHECK_LAUNCH("rode::sddmm_pieces");
     return RODE_OK;
@@ -887,9 +888,8 @@ int sddmm(int m1, int m2, int k, const int *block_r_ind, const int *residue_r_in
 #undef RODE_SDDMM_LAUNCH
 }
 
-// Bytes of an ordering workspace for pieces of at least P nonzeros on average.
-size_t ordering_bytes(long long m1, long long nnz, int P) {
-    return sizeof(OrderHead) + static_cast<size_t>(max_pieces(m1, nnz, P)) * sizeof(unsigned long long);
+size_t piece_bytes(long long m1, long long nnz, int row_vecs) {
+    return piece_len(row_vecs) == 64 ? ordering_bytes<64>(m1, nnz) : ordering_bytes<32>(m1, nnz);
 }
 
 }  // namespace
@@ -905,26 +905,28 @@ int rode_sddmm_f32(int m1, int m2, int n, int k, const int *block_r_ind, const i
                        stream2, nullptr);
 }
 
-int rode_sddmm_order_verdict(int M, int m1, int n, int k, long long nnz, const int *row_offsets, const int *column_indices,
-                             const int *block_r_ind, int *in_range, int *verdict, rode_stream_t stream) {
+int rode_order_verdict(int m1, int n_cols, long long nnz, const int *row_offsets, const int *column_indices,
+                       const int *block_r_ind, int *in_range, int *verdict, rode_stream_t stream) {
     using namespace rode;
-    if (in_range == nullptr || M < 0 || m1 < 0 || n < 0 || k <= 0 || nnz < 0)
-        return fail(RODE_ERR_INVALID_ARGUMENT, "sddmm_order_verdict: bad argument");
-    *in_range = nnz > 0 && order_in_range(M, m1, n, k) ? 1 : 0;
+    if (in_range == nullptr || m1 < 0 || n_cols < 0 || nnz < 0)
+        return fail(RODE_ERR_INVALID_ARGUMENT, "order_verdict: bad argument");
+    *in_range = nnz > 0 && m1 >= kOrderMinSegments && n_cols >= kOrderMinColumns ? 1 : 0;
     if (*in_range == 0 || verdict == nullptr) return RODE_OK;
-    if (!row_offsets || !column_indices || !block_r_ind) return fail(RODE_ERR_INVALID_ARGUMENT, "sddmm_order_verdict: null array");
-    judge_columns<<<1, kJudgeThreads, 0, stream>>>(m1, n, nnz, row_offsets, column_indices, block_r_ind, verdict);
+    if (!row_offsets || !column_indices || !block_r_ind) return fail(RODE_ERR_INVALID_ARGUMENT, "order_verdict: null array");
+    judge_columns<<<1, kJudgeThreads, 0, stream>>>(m1, n_cols, nnz, row_offsets, column_indices, block_r_ind, verdict);
     RODE_CHECK_LAUNCH("rode::judge_columns");
     return RODE_OK;
 }
 
-int rode_sddmm_order_pays(int verdict, int k) { return rode::order_pays(verdict, k) ? 1 : 0; }
+int rode_sddmm_order_pays(int verdict, int M, int m1, int n, int k, long long nnz) {
+    return rode::order_pays(verdict, M, m1, n, k, nnz) ? 1 : 0;
+}
 
 int rode_sddmm_workspace_bytes(int m1, int k, long long nnz, size_t *bytes) {
     using namespace rode;
     if (bytes == nullptr || m1 < 0 || k <= 0 || nnz < 0)
         return fail(RODE_ERR_INVALID_ARGUMENT, "sddmm_workspace_bytes: bad argument");
-    *bytes = ordering_bytes(m1, nnz, piece_len((k + 3) / 4));
+    *bytes = piece_bytes(m1, nnz, (k + 3) / 4);
     return RODE_OK;
 }
 
@@ -937,12 +939,11 @@ int rode_sddmm_f32_ordered(int M, int m1, int m2, int n, int k, long long nnz, c
     Ordering ord = {};
     const bool ordered = workspace != nullptr && m1 > 0 && n > 0 && k > 0 && nnz > 0 && M < kPieceMaxRows;
     if (ordered) {
-        const size_t need = ordering_bytes(m1, nnz, piece_len((k + 3) / 4));
+        const size_t need = piece_bytes(m1, nnz, (k + 3) / 4);
         if (workspace_bytes < need)
             return fail(RODE_ERR_WORKSPACE, "sddmm: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
         if (!aligned_to(workspace, 16)) return fail(RODE_ERR_WORKSPACE, "sddmm: workspace must be 16-byte aligned");
         ord.head = static_cast<OrderHead *>(workspace);
-        ord.list = reinterpret_cast<unsigned long long *>(ord.head + 1);
         ord.capacity = static_cast<int>(max_pieces(m1, nnz, piece_len((k + 3) / 4)));
         ord.n_cols = n;
     }

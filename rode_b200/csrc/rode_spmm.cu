@@ -50,6 +50,7 @@
 #include <type_traits>
 
 #include "rode_common.cuh"
+#include "rode_order.cuh"
 
 namespace rode {
 namespace {
@@ -128,14 +129,17 @@ constexpr int kLoadsInFlight = 8;
 // L * VPL vectors.  U = dense rows per batch: 8 loads of 16 bytes per lane, with which 64 registers keep 32 warps
 // per SM resident.
 //
+// kOrdered: the segments as `order` lists them, whose entries hold what the warp needs of the row pointer too.
+//
 // kRagged: the width is not a multiple of the tile; the last tile's lanes beyond the row's end neither
 // load nor store (widths the reference's tiles do not serve: any multiple of 4 columns).
-template <typename T, int VB, int L, int VPL, int U, int W, int S, bool kHints, bool kClaim, bool kRagged>
+template <typename T, int VB, int L, int VPL, int U, int W, int S, bool kHints, bool kClaim, bool kRagged, bool kOrdered = false>
 __global__ void __launch_bounds__(32 * W, 32 / W)
 spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ column_indices,
            const int *__restrict__ row_offsets, const int *__restrict__ block_r_ind,
            const int *__restrict__ st_off, const T *__restrict__ B, T *__restrict__ C, T *__restrict__ partial,
-           const unsigned *__restrict__ hot, int hot_flag_word, int *__restrict__ next_segment) {
+           const unsigned *__restrict__ hot, int hot_flag_word, int *__restrict__ next_segment,
+           const WholeSegment *__restrict__ order) {
     using V = typename VecB<T, VB>::type;
     constexpr int kLen = VecB<T, VB>::kLen;
     constexpr int G = 32 / L;             // lane groups, each takes every G-th nonzero
@@ -170,21 +174,35 @@ spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ 
     // warp slot waits for a new CTA to be launched into it (one-warp CTAs of a few microseconds
     // each left a fifth of the slots empty at any time).  The claim is issued before the segment's
     // work and read after it, so its latency is hidden.  Otherwise one segment per warp.
-    int seg = S == 1 ? blockIdx.x * W + (threadIdx.x >> 5) : blockIdx.x;
-    while (seg < m1) {
+    if constexpr (kOrdered) chain_wait();  // the list
+    int item = S == 1 ? blockIdx.x * W + (threadIdx.x >> 5) : blockIdx.x;
+    while (item < m1) {
     int claimed = INT_MAX;
     if constexpr (kClaim) {
         if (next_segment != nullptr && lane == 0)
             claimed = static_cast<int>(gridDim.x) * W + atomicAdd(next_segment + blockIdx.y, 1);
     }
-    const int row = __ldg(block_r_ind + seg);
-    const int seg_off = __ldg(st_off + seg);
+    int seg, row, seg_off, end;
+    bool whole_row;
+    if constexpr (kOrdered) {
+        const int4 e = __ldcg(reinterpret_cast<const int4 *>(order) + item);
+        const WholeSegment w = {e.x, e.y, e.z, e.w};
+        seg = w.number();
+        row = w.row;
+        seg_off = w.off;
+        end = w.end;
+        whole_row = w.whole_row();
+    } else {
+        seg = item;
+        row = __ldg(block_r_ind + seg);
+        seg_off = __ldg(st_off + seg);
+        const int next = (seg + 1 < m1) ? __ldg(st_off + seg + 1) : INT_MAX;
+        const int row_begin = __ldg(row_offsets + row);
+        const int row_end = __ldg(row_offsets + row + 1);
+        end = min(row_end, next);
+        whole_row = (seg_off == row_begin) && (next >= row_end);
+    }
     const int off = seg_off + part * 32;
-    const int next = (seg + 1 < m1) ? __ldg(st_off + seg + 1) : INT_MAX;
-    const int row_begin = __ldg(row_offsets + row);
-    const int row_end = __ldg(row_offsets + row + 1);
-    const int end = min(row_end, next);
-    const bool whole_row = (seg_off == row_begin) && (next >= row_end);
 
     // (column, value) of this lane's nonzero in the current and in the next chunk
     int c_cur = 0, c_nxt = 0;
@@ -296,7 +314,7 @@ spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ 
                 reinterpret_cast<V *>(partial)[static_cast<size_t>(seg) * row_vecs + col_vec + v * L] = acc[v];
         }
     }
-    seg = kClaim ? __shfl_sync(kFull, claimed, 0) : INT_MAX;
+    item = kClaim ? __shfl_sync(kFull, claimed, 0) : INT_MAX;
     }  // segments of this warp
 }
 
@@ -995,6 +1013,22 @@ spmm_rows_wide(int m2, int n, const T *__restrict__ values, const int *__restric
     }
 }
 
+// When an order of the segments pays (rode_order.cuh): with uniform columns from an operand beyond the L2 on, on skewed ones for
+// 256-byte rows only.  Whole calls, row by row / ordered, us.  Zipf 671,008 x 929,297 of mean 40 N = 32 (113 MB) 329 / 282, N = 64 830 /
+// 510, N = 128 1750 / 934, fp64 N = 64 1750 / 981; Zipf 2^20 of mean 8 N = 64 353 / 290; Pareto 2^20 of mean 32 N = 32 (128 MB) 517 / 509,
+// N = 64 1104 / 1006, N = 256 4579 / 4126, of mean 16 N = 64 640 / 599, of mean 8 N = 64 390 / 386, N = 128 675 / 677; 2^22 of mean 8
+// N = 32 1023 / 1039, N = 128 2841 / 2820.  R-MAT 23, 22, 21, 20 N = 64 3299 / 3112, 1485 / 1414, 697 / 687, 353 / 345, but N = 32 863 / 876
+// (22), N = 128 5347 / 5818 (23, against popularity hints), fp64 N = 32 785 / 832 (21).
+//
+// The more of the nonzeros are in rows of many segments, the more an order gives: Zipf matrices have 370 to 410 nonzeros per segment,
+// Pareto 170 to 310, where it takes more references per column and a larger grid (2^22 rows of mean 8 above; 262,144 x 2^20 of mean
+// 16, 19,043 segments, N = 128 331 / 333; Zipf of the same size, 10,953 segments, 316 / 284).
+bool order_pays(int verdict, long long m1, long long k, long long n, long long nnz, int elem_size) {
+    if (m1 < kOrderMinSegments || k * n * elem_size < 160ll << 20) return false;
+    if (nnz < kOrderLongRows * m1 && (m1 < 1 << 16 || nnz < 12 * k)) return false;
+    return verdict == kOrderHelps || (verdict == kOrderSkewed && n * elem_size == 256 && elem_size == 4);
+}
+
 template <typename T, int VB, int L, int VPL, bool kRagged>
 int launch_rows(int m2, int n, const T *values, const int *col, const int *row_offsets, const int *residue_r_ind,
                 const T *B, T *C, int *counters, bool chained, bool counters_clear, bool two_rows,
@@ -1004,7 +1038,8 @@ int launch_rows(int m2, int n, const T *values, const int *col, const int *row_o
 template <typename T, typename Block, typename Rows, bool kRagged = false, bool kRowsRagged = kRagged>
 int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, const int *row_offsets,
                  const int *block_r_ind, const int *residue_r_ind, const int *st_off, const T *B, T *C,
-                 T *partial, int *counters, const unsigned *hot, long long nnz, cudaStream_t s1, cudaStream_t s2) {
+                 T *partial, int *counters, const unsigned *hot, long long nnz, const Ordering *ord, cudaStream_t s1,
+                 cudaStream_t s2) {
     constexpr int VB = Block::VB, L = Block::L, VPL = Block::VPL;
     constexpr int kTileWidth = L * VPL * VecB<T, VB>::kLen;
     constexpr int U = kLoadsInFlight * 16 / VB / VPL;            // rows per batch
@@ -1028,20 +1063,27 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
         if (persistent || counters_clear) RODE_CUDA_TRY(cudaMemsetAsync(counters, 0, 2 * kClaimTiles * sizeof(int), s1));
         int *claim = persistent ? counters : nullptr;
         dim3 grid(persistent ? (resident + tiles - 1) / tiles : ctas_needed, tiles);
-        bool launched = false;  // one of the two special forms
+        bool launched = false;  // one of the special forms
+        if (ord != nullptr) {  // segments in the order of their columns
+            if (int rc = launch_order<0>(*ord, m1, row_offsets, col, block_r_ind, st_off, s1)) return rc;
+            RODE_CUDA_TRY(launch_chained(spmm_block<T, VB, L, VPL, U, kCtaWarps, 1, false, true, kRagged, true>, grid,
+                                         dim3(kCtaThreads), s1, true, m1, n, values, col, row_offsets, block_r_ind, st_off, B, C,
+                                         partial, nullptr, 0, claim, ord->list<0>()));
+            launched = true;
+        }
         // Popularity hints: block kernel of the 512-byte tile only.  In the residue-row kernel
         // the marks saved DRAM bytes (5.36 -> 4.79 GB on R-MAT scale 23) but the extra registers
         // cost more time than that returned (1.41 -> 1.52 ms).
         if constexpr (L * VPL * VB == 512 && !kRagged) {
-            if (hot && !small_grid) {
+            if (!launched && hot && !small_grid) {
                 spmm_block<T, VB, L, VPL, U, kCtaWarps, 1, true, true, false><<<grid, kCtaThreads, 0, s1>>>(
-                    m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, hot, (k + 31) / 32, claim);
+                    m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, hot, (k + 31) / 32, claim, nullptr);
                 launched = true;
             }
         }
         // Up to 40 MB of gathers the host's launches are what a call waits for: one for segments and rows.  (Beyond
         // that the separate kernels win back their launch: R-MAT 13 N = 128, 64 MB, 16.7 us with them, 18.7 in one.)
-        const bool one_launch = chained && nnz >= 0 && nnz * n * static_cast<long long>(sizeof(T)) <= 40LL << 20 &&
+        const bool one_launch = !launched && chained && nnz >= 0 && nnz * n * static_cast<long long>(sizeof(T)) <= 40LL << 20 &&
                                 small_grid && static_cast<long long>(m2) * tiles <= 2LL * 32 * sm_count();
         if (one_launch) {
             constexpr int UOne = 2 * U <= L ? 2 * U : L;
@@ -1054,13 +1096,13 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
         const long long warps = static_cast<long long>(m1) * tiles;
         if (!launched && warps <= kSplit4WarpsPerSm * sm_count()) {
             spmm_block<T, VB, L, VPL, U, 4, 4, false, false, kRagged><<<dim3(m1, tiles), 4 * 32, 0, s1>>>(
-                m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0, nullptr);
+                m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0, nullptr, nullptr);
         } else if (!launched && warps <= kSplit2WarpsPerSm * sm_count()) {
             spmm_block<T, VB, L, VPL, U, 2, 2, false, false, kRagged><<<dim3(m1, tiles), 2 * 32, 0, s1>>>(
-                m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0, nullptr);
+                m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0, nullptr, nullptr);
         } else if (!launched) {
             spmm_block<T, VB, L, VPL, U, kCtaWarps, 1, false, true, kRagged><<<grid, kCtaThreads, 0, s1>>>(
-                m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0, claim);
+                m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0, claim, nullptr);
         }
         RODE_CHECK_LAUNCH("rode::spmm_block");
     }
@@ -1137,7 +1179,7 @@ template <typename T>
 int spmm(int m1, int m2, int k, int n, const T *values, const int *col, const int *row_offsets,
          const int *block_r_ind, const int *residue_r_ind, const int *st_off, const T *B, T *C, void *workspace,
          size_t workspace_bytes, const unsigned *hot, rode_stream_t stream1, rode_stream_t stream2,
-         bool all_rows = false, long long nnz = -1) {
+         bool all_rows = false, long long nnz = -1, bool ordered = false) {
     constexpr int kLen = Vec16<T>::kLen;
     if (m1 < 0 || m2 < 0 || n <= 0) return fail(RODE_ERR_INVALID_ARGUMENT, "spmm: m1, m2 >= 0 and n > 0 required");
     if (hot != nullptr && k <= 0)
@@ -1163,6 +1205,14 @@ int spmm(int m1, int m2, int k, int n, const T *values, const int *col, const in
                         workspace ? workspace_bytes : static_cast<size_t>(0));
         if (!aligned_to(workspace, 16)) return fail(RODE_ERR_WORKSPACE, "spmm: workspace must be 16-byte aligned");
     }
+    Ordering ordering = {}, *ord = nullptr;
+    if (ordered && m1 > 0 && m1 < kWholeMaxSegments && k > 0) {
+        const size_t more = ordering_bytes<0>(m1, 0);
+        if (workspace_bytes < need + more)
+            return fail(RODE_ERR_WORKSPACE, "spmm: workspace of %zu bytes needed, %zu given", need + more, workspace_bytes);
+        ordering = {reinterpret_cast<OrderHead *>(static_cast<char *>(workspace) + need), m1, k};
+        ord = &ordering;
+    }
     T *partial = static_cast<T *>(workspace);
     // the claim counters of the persistent block kernel sit behind the partial rows
     int *counters = workspace != nullptr
@@ -1170,7 +1220,7 @@ int spmm(int m1, int m2, int k, int n, const T *values, const int *col, const in
     // Widest tile (32, 16 or 8 vectors of 16 bytes) that divides the row.
 #define RODE_LAUNCH(...)                                                                                             \
     launch_shape<T, __VA_ARGS__>(m1, m2, k, n, values, col, row_offsets, block_r_ind, residue_r_ind, st_off, B, C, partial, \
-                                 counters, hot, nnz, stream1, stream2)
+                                 counters, hot, nnz, ord, stream1, stream2)
     const bool aligned32 = aligned_to(B, 32) && aligned_to(C, 32) && aligned_to(workspace, 32);
     const int vecs = n / kLen;
     // Widths of whole lines that the 512-byte tile does not divide (N = 96, 160, 192, 224 ...): 512-byte tiles with a
@@ -1275,6 +1325,30 @@ int rode_spmm_f64_all(int M, int m1, int k, int n, long long nnz, const double *
                       rode_stream_t stream2) {
     return rode::spmm<double>(m1, M, k, n, values, column_indices, row_offsets, block_r_ind, nullptr, st_off, B, C,
                               workspace, workspace_bytes, hot_columns, stream1, stream2, /*all_rows=*/true, nnz);
+}
+
+int rode_spmm_order_pays(int verdict, int m1, int k, int n, long long nnz, int elem_size) {
+    return rode::order_pays(verdict, m1, k, n, nnz, elem_size) ? 1 : 0;
+}
+
+int rode_spmm_ordered_workspace_bytes(int m1, int n, int elem_size, size_t *bytes) {
+    if (int rc = rode_spmm_workspace_bytes(m1, n, elem_size, bytes)) return rc;
+    *bytes += rode::ordering_bytes<0>(m1, 0);
+    return RODE_OK;
+}
+
+int rode_spmm_f32_ordered(int M, int m1, int k, int n, long long nnz, const float *values, const int *column_indices,
+                          const int *row_offsets, const int *block_r_ind, const int *st_off, const float *B, float *C,
+                          void *workspace, size_t workspace_bytes, rode_stream_t stream1, rode_stream_t stream2) {
+    return rode::spmm<float>(m1, M, k, n, values, column_indices, row_offsets, block_r_ind, nullptr, st_off, B, C,
+                             workspace, workspace_bytes, nullptr, stream1, stream2, /*all_rows=*/true, nnz, /*ordered=*/true);
+}
+
+int rode_spmm_f64_ordered(int M, int m1, int k, int n, long long nnz, const double *values, const int *column_indices,
+                          const int *row_offsets, const int *block_r_ind, const int *st_off, const double *B, double *C,
+                          void *workspace, size_t workspace_bytes, rode_stream_t stream1, rode_stream_t stream2) {
+    return rode::spmm<double>(m1, M, k, n, values, column_indices, row_offsets, block_r_ind, nullptr, st_off, B, C,
+                              workspace, workspace_bytes, nullptr, stream1, stream2, /*all_rows=*/true, nnz, /*ordered=*/true);
 }
 
 }  // extern "C"

@@ -36,7 +36,7 @@ class RoDeCSR:
     }
     MAX_K = 256
     _entry_range = None  # (row_offsets[0], row_offsets[m]) as of construction
-    _ordered = False     # rode_sddmm orders the segments by their columns
+    _verdict = -1        # what an order of the segments by their columns can give, judged at construction
 
     @classmethod
     def config_for(cls, k: int) -> dict:
@@ -77,7 +77,7 @@ class RoDeCSR:
         self.m2 = m2
         if self.column_indices.numel() == self.nnz:
             with torch.cuda.device(self.device):
-                self._ordered = rode_sddmm_cuda.order_pays(blk, m1, self.row_offsets, self.column_indices, self.m, self.n, self.k)
+                self._verdict = rode_sddmm_cuda.order_verdict(blk, m1, self.row_offsets, self.column_indices, self.n)
 
     @classmethod
     def from_random(cls, m: int, n: int, nnz_per_row: int, device: torch.device, k: int = 128) -> "RoDeCSR":
@@ -122,11 +122,13 @@ def rode_sddmm(sparse_matrix: RoDeCSR, lhs: torch.Tensor, rhs: torch.Tensor) -> 
     m, n, k = sparse_matrix.m, sparse_matrix.n, sparse_matrix.k
     _check_dense("lhs_matrix", lhs, (m, k), sparse_matrix)
     _check_dense("rhs_matrix", rhs, (n, k), sparse_matrix)
+    ordered = sparse_matrix._verdict >= 0 and rode_sddmm_cuda.sddmm_order_pays(
+        sparse_matrix._verdict, m, sparse_matrix.m1, n, k, sparse_matrix.nnz)
     return rode_sddmm_cuda.sddmm_forward(
         sparse_matrix.block_indices, sparse_matrix.residue_indices, sparse_matrix.st_offsets, sparse_matrix.m1,
         sparse_matrix.m2, sparse_matrix.row_offsets, sparse_matrix.column_indices, sparse_matrix.values, m, n,
         lhs.contiguous(), rhs.contiguous(), k, sparse_matrix._entry_range == (0, sparse_matrix.values.numel()),
-        sparse_matrix._ordered)
+        ordered)
 
 
 def rode_spmm(sparse_matrix: RoDeCSR, dense: torch.Tensor, hints: bool = True) -> torch.Tensor:
@@ -134,15 +136,18 @@ def rode_spmm(sparse_matrix: RoDeCSR, dense: torch.Tensor, hints: bool = True) -
     them are decomposed with k_block 32; segments of 512, k other than 128 at construction, serve it
     best); the reference has no Python SpMM.
 
-    ``hints``: gather popular columns' rows with an L2 policy that keeps them resident
-    (same results, fewer DRAM bytes on skewed matrices).  The popularity bitmap is built on
-    the first call for a given width and cached on ``sparse_matrix``."""
+    ``hints``: what keeps dense rows in the L2 (same results, fewer DRAM bytes): the segments in the order of their columns
+    where the matrix and the width are such that it pays; else popular columns' rows gathered with an L2 policy that keeps
+    them resident on skewed matrices, whose popularity bitmap is built on the first call for a given width and cached on
+    ``sparse_matrix``."""
     shape = dense.shape
     if len(shape) != 2 or shape[0] != sparse_matrix.n:
         raise ValueError(f"dense must be ({sparse_matrix.n}, width), got {tuple(shape)}")
     assert dense.device == sparse_matrix.device and dense.dtype == torch.float32
     hot = None
-    if hints and shape[1] % 128 == 0:
+    ordered = hints and sparse_matrix._verdict >= 0 and rode_sddmm_cuda.spmm_order_pays(
+        sparse_matrix._verdict, sparse_matrix.m1, sparse_matrix.n, shape[1], sparse_matrix.nnz, dense.element_size())
+    if hints and not ordered and shape[1] % 128 == 0:
         cache = sparse_matrix.__dict__.setdefault("_hot_columns", {})
         row_bytes = shape[1] * dense.element_size()
         if row_bytes not in cache:
@@ -151,7 +156,7 @@ def rode_spmm(sparse_matrix: RoDeCSR, dense: torch.Tensor, hints: bool = True) -
     return rode_sddmm_cuda.spmm_forward(
         sparse_matrix.block_indices, sparse_matrix.residue_indices, sparse_matrix.st_offsets, sparse_matrix.m1,
         sparse_matrix.m2, sparse_matrix.row_offsets, sparse_matrix.column_indices, sparse_matrix.values,
-        sparse_matrix.m, sparse_matrix.n, dense.contiguous(), hot)
+        sparse_matrix.m, sparse_matrix.n, dense.contiguous(), hot, ordered)
 
 
 def torch_sddmm_reference(sparse_csr: torch.Tensor, lhs_matrix: torch.Tensor, rhs_matrix: torch.Tensor) -> torch.Tensor:

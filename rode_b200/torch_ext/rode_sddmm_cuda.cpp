@@ -16,8 +16,8 @@
 //   * k_version may be any multiple of 4 up to 256.
 //   * covers_values (default false) says that row_offsets runs from 0 to the number of values, so that the result
 //     need not be zero-filled first.
-//   * ordered (default false) gives the call scratch memory in which it orders the segments by their columns; order_pays
-//     says whether that helps.
+//   * ordered (default false) gives the call scratch memory in which it orders the segments by their columns; order_verdict
+//     and *_order_pays say whether that helps.
 //   * spmm_forward and hot_columns are new: the reference has no Python entry for SpMM.
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
@@ -134,27 +134,24 @@ torch::Tensor py_sddmm_forward(torch::Tensor block_indices, torch::Tensor residu
     return out;
 }
 
-// Whether sddmm_forward should order the segments of this matrix by their columns (rode_sddmm_order_verdict).  Reads the verdict
-// back where the sizes are in range.
-bool py_order_pays(torch::Tensor block_indices, int m1, torch::Tensor row_offsets, torch::Tensor column_indices, int m, int n,
-                   int k) {
+// What rode_order_verdict says of the columns, -1 where the sizes are out of its range.  Reads the verdict back.
+int py_order_verdict(torch::Tensor block_indices, int m1, torch::Tensor row_offsets, torch::Tensor column_indices, int n) {
     RODE_CHECK_INPUT(block_indices);
     RODE_CHECK_INPUT(row_offsets);
     RODE_CHECK_INPUT(column_indices);
     RODE_CHECK_INT(block_indices);
     RODE_CHECK_INT(row_offsets);
     RODE_CHECK_INT(column_indices);
-    TORCH_CHECK(row_offsets.size(0) == static_cast<long long>(m) + 1, "row_offsets must have m + 1 entries");
     const c10::cuda::CUDAGuard guard(column_indices.device());
     const long long nnz = column_indices.numel();
     int in_range = 0;
-    check_status(rode_sddmm_order_verdict(m, m1, n, k, nnz, nullptr, nullptr, nullptr, &in_range, nullptr, nullptr));
-    if (!in_range) return false;
+    check_status(rode_order_verdict(m1, n, nnz, nullptr, nullptr, nullptr, &in_range, nullptr, nullptr));
+    if (!in_range) return -1;
     torch::Tensor verdict = torch::empty({1}, column_indices.options());
-    check_status(rode_sddmm_order_verdict(m, m1, n, k, nnz, row_offsets.data_ptr<int>(), column_indices.data_ptr<int>(),
-                                          block_indices.data_ptr<int>(), &in_range, verdict.data_ptr<int>(),
-                                          at::cuda::getCurrentCUDAStream(column_indices.device().index()).stream()));
-    return rode_sddmm_order_pays(verdict.item<int>(), k) != 0;
+    check_status(rode_order_verdict(m1, n, nnz, row_offsets.data_ptr<int>(), column_indices.data_ptr<int>(),
+                                    block_indices.data_ptr<int>(), &in_range, verdict.data_ptr<int>(),
+                                    at::cuda::getCurrentCUDAStream(column_indices.device().index()).stream()));
+    return verdict.item<int>();
 }
 
 // Popularity bitmap of the columns for spmm_forward's `hot_columns` argument (rode_hot_columns),
@@ -184,7 +181,7 @@ c10::optional<torch::Tensor> py_hot_columns(torch::Tensor column_indices, int n_
 torch::Tensor py_spmm_forward(torch::Tensor block_indices, torch::Tensor residue_indices, torch::Tensor st_offsets,
                                 int m1, int m2, torch::Tensor row_offsets, torch::Tensor column_indices,
                                 torch::Tensor values, int m, int k, torch::Tensor dense,
-                                c10::optional<torch::Tensor> hot_columns) {
+                                c10::optional<torch::Tensor> hot_columns, bool ordered) {
     RODE_CHECK_INPUT(block_indices);
     RODE_CHECK_INPUT(residue_indices);
     RODE_CHECK_INPUT(st_offsets);
@@ -213,7 +210,8 @@ torch::Tensor py_spmm_forward(torch::Tensor block_indices, torch::Tensor residue
     torch::Tensor ws;
     void *ws_ptr = nullptr;
     if (m1 > 0 || m >= 1 << 19) {
-        check_status(rode_spmm_workspace_bytes(m1, n, static_cast<int>(dense.element_size()), &ws_bytes));
+        check_status((ordered ? rode_spmm_ordered_workspace_bytes : rode_spmm_workspace_bytes)(
+            m1, n, static_cast<int>(dense.element_size()), &ws_bytes));
         ws = empty_cuda({static_cast<long long>(ws_bytes)}, torch::kUInt8, dense.device());
         ws_ptr = ws.data_ptr();
     }
@@ -226,6 +224,19 @@ torch::Tensor py_spmm_forward(torch::Tensor block_indices, torch::Tensor residue
         hot = reinterpret_cast<const unsigned *>(hot_columns->data_ptr<int>());
     }
     const cudaStream_t s = at::cuda::getCurrentCUDAStream(values.device().index()).stream();
+    if (ordered) {
+        const auto call = [&](auto *entry, auto *type) {
+            using T = std::remove_pointer_t<decltype(type)>;
+            check_status(entry(m, m1, k, n, values.size(0), values.data_ptr<T>(), column_indices.data_ptr<int>(),
+                               row_offsets.data_ptr<int>(), block_indices.data_ptr<int>(), st_offsets.data_ptr<int>(),
+                               dense.data_ptr<T>(), out.data_ptr<T>(), ws_ptr, ws_bytes, s, s));
+        };
+        if (dense.dtype() == torch::kFloat32)
+            call(&rode_spmm_f32_ordered, static_cast<float *>(nullptr));
+        else
+            call(&rode_spmm_f64_ordered, static_cast<double *>(nullptr));
+        return out;
+    }
     if (dense.dtype() == torch::kFloat32)
         check_status(rode_spmm_f32_all(m, m1, k, n, values.size(0), values.data_ptr<float>(), column_indices.data_ptr<int>(),
                                        row_offsets.data_ptr<int>(), block_indices.data_ptr<int>(),
@@ -248,12 +259,16 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           py::arg("residue_indices"), py::arg("st_offsets"), py::arg("m1"), py::arg("m2"), py::arg("row_offsets"),
           py::arg("column_indices"), py::arg("values"), py::arg("m"), py::arg("n"), py::arg("lhs_matrix"),
           py::arg("rhs_matrix"), py::arg("k_version"), py::arg("covers_values") = false, py::arg("ordered") = false);
-    m.def("order_pays", &py_order_pays, "Whether ordered=True pays in sddmm_forward (CUDA)", py::arg("block_indices"),
-          py::arg("m1"), py::arg("row_offsets"), py::arg("column_indices"), py::arg("m"), py::arg("n"), py::arg("k"));
+    m.def("order_verdict", &py_order_verdict, "What an order of the segments by their columns can give (CUDA)",
+          py::arg("block_indices"), py::arg("m1"), py::arg("row_offsets"), py::arg("column_indices"), py::arg("n"));
+    m.def("spmm_order_pays", &rode_spmm_order_pays, py::arg("verdict"), py::arg("m1"), py::arg("k"), py::arg("n"),
+          py::arg("nnz"), py::arg("elem_size"));
+    m.def("sddmm_order_pays", &rode_sddmm_order_pays, py::arg("verdict"), py::arg("m"), py::arg("m1"), py::arg("n"), py::arg("k"),
+          py::arg("nnz"));
     m.def("spmm_forward", &py_spmm_forward, "RoDe SpMM forward (CUDA)", py::arg("block_indices"),
           py::arg("residue_indices"), py::arg("st_offsets"), py::arg("m1"), py::arg("m2"), py::arg("row_offsets"),
           py::arg("column_indices"), py::arg("values"), py::arg("m"), py::arg("k"), py::arg("dense"),
-          py::arg("hot_columns") = py::none());
+          py::arg("hot_columns") = py::none(), py::arg("ordered") = false);
     m.def("hot_columns", &py_hot_columns, "Column popularity bitmap for spmm_forward, or None (CUDA)",
           py::arg("column_indices"), py::arg("n_cols"), py::arg("dense_row_bytes"), py::arg("budget_bytes") = 0);
 }

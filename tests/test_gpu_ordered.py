@@ -1,4 +1,4 @@
-"""SDDMM with the segments in the order of their columns (rode_sddmm_f32_ordered), and the verdict on where that pays."""
+"""SpMM and SDDMM with the segments in the order of their columns (rode_*_ordered), and the verdict on where that pays."""
 import numpy as np
 import pytest
 import torch
@@ -55,8 +55,60 @@ def test_ordered_matches_oracle_and_stays_inside_its_workspace(oracle_cpu, k, se
     assert float((ordered - plain).norm() / plain.norm()) < 1e-6
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("n", [4, 32, 64, 96, 100, 128, 132, 256])
+def test_ordered_spmm_is_the_same_product(n, dtype):
+    A = _matrix(4099)
+    d, B = A.to("cuda"), W.dense(A.n, n, seed=6, dtype=dtype).cuda()
+    val = d.val.to(dtype)
+    for seg_len in (32, 512):
+        meta = capi.preprocess(d.row_ptr, d.nnz, seg_len)
+        want = capi.spmm(meta, d.row_ptr, d.col, val, B)
+        need = capi.spmm_ordered_workspace_bytes(meta.m1, n, B.element_size())
+        ws = torch.full((need + 256,), 0xAB, dtype=torch.uint8, device="cuda")
+        C = torch.full((A.m, n), float("nan"), device="cuda", dtype=dtype)
+        call = [dtype, A.m, meta.m1, A.n, n, A.nnz, val.data_ptr(), d.col.data_ptr(), d.row_ptr.data_ptr(), meta.block_r_ind.data_ptr(),
+                meta.st_off.data_ptr(), B.data_ptr(), C.data_ptr(), ws.data_ptr()]
+        capi.spmm_ordered_raw(*call, need)
+        torch.cuda.synchronize()
+        # grids of this size take another kernel without the order: the same sums in another order
+        assert float((C - want).norm() / want.norm()) < (1e-6 if dtype == torch.float32 else 1e-15)
+        assert bool((ws[need:] == 0xAB).all())
+        again = torch.full_like(C, float("nan"))
+        call[12] = again.data_ptr()
+        capi.spmm_ordered_raw(*call, need)
+        assert torch.equal(C, again)
+        with pytest.raises(capi.RodeError):
+            capi.spmm_ordered_raw(*call, need - 1)
+
+
+def test_ordered_calls_captured_and_on_two_streams():
+    k = 64
+    A = _matrix(4099).to("cuda")
+    meta = capi.preprocess(A.row_ptr, A.nnz)
+    lhs, rhs = W.dense(A.m, k, seed=5).cuda(), W.dense(A.n, k, seed=6).cuda()
+    want = capi.sddmm(meta, A.row_ptr, A.col, A.val, lhs, rhs, ordered=True)
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    got = capi.sddmm(meta, A.row_ptr, A.col, A.val, lhs, rhs, stream1=s1, stream2=s2, ordered=True)
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    out = torch.empty_like(want)
+    ws = torch.empty(capi.sddmm_workspace_bytes(meta.m1, k, A.nnz), dtype=torch.uint8, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        capi.sddmm_ordered_raw(A.m, meta.m1, meta.m2, A.n, k, A.nnz, meta.block_r_ind.data_ptr(), meta.residue_r_ind.data_ptr(),
+                               meta.st_off.data_ptr(), A.row_ptr.data_ptr(), A.col.data_ptr(), A.val.data_ptr(), lhs.data_ptr(),
+                               rhs.data_ptr(), out.data_ptr(), ws.data_ptr(), ws.numel(), torch.cuda.current_stream(),
+                               torch.cuda.current_stream())
+    for _ in range(2):
+        out.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out[5:-3], want[5:-3])
+
+
 def test_verdict():
-    n, per, m = 700_001, 40, 40_000
+    n, per, m = 700_001, 40, 70_000
     g = torch.Generator(device="cuda")
     g.manual_seed(1)
     u = torch.rand((m, per), generator=g, device="cuda", dtype=torch.float64)
@@ -66,6 +118,10 @@ def test_verdict():
         col = c.clamp(0, n - 1).to(torch.int32).sort(1).values.reshape(-1).contiguous()
         meta = capi.preprocess(row_ptr, col.numel())
         assert meta.m1 == m
-        pays = [capi.sddmm_order_pays(meta, row_ptr, col, n, k) for k in (32, 64, 128)]
+        verdict = capi.order_verdict(meta, row_ptr, col, n)
+        pays = [capi.sddmm_order_pays(verdict, m, meta.m1, n, k, col.numel()) for k in (32, 64, 128)]
+        nnz = 12 * n  # as if there were a few more references per column
+        assert [capi.spmm_order_pays(verdict, meta.m1, n, k, nnz) for k in (32, 64, 128)] == {
+            "uniform": [False, True, True], "skewed": [False, True, False], "band": [False] * 3}[kind], kind
         # 90 MB, 179 MB, 358 MB of rhs
         assert pays == {"uniform": [False, True, True], "skewed": [False, False, True], "band": [False] * 3}[kind], kind
