@@ -305,14 +305,34 @@ __device__ __forceinline__ unsigned group_mask(int lane) {
 // flushed their stores.  In the kernels whose code generation suffers from a common exit (the per-row
 // kernel of the stencil 0.695 -> 0.750 ms) that is a CTA of its own behind the last row.  Launched without
 // the attribute, both are no-ops.
+//
+// The first grid of a call is a programmatic dependent too, of whatever the stream holds before it (its launch latency then
+// overlaps the end of that: calls back to back, SDDMM Bernoulli 4096^2 K = 32 8.2 -> 6.8 us).  Every CTA of it waits before it
+// touches memory (after_chain), and before it lets the next grid start: so the in-chain grids, which do not wait at
+// their beginning, start behind everything that came before the call.
 __device__ __forceinline__ void chain_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// chain_wait(), then i: read-only loads, which a memory clobber does not hold back, stay behind the wait if they are indexed
+// by the result.
+__device__ __forceinline__ unsigned after_chain(unsigned i) {
+    asm volatile("griddepcontrol.wait;" : "+r"(i)::"memory");
+    return i;
+}
+// The same where `first`, without a branch (which cost spmm_rows 140 bytes of spills).
+__device__ __forceinline__ unsigned after_chain_if(bool first, unsigned i) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.s32 p, %1, 0;\n@p griddepcontrol.wait;\n}"
+        : "+r"(i)
+        : "r"(static_cast<int>(first))
+        : "memory");
+    return i;
+}
 
 #endif  // __CUDACC__
 
 #ifdef __CUDACC__
 // kernel<<<grid, block, 0, stream>>>(args...), with `chained` as a programmatic dependent of the grid
-// before it on the stream.
+// before it on the stream (no difference behind a copy, a fill or an event that is waited for).
 template <typename... P, typename... A>
 cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t stream, bool chained, A... args) {
     cudaLaunchConfig_t cfg = {};

@@ -192,7 +192,7 @@ template <int L, int VPL, int U, bool kClaim, bool kRagged>
 __device__ __forceinline__ void block_segments(int m1, const int *__restrict__ block_r_ind, const int *__restrict__ st_off,
             const int *__restrict__ row_offsets, const int *__restrict__ column_indices,
             const float *__restrict__ values, const float *__restrict__ lhs, const float *__restrict__ rhs,
-            float *__restrict__ out, int *__restrict__ next_segment, int row_vecs_arg) {
+            float *__restrict__ out, int *__restrict__ next_segment, int row_vecs_arg, int seg) {
     constexpr int G = 32 / L;
     static_assert(L % U == 0 && U >= 2, "a chunk is a whole number of batches");
     const unsigned row_vecs = kRagged ? static_cast<unsigned>(row_vecs_arg) : L * VPL;
@@ -204,7 +204,6 @@ __device__ __forceinline__ void block_segments(int m1, const int *__restrict__ b
     // (with four vectors per lane a second form only spills; L = 16 is the form of the large grids)
     constexpr bool kFullPath = VPL <= 3 && L == 8;
     const int pos = l * G + g;  // this lane's nonzero of a chunk: group g holds positions g, g + G, ...
-    int seg = blockIdx.x;
     while (seg < m1) {
     int claimed = INT_MAX;  // never used in arithmetic: the loop test compares it with m1 as it is
     if constexpr (kClaim) {
@@ -304,9 +303,10 @@ sddmm_block(int m1, const int *__restrict__ block_r_ind, const int *__restrict__
             const int *__restrict__ row_offsets, const int *__restrict__ column_indices,
             const float *__restrict__ values, const float *__restrict__ lhs, const float *__restrict__ rhs,
             float *__restrict__ out, int *__restrict__ next_segment, int row_vecs) {
+    const int seg = after_chain(blockIdx.x);  // (the first grid of the call)
     chain_begin();
     block_segments<L, VPL, U, kClaim, kRagged>(m1, block_r_ind, st_off, row_offsets, column_indices, values, lhs, rhs, out,
-                                               next_segment, row_vecs);
+                                               next_segment, row_vecs, seg);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(32, (VPL > 1 || BL > 0) ? 24 : kItemsCtas)
 sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, const int *__restrict__ st_off,
             const int *__restrict__ row_offsets, const int *__restrict__ column_indices,
             const float *__restrict__ values, const float *__restrict__ lhs, const float *__restrict__ rhs,
-            float *__restrict__ out, int row_vecs_arg, int row_mode_min, int m1, const int *__restrict__ seg_rows) {
+            float *__restrict__ out, int row_vecs_arg, int row_mode_min, int m1, const int *__restrict__ seg_rows, bool first) {
     constexpr int G = 32 / L;
     constexpr int kBatch = kLoadsInFlight / VPL;  // nonzeros per batch
     const size_t row_vecs = kRagged ? static_cast<size_t>(row_vecs_arg) : L * VPL;  // float4 per dense row (K / 4)
@@ -351,14 +351,14 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
     const int lane = threadIdx.x;
     const int g = lane / L, l = lane % L;
     const unsigned gmask = group_mask<L>(lane);
-    int bundle = blockIdx.x;
+    int bundle = kSegments || BL > 0 ? after_chain(blockIdx.x) : after_chain_if(first, blockIdx.x);
+    chain_begin();
     if constexpr (BL > 0) {
         if (bundle < m1)
             return block_segments<BL, BVPL, BU, false, kRagged>(m1, seg_rows, st_off, row_offsets, column_indices, values, lhs,
-                                                                rhs, out, nullptr, row_vecs_arg);
+                                                                rhs, out, nullptr, row_vecs_arg, bundle);
         bundle -= m1;
     }
-    if constexpr (kSegments) chain_begin();
     const long long item0 = static_cast<long long>(bundle) * items_per_warp;
     if (item0 >= n_items) return chain_wait();  // the CTA behind the items
 
@@ -804,9 +804,9 @@ int launch_k(int m1, int m2, int k, const int *block_r_ind, const int *residue_r
         // (a warp per 32-long segment, K = 128, pays while they all fit at once: Bernoulli 4096^2 13.5 us with the two
         // kernels, 14.7 in one; 2000^2 12.3 and 10.3)
         if (ord == nullptr && m1 > 0 && m2 > 0 && s1 == s2 && ctas <= (kLongSegments ? 4LL : 1LL) * 24 * sm_count()) {
-            sddmm_items<L, VPL, false, kRagged, BL, BVPL, kRowU, BL, BVPL, BU><<<static_cast<unsigned>(ctas), 32, 0, s1>>>(
-                m2, per, residue_r_ind, st_off, row_offsets, col, values, lhs, rhs, out, row_vecs, row_mode_min, m1,
-                block_r_ind);
+            RODE_CUDA_TRY(launch_chained(sddmm_items<L, VPL, false, kRagged, BL, BVPL, kRowU, BL, BVPL, BU>,
+                                         dim3(static_cast<unsigned>(ctas)), dim3(32), s1, true, m2, per, residue_r_ind, st_off,
+                                         row_offsets, col, values, lhs, rhs, out, row_vecs, row_mode_min, m1, block_r_ind, true));
             RODE_CHECK_LAUNCH("rode::sddmm_items<segments and rows>");
             return RODE_OK;
         }
@@ -827,17 +827,19 @@ int launch_k(int m1, int m2, int k, const int *block_r_ind, const int *residue_r
             }
             if (claim.ptr != nullptr) {
                 RODE_CUDA_TRY(cudaMemsetAsync(claim.ptr, 0, sizeof(int), s1));
-                sddmm_block<Claimed::L, Claimed::VPL, Claimed::U, true, kRagged><<<resident, 32, 0, s1>>>(
-                    m1, block_r_ind, st_off, row_offsets, col, values, lhs, rhs, out, claim.ptr, row_vecs);
+                RODE_CUDA_TRY(launch_chained(sddmm_block<Claimed::L, Claimed::VPL, Claimed::U, true, kRagged>, dim3(resident), dim3(32),
+                                             s1, true, m1, block_r_ind, st_off, row_offsets, col, values, lhs, rhs, out, claim.ptr,
+                                             row_vecs));
             } else {
-                sddmm_block<BL, BVPL, BU, false, kRagged><<<m1, 32, 0, s1>>>(m1, block_r_ind, st_off, row_offsets, col, values,
-                                                                            lhs, rhs, out, nullptr, row_vecs);
+                RODE_CUDA_TRY(launch_chained(sddmm_block<BL, BVPL, BU, false, kRagged>, dim3(m1), dim3(32), s1, true, m1, block_r_ind,
+                                             st_off, row_offsets, col, values, lhs, rhs, out, nullptr, row_vecs));
             }
             RODE_CHECK_LAUNCH("rode::sddmm_block");
         } else {
             const int per = items_per_warp(m1, 32, 4);
-            sddmm_items<L, VPL, true, kRagged, 0, 1, 1><<<(m1 + per - 1) / per, 32, 0, s1>>>(
-                m1, per, block_r_ind, st_off, row_offsets, col, values, lhs, rhs, out, row_vecs, 0, 0, nullptr);
+            RODE_CUDA_TRY(launch_chained(sddmm_items<L, VPL, true, kRagged, 0, 1, 1>, dim3((m1 + per - 1) / per), dim3(32), s1, true,
+                                         m1, per, block_r_ind, st_off, row_offsets, col, values, lhs, rhs, out, row_vecs, 0, 0,
+                                         nullptr, true));
             RODE_CHECK_LAUNCH("rode::sddmm_items<segments>");
         }
     }
@@ -846,8 +848,8 @@ int launch_k(int m1, int m2, int k, const int *block_r_ind, const int *residue_r
         // whole rounds of the row mode (30,000 rows of 25, 3 -> 4 rows per warp: K = 128 28.6 -> 25.3 us, K = 96 28.8 -> 22.6)
         if (L == 32 && per > 1) per = (per + 32 / RL - 1) / (32 / RL) * (32 / RL);
         RODE_CUDA_TRY(launch_chained(sddmm_items<L, VPL, false, kRagged, RL, RVPL, RU>, dim3((m2 + per - 1) / per + 1), dim3(32), s2,
-                                     m1 > 0 && s1 == s2, m2, per, residue_r_ind, nullptr, row_offsets, col, values, lhs,
-                                     rhs, out, row_vecs, row_mode_min, 0, nullptr));
+                                     true, m2, per, residue_r_ind, nullptr, row_offsets, col, values, lhs, rhs, out, row_vecs,
+                                     row_mode_min, 0, nullptr, !(m1 > 0 && s1 == s2)));
         RODE_CHECK_LAUNCH("rode::sddmm_items<rows>");
     }
     return RODE_OK;

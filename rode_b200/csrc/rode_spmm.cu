@@ -146,6 +146,8 @@ spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ 
     constexpr int kSteps = 32 / G;        // nonzeros per group per 32-nonzero chunk
     constexpr int NB = (kSteps + U - 1) / U;
     constexpr unsigned kFull = 0xffffffffu;
+    // (the first grid of the call, or behind the kernels that make the list)
+    int item = after_chain(S == 1 ? blockIdx.x * W + (threadIdx.x >> 5) : blockIdx.x);
     chain_begin();
     static_assert(W % S == 0 && (S == 1 || (W == S && !kClaim)), "a CTA per split segment");
     const int part = S == 1 ? 0 : threadIdx.x >> 5;  // this warp takes every S-th chunk of its segment
@@ -174,8 +176,6 @@ spmm_block(int m1, int n, const T *__restrict__ values, const int *__restrict__ 
     // warp slot waits for a new CTA to be launched into it (one-warp CTAs of a few microseconds
     // each left a fifth of the slots empty at any time).  The claim is issued before the segment's
     // work and read after it, so its latency is hidden.  Otherwise one segment per warp.
-    if constexpr (kOrdered) chain_wait();  // the list
-    int item = S == 1 ? blockIdx.x * W + (threadIdx.x >> 5) : blockIdx.x;
     while (item < m1) {
     int claimed = INT_MAX;
     if constexpr (kClaim) {
@@ -346,6 +346,7 @@ spmm_one_launch(int m1, int seg_ctas, int rows, int n, const T *__restrict__ val
     __shared__ __align__(16) int s_col[W][2][32];
     __shared__ __align__(16) T s_val[W][2][32];
     __shared__ __align__(32) V s_acc[W][W][L * VPL];  // [warp][segment]
+    const int cta = after_chain(blockIdx.x);
     chain_begin();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane / L, l = lane % L;
@@ -396,8 +397,8 @@ spmm_one_launch(int m1, int seg_ctas, int rows, int n, const T *__restrict__ val
             for (int w = L; w < 32; w <<= 1) vadd(acc[v], vshfl_xor(kFull, acc[v], w));
     };
 
-    if (static_cast<int>(blockIdx.x) >= seg_ctas) {  // ---- a row per warp -----------------------------------
-        const int item = (static_cast<int>(blockIdx.x) - seg_ctas) * W + warp;
+    if (cta >= seg_ctas) {  // ---- a row per warp -----------------------------------
+        const int item = (cta - seg_ctas) * W + warp;
         if (item >= rows) return;
         const int row = residue_r_ind != nullptr ? __ldg(residue_r_ind + item) : item;
         const int begin = __ldg(row_offsets + row), end = __ldg(row_offsets + row + 1);
@@ -423,7 +424,7 @@ spmm_one_launch(int m1, int seg_ctas, int rows, int n, const T *__restrict__ val
     }
 
     // ---- four segments, far apart: lane j < W of every warp holds segment j ---------------------------------
-    const int my_seg = static_cast<int>(blockIdx.x) + lane * seg_ctas;
+    const int my_seg = cta + lane * seg_ctas;
     int row = 0, off = 0, end = 0;
     bool whole = false;
     if (lane < W && my_seg < m1) {
@@ -494,7 +495,7 @@ spmm_one_launch(int m1, int seg_ctas, int rows, int n, const T *__restrict__ val
     }
     __syncthreads();
     // warp s adds the partial rows of segment s, in the order of the warps
-    const int seg = static_cast<int>(blockIdx.x) + warp * seg_ctas;
+    const int seg = cta + warp * seg_ctas;
     if (seg >= m1) return;
     const int first = __shfl_sync(kFull, incl - chunks, warp) / per, last = (__shfl_sync(kFull, incl, warp) - 1) / per;
     const int out_row = __shfl_sync(kFull, row, warp);
@@ -560,6 +561,7 @@ spmm_fixup(int m1, int segs_per_cta, int n, const int *__restrict__ row_offsets,
     __shared__ int s_row[kFixupThreads], s_first[kFixupThreads], s_cnt[kFixupThreads];
     __shared__ int n_narrow, n_wide;
     __shared__ double s_part[kFixupWarps][32][kLen];
+    chain_begin();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) n_narrow = n_wide = 0;
     __syncthreads();
@@ -660,7 +662,7 @@ __global__ void __launch_bounds__(kCtaThreads, (sizeof(T) == 4 ? 32 : 16) / kCta
 spmm_rows(int m2, int rows_per_group, int n, const T *__restrict__ values,
           const int *__restrict__ column_indices, const int *__restrict__ row_offsets,
           const int *__restrict__ residue_r_ind, const T *__restrict__ B, T *__restrict__ C,
-          int *__restrict__ next_group) {
+          int *__restrict__ next_group, bool first) {
     using V = typename Vec16<T>::type;
     constexpr int kLen = Vec16<T>::kLen;
     constexpr int U = (kLoadsInFlight < L) ? kLoadsInFlight : L;  // rows per batch
@@ -681,7 +683,8 @@ spmm_rows(int m2, int rows_per_group, int n, const T *__restrict__ values,
     // the bundle of rows of its own index and claims further bundles from a counter per column
     // tile; the claim is issued before the bundle's work and read after it.
     const long long n_groups = (static_cast<long long>(m2) + rows_per_group - 1) / rows_per_group;
-    long long group = (static_cast<long long>(blockIdx.x) * kCtaThreads + threadIdx.x) / L;
+    const unsigned cta = after_chain_if(first, blockIdx.x);
+    long long group = (static_cast<long long>(cta) * kCtaThreads + threadIdx.x) / L;
     while (group < n_groups) {
     int claimed = INT_MAX;
     constexpr bool kClaim = sizeof(T) == 4;  // fp64: 12 more registers for it cost more than it gains
@@ -819,7 +822,7 @@ spmm_rows(int m2, int rows_per_group, int n, const T *__restrict__ values,
 constexpr int kRowsCtaThreads = 32;
 constexpr long long kWideRowsWaves = 2;  // spmm_rows_wide (a warp per row) serves lists of at most so many waves of 32 warps per SM
 
-template <typename T, int VB, int L, int VPL, int R, bool kRagged>
+template <typename T, int VB, int L, int VPL, int R, bool kRagged, bool kFirst>
 __global__ void __launch_bounds__(kRowsCtaThreads, 1024 / kRowsCtaThreads)  // 64 registers: 32 warps per SM
 spmm_rows_simple(int m2, int n, const T *__restrict__ values, const int *__restrict__ column_indices,
                  const int *__restrict__ row_offsets, const int *__restrict__ residue_r_ind,
@@ -834,7 +837,9 @@ spmm_rows_simple(int m2, int n, const T *__restrict__ values, const int *__restr
     const int lane = threadIdx.x & 31;
     const int l = lane % L;
     const unsigned gmask = group_mask<L>(lane);
-    const long long item0 = ((static_cast<long long>(blockIdx.x) * kRowsCtaThreads + threadIdx.x) / L) * R;
+    unsigned cta = blockIdx.x;
+    if constexpr (kFirst) cta = after_chain(cta);
+    const long long item0 = ((static_cast<long long>(cta) * kRowsCtaThreads + threadIdx.x) / L) * R;
     int row[R], begin[R], end[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -940,7 +945,7 @@ template <typename T, int VB, int L, int VPL, bool kRagged>
 __global__ void __launch_bounds__(32 * kSmallGridWarps, 1)
 spmm_rows_wide(int m2, int n, const T *__restrict__ values, const int *__restrict__ column_indices,
                const int *__restrict__ row_offsets, const int *__restrict__ residue_r_ind,
-               const T *__restrict__ B, T *__restrict__ C) {
+               const T *__restrict__ B, T *__restrict__ C, bool first) {
     using V = typename VecB<T, VB>::type;
     constexpr int kLen = VecB<T, VB>::kLen;
     constexpr int G = 32 / L;    // lane groups; a group takes at most 32 / G = L nonzeros
@@ -948,7 +953,8 @@ spmm_rows_wide(int m2, int n, const T *__restrict__ values, const int *__restric
     constexpr int kBlockK = 32;  // k_block of the preprocessing
     constexpr unsigned kFull = 0xffffffffu;
     if (blockIdx.x == gridDim.x - 1) return chain_wait();  // the CTA behind the rows
-    const int item = blockIdx.x * kSmallGridWarps + (threadIdx.x >> 5);
+    const int cta = after_chain_if(first, blockIdx.x);
+    const int item = cta * kSmallGridWarps + (threadIdx.x >> 5);
     if (item >= m2) return;
     const int lane = threadIdx.x & 31;
     const int g = lane / L, l = lane % L;
@@ -1076,8 +1082,8 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
         // cost more time than that returned (1.41 -> 1.52 ms).
         if constexpr (L * VPL * VB == 512 && !kRagged) {
             if (!launched && hot && !small_grid) {
-                spmm_block<T, VB, L, VPL, U, kCtaWarps, 1, true, true, false><<<grid, kCtaThreads, 0, s1>>>(
-                    m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, hot, (k + 31) / 32, claim, nullptr);
+                RODE_CUDA_TRY(launch_chained(spmm_block<T, VB, L, VPL, U, kCtaWarps, 1, true, true, false>, grid, dim3(kCtaThreads), s1, true,
+                    m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, hot, (k + 31) / 32, claim, nullptr));
                 launched = true;
             }
         }
@@ -1089,20 +1095,24 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
             constexpr int UOne = 2 * U <= L ? 2 * U : L;
             const int seg_ctas = (m1 + kOneLaunchWarps - 1) / kOneLaunchWarps;
             const int row_ctas = (m2 + kOneLaunchWarps - 1) / kOneLaunchWarps;
-            spmm_one_launch<T, VB, L, VPL, UOne, kRagged><<<dim3(seg_ctas + row_ctas, tiles), 32 * kOneLaunchWarps, 0, s1>>>(
-                m1, seg_ctas, m2, n, values, col, row_offsets, block_r_ind, st_off, residue_r_ind, B, C, partial);
+            RODE_CUDA_TRY(launch_chained(spmm_one_launch<T, VB, L, VPL, UOne, kRagged>, dim3(seg_ctas + row_ctas, tiles),
+                                         dim3(32 * kOneLaunchWarps), s1, true, m1, seg_ctas, m2, n, values, col, row_offsets,
+                                         block_r_ind, st_off, residue_r_ind, B, C, partial));
             rows_done = launched = true;
         }
         const long long warps = static_cast<long long>(m1) * tiles;
         if (!launched && warps <= kSplit4WarpsPerSm * sm_count()) {
-            spmm_block<T, VB, L, VPL, U, 4, 4, false, false, kRagged><<<dim3(m1, tiles), 4 * 32, 0, s1>>>(
-                m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0, nullptr, nullptr);
+            RODE_CUDA_TRY(launch_chained(spmm_block<T, VB, L, VPL, U, 4, 4, false, false, kRagged>, dim3(m1, tiles), dim3(4 * 32), s1,
+                                         true, m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0,
+                                         nullptr, nullptr));
         } else if (!launched && warps <= kSplit2WarpsPerSm * sm_count()) {
-            spmm_block<T, VB, L, VPL, U, 2, 2, false, false, kRagged><<<dim3(m1, tiles), 2 * 32, 0, s1>>>(
-                m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0, nullptr, nullptr);
+            RODE_CUDA_TRY(launch_chained(spmm_block<T, VB, L, VPL, U, 2, 2, false, false, kRagged>, dim3(m1, tiles), dim3(2 * 32), s1,
+                                         true, m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0,
+                                         nullptr, nullptr));
         } else if (!launched) {
-            spmm_block<T, VB, L, VPL, U, kCtaWarps, 1, false, true, kRagged><<<grid, kCtaThreads, 0, s1>>>(
-                m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0, claim, nullptr);
+            RODE_CUDA_TRY(launch_chained(spmm_block<T, VB, L, VPL, U, kCtaWarps, 1, false, true, kRagged>, grid, dim3(kCtaThreads), s1,
+                                         true, m1, n, values, col, row_offsets, block_r_ind, st_off, B, C, partial, nullptr, 0,
+                                         claim, nullptr));
         }
         RODE_CHECK_LAUNCH("rode::spmm_block");
     }
@@ -1150,12 +1160,12 @@ int launch_rows(int m2, int n, const T *values, const int *col, const int *row_o
             if (!counters_clear) RODE_CUDA_TRY(cudaMemsetAsync(claim, 0, kClaimTiles * sizeof(int), s2));
         }
         const dim3 grid(static_cast<unsigned>(persistent ? (resident + tiles - 1) / tiles : ctas_needed), tiles);
-        RODE_CUDA_TRY(launch_chained(spmm_rows<T, 32, kRagged>, grid, dim3(kCtaThreads), s2, chained, m2, per_group, n, values,
-                                     col, row_offsets, residue_r_ind, B, C, claim));
+        RODE_CUDA_TRY(launch_chained(spmm_rows<T, 32, kRagged>, grid, dim3(kCtaThreads), s2, true, m2, per_group, n, values,
+                                     col, row_offsets, residue_r_ind, B, C, claim, !chained));
     } else if (static_cast<long long>(m2) * tiles <= kWideRowsWaves * 32 * sm_count()) {
         const dim3 grid((m2 + kSmallGridWarps - 1) / kSmallGridWarps + 1, tiles);
-        RODE_CUDA_TRY(launch_chained(spmm_rows_wide<T, VB, L, VPL, kRagged>, grid, dim3(32 * kSmallGridWarps), s2, chained, m2,
-                                     n, values, col, row_offsets, residue_r_ind, B, C));
+        RODE_CUDA_TRY(launch_chained(spmm_rows_wide<T, VB, L, VPL, kRagged>, grid, dim3(32 * kSmallGridWarps), s2, true, m2,
+                                     n, values, col, row_offsets, residue_r_ind, B, C, !chained));
     } else {
         // Two rows per lane group where rows are short: both rows' bounds and first columns are then fetched together, and a
         // short row's life is that chain of loads; long even rows lose it again to the longer life of a warp.
@@ -1163,8 +1173,12 @@ int launch_rows(int m2, int n, const T *values, const int *col, const int *row_o
             constexpr int R = decltype(two)::value ? 2 : 1;
             constexpr int kRowsPerCta = R * kRowsCtaThreads / L;
             const dim3 grid(static_cast<unsigned>((static_cast<long long>(m2) + kRowsPerCta - 1) / kRowsPerCta + 1), tiles);
-            return launch_chained(spmm_rows_simple<T, VB, L, VPL, R, kRagged>, grid, dim3(kRowsCtaThreads), s2, chained, m2, n,
-                                  values, col, row_offsets, residue_r_ind, B, C);
+            // (first grid of the call: an early start is worth a microsecond, and a wait in each of half a million CTAs costs
+            // more than that: stencil 128^3 N = 64 +1.7 %)
+            const bool early = !chained && grid.x <= 64u * 32u * sm_count();
+            const auto kernel = early ? spmm_rows_simple<T, VB, L, VPL, R, kRagged, true> : spmm_rows_simple<T, VB, L, VPL, R, kRagged, false>;
+            return launch_chained(kernel, grid, dim3(kRowsCtaThreads), s2, chained || early, m2, n, values, col, row_offsets,
+                                  residue_r_ind, B, C);
         };
         if (two_rows)
             RODE_CUDA_TRY(launch(std::true_type{}));
