@@ -318,7 +318,18 @@ __device__ __forceinline__ unsigned after_chain(unsigned i) {
     asm volatile("griddepcontrol.wait;" : "+r"(i)::"memory");
     return i;
 }
-// The same where `first`, without a branch (which cost spmm_rows 140 bytes of spills).
+// Loads of what the grids before this one have written, that stay behind a wait (__ldcg alone is not held back by one).
+__device__ __forceinline__ int ld_behind_wait(const int *p) {
+    int v;
+    asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ int2 ld_behind_wait(const int2 *p) {
+    int2 v;
+    asm volatile("ld.global.cg.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+    return v;
+}
+// after_chain() where `first`, without a branch (which cost spmm_rows 140 bytes of spills).
 __device__ __forceinline__ unsigned after_chain_if(bool first, unsigned i) {
     asm volatile(
         "{\n.reg .pred p;\nsetp.ne.s32 p, %1, 0;\n@p griddepcontrol.wait;\n}"

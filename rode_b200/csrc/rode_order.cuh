@@ -206,7 +206,7 @@ order_pieces(int m1, int n_cols, const int *__restrict__ row_offsets, const int 
     int my_start = 0;       // where bucket t starts in the list
     if constexpr (kPlace) {
         chain_wait();  // the counts
-        my_start = scan(__ldcg(&head->counts[t]), unused);
+        my_start = scan(ld_behind_wait(&head->counts[t]), unused);
     }
     __syncthreads();
     constexpr int N = P > 0 ? kOrderPerThread : 1;

@@ -273,12 +273,12 @@ fill_tiles(Params p, int M, int group, const int *__restrict__ row_ptr, const in
         const int groups = tile / group;
 #pragma unroll 4
         for (int g = threadIdx.x; g < groups; g += kThreads) {
-            const int2 v = __ldcg(sums + (static_cast<size_t>(g) + 1) * group - 1);
+            const int2 v = ld_behind_wait(sums + (static_cast<size_t>(g) + 1) * group - 1);
             b += v.x;
             r += v.y;
         }
         if (threadIdx.x == 0 && tile % group != 0) {
-            const int2 v = __ldcg(sums + tile - 1);
+            const int2 v = ld_behind_wait(sums + tile - 1);
             b += v.x;
             r += v.y;
         }

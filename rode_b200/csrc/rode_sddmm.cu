@@ -592,7 +592,7 @@ sddmm_pieces(OrderHead *head, const unsigned long long *__restrict__ list, int c
     chain_wait();
     int total = 0;
 #pragma unroll
-    for (int i = 0; i < kOrderBuckets / 32; ++i) total += __ldcg(&head->counts[lane + 32 * i]);
+    for (int i = 0; i < kOrderBuckets / 32; ++i) total += ld_behind_wait(&head->counts[lane + 32 * i]);
     total = min(__reduce_add_sync(kFull, total), capacity);
     const int bundles = (total + kPieceRounds - 1) / kPieceRounds;
     const float4 *lhs_lane = reinterpret_cast<const float4 *>(lhs) + l;

@@ -1019,20 +1019,22 @@ spmm_rows_wide(int m2, int n, const T *__restrict__ values, const int *__restric
     }
 }
 
-// When an order of the segments pays (rode_order.cuh): with uniform columns from an operand beyond the L2 on, on skewed ones for
-// 256-byte rows only.  Whole calls, row by row / ordered, us.  Zipf 671,008 x 929,297 of mean 40 N = 32 (113 MB) 329 / 282, N = 64 830 /
+// When an order of the segments pays (rode_order.cuh): from an operand beyond the L2 on, on skewed columns for the 256- and 512-byte
+// tiles of float only.  Whole calls, row by row / ordered, us.  Zipf 671,008 x 929,297 of mean 40 N = 32 (113 MB) 329 / 282, N = 64 830 /
 // 510, N = 128 1750 / 934, fp64 N = 64 1750 / 981; Zipf 2^20 of mean 8 N = 64 353 / 290; Pareto 2^20 of mean 32 N = 32 (128 MB) 517 / 509,
 // N = 64 1104 / 1006, N = 256 4579 / 4126, of mean 16 N = 64 640 / 599, of mean 8 N = 64 390 / 386, N = 128 675 / 677; 2^22 of mean 8
 // N = 32 1023 / 1039, N = 128 2841 / 2820.  R-MAT 23, 22, 21, 20 N = 64 3299 / 3112, 1485 / 1414, 697 / 687, 353 / 345, but N = 32 863 / 876
-// (22), N = 128 5347 / 5818 (23, against popularity hints), fp64 N = 32 785 / 832 (21).
+// (22), fp64 N = 32 785 / 832 (21).  R-MAT N = 128 with popularity hints / ordered, calls back to back under the power cap: scale 23
+// 5862 / 5728, 22 2690 / 2669 (in short bursts 2268 / 2364), 21 1269 / 1254, of 32 per row 2295 / 2157, 20 of 64 1957 / 1792, 19 286 / 286; N = 256
+// 2576 / 2474; 22 of 6 per row 1280 / 1311; and the first call on a matrix, which builds no bitmap then, scale 23 6257 / 5000, 21 1687 / 1152.
 //
 // The more of the nonzeros are in rows of many segments, the more an order gives: Zipf matrices have 370 to 410 nonzeros per segment,
 // Pareto 170 to 310, where it takes more references per column and a larger grid (2^22 rows of mean 8 above; 262,144 x 2^20 of mean
 // 16, 19,043 segments, N = 128 331 / 333; Zipf of the same size, 10,953 segments, 316 / 284).
 bool order_pays(int verdict, long long m1, long long k, long long n, long long nnz, int elem_size) {
     if (m1 < kOrderMinSegments || k * n * elem_size < 160ll << 20) return false;
-    if (nnz < kOrderLongRows * m1 && (m1 < 1 << 16 || nnz < 12 * k)) return false;
-    return verdict == kOrderHelps || (verdict == kOrderSkewed && n * elem_size == 256 && elem_size == 4);
+    if (nnz < kOrderLongRows * m1 && (m1 < 1 << 15 || nnz < 12 * k)) return false;
+    return verdict == kOrderHelps || (verdict == kOrderSkewed && elem_size == 4 && (n == 64 || n % 128 == 0));
 }
 
 template <typename T, int VB, int L, int VPL, bool kRagged>

@@ -137,8 +137,8 @@ def rode_spmm(sparse_matrix: RoDeCSR, dense: torch.Tensor, hints: bool = True) -
     best); the reference has no Python SpMM.
 
     ``hints``: what keeps dense rows in the L2 (same results, fewer DRAM bytes): the segments in the order of their columns
-    where the matrix and the width are such that it pays; else popular columns' rows gathered with an L2 policy that keeps
-    them resident on skewed matrices, whose popularity bitmap is built on the first call for a given width and cached on
+    where the matrix and the width are such that it pays; else, on skewed matrices, popular columns' rows gathered with an L2
+    policy that keeps them resident, whose popularity bitmap is built on the first call for a given width and cached on
     ``sparse_matrix``."""
     shape = dense.shape
     if len(shape) != 2 or shape[0] != sparse_matrix.n:

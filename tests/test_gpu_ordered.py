@@ -122,6 +122,6 @@ def test_verdict():
         pays = [capi.sddmm_order_pays(verdict, m, meta.m1, n, k, col.numel()) for k in (32, 64, 128)]
         nnz = 12 * n  # as if there were a few more references per column
         assert [capi.spmm_order_pays(verdict, meta.m1, n, k, nnz) for k in (32, 64, 128)] == {
-            "uniform": [False, True, True], "skewed": [False, True, False], "band": [False] * 3}[kind], kind
+            "uniform": [False, True, True], "skewed": [False, True, True], "band": [False] * 3}[kind], kind
         # 90 MB, 179 MB, 358 MB of rhs
         assert pays == {"uniform": [False, True, True], "skewed": [False, False, True], "band": [False] * 3}[kind], kind
