@@ -35,7 +35,7 @@
 //    dependent chain row index -> row pointer -> column -> dense row is paid once per 32
 //    rows, not per row.  The nonzeros of the 32 rows form one entry stream that runs through
 //    the same batched gather; a row is stored when the stream passes its end.
-//    spmm_rows_simple (L < 32): one lane group per residue row, or per two short ones; spmm_rows_wide: one warp per
+//    spmm_rows_simple, spmm_rows_simple_staged (L < 32): one lane group per residue row, or per two short ones; spmm_rows_wide: one warp per
 //    row, for lists too short to fill the GPU.  All of them also take the rows of the whole matrix in the place of
 //    a list, and then store zeros in those without a nonzero.
 //    Rows of the list without a nonzero are not touched (the reference stores zeros there,
@@ -935,6 +935,118 @@ spmm_rows_simple(int m2, int n, const T *__restrict__ values, const int *__restr
 }
 
 // ---------------------------------------------------------------------------------------
+// The same rows, R per lane group one after the other, with all pairs of the warp's rows fetched at once: a load per row
+// and array, coalesced over the row's nonzeros (fewer than 32), instead of one per chunk of L nonzeros of several rows.  That
+// is three memory round trips before a warp only waits for dense rows, and a third fewer wavefronts for the pairs on the SM's
+// load path, which bounds rows that share their columns (27-point stencil 128^3, us, one chunk after the other / staged: N = 16
+// 353 / 286, N = 32 390 / 368, N = 64 673 / 628, N = 96 1179 / 1090, fp64 N = 32 792 / 665; 300,000 rows of 15 to 24 N = 64 116 / 97; 1,000,000 of 0
+// to 12 N = 32 133 / 118, N = 64 267 / 226; Pareto 2^20 rows alone N = 64 434 / 358).
+//
+// It serves matrices without segments and lists of 2^19 rows and more.  Shorter lists beside a block grid keep spmm_rows_simple:
+// there the rows are the smaller part, and their loads get in the way of the last segments (R-MAT 17 N = 64 51 / 54, the rows
+// alone 25 / 22; Pareto 300,007 N = 32 87 / 93; but R-MAT 21 N = 64 697 / 679, Pareto 2^20 N = 64 1105 / 1064).
+//
+// R = 2 where rows are not known to be long (rows alone, R = 1 / 2: R-MAT 21 N = 64 278 / 226, Pareto 2^20 N = 64 371 / 358; stencil N = 64
+// 633 / 650; rows of 15 to 24 N = 32 56 / 58, N = 64 102 / 97); the 128-byte tile of fp64 has no room for two (8 rows x 32
+// pairs are 3 KB per CTA; 1,000,000 rows of 0 to 12 N = 16 131 / 188) and leaves short rows to spmm_rows_simple (R-MAT 21 N = 16 456 /
+// 466).
+constexpr int kStagedRows = 1 << 19;
+template <typename T, int VB, int L, int VPL, int R, bool kRagged, bool kFirst>
+__global__ void __launch_bounds__(kRowsCtaThreads, 1024 / kRowsCtaThreads)  // 64 registers: 32 warps per SM
+spmm_rows_simple_staged(int m2, int n, const T *__restrict__ values, const int *__restrict__ column_indices,
+                 const int *__restrict__ row_offsets, const int *__restrict__ residue_r_ind,
+                 const T *__restrict__ B, T *__restrict__ C) {
+    using V = typename VecB<T, VB>::type;
+    constexpr int kLen = VecB<T, VB>::kLen;
+    constexpr int U = kLoadsInFlight * 16 / VB / VPL;  // dense rows per batch
+    constexpr int G = 32 / L;                          // rows side by side
+    constexpr int N = G * R;                           // rows of the warp
+    constexpr int kAlign = 4;    // vec_len of the preprocessing
+    constexpr int kBlockK = 32;  // k_block of the preprocessing
+    constexpr unsigned kFull = 0xffffffffu;
+    static_assert(U == 4 && N <= 32, "quadruples; a descriptor per lane");
+    if (blockIdx.x == gridDim.x - 1) return chain_wait();  // the CTA behind the rows
+    __shared__ __align__(16) int s_col[N * 32];
+    __shared__ __align__(16) T s_val[N * 32];
+    const int lane = threadIdx.x;
+    const int g = lane / L, l = lane % L;
+    unsigned cta = blockIdx.x;
+    if constexpr (kFirst) cta = after_chain(cta);
+    const long long item0 = static_cast<long long>(cta) * N;
+    // lane j of the warp reads the descriptor of row item0 + j; group g takes rows g, G + g, ...
+    int row = -1, begin = 0, len = 0;
+    if (lane < N && item0 + lane < m2) {
+        row = residue_r_ind != nullptr ? __ldg(residue_r_ind + item0 + lane) : static_cast<int>(item0) + lane;
+        begin = __ldg(row_offsets + row);
+        const int end = __ldg(row_offsets + row + 1);
+        // aligned length >= k_block: a block part exists and its last segment took the tail;
+        // list form, no nonzero: the row stays as the caller zero-filled it (all rows: zeros are stored below)
+        if (end - begin + (begin % kAlign) >= kBlockK || (end == begin && residue_r_ind != nullptr))
+            row = -1;
+        else
+            len = end - begin;
+    }
+    int c[N];
+    T v[N];
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+        const int b = __shfl_sync(kFull, begin, r), e = __shfl_sync(kFull, len, r);
+        c[r] = 0;
+        v[r] = T(0);
+        if (lane < e) {
+            c[r] = ld_stream(column_indices + b + lane);
+            v[r] = ld_stream(values + b + lane);
+        }
+    }
+    // quadruple q of row r: rotated so that the lane groups read the same one of neighbouring rows from different banks
+    auto at = [](int r, int q) { return r * 32 + ((q ^ (r & 7)) << 2); };
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+        s_col[at(r, lane / 4) + lane % 4] = c[r];
+        s_val[at(r, lane / 4) + lane % 4] = v[r];
+    }
+    __syncwarp();
+    const size_t row_vecs = static_cast<size_t>(n) / kLen;
+    const size_t col_vec = static_cast<size_t>(blockIdx.y) * L * VPL + l;
+    const unsigned row_bytes = static_cast<unsigned>(n) * static_cast<unsigned>(sizeof(T));  // n < 2^21 elements
+    const V *b_lane = reinterpret_cast<const V *>(B) + col_vec;
+    auto inside = [&](int v) { return !kRagged || col_vec + v * L < row_vecs; };
+#pragma unroll 1
+    for (int i = 0; i < R; ++i) {
+        const int row_i = __shfl_sync(kFull, row, i * G + g), len_i = __shfl_sync(kFull, len, i * G + g);
+        const int longest = __reduce_max_sync(kFull, len_i);
+        V acc[VPL];
+#pragma unroll
+        for (int v = 0; v < VPL; ++v) acc[v] = vzero(static_cast<V *>(nullptr));
+        for (int t0 = 0; t0 < longest; t0 += U) {
+            int cc[U];
+            T vv[U];
+            V bb[U][VPL];
+            ld_shared_run<U>(s_col + at(i * G + g, t0 / 4), cc);
+            ld_shared_run<U>(s_val + at(i * G + g, t0 / 4), vv);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int v = 0; v < VPL; ++v) {
+                    bb[u][v] = vzero(static_cast<V *>(nullptr));
+                    if (t0 + u < len_i && inside(v))
+                        bb[u][v] = ld_dense(dense_row(b_lane + v * L, static_cast<unsigned>(cc[u]), row_bytes));
+                }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int v = 0; v < VPL; ++v) vfma(acc[v], vv[u], bb[u][v]);
+        }
+        if (row_i >= 0) {
+#pragma unroll
+            for (int v = 0; v < VPL; ++v)
+                if (inside(v))
+                    st_stream(reinterpret_cast<V *>(C) + static_cast<size_t>(row_i) * row_vecs + col_vec + v * L, acc[v]);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------
 // The same rows, one WARP per row: for residue lists too short to fill the GPU, where the
 // time of the launch is the dependent chain of one row, not throughput.  The 32 lanes fetch
 // the row's (fewer than 32) pairs in one coalesced load; the 32 / L lane groups then take
@@ -1039,7 +1151,7 @@ bool order_pays(int verdict, long long m1, long long k, long long n, long long n
 
 template <typename T, int VB, int L, int VPL, bool kRagged>
 int launch_rows(int m2, int n, const T *values, const int *col, const int *row_offsets, const int *residue_r_ind,
-                const T *B, T *C, int *counters, bool chained, bool counters_clear, bool two_rows,
+                const T *B, T *C, int *counters, bool chained, bool counters_clear, int m1, long long nnz,
                 cudaStream_t s2);
 
 // Block kernel of one shape and residue-row kernel of another; each walks the columns in tiles of its own.
@@ -1122,7 +1234,7 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
     // they are a plain launch.
     if (m2 > 0 && !rows_done) {
         if (int rc = launch_rows<T, Rows::VB, Rows::L, Rows::VPL, kRowsRagged>(m2, n, values, col, row_offsets, residue_r_ind, B, C, counters,
-                                                            chained, counters_clear, short_rows(nnz, m1, m2, Rows::VB * Rows::L * Rows::VPL), s2))
+                                                            chained, counters_clear, m1, nnz, s2))
             return rc;
     }
     if (m1 > 1) {  // (a row that was cut has two segments at least)
@@ -1140,7 +1252,7 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
 
 template <typename T, int VB, int L, int VPL, bool kRagged>
 int launch_rows(int m2, int n, const T *values, const int *col, const int *row_offsets, const int *residue_r_ind,
-                const T *B, T *C, int *counters, bool chained, bool counters_clear, bool two_rows,
+                const T *B, T *C, int *counters, bool chained, bool counters_clear, int m1, long long nnz,
                 cudaStream_t s2) {
     constexpr int kTileWidth = L * VPL * VecB<T, VB>::kLen;
     const unsigned tiles = static_cast<unsigned>(kRagged ? (n + kTileWidth - 1) / kTileWidth : n / kTileWidth);
@@ -1169,23 +1281,39 @@ int launch_rows(int m2, int n, const T *values, const int *col, const int *row_o
         RODE_CUDA_TRY(launch_chained(spmm_rows_wide<T, VB, L, VPL, kRagged>, grid, dim3(32 * kSmallGridWarps), s2, true, m2,
                                      n, values, col, row_offsets, residue_r_ind, B, C, !chained));
     } else {
-        // Two rows per lane group where rows are short: both rows' bounds and first columns are then fetched together, and a
-        // short row's life is that chain of loads; long even rows lose it again to the longer life of a warp.
-        auto launch = [&](auto two) {
-            constexpr int R = decltype(two)::value ? 2 : 1;
-            constexpr int kRowsPerCta = R * kRowsCtaThreads / L;
-            const dim3 grid(static_cast<unsigned>((static_cast<long long>(m2) + kRowsPerCta - 1) / kRowsPerCta + 1), tiles);
-            // (first grid of the call: an early start is worth a microsecond, and a wait in each of half a million CTAs costs
-            // more than that: stencil 128^3 N = 64 +1.7 %)
+        // (first grid of the call: an early start is worth a microsecond, and a wait in each of half a million CTAs costs
+        // more than that: stencil 128^3 N = 64 +1.7 %)
+        auto launch = [&](auto plain, auto first, int rows_per_group) {
+            const int rows_per_cta = rows_per_group * kRowsCtaThreads / L;
+            const dim3 grid(static_cast<unsigned>((static_cast<long long>(m2) + rows_per_cta - 1) / rows_per_cta + 1), tiles);
             const bool early = !chained && grid.x <= 64u * 32u * sm_count();
-            const auto kernel = early ? spmm_rows_simple<T, VB, L, VPL, R, kRagged, true> : spmm_rows_simple<T, VB, L, VPL, R, kRagged, false>;
-            return launch_chained(kernel, grid, dim3(kRowsCtaThreads), s2, chained || early, m2, n, values, col, row_offsets,
-                                  residue_r_ind, B, C);
+            return launch_chained(early ? first : plain, grid, dim3(kRowsCtaThreads), s2, chained || early, m2, n, values, col,
+                                  row_offsets, residue_r_ind, B, C);
         };
-        if (two_rows)
-            RODE_CUDA_TRY(launch(std::true_type{}));
-        else
-            RODE_CUDA_TRY(launch(std::false_type{}));
+        constexpr int kTileBytes = VB * L * VPL;
+        constexpr bool kRoomForTwo = sizeof(T) == 4 || kTileBytes > 128;
+        const bool shorts = short_rows(nnz, m1, m2, kTileBytes);
+        const bool staged = (m1 == 0 || m2 >= kStagedRows) && (kRoomForTwo || !shorts);
+        if constexpr (kRoomForTwo) {
+            if (staged && !rows_hold(nnz, m1, m2, kTileBytes == 128 ? 10 : 20)) {
+                RODE_CUDA_TRY(launch(spmm_rows_simple_staged<T, VB, L, VPL, 2, kRagged, false>,
+                                     spmm_rows_simple_staged<T, VB, L, VPL, 2, kRagged, true>, 2));
+                RODE_CHECK_LAUNCH("rode::spmm_rows");
+                return RODE_OK;
+            }
+        }
+        if (staged) {
+            RODE_CUDA_TRY(launch(spmm_rows_simple_staged<T, VB, L, VPL, 1, kRagged, false>,
+                                 spmm_rows_simple_staged<T, VB, L, VPL, 1, kRagged, true>, 1));
+        } else if (shorts) {
+            // Two rows per lane group where rows are short: both rows' bounds and first columns are then fetched together, and
+            // a short row's life is that chain of loads; long even rows lose it again to the longer life of a warp.
+            RODE_CUDA_TRY(launch(spmm_rows_simple<T, VB, L, VPL, 2, kRagged, false>,
+                                 spmm_rows_simple<T, VB, L, VPL, 2, kRagged, true>, 2));
+        } else {
+            RODE_CUDA_TRY(launch(spmm_rows_simple<T, VB, L, VPL, 1, kRagged, false>,
+                                 spmm_rows_simple<T, VB, L, VPL, 1, kRagged, true>, 1));
+        }
     }
     RODE_CHECK_LAUNCH("rode::spmm_rows");
     return RODE_OK;
