@@ -24,8 +24,7 @@
 //    matching values, so results are stored coalesced.
 //  * Row mode of the residue-row kernel: a warp whose rows are long enough (6 nonzeros on average, 16 where the stream has
 //    one lane group) and, in short lists and wide rows, about equally long does not form a stream; its lane groups
-//    take the rows one each, neighbouring rows side by side, each row by the plain per-row loop
-//    sddmm_one_row.  The warp decides from the row lengths it has just loaded (27-point stencil, K = 64:
+//    take the rows one each, neighbouring rows side by side (sddmm_rows_one_by_one).  The warp decides from the row lengths it has just loaded (27-point stencil, K = 64:
 //    1.26 -> 0.81 ms, rhs rows shared by neighbouring rows now hit in L1; power-law rows,
 //    K = 64: 0.51 -> 0.44 ms; graphs with many empty rows keep the stream).
 //  * The column indices of a chunk reach the lanes that gather with them through a small
@@ -37,6 +36,7 @@
 //    warp of its own; chunk loads are then plain coalesced loads without any search and the
 //    lhs slice never changes (power-law K = 32: 370 us against 744 us through sddmm_items).
 //    Small grids run segments and rows in one launch.
+//  * sddmm_pieces: the segments of large operands, cut into pieces that are sorted by their columns (rode_order.cuh).
 //  * One-warp CTAs: a CTA's slot is held until its slowest warp finishes.
 //
 // Per nonzero: 12 B of CSR data/output plus 4*K bytes of rhs (L1/L2/HBM by reuse); per item
@@ -96,65 +96,86 @@ __device__ __forceinline__ float reduce_batch(float (&p)[NB], int l, unsigned gm
     return r;
 }
 
-// All nonzeros [begin, end) of ONE row, by the lane group (L lanes x VPL loads per lane) that
-// `lane` belongs to; every lane of the group must call with the same row.  Lane l fetches the
-// pair of nonzero l of a chunk of L one chunk ahead; batches of kLoadsInFlight loads per lane.
-// `stage` = 2 x 32 ints of shared memory owned by this warp (two chunk buffers), `stage_buf` the
-// buffer to use next; both are carried from row to row so that a group never stores into a
-// buffer that one of its lanes may still read.
+// The rows of up to 32 items one by one, 32 / L neighbouring ones side by side, a lane group (L lanes x VPL loads per lane)
+// each.  Lane j of the warp holds bounds and row of item j (len = 0: nothing to do); all lanes call.  The columns and values of a
+// round's rows, fewer than 32 each, are fetched by one coalesced load per row and array, a round ahead; the columns
+// reach the groups, and the dot products the lanes that hold the values, through shared memory.
+// `stage` = 2 x 32 / L x 32 words of shared memory.  (Chunks of L nonzeros fetched by each group for itself, and the results
+// stored from the lanes of the group, took more wavefronts on the SM's load path, which bounds rows that share columns, and
+// more round trips: calls, us, before / after: stencil 128^3 K = 32 524 / 506, K = 64 761 / 727, K = 96 1217 / 1195; 300,000 rows of 0 to 28 K =
+// 64 138 / 127; rows of Pareto 2^20 K = 64 431 / 402, of R-MAT 21 K = 200 1181 / 1078.)
 // kRagged: the dense rows hold row_vecs_arg <= L * VPL vectors, the rest of the lanes idle.
 template <int L, int VPL, int kBatch, bool kRagged>
-__device__ __forceinline__ void sddmm_one_row(int row, int begin, int end, int lane, int row_vecs_arg,
-                                              const int *__restrict__ column_indices,
-                                              const float *__restrict__ values, const float *__restrict__ lhs,
-                                              const float *__restrict__ rhs, float *__restrict__ out, int *stage,
-                                              int &stage_buf) {
+__device__ __forceinline__ void sddmm_rows_one_by_one(int n_items, int row, int begin, int len, int lane, int row_vecs_arg,
+                                                      const int *__restrict__ column_indices,
+                                                      const float *__restrict__ values, const float *__restrict__ lhs,
+                                                      const float *__restrict__ rhs, float *__restrict__ out, int *stage) {
+    constexpr int G = 32 / L;
     const size_t row_vecs = kRagged ? static_cast<unsigned>(row_vecs_arg) : L * VPL;
-    const int l = lane % L;
-    const unsigned gmask = group_mask<L>(lane);
+    const int g = lane / L, l = lane % L;
     const float4 *rhs_lane = reinterpret_cast<const float4 *>(rhs) + l;
     auto inside = [&](int v) { return !kRagged || static_cast<size_t>(l + v * L) < row_vecs; };
-    float4 a[VPL];
+    int *s_col = stage;
+    float *s_dot = reinterpret_cast<float *>(stage + G * 32);
+    // quadruple q of row r, rotated so that the groups read the same one of neighbouring rows from different banks
+    auto at = [](int r, int q) { return r * 32 + ((q ^ (r & 7)) << 2); };
+    int c_nxt[G];
+    float v_nxt[G];
+    auto fetch = [&](int j0) {
 #pragma unroll
-    for (int v = 0; v < VPL; ++v)
-        a[v] = inside(v) ? __ldg(reinterpret_cast<const float4 *>(lhs) + static_cast<size_t>(row) * row_vecs + v * L + l)
-                         : make_float4(0.f, 0.f, 0.f, 0.f);
-    int c_nxt = 0;
-    float v_nxt = 0.f;
-    if (begin + l < end) {
-        c_nxt = ld_stream(column_indices + begin + l);
-        v_nxt = ld_stream(values + begin + l);
-    }
-    for (int base = begin; base < end; base += L) {
-        const int c = c_nxt;
-        const float val = v_nxt;
-        const int e = base + L + l;
-        c_nxt = 0;
-        v_nxt = 0.f;
-        if (e < end) {
-            c_nxt = ld_stream(column_indices + e);
-            v_nxt = ld_stream(values + e);
+        for (int r = 0; r < G; ++r) {
+            const int b = __shfl_sync(kFull, begin, (j0 + r) & 31), n = __shfl_sync(kFull, len, (j0 + r) & 31);
+            c_nxt[r] = 0;
+            v_nxt[r] = 0.f;
+            if (j0 + r < n_items && lane < n) {
+                c_nxt[r] = ld_stream(column_indices + b + lane);
+                v_nxt[r] = ld_stream(values + b + lane);
+            }
         }
-        const int cnt = min(L, end - base);
-        float mine = 0.f;
-        int *my_stage = stage + stage_buf * 32 + (lane - l);  // this group's region of the buffer
-        my_stage[l] = c;
-        __syncwarp(gmask);
-        stage_buf ^= 1;
+    };
+    fetch(0);
+#pragma unroll 1
+    for (int j0 = 0; j0 < n_items; j0 += G) {
+        const int j = (j0 + g) & 31;
+        const int my_row = __shfl_sync(kFull, row, j);
+        int my_len = __shfl_sync(kFull, len, j);
+        if (j0 + g >= n_items) my_len = 0;
+        const int longest = __reduce_max_sync(kFull, my_len);
+        float val[G];
 #pragma unroll
-        for (int b = 0; b < L / kBatch; ++b) {
-            if (b * kBatch < cnt) {  // uniform inside the group
+        for (int r = 0; r < G; ++r) {
+            s_col[at(r, lane / 4) + lane % 4] = c_nxt[r];
+            val[r] = v_nxt[r];
+        }
+        __syncwarp();
+        if (j0 + G < n_items) fetch(j0 + G);
+        float4 a[VPL];
+#pragma unroll
+        for (int v = 0; v < VPL; ++v)
+            a[v] = my_len > 0 && inside(v) ? __ldg(reinterpret_cast<const float4 *>(lhs) + static_cast<size_t>(my_row) * row_vecs + v * L + l)
+                                           : make_float4(0.f, 0.f, 0.f, 0.f);
+        constexpr int kQuad = kBatch < 4 ? 4 : kBatch;  // columns read at a time
+#pragma unroll 1
+        for (int t0 = 0; t0 < longest; t0 += kQuad) {
+            int cc[kQuad];
+#pragma unroll
+            for (int x = 0; x < kQuad; x += 4) {
+                int quad[4];
+                ld_shared_run<4>(s_col + at(g, (t0 + x) / 4), quad);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) cc[x + u] = quad[u];
+            }
+#pragma unroll
+            for (int x = 0; x < kQuad; x += kBatch) {
+                if (x > 0 && t0 + x >= longest) break;  // warp-uniform
                 float4 bb[kBatch][VPL];
-                int cc[kBatch];
-                ld_shared_run<kBatch>(my_stage + b * kBatch, cc);
 #pragma unroll
                 for (int u = 0; u < kBatch; ++u) {
-                    const int t = b * kBatch + u;
 #pragma unroll
                     for (int v = 0; v < VPL; ++v) {
                         bb[u][v] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (t < cnt && inside(v))
-                            bb[u][v] = ld_dense(rhs_row<kRagged && VPL < 4>(rhs_lane, cc[u], row_vecs) + v * L);
+                        if (t0 + x + u < my_len && inside(v))
+                            bb[u][v] = ld_dense(rhs_row<kRagged && VPL < 4>(rhs_lane, cc[x + u], row_vecs) + v * L);
                     }
                 }
                 float p[kBatch];
@@ -165,12 +186,18 @@ __device__ __forceinline__ void sddmm_one_row(int row, int begin, int end, int l
                     for (int v = 0; v < VPL; ++v) d = dot4(a[v], bb[u][v], d);
                     p[u] = d;
                 }
-                const float r = reduce_batch<L, kBatch>(p, l, gmask);
-                const float got = (L == kBatch) ? r : __shfl_sync(gmask, r, (l & (kBatch - 1)) * (L / kBatch), L);
-                if ((l / kBatch) == b) mine = got;
+                // nonzero u of the batch sits in lanes u * (L / kBatch) ..
+                const float r = reduce_batch<L, kBatch>(p, l, kFull);
+                if (l % (L / kBatch) == 0) s_dot[g * 32 + t0 + x + l / (L / kBatch)] = r;
             }
         }
-        if (base + l < end) st_stream(out + base + l, val * mine);
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < G; ++r) {
+            const int b = __shfl_sync(kFull, begin, (j0 + r) & 31), n = __shfl_sync(kFull, len, (j0 + r) & 31);
+            if (j0 + r < n_items && lane < n) st_stream(out + b + lane, val[r] * s_dot[r * 32 + lane]);
+        }
+        __syncwarp();
     }
 }
 
@@ -344,9 +371,12 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
     const size_t row_vecs = kRagged ? static_cast<size_t>(row_vecs_arg) : L * VPL;  // float4 per dense row (K / 4)
     constexpr int kAlign = 4;             // vec_len of the preprocessing
     constexpr int kBlockK = 32;           // k_block of the preprocessing
-    __shared__ int s_end[32];             // stream position where item j ends
-    __shared__ int s_row[32];             // row of item j
-    __shared__ __align__(16) int s_col[2][32];  // column indices of the current chunk, two buffers
+    // the stream's tables, or the row mode's columns and dot products
+    constexpr int kRowWords = LB > 0 ? 2 * 32 / (LB > 0 ? LB : 1) * 32 : 0;
+    __shared__ __align__(16) int s_words[kRowWords > 128 ? kRowWords : 128];
+    int *const s_end = s_words;           // stream position where item j ends
+    int *const s_row = s_words + 32;      // row of item j
+    int *const s_col = s_words + 64;      // column indices of the current chunk, two buffers
     int stage_buf = 0;
     const int lane = threadIdx.x;
     const int g = lane / L, l = lane % L;
@@ -384,10 +414,8 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
         if (lane >= d) start += up;
     }
     const int total = __shfl_sync(kFull, start, 31);
-    s_end[lane] = start;  // inclusive sum = end position
-    s_row[lane] = row;
+    const int stop = start;  // inclusive sum = end position
     start -= len;
-    const unsigned nonempty = __ballot_sync(kFull, len > 0);
     if (total == 0) return;
     if constexpr (LB > 0 && !kSegments) {
         static_assert(LB * VPLB == L * VPL || kRagged, "both lane-group shapes must cover the same dense row");
@@ -412,21 +440,13 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
                              (items_per_warp >= 32 / LB && __reduce_max_sync(kFull, len) * items_per_warp <= 2 * total);
             }
         }
-        if (one_by_one) {
-            constexpr int GB = 32 / LB;
-            const int gb = lane / LB;
-            for (int j0 = 0; j0 < items_per_warp; j0 += GB) {
-                const int j = j0 + gb;  // items_per_warp <= 32, a multiple of GB or the tail is empty
-                const int r = __shfl_sync(kFull, row, j & 31);
-                const int b0 = __shfl_sync(kFull, begin, j & 31);
-                const int n0 = __shfl_sync(kFull, len, j & 31);
-                if (j < items_per_warp && n0 > 0)
-                    sddmm_one_row<LB, VPLB, UB, kRagged>(
-                        r, b0, b0 + n0, lane, row_vecs_arg, column_indices, values, lhs, rhs, out, &s_col[0][0], stage_buf);
-            }
-            return;
-        }
+        if (one_by_one)
+            return sddmm_rows_one_by_one<LB, VPLB, UB, kRagged>(items_per_warp, row, begin, len, lane, row_vecs_arg, column_indices,
+                                                                values, lhs, rhs, out, s_words);
     }
+    s_end[lane] = stop;
+    s_row[lane] = row;
+    const unsigned nonempty = __ballot_sync(kFull, len > 0);
     __syncwarp();
 
     // ---- this group's contiguous part of the stream: [p0, p1) ----------------------------------
@@ -498,7 +518,7 @@ sddmm_items(int n_items, int items_per_warp, const int *__restrict__ item_rows, 
         fetch(p0 + (ch + 2) * L + l, e_pre, c_pre, v_pre);
         const int cnt = min(L, p1 - (p0 + ch * L));  // valid nonzeros of this chunk (may be <= 0)
         float mine = 0.f;
-        int *my_stage = &s_col[stage_buf][lane - l];  // this group's region of the chunk buffer
+        int *my_stage = s_col + stage_buf * 32 + lane - l;  // this group's region of the chunk buffer
         my_stage[l] = c_cur;
         __syncwarp();  // every group runs the same number of chunks
         stage_buf ^= 1;
