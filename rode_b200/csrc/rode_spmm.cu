@@ -1393,14 +1393,23 @@ int spmm(int m1, int m2, int k, int n, const T *values, const int *col, const in
         if (aligned_to(B, 32) && aligned_to(C, 32)) return RODE_LAUNCH(Tile512, Aligned128, true, false);
         return RODE_LAUNCH(Tile512, Rows128, true, false);
     }
+    // Matrices without segments whose rows are not short take the 256-byte tile's row kernel, in two or more passes, in the place of
+    // the stream of spmm_rows: the passes read the pairs again, but four rows run side by side and wait for dense rows only.  us,
+    // stream / 256-byte tiles, N = 128: stencil 128^3 1415 / 1257, 61^3 193 / 156, rows of 15 to 24 271 / 198, of 0 to 27 211 / 177, of 4 to 8
+    // 223 / 186, of 4 to 6 195 / 172, of 2 to 6 165 / 160, of 0 to 4 231 / 246; fp64 N = 64 stencil 128^3 1705 / 1351, rows of 15 to 24
+    // 308 / 220, of 0 to 4 231 / 258.  Ragged widths idle lanes in the last tile of either, and need longer rows: stencil 61^3
+    // N = 68 191 / 139, N = 100 197 / 163, N = 132 340 / 217, N = 200 344 / 297; rows of 0 to 27 145 / 162, 180 / 211, 349 / 305, 426 / 403.
+    const bool long_rows_only = m1 == 0 && rows_hold(nnz, 0, m2, vecs % 32 == 0 ? 5 : 20);
     // Widths the tiles do not divide (any other multiple of 4 columns; the reference has none of them): the narrowest
     // shape that covers the row, or 512-byte tiles with a partly empty last one.  No popularity hints.
     if (vecs % 8 != 0) {
         if (vecs < 8) return RODE_LAUNCH(Block128, Rows128, true);
         if (vecs < 16) return RODE_LAUNCH(Tile256, Tile256, true);
+        if (long_rows_only) return RODE_LAUNCH(Tile512, Tile256, true);
         return RODE_LAUNCH(Tile512, Tile512, true);
     }
     // (32-byte loads measured no faster than 16-byte ones in the wider tiles: the gathers are bound by bytes through L1 and L2)
+    if (vecs % 32 == 0 && long_rows_only) return RODE_LAUNCH(Tile512, Tile256);
     if (vecs % 32 == 0) return RODE_LAUNCH(Tile512, Tile512);
     if (vecs % 16 == 0) return RODE_LAUNCH(Tile256, Tile256);
     if (aligned32) return RODE_LAUNCH(Aligned128, Aligned128);

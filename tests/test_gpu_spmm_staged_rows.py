@@ -28,11 +28,11 @@ def test_rows_against_fp64(m, long_rows, dtype):
     val = A.val.to(dtype)
     sparse = torch.sparse_csr_tensor(A.row_ptr.long(), A.col.long(), val.double(), size=(A.m, A.n))
     size = 4 if dtype == torch.float32 else 8
-    for n in (4, 16, 128 // size, 36, 256 // size, 96):
+    for n in (4, 16, 128 // size, 36, 256 // size, 96, 512 // size, 1024 // size):  # (512 bytes and more: the 256-byte tile's kernel)
         B = W.dense(A.n, n, device="cuda", seed=n, dtype=dtype)
         out = []
         nodes = graph_nodes(lambda: out.append(capi.spmm(meta, A.row_ptr, A.col, val, B)))
-        if n * size <= 256:
+        if n * size <= 256 or (long_rows == 0 and n * size % 512 == 0):
             assert any("spmm_rows_simple" in k for k in nodes), nodes
         C = capi.spmm(meta, A.row_ptr, A.col, val, B)
         want = sparse @ B.double()
