@@ -83,10 +83,10 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, int, int> py_preprocess(
     return std::make_tuple(blk.contiguous(), st.contiguous(), res.contiguous(), n_blk, n_res);
 }
 
-torch::Tensor py_sddmm_forward(torch::Tensor block_indices, torch::Tensor residue_indices, torch::Tensor st_offsets,
-                                 int m1, int m2, torch::Tensor row_offsets, torch::Tensor column_indices,
-                                 torch::Tensor values, int m, int n, torch::Tensor lhs_matrix,
-                                 torch::Tensor rhs_matrix, int k_version, bool covers_values, bool ordered) {
+torch::Tensor py_sddmm_forward(const torch::Tensor &block_indices, const torch::Tensor &residue_indices,
+                                 const torch::Tensor &st_offsets, int m1, int m2, const torch::Tensor &row_offsets, const torch::Tensor &column_indices,
+                                 const torch::Tensor &values, int m, int n, const torch::Tensor &lhs_matrix,
+                                 const torch::Tensor &rhs_matrix, int k_version, bool covers_values, bool ordered) {
     RODE_CHECK_INPUT(block_indices);
     RODE_CHECK_INPUT(residue_indices);
     RODE_CHECK_INPUT(st_offsets);
@@ -135,7 +135,8 @@ torch::Tensor py_sddmm_forward(torch::Tensor block_indices, torch::Tensor residu
 }
 
 // What rode_order_verdict says of the columns, -1 where the sizes are out of its range.  Reads the verdict back.
-int py_order_verdict(torch::Tensor block_indices, int m1, torch::Tensor row_offsets, torch::Tensor column_indices, int n) {
+int py_order_verdict(const torch::Tensor &block_indices, int m1, const torch::Tensor &row_offsets,
+                     const torch::Tensor &column_indices, int n) {
     RODE_CHECK_INPUT(block_indices);
     RODE_CHECK_INPUT(row_offsets);
     RODE_CHECK_INPUT(column_indices);
@@ -156,7 +157,7 @@ int py_order_verdict(torch::Tensor block_indices, int m1, torch::Tensor row_offs
 
 // Popularity bitmap of the columns for spmm_forward's `hot_columns` argument (rode_hot_columns),
 // or None when the library finds that marks would not help.  Reads the flag word back.
-c10::optional<torch::Tensor> py_hot_columns(torch::Tensor column_indices, int n_cols, int64_t dense_row_bytes,
+c10::optional<torch::Tensor> py_hot_columns(const torch::Tensor &column_indices, int n_cols, int64_t dense_row_bytes,
                                             int64_t budget_bytes) {
     RODE_CHECK_INPUT(column_indices);
     RODE_CHECK_INT(column_indices);
@@ -178,10 +179,10 @@ c10::optional<torch::Tensor> py_hot_columns(torch::Tensor column_indices, int n_
     return bitmap;
 }
 
-torch::Tensor py_spmm_forward(torch::Tensor block_indices, torch::Tensor residue_indices, torch::Tensor st_offsets,
-                                int m1, int m2, torch::Tensor row_offsets, torch::Tensor column_indices,
-                                torch::Tensor values, int m, int k, torch::Tensor dense,
-                                c10::optional<torch::Tensor> hot_columns, bool ordered) {
+torch::Tensor py_spmm_forward(const torch::Tensor &block_indices, const torch::Tensor &residue_indices,
+                                const torch::Tensor &st_offsets, int m1, int m2, const torch::Tensor &row_offsets, const torch::Tensor &column_indices,
+                                const torch::Tensor &values, int m, int k, const torch::Tensor &dense,
+                                const c10::optional<torch::Tensor> &hot_columns, bool ordered) {
     RODE_CHECK_INPUT(block_indices);
     RODE_CHECK_INPUT(residue_indices);
     RODE_CHECK_INPUT(st_offsets);
