@@ -959,7 +959,8 @@ int rode_sddmm_f32_ordered(int M, int m1, int m2, int n, int k, long long nnz, c
     using namespace rode;
     if (M < 0 || nnz < 0) return fail(RODE_ERR_INVALID_ARGUMENT, "sddmm: M, nnz must be >= 0");
     Ordering ord = {};
-    const bool ordered = workspace != nullptr && m1 > 0 && n > 0 && k > 0 && nnz > 0 && M < kPieceMaxRows;
+    // (the cuts of a segment are multiples of up to 64 beyond its ends)
+    const bool ordered = workspace != nullptr && m1 > 0 && n > 0 && k > 0 && nnz > 0 && nnz < INT_MAX - 256 && M < kPieceMaxRows;
     if (ordered) {
         const size_t need = piece_bytes(m1, nnz, (k + 3) / 4);
         if (workspace_bytes < need)
