@@ -1178,9 +1178,11 @@ int launch_shape(int m1, int m2, int k, int n, const T *values, const int *col, 
         const int resident_per_tile = resident / static_cast<int>(tiles <= kClaimTiles ? tiles : 1);
         const bool claims = counters != nullptr && claims_work<T>(n, tiles);
         const bool persistent = claims && !small_grid && ctas_needed > kPersistentMinWaves * resident_per_tile;
-        // in a chain the residue kernel's counters are zeroed here too: nothing may stand between two of its grids
+        // in a chain the residue kernel's counters are zeroed here too: nothing may stand between two of its grids.  On a stream
+        // of its own it may be at work already, and zeroes them itself
         counters_clear = claims && chained && m2 > 32LL * kPersistentMinWaves * resident_per_tile;
-        if (persistent || counters_clear) RODE_CUDA_TRY(cudaMemsetAsync(counters, 0, 2 * kClaimTiles * sizeof(int), s1));
+        if (persistent || counters_clear)
+            RODE_CUDA_TRY(cudaMemsetAsync(counters, 0, (counters_clear ? 2 : 1) * kClaimTiles * sizeof(int), s1));
         int *claim = persistent ? counters : nullptr;
         dim3 grid(persistent ? (resident + tiles - 1) / tiles : ctas_needed, tiles);
         bool launched = false;  // one of the special forms
