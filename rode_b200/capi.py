@@ -208,10 +208,13 @@ _NULL = contextlib.nullcontext()
 
 
 def _stream_object(s, dev: torch.device) -> torch.cuda.Stream:
-    """The stream of a torch stream, a raw handle, or None (torch's current one)."""
+    """The stream of a torch stream, a raw handle (0: the default stream), or None (torch's current one)."""
     if s is None:
         return torch.cuda.current_stream(dev)
-    return s if isinstance(s, torch.cuda.Stream) else torch.cuda.ExternalStream(int(s), device=dev)
+    if isinstance(s, torch.cuda.Stream):
+        return s
+    # (ExternalStream(0) would be a stream of torch's pool)
+    return torch.cuda.ExternalStream(int(s), device=dev) if int(s) else torch.cuda.default_stream(dev)
 
 
 def _current(dev: torch.device) -> int:
