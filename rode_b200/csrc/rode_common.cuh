@@ -318,7 +318,15 @@ __device__ __forceinline__ unsigned after_chain(unsigned i) {
     asm volatile("griddepcontrol.wait;" : "+r"(i)::"memory");
     return i;
 }
-// Loads of what the grids before this one have written, that stay behind a wait (__ldcg alone is not held back by one).
+// The same for a pointer to what the grids before this one write: loads through the result stay behind the wait.
+template <typename T>
+__device__ __forceinline__ const T *after_chain(const T *p) {
+    unsigned long long a = reinterpret_cast<unsigned long long>(p);
+    asm volatile("griddepcontrol.wait;" : "+l"(a)::"memory");
+    return reinterpret_cast<const T *>(a);
+}
+// Loads of what the grids before this one have written, that stay behind a wait (__ldcg alone, through a pointer that was known
+// before, is not held back by one).
 __device__ __forceinline__ int ld_behind_wait(const int *p) {
     int v;
     asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");

@@ -594,12 +594,12 @@ spmm_fixup(int m1, int segs_per_cta, int n, const int *__restrict__ row_offsets,
         // before spmm_block has completed and flushed its stores: whatever the caller enqueues
         // on the stream afterwards (an event, a copy of C, the next kernel) is then ordered
         // after the block grid through this grid, as with a plain launch.
-        if (blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (blockIdx.x == 0) chain_wait();
         return;
     }
     // Everything above read only the caller's metadata; the workspace is written by the
     // preceding spmm_block grid: wait for it (no-op when launched without the attribute).
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const T *const finished = after_chain(partial);
 
     // `width` lanes cover a row of up to 32 vectors; narrower rows leave 32 / width groups of lanes that
     // take alternate slots and are combined by shuffles.
@@ -620,7 +620,7 @@ spmm_fixup(int m1, int segs_per_cta, int n, const int *__restrict__ row_offsets,
         st_stream(reinterpret_cast<V *>(C) + static_cast<size_t>(row) * row_vecs + x, *reinterpret_cast<const V *>(e));
     };
     for (int i = warp; i < narrow; i += kFixupWarps) {
-        const V *slots = reinterpret_cast<const V *>(partial) + static_cast<size_t>(s_first[i]) * row_vecs;
+        const V *slots = reinterpret_cast<const V *>(finished) + static_cast<size_t>(s_first[i]) * row_vecs;
         const int row = s_row[i], cnt = s_cnt[i];
         for (int x0 = 0; x0 < row_vecs; x0 += 32) {
             const int x = x0 + l;
@@ -632,7 +632,7 @@ spmm_fixup(int m1, int segs_per_cta, int n, const int *__restrict__ row_offsets,
     }
     for (int i = 0; i < wide; ++i) {
         const int at = kFixupThreads - 1 - i;
-        const V *slots = reinterpret_cast<const V *>(partial) + static_cast<size_t>(s_first[at]) * row_vecs;
+        const V *slots = reinterpret_cast<const V *>(finished) + static_cast<size_t>(s_first[at]) * row_vecs;
         const int row = s_row[at], cnt = s_cnt[at];
         for (int x0 = 0; x0 < row_vecs; x0 += 32) {
             const int x = x0 + l;
