@@ -29,7 +29,8 @@ constexpr int kOrderPerThread = 8;   // pieces a thread holds per round (1 where
 struct OrderHead {
     int counts[kOrderBuckets];  // pieces per bucket
     int used[kOrderBuckets];    // of them already placed in the list
-    int claim[64];              // claim counter of the kernel that works through the list
+    int claim;                  // claim counter of the kernel that works through the list
+    int unused[63];             // (the list starts on a 256-byte boundary of the head)
 };
 
 // A piece: some consecutive nonzeros of one row, packed into 64 bits.
@@ -94,58 +95,6 @@ size_t ordering_bytes(long long m1, long long nnz) {
 // columns far more often than the S^2 / 2n times of uniform ones, on R-MAT graphs of scale 18 to 21 50 to 150 times as often,
 // whatever the numbering of the columns.
 enum { kOrderHelps = 0, kOrderSkewed = 1, kOrderLocal = 2 };
-constexpr int kJudgeThreads = 1024;
-constexpr int kJudgeSamples = 4 * kJudgeThreads;
-constexpr int kJudgeSlots = 2 * kJudgeSamples;
-static __global__ void __launch_bounds__(kJudgeThreads)
-judge_columns(int m1, int n_cols, long long nnz, const int *__restrict__ row_offsets,
-              const int *__restrict__ column_indices, const int *__restrict__ block_r_ind, int *__restrict__ verdict) {
-    __shared__ int s_slot[kJudgeSlots];
-    __shared__ int s_repeats;
-    __shared__ float s_span[kJudgeThreads / 32];
-    const int t = threadIdx.x;
-    int c[kJudgeSamples / kJudgeThreads];
-    const int row = __ldg(block_r_ind + static_cast<int>(static_cast<long long>(t) * m1 / kJudgeThreads));
-    const int begin = __ldg(row_offsets + row), end = __ldg(row_offsets + row + 1);
-#pragma unroll
-    for (int i = 0; i < kJudgeSamples / kJudgeThreads; ++i)
-        c[i] = __ldg(column_indices + (static_cast<long long>(i) * kJudgeThreads + t) * nnz / kJudgeSamples);
-    float span = 0.f;
-    if (end > begin) span = fabsf(static_cast<float>(__ldg(column_indices + end - 1)) - static_cast<float>(__ldg(column_indices + begin)));
-    for (int i = t; i < kJudgeSlots; i += kJudgeThreads) s_slot[i] = -1;
-    if (t == 0) s_repeats = 0;
-    __syncthreads();
-    int repeats = 0;
-#pragma unroll
-    for (int i = 0; i < kJudgeSamples / kJudgeThreads; ++i) {
-        int at = static_cast<int>(static_cast<unsigned>(c[i]) * 2654435761u / (0x100000000ull / kJudgeSlots));
-        while (true) {  // ends: there are fewer samples than slots
-            const int old = atomicCAS(&s_slot[at], -1, c[i]);
-            if (old == -1) break;
-            if (old == c[i]) {
-                ++repeats;
-                break;
-            }
-            at = (at + 1) % kJudgeSlots;
-        }
-    }
-    repeats = __reduce_add_sync(0xffffffffu, repeats);
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) span += __shfl_xor_sync(0xffffffffu, span, d);
-    if (t % 32 == 0) {
-        atomicAdd(&s_repeats, repeats);
-        s_span[t / 32] = span;
-    }
-    __syncthreads();
-    if (t == 0) {
-        float sum = 0.f;
-        for (int w = 0; w < kJudgeThreads / 32; ++w) sum += s_span[w];
-        const float uniform = 0.5f * kJudgeSamples * kJudgeSamples / n_cols;
-        const bool skewed = s_repeats > 8.f * uniform + 16.f;
-        const bool local = sum / kJudgeThreads < n_cols / 32.f;
-        *verdict = local ? kOrderLocal : skewed ? kOrderSkewed : kOrderHelps;
-    }
-}
 
 // One CTA takes 256 consecutive segments, their pieces in rounds of 2048.  kPlace = false counts the pieces of each bucket,
 // kPlace = true puts them into the list, bucket after bucket; inside a bucket they stand in any order.  capacity: entries that the
