@@ -89,9 +89,9 @@ size_t ordering_bytes(long long m1, long long nnz) {
 }
 
 #ifdef __CUDACC__
-// What keeps an order by columns from helping, judged from samples at even distances.  kOrderLocal: rows are narrow bands already
+// What keeps an order by columns from helping, judged from 4096 samples of the nonzeros.  kOrderLocal: rows are narrow bands already
 // (1024 rows span less than a thirtieth of the columns on average).  kOrderSkewed: a few columns get most of the references, and
-// their rows stay in the L2 in any order (R-MAT 21 K = 64 block 457 us row by row, 486 ordered); 4096 nonzeros then repeat
+// their rows stay in the L2 in any order (R-MAT 21 K = 64 block 457 us row by row, 486 ordered); the samples then repeat
 // columns far more often than the S^2 / 2n times of uniform ones, on R-MAT graphs of scale 18 to 21 50 to 150 times as often,
 // whatever the numbering of the columns.
 enum { kOrderHelps = 0, kOrderSkewed = 1, kOrderLocal = 2 };

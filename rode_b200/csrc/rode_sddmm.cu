@@ -925,8 +925,14 @@ judge_columns(int m1, int n_cols, long long nnz, const int *__restrict__ row_off
     const int row = __ldg(block_r_ind + static_cast<int>(static_cast<long long>(t) * m1 / kJudgeThreads));
     const int begin = __ldg(row_offsets + row), end = __ldg(row_offsets + row + 1);
 #pragma unroll
-    for (int i = 0; i < kJudgeSamples / kJudgeThreads; ++i)
-        c[i] = __ldg(column_indices + (static_cast<long long>(i) * kJudgeThreads + t) * nnz / kJudgeSamples);
+    for (int i = 0; i < kJudgeSamples / kJudgeThreads; ++i) {
+        const unsigned at = static_cast<unsigned>(i * kJudgeThreads + t);
+        // (somewhere in the sample's share of the nonzeros: at even distances rows of equal length would be asked at the
+        // same place, where ascending columns repeat without being popular)
+        const unsigned within = (at * 2654435761u) >> 16;
+        c[i] = __ldg(column_indices + ((static_cast<long long>(at) << 16) + within) * nnz /
+                                          (static_cast<long long>(kJudgeSamples) << 16));
+    }
     float span = 0.f;
     if (end > begin) span = fabsf(static_cast<float>(__ldg(column_indices + end - 1)) - static_cast<float>(__ldg(column_indices + begin)));
     for (int i = t; i < kJudgeSlots; i += kJudgeThreads) s_slot[i] = -1;

@@ -1,0 +1,26 @@
+"""Which matrices an order of the segments by their columns is taken for: the samples that the verdict rests on, and the lines
+of rode_spmm_order_pays and rode_sddmm_order_pays between matrices on which both sides were timed."""
+import pytest
+import torch
+
+from rode_b200 import capi
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows_of(length, rows, n, seed=1):
+    """Rows of one length with uniform columns, ascending."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    col = torch.randint(0, n, (rows, length), generator=g, device="cuda", dtype=torch.int32).sort(1).values
+    row_ptr = (torch.arange(rows + 1, device="cuda") * length).to(torch.int32)
+    meta = capi.preprocess(row_ptr, col.numel())
+    col = col.reshape(-1).contiguous()
+    return meta, col.numel(), capi.order_verdict(meta, row_ptr, col, n)
+
+
+@pytest.mark.parametrize("length", [1000, 1024, 1536])
+def test_rows_as_long_as_the_distance_of_the_samples_are_not_skewed(length):
+    n = 1 << 20
+    meta, nnz, verdict = _rows_of(length, 8192, n)
+    assert capi.spmm_order_pays(verdict, meta.m1, n, 96, nnz)  # (skewed columns take no order at this width)
