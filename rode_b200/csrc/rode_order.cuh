@@ -20,7 +20,7 @@ namespace rode {
 // Below so many segments an order does not pay for itself, below so many columns the dense operand fits the L2 at any width in
 // use (1 KB per row: 160 MB).
 constexpr int kOrderMinSegments = 1 << 13;
-constexpr int kOrderLongRows = 330;  // nonzeros of the matrix per segment: most are in rows of many (512-long) segments
+constexpr int kOrderLongRows = 330;  // SDDMM: nonzeros of the matrix per segment, most are in rows of many (512-long) segments
 constexpr int kOrderMinColumns = 160 << 10;
 constexpr int kOrderBuckets = 256;   // one per thread of an ordering CTA
 constexpr int kOrderThreads = kOrderBuckets;
@@ -94,7 +94,10 @@ size_t ordering_bytes(long long m1, long long nnz) {
 // their rows stay in the L2 in any order (R-MAT 21 K = 64 block 457 us row by row, 486 ordered); the samples then repeat
 // columns far more often than the S^2 / 2n times of uniform ones, on R-MAT graphs of scale 18 to 21 50 to 150 times as often,
 // whatever the numbering of the columns.
-enum { kOrderHelps = 0, kOrderSkewed = 1, kOrderLocal = 2 };
+//
+// How much of the columns a segment spans (a row's span over the number of its segments, 1024 samples) is what whole segments in
+// order depend on, and goes with it: kOrderNarrow: less than three quarters on average; kOrderWide: more than nine tenths.
+enum { kOrderHelps = 0, kOrderSkewed = 1, kOrderLocal = 2, kOrderKind = 3, kOrderNarrow = 4, kOrderWide = 8 };
 
 // One CTA takes 256 consecutive segments, their pieces in rounds of 2048.  kPlace = false counts the pieces of each bucket,
 // kPlace = true puts them into the list, bucket after bucket; inside a bucket they stand in any order.  capacity: entries that the

@@ -786,8 +786,8 @@ constexpr int piece_len(int row_vecs) { return row_vecs <= 16 ? 64 : 32; }
 // Pareto 394 / 355; 10,953 segments Zipf of mean 16 K = 64 159 / 156, K = 96 265 / 241.  Bands: 1M rows of 60 in 3000 columns K = 128 1775 / 1921.
 bool order_pays(int verdict, long long M, long long m1, long long n, int k, long long nnz) {
     const bool enough = m1 >= 1 << 15 || (k > 64 && m1 >= kOrderMinSegments && nnz >= kOrderLongRows * m1);
-    return M < kPieceMaxRows && enough && n * k * 4 >= (k > 96 ? 128ll << 20 : 160ll << 20) &&
-           (verdict == kOrderHelps || (verdict == kOrderSkewed && k > 96));
+    return verdict >= 0 && M < kPieceMaxRows && enough && n * k * 4 >= (k > 96 ? 128ll << 20 : 160ll << 20) &&
+           ((verdict & kOrderKind) == kOrderHelps || ((verdict & kOrderKind) == kOrderSkewed && k > 96));
 }
 // The block segments through sddmm_pieces.
 template <int L, int VPL, int U>
@@ -919,10 +919,16 @@ judge_columns(int m1, int n_cols, long long nnz, const int *__restrict__ row_off
               const int *__restrict__ column_indices, const int *__restrict__ block_r_ind, int *__restrict__ verdict) {
     __shared__ int s_slot[kJudgeSlots];
     __shared__ int s_repeats;
-    __shared__ float s_span[kJudgeThreads / 32];
+    __shared__ float s_span[kJudgeThreads / 32], s_seg_span[kJudgeThreads / 32];
     const int t = threadIdx.x;
     int c[kJudgeSamples / kJudgeThreads];
-    const int row = __ldg(block_r_ind + static_cast<int>(static_cast<long long>(t) * m1 / kJudgeThreads));
+    const int seg = static_cast<int>(static_cast<long long>(t) * m1 / kJudgeThreads);
+    const int row = __ldg(block_r_ind + seg);
+    // segments of the row, up to two on either side of this one: from five on it is narrow enough
+    int segs = 1;
+#pragma unroll
+    for (int d = -2; d <= 2; ++d)
+        if (d != 0 && seg + d >= 0 && seg + d < m1 && __ldg(block_r_ind + seg + d) == row) ++segs;
     const int begin = __ldg(row_offsets + row), end = __ldg(row_offsets + row + 1);
 #pragma unroll
     for (int i = 0; i < kJudgeSamples / kJudgeThreads; ++i) {
@@ -953,20 +959,30 @@ judge_columns(int m1, int n_cols, long long nnz, const int *__restrict__ row_off
         }
     }
     repeats = __reduce_add_sync(0xffffffffu, repeats);
+    float seg_span = span / static_cast<float>(segs);
 #pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) span += __shfl_xor_sync(0xffffffffu, span, d);
+    for (int d = 16; d >= 1; d >>= 1) {
+        span += __shfl_xor_sync(0xffffffffu, span, d);
+        seg_span += __shfl_xor_sync(0xffffffffu, seg_span, d);
+    }
     if (t % 32 == 0) {
         atomicAdd(&s_repeats, repeats);
         s_span[t / 32] = span;
+        s_seg_span[t / 32] = seg_span;
     }
     __syncthreads();
     if (t == 0) {
-        float sum = 0.f;
-        for (int w = 0; w < kJudgeThreads / 32; ++w) sum += s_span[w];
+        float sum = 0.f, seg_sum = 0.f;
+        for (int w = 0; w < kJudgeThreads / 32; ++w) {
+            sum += s_span[w];
+            seg_sum += s_seg_span[w];
+        }
+        const float of_columns = seg_sum / (static_cast<float>(kJudgeThreads) * n_cols);
         const float uniform = 0.5f * kJudgeSamples * kJudgeSamples / n_cols;
         const bool skewed = s_repeats > 8.f * uniform + 16.f;
         const bool local = sum / kJudgeThreads < n_cols / 32.f;
-        *verdict = local ? kOrderLocal : skewed ? kOrderSkewed : kOrderHelps;
+        *verdict = (local ? kOrderLocal : skewed ? kOrderSkewed : kOrderHelps) |
+                   (of_columns < 0.75f ? kOrderNarrow : of_columns > 0.9f ? kOrderWide : 0);
     }
 }
 

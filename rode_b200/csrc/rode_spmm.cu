@@ -1132,21 +1132,41 @@ spmm_rows_wide(int m2, int n, const T *__restrict__ values, const int *__restric
 }
 
 // When an order of the segments pays (rode_order.cuh): from an operand beyond the L2 on, on skewed columns for the 256- and 512-byte
-// tiles of float only.  Whole calls, row by row / ordered, us.  Zipf 671,008 x 929,297 of mean 40 N = 32 (113 MB) 329 / 282, N = 64 830 /
-// 510, N = 128 1750 / 934, fp64 N = 64 1750 / 981; Zipf 2^20 of mean 8 N = 64 353 / 290; Pareto 2^20 of mean 32 N = 32 (128 MB) 517 / 509,
-// N = 64 1104 / 1006, N = 256 4579 / 4126, of mean 16 N = 64 640 / 599, of mean 8 N = 64 390 / 386, N = 128 675 / 677; 2^22 of mean 8
-// N = 32 1023 / 1039, N = 128 2841 / 2820.  R-MAT 23, 22, 21, 20 N = 64 3299 / 3112, 1485 / 1414, 697 / 687, 353 / 345, but N = 32 863 / 876
-// (22), fp64 N = 32 785 / 832 (21).  R-MAT N = 128 with popularity hints / ordered, calls back to back under the power cap: scale 23
-// 5862 / 5728, 22 2690 / 2669 (in short bursts 2268 / 2364), 21 1269 / 1254, of 32 per row 2295 / 2157, 20 of 64 1957 / 1792, 19 286 / 286; N = 256
-// 2576 / 2474; 22 of 6 per row 1280 / 1311; and the first call on a matrix, which builds no bitmap then, scale 23 6257 / 5000, 21 1687 / 1152.
+// tiles of float only.  Whole calls, row by row / ordered, us.
 //
-// The more of the nonzeros are in rows of many segments, the more an order gives: Zipf matrices have 370 to 410 nonzeros per segment,
-// Pareto 170 to 310, where it takes more references per column and a larger grid (2^22 rows of mean 8 above; 262,144 x 2^20 of mean
-// 16, 19,043 segments, N = 128 331 / 333; Zipf of the same size, 10,953 segments, 316 / 284).
+// What it gives is a matter of how much of the columns a segment spans.  N = 64, 2^20 columns (256 MB): Zipf of mean 16 (segments
+// span 0.46 of the columns on average) 598 / 395, log-normal lengths of sigma 3 (0.70) 640 / 494, Pareto of mean 32 (0.86) 1063 / 912, of
+// mean 16 603 / 546; 2^21 columns: log-normal of sigma 1 (0.96), mean 16 and 32, 1273 / 1538 and 2435 / 3018, Pareto of shape 2
+// (0.95) 2401 / 2986.  Segments that are rows of one length (span 0.99; three segments: 0.33): rows of 256, 400, 500 N = 128
+// 662 / 678, 523 / 540, 478 / 505, N = 256 1395 / 1428, 1136 / 1181, 980 / 1083, N = 32 401 / 415, 388 / 396, 370 / 380, rows of
+// 1500 N = 128 523 / 371.  So wide segments keep the order of the rows, except short ones in grids that are not too large (up
+// to 2^17 of less than 192 nonzeros: rows of 160 N = 128 803 / 802, of 96 824 / 828, log-normal of sigma 2 1212 / 1203); narrow ones
+// are ordered from 8192 on (Pareto of shape 0.8 and mean 4, 11,607 segments, N = 128 418 / 406; rows of 600, 13,980 segments, 250 /
+// 172), and those between them where there are more segments and references per column (Pareto of mean 8, 31,336 segments,
+// N = 128 673 / 675, 2^22 of mean 8 N = 32 1023 / 1039, N = 128 2841 / 2820).
+//
+// In the 256-byte tile of float the ordered form is the faster one whatever the segments
+// span, up to 2^17 of them and from 4 references per column on (rows of 256, 400, 500 N = 64 323 / 308, 275 / 264, 273 / 258, Pareto of
+// mean 4 and 8 243 / 230, 366 / 344, of mean 4 N = 48 232 / 224; of 2 references per column rows of 96, 160 N = 64 73 / 77, 74 / 77).
+//
+// Skewed columns, against the popularity hints at N = 128 and 256 and without at 64: R-MAT 23, 22, 21, 20 N = 64 3136 / 2764, 1441 / 1326,
+// 693 / 668, 355 / 334, but N = 32 863 / 876 (22), fp64 N = 32 785 / 832 (21); N = 128, calls one by one 5072 / 4900, 2275 / 2224, 1081 / 1064,
+// 531 / 522 (19: 271 / 275), back to back under the power cap 5879 / 5799, 2743 / 2677, 1266 / 1253, 605 / 581, between GEMMs 5800 / 5671, 2643 /
+// 2595, 1221 / 1222, 581 / 570; with rows and columns in random order 5132 / 5019, 2284 / 2225, 1070 / 1045, 532 / 503; of 32 per row (21)
+// 1900 / 1807, 20 of 64 1635 / 1543, N = 256 (22) 4837 / 4560; 22 of 6 per row 1119 / 1136, which the references per column leave out.
+// Columns skewed by themselves (Pareto 2^21 of mean 16, columns repeat 13, 81, 334 times as often as uniform ones) N = 64 1124 /
+// 1097, 977 / 947, 781 / 742, but N = 128 2074 / 2087, 1681 / 1721, 1134 / 1201: there hints are better from some fifteen calls on,
+// for an ordered first call needs no bitmap (0.5 to 2 ms).
 bool order_pays(int verdict, long long m1, long long k, long long n, long long nnz, int elem_size) {
-    if (m1 < kOrderMinSegments || k * n * elem_size < 160ll << 20) return false;
-    if (nnz < kOrderLongRows * m1 && (m1 < 1 << 15 || nnz < 12 * k)) return false;
-    return verdict == kOrderHelps || (verdict == kOrderSkewed && elem_size == 4 && (n == 64 || n % 128 == 0));
+    if (verdict < 0 || m1 < kOrderMinSegments || k * n * elem_size < 160ll << 20) return false;
+    const int kind = verdict & kOrderKind;
+    const long long row_bytes = n * elem_size;
+    const bool moderate = m1 <= 1 << 17 && row_bytes > 128;
+    const bool narrow_tile = moderate && elem_size == 4 && row_bytes <= 256 && kind == kOrderHelps && nnz >= 4 * k;
+    if ((verdict & kOrderWide) != 0 && !narrow_tile && !(moderate && nnz < 192 * m1)) return false;
+    const bool narrow = (verdict & kOrderNarrow) != 0 && kind == kOrderHelps;
+    if (!narrow && !narrow_tile && (m1 < 1 << 15 || nnz < 12 * k)) return false;
+    return kind == kOrderHelps || (kind == kOrderSkewed && elem_size == 4 && (n == 64 || n % 128 == 0));
 }
 
 template <typename T, int VB, int L, int VPL, bool kRagged>

@@ -24,3 +24,21 @@ def test_rows_as_long_as_the_distance_of_the_samples_are_not_skewed(length):
     n = 1 << 20
     meta, nnz, verdict = _rows_of(length, 8192, n)
     assert capi.spmm_order_pays(verdict, meta.m1, n, 96, nnz)  # (skewed columns take no order at this width)
+
+
+@pytest.mark.parametrize("length,rows,pays", [  # 256-byte and 512-byte rows
+    (256, 40000, (True, False)), (400, 30000, (True, False)), (500, 30000, (True, False)), (500, 9000, (True, False)),
+    (100, 200000, (False, False)), (160, 80000, (True, True)), (600, 7000, (True, True)), (1500, 4000, (True, True)),
+    (100, 20000, (False, False))])
+def test_spmm_orders_segments_that_span_little_of_the_columns(length, rows, pays):
+    n = 700_001
+    meta, nnz, verdict = _rows_of(length, rows, n)
+    assert tuple(capi.spmm_order_pays(verdict, meta.m1, n, width, nnz) for width in (64, 128)) == pays
+    assert not capi.spmm_order_pays(-1, meta.m1, n, 128, nnz)
+
+
+def test_spmm_of_128_byte_rows_orders_no_wide_segments():
+    meta, nnz, verdict = _rows_of(100, 200_000, 1_400_001)
+    assert not capi.spmm_order_pays(verdict, 100_000, 1_400_001, 32, nnz)
+    meta, nnz, verdict = _rows_of(3000, 8000, 1_400_001)
+    assert capi.spmm_order_pays(verdict, meta.m1, 1_400_001, 32, nnz)
