@@ -784,9 +784,16 @@ constexpr int piece_len(int row_vecs) { return row_vecs <= 16 ? 64 : 32; }
 // Uniform columns, us: K = 32 512 MB Pareto of mean 16 1912 / 1495, 128 MB 347 / 345 and of mean 8 228 / 241; K = 64 256 MB 1090 / 919
 // (mean 32), 364 / 368 (mean 8, 31,336 segments); Zipf 671,008 x 929,297 of mean 40 K = 64 800 / 517, K = 128 1797 / 942; K = 128 128 MB
 // Pareto 394 / 355; 10,953 segments Zipf of mean 16 K = 64 159 / 156, K = 96 265 / 241.  Bands: 1M rows of 60 in 3000 columns K = 128 1775 / 1921.
+//
+// An order also needs references to bring together (rows of one length, uniform columns, references per column, row by row / ordered): K = 32
+// 2 80 / 95 (rows of 64), 78 / 85 (of 128), 4 214 / 174, 145 / 136; K = 64 2 69 / 83 and 77 / 89 (of 40), 3 98 / 116 and 129 / 130, 4 129 /
+// 148 and 171 / 159, 6 207 / 212 (of 64), 8 248 / 214 (of 128); K = 96 2 128 / 138 (of 40), in long rows (of 2000; 8388 and 12,580
+// segments) 4 158 / 171, K = 80 4 150 / 169, 6 205 / 212, but Zipf of mean 4 and 8, K = 96, 370 / 349 and 581 / 445; K = 128 1 80 / 85 and 79 / 89 (of 64 and
+// 128), 2 157 / 139 (of 96); Pareto 2^21 K = 32 of mean 4 323 / 339, of 8 480 / 474, 2^20 K = 128 of mean 2 234 / 245, of 4 403 / 398.
 bool order_pays(int verdict, long long M, long long m1, long long n, int k, long long nnz) {
     const bool enough = m1 >= 1 << 15 || (k > 64 && m1 >= kOrderMinSegments && nnz >= kOrderLongRows * m1);
-    return verdict >= 0 && M < kPieceMaxRows && enough && n * k * 4 >= (k > 96 ? 128ll << 20 : 160ll << 20) &&
+    const bool shared = k > 96 ? nnz >= 2 * n : m1 < 1 << 15 ? nnz >= 6 * n : 2 * nnz >= 7 * n;
+    return verdict >= 0 && M < kPieceMaxRows && enough && shared && n * k * 4 >= (k > 96 ? 128ll << 20 : 160ll << 20) &&
            ((verdict & kOrderKind) == kOrderHelps || ((verdict & kOrderKind) == kOrderSkewed && k > 96));
 }
 // The block segments through sddmm_pieces.

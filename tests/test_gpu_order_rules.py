@@ -42,3 +42,15 @@ def test_spmm_of_128_byte_rows_orders_no_wide_segments():
     assert not capi.spmm_order_pays(verdict, 100_000, 1_400_001, 32, nnz)
     meta, nnz, verdict = _rows_of(3000, 8000, 1_400_001)
     assert capi.spmm_order_pays(verdict, meta.m1, 1_400_001, 32, nnz)
+
+
+@pytest.mark.parametrize("n,k,length,per_column,pays", [
+    (1_400_001, 32, 64, 2, False), (1_400_001, 32, 64, 4, True), (700_001, 64, 40, 3, False), (700_001, 64, 128, 7, True),
+    (700_001, 96, 40, 3, False), (700_001, 96, 40, 4, True), (1_400_001, 96, 2000, 4, False),
+    (1_400_001, 96, 2000, 7, True), (700_001, 128, 32, 1, False), (700_001, 128, 32, 3, True)])
+def test_sddmm_orders_where_columns_are_shared(n, k, length, per_column, pays):
+    meta, nnz, verdict = _rows_of(length, per_column * n // length + 1, n)
+    assert verdict >= 0
+    m1 = meta.m1 if length > 512 else max(meta.m1, 1 << 15)
+    assert capi.sddmm_order_pays(verdict, nnz // length, m1, n, k, nnz) is pays
+    assert not capi.sddmm_order_pays(-1, meta.m1, 1 << 15, n, k, nnz) and not capi.sddmm_order_pays(-3, meta.m1, 1 << 15, n, k, nnz)
