@@ -120,14 +120,16 @@ def rode_sddmm(sparse_matrix: RoDeCSR, lhs: torch.Tensor, rhs: torch.Tensor) -> 
     """out = S ⊙ (lhs @ rhs^T) sampled at the stored entries of S; returns values [nnz], zero for entries that
     belong to no row (mirrors ``rode_sddmm.py:194-248``)."""
     m, n, k = sparse_matrix.m, sparse_matrix.n, sparse_matrix.k
-    _check_dense("lhs_matrix", lhs, (m, k), sparse_matrix)
-    _check_dense("rhs_matrix", rhs, (n, k), sparse_matrix)
+    if not rode_sddmm_cuda.sddmm_operands_fit(lhs, rhs, sparse_matrix.values, m, n, k):
+        _check_dense("lhs_matrix", lhs, (m, k), sparse_matrix)
+        _check_dense("rhs_matrix", rhs, (n, k), sparse_matrix)
+        lhs, rhs = lhs.contiguous(), rhs.contiguous()
     ordered = sparse_matrix._verdict >= 0 and rode_sddmm_cuda.sddmm_order_pays(
         sparse_matrix._verdict, m, sparse_matrix.m1, n, k, sparse_matrix.nnz)
     return rode_sddmm_cuda.sddmm_forward(
         sparse_matrix.block_indices, sparse_matrix.residue_indices, sparse_matrix.st_offsets, sparse_matrix.m1,
         sparse_matrix.m2, sparse_matrix.row_offsets, sparse_matrix.column_indices, sparse_matrix.values, m, n,
-        lhs.contiguous(), rhs.contiguous(), k, sparse_matrix._entry_range == (0, sparse_matrix.values.numel()),
+        lhs, rhs, k, sparse_matrix._entry_range == (0, sparse_matrix.values.numel()),
         ordered)
 
 

@@ -18,6 +18,7 @@
 //     need not be zero-filled first.
 //   * ordered (default false) gives the call scratch memory in which it orders the segments by their columns; order_verdict
 //     and *_order_pays say whether that helps.
+//   * sddmm_operands_fit checks both dense operands in one call.
 //   * spmm_forward and hot_columns are new: the reference has no Python entry for SpMM.
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
@@ -81,6 +82,18 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, int, int> py_preprocess(
     res = res.narrow(0, 0, std::max(n_res, 1));
     if (on_host) return std::make_tuple(blk.cpu(), st.cpu(), res.cpu(), n_blk, n_res);
     return std::make_tuple(blk.contiguous(), st.contiguous(), res.contiguous(), n_blk, n_res);
+}
+
+// Both dense operands are as sddmm_forward takes them: float32, row-major, of these shapes, where `values` is.  (One call in the
+// place of a dozen attributes of two tensors, which cost a small call from Python a microsecond; who gets false finds out
+// what is wrong in his own time.)
+bool py_sddmm_operands_fit(const torch::Tensor &lhs, const torch::Tensor &rhs, const torch::Tensor &values, int64_t m, int64_t n,
+                           int64_t k) {
+    const auto fits = [&](const torch::Tensor &t, int64_t rows) {
+        return t.dim() == 2 && t.size(0) == rows && t.size(1) == k && t.scalar_type() == torch::kFloat32 &&
+               t.device() == values.device() && t.is_contiguous();
+    };
+    return fits(lhs, m) && fits(rhs, n);
 }
 
 torch::Tensor py_sddmm_forward(const torch::Tensor &block_indices, const torch::Tensor &residue_indices,
@@ -260,6 +273,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           py::arg("residue_indices"), py::arg("st_offsets"), py::arg("m1"), py::arg("m2"), py::arg("row_offsets"),
           py::arg("column_indices"), py::arg("values"), py::arg("m"), py::arg("n"), py::arg("lhs_matrix"),
           py::arg("rhs_matrix"), py::arg("k_version"), py::arg("covers_values") = false, py::arg("ordered") = false);
+    m.def("sddmm_operands_fit", &py_sddmm_operands_fit, py::arg("lhs"), py::arg("rhs"), py::arg("values"), py::arg("m"),
+          py::arg("n"), py::arg("k"));
     m.def("order_verdict", &py_order_verdict, "What an order of the segments by their columns can give (CUDA)",
           py::arg("block_indices"), py::arg("m1"), py::arg("row_offsets"), py::arg("column_indices"), py::arg("n"));
     m.def("spmm_order_pays", &rode_spmm_order_pays, py::arg("verdict"), py::arg("m1"), py::arg("k"), py::arg("n"),
