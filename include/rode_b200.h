@@ -189,11 +189,15 @@ int rode_spmm_f64_all(int M, int m1, int k, int n, long long nnz, const double *
  *
  * Whether it helps on a matrix: rode_order_verdict sets *in_range (host) to 1 where the number of segments and columns is such
  * that it can, and then, unless verdict (device, one int) is null, enqueues a kernel that looks at samples of the columns and
- * writes its verdict (narrow bands anyway, a few columns with most of the references, neither).  rode_spmm_order_pays and
- * rode_sddmm_order_pays turn that number, read back, into yes or no for one width.
+ * writes its verdict, a number of 0 and above (narrow bands anyway, a few columns with most of the references, neither, and how
+ * much of the columns a segment spans).  rode_spmm_order_pays and rode_sddmm_order_pays turn that number, read back, into yes or
+ * no for one width; for a negative one, as where nothing was judged, they say no.
  *
- * SpMM: everything as for rode_spmm_f32_all / _f64_all without hot_columns, bit for bit; the workspace is
- * rode_spmm_ordered_workspace_bytes() large, 16-byte aligned. */
+ * SpMM: everything as for rode_spmm_f32_all / _f64_all without hot_columns; the workspace is
+ * rode_spmm_ordered_workspace_bytes() large, 16-byte aligned.  A row's sum is formed in the same order with and without the order
+ * of the segments, so results are the same bit for bit in grids of more than 22 warps (segments times column tiles) per SM that
+ * gather more than 40 MB; smaller ones, for which rode_spmm_order_pays never says yes, take other kernels without an order
+ * and round differently.  From 2^30 segments on the call is the one without an order. */
 int rode_order_verdict(int m1, int n_cols, long long nnz, const int *row_offsets, const int *column_indices,
                        const int *block_r_ind, int *in_range, int *verdict, rode_stream_t stream);
 int rode_spmm_order_pays(int verdict, int m1, int k, int n, long long nnz, int elem_size);
@@ -275,7 +279,8 @@ int rode_sddmm_f32(int m1, int m2, int n, int k, const int *block_r_ind, const i
  * gather from (see above).  Same results as rode_sddmm_f32 up to the rounding of the dot products.
  *   M, nnz     rows of the matrix, length of values and column_indices
  *   workspace  rode_sddmm_workspace_bytes() bytes, 16-byte aligned, contents don't-care before and after, not shared by
- *              calls that may overlap in time; null: the call is rode_sddmm_f32.  From 2^26 rows on it is not used.
+ *              calls that may overlap in time; null: the call is rode_sddmm_f32.  From 2^26 rows, or an nnz of
+ *              2^31 - 257, on it is not used (nor looked at).
  * The ordering runs on stream1.
  *
  * Whether that pays: rode_sddmm_order_pays, with the verdict of rode_order_verdict on the matrix. */

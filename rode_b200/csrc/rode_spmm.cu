@@ -945,6 +945,8 @@ spmm_rows_simple(int m2, int n, const T *__restrict__ values, const int *__restr
 // It serves matrices without segments and lists of 2^19 rows and more.  Shorter lists beside a block grid keep spmm_rows_simple:
 // there the rows are the smaller part, and their loads get in the way of the last segments (R-MAT 17 N = 64 51 / 54, the rows
 // alone 25 / 22; Pareto 300,007 N = 32 87 / 93; but R-MAT 21 N = 64 697 / 679, Pareto 2^20 N = 64 1105 / 1064).
+// (That is said of block grids that fill the GPU.  A handful of segments takes a short list off this kernel as well, for nothing: stencil
+// 61^3 without / with one row of 600 nonzeros N = 64 84 / 90.)
 //
 // R = 2 where rows are not known to be long (rows alone, R = 1 / 2: R-MAT 21 N = 64 278 / 226, Pareto 2^20 N = 64 371 / 358; stencil N = 64
 // 633 / 650; rows of 15 to 24 N = 32 56 / 58, N = 64 102 / 97); the 128-byte tile of fp64 has no room for two (8 rows x 32
@@ -1421,6 +1423,8 @@ int spmm(int m1, int m2, int k, int n, const T *values, const int *col, const in
     // 223 / 186, of 4 to 6 195 / 172, of 2 to 6 165 / 160, of 0 to 4 231 / 246; fp64 N = 64 stencil 128^3 1705 / 1351, rows of 15 to 24
     // 308 / 220, of 0 to 4 231 / 258.  Ragged widths idle lanes in the last tile of either, and need longer rows: stencil 61^3
     // N = 68 191 / 139, N = 100 197 / 163, N = 132 340 / 217, N = 200 344 / 297; rows of 0 to 27 145 / 162, 180 / 211, 349 / 305, 426 / 403.
+    // (With segments beside them those passes lose, R-MAT 21 N = 128 1109 / 1291; that a few segments do no harm this line does not know:
+    // stencil 61^3 without / with one row of 600 nonzeros N = 128 160 / 194, N = 132 224 / 369.)
     const bool long_rows_only = m1 == 0 && rows_hold(nnz, 0, m2, vecs % 32 == 0 ? 5 : 20);
     // Widths the tiles do not divide (any other multiple of 4 columns; the reference has none of them): the narrowest
     // shape that covers the row, or 512-byte tiles with a partly empty last one.  No popularity hints.
