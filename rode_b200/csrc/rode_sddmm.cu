@@ -609,7 +609,9 @@ sddmm_pieces(OrderHead *head, const unsigned long long *__restrict__ list, int c
     __shared__ __align__(16) int s_col[2][32];
     int stage_buf = 0;
     chain_begin();
-    const unsigned long long *const placed = after_chain(list);
+    // position of the piece two ahead: round `r2` of bundle `b2`.  Behind the wait, as is whatever is claimed from the head: the
+    // list is not read before it is complete.
+    int b2 = after_chain(blockIdx.x), r2 = 0;
     int total = 0;
 #pragma unroll
     for (int i = 0; i < kOrderBuckets / 32; ++i) total += ld_behind_wait(&head->counts[lane + 32 * i]);
@@ -620,10 +622,8 @@ sddmm_pieces(OrderHead *head, const unsigned long long *__restrict__ list, int c
     auto inside = [&](int v) { return !kRagged || static_cast<unsigned>(l + v * L) < row_vecs; };
     auto entry = [&](int bundle, int round) {
         const long long i = static_cast<long long>(bundle) * kPieceRounds + round;
-        return bundle < bundles && i < total ? __ldcg(placed + i) : 0ull;
+        return bundle < bundles && i < total ? __ldcg(list + i) : 0ull;
     };
-    // Position of the piece two ahead: round `r2` of bundle `b2`.
-    int b2 = blockIdx.x, r2 = 0;
     if (b2 >= bundles) return;
     int claimed = INT_MAX;
     auto claim = [&]() {
